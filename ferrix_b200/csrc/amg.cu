@@ -465,23 +465,32 @@ __global__ void k_prolong(int ndof, int bs, const int32_t* __restrict__ agg, con
 
 // ------------------------------------------------------------------ coarsest level
 
-__global__ void k_dense_from_bsr(int n, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ cols,
-                                 const double* __restrict__ vals, double* __restrict__ A) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+// A (zeroed) = the dense matrix of a block CSR; a warp per block row, lanes over its values (a thread
+// per row took 39-187 us on the rows of up to a hundred blocks that a smoothed transfer gives)
+template <int BS>
+__global__ void __launch_bounds__(128) k_dense_from_bsr(int n, const int32_t* __restrict__ row_ptr,
+                                                        const int32_t* __restrict__ cols,
+                                                        const double* __restrict__ vals, double* __restrict__ A) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= n) return;
-    const int nd = 6 * n;
-    for (int b = row_ptr[i]; b < row_ptr[i + 1]; ++b)
-        for (int r = 0; r < 6; ++r)
-            for (int c = 0; c < 6; ++c)
-                A[(int64_t)(6 * i + r) * nd + 6 * cols[b] + c] = vals[(int64_t)b * 36 + r * 6 + c];
+    const int64_t nd = (int64_t)BS * n;
+    const int64_t v0 = (int64_t)row_ptr[i] * (BS * BS), v1 = (int64_t)row_ptr[i + 1] * (BS * BS);
+    for (int64_t v = v0 + lane; v < v1; v += 32) {
+        const int64_t b = v / (BS * BS);
+        const int e = (int)(v - b * (BS * BS)), r = e / BS, c = e - r * BS;
+        A[(BS * (int64_t)i + r) * nd + (int64_t)BS * cols[b] + c] = vals[v];
+    }
 }
 
-// Coarsest level: in-place blocked Gauss-Jordan inverse of the dense SPD matrix
-// (no pivoting), panels of kPanel pivots. Per panel K: the pivot block is
-// inverted by one CTA (P), the panel rows become P A[K, j], every other row i
-// gets A[i, j] -= A[i, K] (P A[K, j]) and A[i, K] = -A[i, K] P. DOFs with a
-// vanishing diagonal are decoupled first and get zero rows/columns in the inverse.
+// Coarsest level: blocked Gauss-Jordan inverse of the dense SPD matrix (no pivoting), kPanel
+// pivots per launch. With P the inverse of the pivot block A[K, K], panel K maps A to
+//   B[K, K] = P, B[K, j] = P A[K, j], B[i, K] = -A[i, K] P, B[i, j] = A[i, j] - A[i, K] P A[K, j].
+// A and B alternate between two buffers, so that every tile is computed from A alone by its own
+// CTA and a panel is one launch; the CTA that holds the next pivot block inverts it as
+// soon as it is updated. DOFs with a vanishing diagonal are decoupled first and get
+// zero rows/columns in the inverse.
 constexpr int kPanel = 32;
+constexpr int kTileRows = 64;  // rows of a tile (kPanel columns): P A[K, j] is formed once per tile
 
 __global__ void __launch_bounds__(1024) k_dense_decouple(int nd, double* __restrict__ A, uint8_t* __restrict__ dead,
                                                          double* __restrict__ diag) {
@@ -509,100 +518,129 @@ __global__ void __launch_bounds__(1024) k_dense_decouple(int nd, double* __restr
 // matrix keeps each pivot at or above 1 / cond of the original diagonal).
 constexpr double kSingularPivot = 1e-12;
 
-// P = inverse of the pivot block A[k0:k0+b, k0:k0+b], written in place (one CTA, 32 warps);
-// *singular |= 1 when a pivot is not above kSingularPivot times its original diagonal
-__global__ void __launch_bounds__(1024) k_panel_inverse(int nd, int k0, int b, double* __restrict__ A,
-                                                        const double* __restrict__ diag, int* __restrict__ singular) {
-    __shared__ double S[kPanel][kPanel + 1];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    S[w][lane] = (w < b && lane < b) ? A[(int64_t)(k0 + w) * nd + k0 + lane] : (w == lane ? 1.0 : 0.0);
-    __syncthreads();
+// P = inverse of the pivot block that the 256 threads hold (thread (ty, tx): entries (ty + 8 u, tx)),
+// b pivots from k0, the rest the identity; *singular |= 1 when a pivot is not above
+// kSingularPivot times its original diagonal. One barrier per pivot: its row and column go
+// through alternating shared buffers, everything else stays in registers.
+__device__ __forceinline__ void invert_pivot(double (&a)[4], int k0, int b, const double* __restrict__ diag,
+                                             int* __restrict__ singular, double* __restrict__ P) {
+    __shared__ double s_row[2][kPanel], s_col[2][kPanel];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     for (int t = 0; t < b; ++t) {
-        if (threadIdx.x == 0 && !(S[t][t] > kSingularPivot * diag[k0 + t])) *singular = 1;
-        const double ip = 1.0 / S[t][t];
-        __syncthreads();
-        if (w == t && lane != t) S[t][lane] *= ip;
-        __syncthreads();
-        const double f = S[w][t];
-        __syncthreads();
-        if (w != t) {
-            if (lane != t) S[w][lane] -= f * S[t][lane];
-            else S[w][t] = -f * ip;
+        const int q = t & 1;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (tx == t) s_col[q][ty + 8 * u] = a[u];
+            if (ty + 8 * u == t) s_row[q][tx] = a[u];
         }
         __syncthreads();
-        if (threadIdx.x == 0) S[t][t] = ip;
-        __syncthreads();
-    }
-    if (w < b && lane < b) A[(int64_t)(k0 + w) * nd + k0 + lane] = S[w][lane];
-}
-
-__device__ __forceinline__ void load_panel(int nd, int k0, int b, const double* A, double (*P)[kPanel]) {
-    for (int e = threadIdx.x; e < kPanel * kPanel; e += blockDim.x) {
-        const int r = e / kPanel, c = e % kPanel;
-        P[r][c] = (r < b && c < b) ? A[(int64_t)(k0 + r) * nd + k0 + c] : 0.0;
-    }
-    __syncthreads();
-}
-
-// panel rows: A[K, j] = P A[K, j] for every column j outside K (one thread per column)
-__global__ void __launch_bounds__(128) k_panel_rows(int nd, int k0, int b, double* __restrict__ A) {
-    __shared__ double P[kPanel][kPanel];
-    load_panel(nd, k0, b, A, P);
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nd || (j >= k0 && j < k0 + b)) return;
-    double col[kPanel];
+        const double p = s_row[q][t], ip = 1.0 / p, rt = s_row[q][tx] * ip;
+        if (threadIdx.x == 0 && !(p > kSingularPivot * diag[k0 + t])) *singular = 1;
 #pragma unroll
-    for (int t = 0; t < kPanel; ++t) col[t] = t < b ? A[(int64_t)(k0 + t) * nd + j] : 0.0;
-    for (int r = 0; r < b; ++r) {
-        double s = 0.0;
-#pragma unroll
-        for (int t = 0; t < kPanel; ++t) s += P[r][t] * col[t];
-        A[(int64_t)(k0 + r) * nd + j] = s;
+        for (int u = 0; u < 4; ++u) {
+            const double f = s_col[q][ty + 8 * u];
+            if (ty + 8 * u == t) a[u] = tx == t ? ip : rt;
+            else a[u] = tx == t ? -f * ip : a[u] - f * rt;
+        }
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) P[(ty + 8 * u) * kPanel + tx] = a[u];
 }
 
-// A[i, j] -= A[i, K] A[K, j] for every i, j outside K: one 32 x 32 tile per CTA,
-// both factors staged in shared memory (k0 is a multiple of 32, so the panel's
-// rows and columns are whole tiles, which are skipped)
-__global__ void __launch_bounds__(256) k_panel_update(int nd, int k0, int b, double* __restrict__ A) {
-    __shared__ double Lt[32][33];  // A[i0 + r, k0 + t]
-    __shared__ double Rt[32][33];  // A[k0 + t, j0 + c]
-    const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
-    if (i0 == k0 || j0 == k0) return;  // CTA-uniform
+// the first pivot block's inverse
+__global__ void __launch_bounds__(256) k_gj_first(int nd, const double* __restrict__ A, const double* __restrict__ diag,
+                                                  int* __restrict__ singular, double* __restrict__ P) {
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int r = ty; r < 32; r += 8) {
-        const int i = i0 + r, j = j0 + tx;
-        Lt[r][tx] = (i < nd && tx < b) ? A[(int64_t)i * nd + k0 + tx] : 0.0;
-        Rt[r][tx] = (r < b && j < nd) ? A[(int64_t)(k0 + r) * nd + j] : 0.0;
-    }
-    __syncthreads();
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-    for (int t = 0; t < 32; ++t) {
-        const double rv = Rt[t][tx];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) acc[u] += Lt[ty + 8 * u][t] * rv;
-    }
-    const int j = j0 + tx;
-    if (j >= nd) return;
+    const int b = min(kPanel, nd);
+    double a[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-        const int i = i0 + ty + 8 * u;
-        if (i < nd) A[(int64_t)i * nd + j] -= acc[u];
+        const int r = ty + 8 * u;
+        a[u] = r < b && tx < b ? A[(int64_t)r * nd + tx] : (r == tx ? 1.0 : 0.0);
     }
+    invert_pivot(a, 0, b, diag, singular, P);
 }
 
-// after the update: A[i, K] = -A[i, K] P for every row i outside K (one warp per row)
-__global__ void __launch_bounds__(256) k_panel_cols(int nd, int k0, int b, double* __restrict__ A) {
-    __shared__ double P[kPanel][kPanel];
-    load_panel(nd, k0, b, A, P);
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (i >= nd || (i >= k0 && i < k0 + b)) return;  // warp-uniform
-    double* Ai = A + (int64_t)i * nd;
-    const double a = lane < b ? Ai[k0 + lane] : 0.0;
-    double acc = 0.0;
-    for (int s = 0; s < b; ++s) acc += __shfl_sync(0xffffffffu, a, s) * P[s][lane];
-    if (lane < b) Ai[k0 + lane] = -acc;
+// One panel: B from A and P (see above). Bound by the launch and, above ~1,000 DOF, by
+// shared-memory loads of the two 32-deep products (pairs of the left factor per load). With
+// separate launches for the pivot inverse (16-18 us), panel rows (9), update (8) and panel
+// columns (4) instead: the NLGEOM beam of 16k DOF, with 85 inverses of 168 DOF, took 370 ms
+// against 355, the 14,883-DOF cantilever 9.44 against 9.15 ms from deck text.
+__global__ void __launch_bounds__(256) k_gj_panel(int nd, int k0, const double* __restrict__ A,
+                                                  double* __restrict__ B, const double* __restrict__ P,
+                                                  double* __restrict__ P_next, const double* __restrict__ diag,
+                                                  int* __restrict__ singular) {
+    __shared__ __align__(16) double Ps[kPanel][kPanel + 2];     // P, zero outside the panel
+    __shared__ double Rs[kPanel][kPanel];                       // A[K, j0 + c], then P A[K, j0 + c]
+    __shared__ __align__(16) double Ls[kTileRows][kPanel + 2];  // A[i0 + r, K]
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int i0 = blockIdx.y * kTileRows, j0 = blockIdx.x * kPanel;
+    const int b = min(kPanel, nd - k0);
+    const bool panel_col = j0 == k0;
+    const int j = j0 + tx;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int r = ty + 8 * u;
+        Ps[r][tx] = r < b && tx < b ? P[r * kPanel + tx] : 0.0;
+        if (!panel_col) Rs[r][tx] = r < b && j < nd ? A[(int64_t)(k0 + r) * nd + j] : 0.0;
+    }
+    double a[kTileRows / 8];
+#pragma unroll
+    for (int u = 0; u < kTileRows / 8; ++u) {
+        const int r = ty + 8 * u, i = i0 + r;
+        Ls[r][tx] = i < nd && tx < b ? A[(int64_t)i * nd + k0 + tx] : 0.0;
+        a[u] = i < nd && j < nd ? A[(int64_t)i * nd + j] : 0.0;
+    }
+    __syncthreads();
+    double m[4] = {0.0, 0.0, 0.0, 0.0};  // R = P A[K, j], or P itself in the panel's own columns
+    if (panel_col) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) m[u] = Ps[ty + 8 * u][tx];
+    } else {
+#pragma unroll
+        for (int t = 0; t < kPanel; t += 2) {
+            const double r0 = Rs[t][tx], r1 = Rs[t + 1][tx];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const double2 p = *reinterpret_cast<const double2*>(&Ps[ty + 8 * u][t]);
+                m[u] += p.x * r0 + p.y * r1;
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) Rs[ty + 8 * u][tx] = m[u];
+    __syncthreads();
+    double acc[kTileRows / 8];
+#pragma unroll
+    for (int u = 0; u < kTileRows / 8; ++u) acc[u] = 0.0;
+#pragma unroll 4
+    for (int t = 0; t < kPanel; t += 2) {
+        const double r0 = Rs[t][tx], r1 = Rs[t + 1][tx];
+#pragma unroll
+        for (int u = 0; u < kTileRows / 8; ++u) {
+            const double2 l = *reinterpret_cast<const double2*>(&Ls[ty + 8 * u][t]);
+            acc[u] += l.x * r0 + l.y * r1;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kTileRows / 8; ++u) {
+        const int i = i0 + ty + 8 * u;
+        if (i >= k0 && i < k0 + b) a[u] = Rs[i - k0][tx];
+        else a[u] = (panel_col ? 0.0 : a[u]) - acc[u];
+        if (i < nd && j < nd) B[(int64_t)i * nd + j] = a[u];
+    }
+    const int kn = k0 + kPanel;
+    if (kn >= nd || j0 != kn || kn < i0 || kn >= i0 + kTileRows) return;  // CTA-uniform
+    const int bn = min(kPanel, nd - kn);
+    double pv[4];  // the next pivot block: rows kn - i0 .. of this tile (i0 and kn are multiples of 32)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const double v = kn == i0 ? a[u] : a[4 + u];
+        const int r = ty + 8 * u;
+        pv[u] = r < bn && tx < bn ? v : (r == tx ? 1.0 : 0.0);
+    }
+    invert_pivot(pv, kn, bn, diag, singular, P_next);
 }
 
 __global__ void __launch_bounds__(256) k_dense_zero_dead(int nd, double* __restrict__ A,
@@ -1634,23 +1672,26 @@ void Amg::coarsest_inverse(AmgLevel& l, cudaStream_t s) {
     const int64_t nd = (int64_t)l.n * l.bs;
     l.dense_inv.alloc((size_t)nd * nd, s);
     l.dense_inv.zero(s);
-    FX_LAUNCH(k_dense_from_bsr, grid_for(l.n, 64), 64, 0, s, l.n, l.row_ptr.ptr, l.cols.ptr, l.vals.ptr,
-              l.dense_inv.ptr);
+    FX_LAUNCH(k_dense_from_bsr<6>, grid_for((int64_t)l.n * 32, 128), 128, 0, s, l.n, l.row_ptr.ptr, l.cols.ptr,
+              l.vals.ptr, l.dense_inv.ptr);
     DBuf<uint8_t> dead;
     dead.alloc(nd, s);
-    DBuf<double> diag0;
+    DBuf<double> diag0, other, pivot;
     DBuf<int> singular;
     diag0.alloc(nd, s);
     singular.alloc(1, s);
     singular.zero(s);
+    other.alloc((size_t)nd * nd, s);
+    pivot.alloc(2 * kPanel * kPanel, s);
     FX_LAUNCH(k_dense_decouple, 1, 1024, 0, s, (int)nd, l.dense_inv.ptr, dead.ptr, diag0.ptr);
+    double* P[2] = {pivot.ptr, pivot.ptr + kPanel * kPanel};
+    FX_LAUNCH(k_gj_first, 1, 256, 0, s, (int)nd, l.dense_inv.ptr, diag0.ptr, singular.ptr, P[0]);
+    const dim3 tiles(grid_for(nd, kPanel), grid_for(nd, kTileRows));
     for (int k0 = 0; k0 < (int)nd; k0 += kPanel) {
-        const int b = std::min<int>(kPanel, (int)nd - k0);
-        FX_LAUNCH(k_panel_inverse, 1, 1024, 0, s, (int)nd, k0, b, l.dense_inv.ptr, diag0.ptr, singular.ptr);
-        FX_LAUNCH(k_panel_rows, grid_for(nd, 128), 128, 0, s, (int)nd, k0, b, l.dense_inv.ptr);
-        const unsigned tiles = (unsigned)((nd + 31) / 32);
-        FX_LAUNCH(k_panel_update, dim3(tiles, tiles), 256, 0, s, (int)nd, k0, b, l.dense_inv.ptr);
-        FX_LAUNCH(k_panel_cols, grid_for(nd * 32), 256, 0, s, (int)nd, k0, b, l.dense_inv.ptr);
+        FX_LAUNCH(k_gj_panel, tiles, 256, 0, s, (int)nd, k0, l.dense_inv.ptr, other.ptr, P[0], P[1], diag0.ptr,
+                  singular.ptr);
+        l.dense_inv.swap(other);
+        std::swap(P[0], P[1]);
     }
     FX_LAUNCH(k_dense_zero_dead, grid_for(nd * 32), 256, 0, s, (int)nd, l.dense_inv.ptr, dead.ptr);
     int sing = 0;
