@@ -10,6 +10,8 @@
 
 #include "amg.hpp"
 #include "coarse_row.cuh"
+#include "corner.cuh"
+#include "transfer.cuh"
 
 namespace fx {
 
@@ -17,12 +19,10 @@ namespace {
 
 constexpr int kCoarseMaxDof = 1200;  // dense inverse at or below this size
 constexpr int kMaxLevels = 8;
-
-int bits_for(int64_t n) {
-    int b = 1;
-    while ((int64_t(1) << b) < n) ++b;
-    return b;
-}
+// Prolongator smoothing weight omega = kSmoothOmega / lmax with lmax the level's estimate, which
+// is 1.1 times the power iteration's value: 4/3 over the latter, the optimum of the analysis
+constexpr double kLmaxMargin = 1.1;
+constexpr double kSmoothOmega = 4.0 / 3.0 * kLmaxMargin;
 
 template <typename Op>
 void cub_call(Op op, DBuf<uint8_t>& tmp, cudaStream_t s) {
@@ -34,38 +34,59 @@ void cub_call(Op op, DBuf<uint8_t>& tmp, cudaStream_t s) {
 
 // ------------------------------------------------------------------ aggregation
 
-// org[0..2] = componentwise minimum of the n points c (one CTA)
-__global__ void __launch_bounds__(1024) k_min3(int n, const double* __restrict__ c, double* __restrict__ org) {
-    __shared__ double sh[3][32];
-    double m[3] = {1e300, 1e300, 1e300};
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
+// order-preserving integer image of a double, and back
+__device__ __forceinline__ unsigned long long ordered(double v) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    return (u >> 63) ? ~u : u | 0x8000000000000000ull;
+}
+__host__ __device__ __forceinline__ unsigned long long unordered_bits(unsigned long long u) {
+    return (u >> 63) ? u & 0x7fffffffffffffffull : ~u;
+}
+
+// box[0..2] = componentwise minimum of the n points c, box[3..5] = maximum, as ordered integers (set to
+// all ones / zero before). One pass over all SMs (one CTA took 79 us for 139k nodes).
+__global__ void __launch_bounds__(256) k_box(int n, const double* __restrict__ c, unsigned long long* __restrict__ box) {
+    unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 #pragma unroll
-        for (int d = 0; d < 3; ++d) m[d] = fmin(m[d], c[3 * (int64_t)i + d]);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        for (int d = 0; d < 3; ++d) {
+            const unsigned long long v = ordered(c[3 * (int64_t)i + d]);
+            lo[d] = min(lo[d], v);
+            hi[d] = max(hi[d], v);
+        }
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        for (int o = 16; o > 0; o >>= 1) m[d] = fmin(m[d], __shfl_xor_sync(0xffffffffu, m[d], o));
-        if (lane == 0) sh[d][w] = m[d];
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        double v = 1e300;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) v = fmin(v, sh[threadIdx.x][k]);
-        org[threadIdx.x] = v;
+        for (int o = 16; o > 0; o >>= 1) {
+            lo[d] = min(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+            hi[d] = max(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+        }
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(box + d, lo[d]);
+            atomicMax(box + 3 + d, hi[d]);
+        }
     }
 }
 
-__global__ void k_cell_keys(int n, const double* __restrict__ c, const double* __restrict__ org, double inv_cell,
-                            uint64_t* __restrict__ keys, int32_t* __restrict__ ids) {
+// Cells of a level: the bounding box cut into k[d] equal parts per direction (none is a sliver at
+// the box's far side; with cells of one edge the 205k-DOF C3D4 box had 3,060 instead of 2,464)
+struct CellGrid {
+    int k[3];
+    double inv[3];  // parts per length
+};
+
+__global__ void k_cell_keys(int n, const double* __restrict__ c, const unsigned long long* __restrict__ box,
+                            CellGrid g, uint64_t* __restrict__ keys, int32_t* __restrict__ ids) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const double ox = org[0], oy = org[1], oz = org[2];
-    auto cell = [&](double v, double o) {
-        double f = floor((v - o) * inv_cell);
-        f = f < 0.0 ? 0.0 : (f > 2097151.0 ? 2097151.0 : f);
-        return (uint64_t)f;
-    };
-    keys[i] = cell(c[3 * i], ox) | (cell(c[3 * i + 1], oy) << 21) | (cell(c[3 * i + 2], oz) << 42);
+    uint64_t key = 0;
+#pragma unroll
+    for (int d = 2; d >= 0; --d) {
+        const double o = __longlong_as_double((long long)unordered_bits(box[d]));
+        const double f = floor((c[3 * (int64_t)i + d] - o) * g.inv[d]);
+        const int q = f > 0.0 ? (f < (double)g.k[d] ? (int)f : g.k[d] - 1) : 0;
+        key = key * (uint64_t)g.k[d] + (uint64_t)q;
+    }
+    keys[i] = key;
     ids[i] = i;
 }
 
@@ -114,183 +135,82 @@ __device__ __forceinline__ double nullspace_row(int bs, int j, int d, int col, c
     return d == 0 ? z : (d == 2 ? -x : 0.0);                  // rotation about y
 }
 
-// One warp per aggregate: Q (rows of the members, in place) and R (6x6).
-__global__ void k_agg_qr(int na, const int32_t* __restrict__ ptr, const int32_t* __restrict__ nodes, int bs,
-                         const double* __restrict__ c, const double* __restrict__ cent,
-                         const double* __restrict__ Rprev, double* __restrict__ Q, double* __restrict__ Rnext) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= na) return;  // warp-uniform
-    const int a = warp;
+// One warp per aggregate: Q (rows of the members) and R (6x6) by modified Gram-Schmidt, twice. The
+// rows (at most kQrRows) are orthogonalised in shared memory, each lane its own rows, and written
+// once; larger aggregates in place in Q (SH false). In global memory throughout, the passes' round
+// trips took 95-108 us per level.
+constexpr int kQrRows = 256, kQrWarps = 2;
+template <bool SH>
+__device__ __forceinline__ void agg_qr(int a, int lane, const int32_t* __restrict__ ptr,
+                                       const int32_t* __restrict__ nodes, int bs, const double* __restrict__ c,
+                                       const double* __restrict__ cent, const double* __restrict__ Rprev,
+                                       double* __restrict__ Q, double* __restrict__ Rnext, double* sh) {
     const int p0 = ptr[a], m = ptr[a + 1] - ptr[a];
     const int rows = m * bs;
-    auto qidx = [&](int r, int col) {
-        int j = nodes[p0 + r / bs];
-        return ((size_t)j * bs + (r % bs)) * 6 + col;
+    auto qidx = [&](int r, int col) -> int64_t {
+        if (SH) return (int64_t)col * kQrRows + r;
+        return ((int64_t)nodes[p0 + r / bs] * bs + (r % bs)) * 6 + col;
     };
+    double* W = SH ? sh : Q;
     for (int r = lane; r < rows; r += 32) {
         int j = nodes[p0 + r / bs];
-        for (int col = 0; col < 6; ++col) Q[qidx(r, col)] = nullspace_row(bs, j, r % bs, col, c, cent, a, Rprev);
+        for (int col = 0; col < 6; ++col) W[qidx(r, col)] = nullspace_row(bs, j, r % bs, col, c, cent, a, Rprev);
     }
     __syncwarp();
     double R[36];
+#pragma unroll
     for (int k = 0; k < 36; ++k) R[k] = 0.0;
+#pragma unroll
     for (int col = 0; col < 6; ++col) {
         double n0 = 0.0;
         for (int r = lane; r < rows; r += 32) {
-            double v = Q[qidx(r, col)];
+            double v = W[qidx(r, col)];
             n0 += v * v;
         }
         n0 = sqrt(warp_sum(n0));
         for (int pass = 0; pass < 2; ++pass)
+#pragma unroll
             for (int k = 0; k < col; ++k) {
                 double dot = 0.0;
-                for (int r = lane; r < rows; r += 32) dot += Q[qidx(r, k)] * Q[qidx(r, col)];
+                for (int r = lane; r < rows; r += 32) dot += W[qidx(r, k)] * W[qidx(r, col)];
                 dot = warp_sum(dot);
                 R[k * 6 + col] += dot;
-                for (int r = lane; r < rows; r += 32) Q[qidx(r, col)] -= dot * Q[qidx(r, k)];
-                __syncwarp();
+                for (int r = lane; r < rows; r += 32) W[qidx(r, col)] -= dot * W[qidx(r, k)];
             }
         double nr = 0.0;
         for (int r = lane; r < rows; r += 32) {
-            double v = Q[qidx(r, col)];
+            double v = W[qidx(r, col)];
             nr += v * v;
         }
         nr = sqrt(warp_sum(nr));
         const bool keep = n0 > 0.0 && nr > 1e-10 * n0;
         R[col * 6 + col] = keep ? nr : 0.0;
-        for (int r = lane; r < rows; r += 32) Q[qidx(r, col)] = keep ? Q[qidx(r, col)] / nr : 0.0;
-        __syncwarp();
+        for (int r = lane; r < rows; r += 32) W[qidx(r, col)] = keep ? W[qidx(r, col)] / nr : 0.0;
     }
+    if (SH)
+        for (int r = lane; r < rows; r += 32) {
+            const int64_t o = ((int64_t)nodes[p0 + r / bs] * bs + (r % bs)) * 6;
+#pragma unroll
+            for (int col = 0; col < 6; ++col) Q[o + col] = W[qidx(r, col)];
+        }
     if (lane == 0)
+#pragma unroll
         for (int k = 0; k < 36; ++k) Rnext[(size_t)a * 36 + k] = R[k];
 }
 
-// ------------------------------------------------------------------ Galerkin coarse matrix
-
-// fine block (row i, col j) and its values at level 0 (planar BSR3) or above (row-major bs x bs)
-struct FineView {
-    int bs;
-    const int32_t* blk_row;  // per block
-    const int32_t* blk_col;  // per block (coarse levels); level 0 uses planar cols
-    const double* vals;
-    // level 0 planar
-    const int32_t* row_ptr;
-    const int32_t* goff;
-    const int32_t* cols4;
-    __device__ __forceinline__ int col(int64_t b, int i) const {
-        if (bs == 6) return blk_col[b];
-        int k = (int)(b - row_ptr[i]);
-        return cols4[4 * (int64_t)goff[i] + k];
-    }
-    template <int BS>
-    __device__ __forceinline__ void load(int64_t b, int i, double* v) const {
-        if (BS == 6) {
-#pragma unroll
-            for (int k = 0; k < 36; ++k) v[k] = vals[b * 36 + k];
-        } else {
-            const int k = (int)(b - row_ptr[i]);
-            const int64_t g0 = goff[i];
-            const int ng = goff[i + 1] - (int)g0;
-            const double* base = vals + (g0 * 9 + k / 4) * 4 + (k & 3);
-#pragma unroll
-            for (int t = 0; t < 9; ++t) v[t] = base[(int64_t)t * ng * 4];
-        }
-    }
-};
-
-__global__ void k_coarse_keys(int64_t nb, FineView F, const int32_t* __restrict__ agg, int nbits,
-                              uint64_t* __restrict__ keys, int64_t* __restrict__ ids) {
-    int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    int i = F.blk_row[b];
-    int j = F.col(b, i);
-    keys[b] = ((uint64_t)agg[i] << nbits) | (uint64_t)agg[j];
-    ids[b] = b;
-}
-
-__global__ void k_heads_u64(int64_t n, const uint64_t* __restrict__ keys, int32_t* __restrict__ head) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) head[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1 : 0;
-}
-
-__global__ void k_coarse_blocks(int64_t n, const uint64_t* __restrict__ keys, const int32_t* __restrict__ bid,
-                                int nbits, int64_t* __restrict__ seg, int32_t* __restrict__ crow,
-                                int32_t* __restrict__ ccol, int32_t* __restrict__ cnt) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (i == 0 || keys[i] != keys[i - 1]) {
-        int b = bid[i] - 1;
-        seg[b] = i;
-        int I = (int)(keys[i] >> nbits);
-        crow[b] = I;
-        ccol[b] = (int)(keys[i] & ((uint64_t(1) << nbits) - 1));
-        atomicAdd(&cnt[I], 1);
-    }
-}
-
-// Coarse block = sum over its fine blocks of Q_i^T A_ij Q_j. One warp per coarse
-// block; lane k takes the k-th contiguous slice of the block's sorted fine blocks
-// (row-major within a key, so each row's blocks are adjacent): T = sum_j A_ij Q_j
-// is accumulated per row and Q_i^T T added when the row changes. The 36 sums are
-// combined by a fixed butterfly: no atomics, the result does not depend on timing.
-template <int BS>
-__global__ void __launch_bounds__(128) k_galerkin(int64_t ncb, const int64_t* __restrict__ seg,
-                                                  const int64_t* __restrict__ sorted_b, FineView F,
-                                                  const double* __restrict__ Q, double* __restrict__ cvals) {
-    const int64_t cb = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (cb >= ncb) return;  // warp-uniform
-    const int64_t s0 = seg[cb], len = seg[cb + 1] - s0;
-    const int64_t per = (len + 31) / 32;
-    const int64_t a = s0 + lane * per, e = min(a + per, s0 + len);
-    double acc[36];
-#pragma unroll
-    for (int k = 0; k < 36; ++k) acc[k] = 0.0;
-    double T[BS * 6];
-    int cur = -1;
-    auto flush = [&]() {
-        const double* Qi = Q + (size_t)cur * BS * 6;
-#pragma unroll
-        for (int k = 0; k < BS; ++k) {
-            double q[6];
-#pragma unroll
-            for (int r = 0; r < 6; ++r) q[r] = Qi[k * 6 + r];
-#pragma unroll
-            for (int r = 0; r < 6; ++r)
-#pragma unroll
-                for (int c = 0; c < 6; ++c) acc[r * 6 + c] += q[r] * T[k * 6 + c];
-        }
-    };
-    for (int64_t s = a; s < e; ++s) {
-        const int64_t b = sorted_b[s];
-        const int i = F.blk_row[b];
-        const int j = F.col(b, i);
-        if (i != cur) {
-            if (cur >= 0) flush();
-            cur = i;
-#pragma unroll
-            for (int k = 0; k < BS * 6; ++k) T[k] = 0.0;
-        }
-        const double* Qj = Q + (size_t)j * BS * 6;
-        double v[BS * BS];
-        F.load<BS>(b, i, v);
-#pragma unroll
-        for (int k = 0; k < BS; ++k) {
-            double q[6];
-#pragma unroll
-            for (int c = 0; c < 6; ++c) q[c] = Qj[k * 6 + c];
-#pragma unroll
-            for (int r = 0; r < BS; ++r)
-#pragma unroll
-                for (int c = 0; c < 6; ++c) T[r * 6 + c] += v[r * BS + k] * q[c];
-        }
-    }
-    if (cur >= 0) flush();
-#pragma unroll
-    for (int k = 0; k < 36; ++k) {
-        const double t = warp_sum(acc[k]);
-        if (lane == 0) cvals[cb * 36 + k] = t;
-    }
+__global__ void __launch_bounds__(32 * kQrWarps) k_agg_qr(int na, const int32_t* __restrict__ ptr,
+                                                          const int32_t* __restrict__ nodes, int bs,
+                                                          const double* __restrict__ c,
+                                                          const double* __restrict__ cent,
+                                                          const double* __restrict__ Rprev, double* __restrict__ Q,
+                                                          double* __restrict__ Rnext) {
+    __shared__ double sh[kQrWarps][6 * kQrRows];
+    const int w = threadIdx.x >> 5, a = blockIdx.x * kQrWarps + w, lane = threadIdx.x & 31;
+    if (a >= na) return;  // warp-uniform
+    if ((ptr[a + 1] - ptr[a]) * bs <= kQrRows)
+        agg_qr<true>(a, lane, ptr, nodes, bs, c, cent, Rprev, Q, Rnext, sh[w]);
+    else
+        agg_qr<false>(a, lane, ptr, nodes, bs, c, cent, Rprev, Q, Rnext, nullptr);
 }
 
 __global__ void k_expand_rows(int n, const int32_t* __restrict__ row_ptr, int32_t* __restrict__ blk_row) {
@@ -350,31 +270,16 @@ __global__ void k_block_inv6(int n, const int32_t* __restrict__ row_ptr, const i
 
 // ------------------------------------------------------------------ level operators
 
-// coarse levels: row-major 6x6 blocks, one warp per block row
-__global__ void __launch_bounds__(256) k_ln_spmv(int n, const int32_t* __restrict__ row_ptr,
-                                                 const int32_t* __restrict__ cols, const double* __restrict__ vals,
-                                                 const double* __restrict__ x, const double* __restrict__ b,
-                                                 double* __restrict__ y) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= n) return;  // warp-uniform
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (int blk = row_ptr[warp] + lane; blk < row_ptr[warp + 1]; blk += 32) {
-        const double* v = vals + (int64_t)blk * 36;
-        const double* xx = x + 6 * (int64_t)cols[blk];
-        double xv[6];
-        for (int c = 0; c < 6; ++c) xv[c] = xx[c];
-        for (int r = 0; r < 6; ++r) {
-            double t = 0.0;
-            for (int c = 0; c < 6; ++c) t += v[r * 6 + c] * xv[c];
-            acc[r] += t;
-        }
-    }
-    for (int r = 0; r < 6; ++r) acc[r] = warp_sum(acc[r]);
-    if (lane < 6) {
-        double v = acc[0];
-        for (int r = 1; r < 6; ++r)
-            if (lane == r) v = acc[r];
-        y[6 * (int64_t)warp + lane] = b ? b[6 * (int64_t)warp + lane] - v : v;
+// The cycle's copy of a 6x6 level's values (coarse_row6): per block row 18 planes of 16-byte pairs
+__global__ void __launch_bounds__(128) k_planar6(int n, const int32_t* __restrict__ row_ptr,
+                                                 const double* __restrict__ vals, double2* __restrict__ out) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const int64_t b0 = row_ptr[i];
+    const int nb = row_ptr[i + 1] - (int)b0;
+    for (int it = lane; it < 18 * nb; it += 32) {
+        const int q = it / nb, k = it - q * nb;
+        out[b0 * 18 + it] = __ldg(reinterpret_cast<const double2*>(vals) + (b0 + k) * 18 + q);
     }
 }
 
@@ -394,73 +299,93 @@ __global__ void k_cheb_init(int n, int bs, const double* __restrict__ dinv, cons
     }
 }
 
-// bc = Q^T rf per aggregate: one warp per aggregate, lanes over member rows
+// b_c = P^T r_f: a CTA of kRestrictWarps warps per aggregate (restrict_agg).
 // Coarse Chebyshev start fused into the restriction (cs.dinv != null): with
-// b = R r the first pre-smoothing step of the coarse level from x = 0 is
+// b = P^T r the first pre-smoothing step of the coarse level from x = 0 is
 // d = c2 D^-1 b, xs = d, r = b (what k_cheb_start does there).
-// b_c = Q^T r_f, warp per aggregate; each lane's rows are loaded four at a time
-// before they are accumulated (in the same order as one row at a time).
-__global__ void k_restrict(int na, const int32_t* __restrict__ ptr, const int32_t* __restrict__ nodes, int bs,
-                           const double* __restrict__ Q, const double* __restrict__ rf, double* __restrict__ bc,
-                           CoarseStart cs) {
-    const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (a >= na) return;  // warp-uniform
-    const int p0 = ptr[a], rows = (ptr[a + 1] - p0) * bs;
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (int r0 = lane; r0 < rows; r0 += 128) {
-        double rv[4], qv[4][6];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int r = r0 + 32 * u;
-            rv[u] = 0.0;
-            if (r < rows) {
-                const int j = nodes[p0 + r / bs];
-                const int64_t row = (int64_t)j * bs + r % bs;
-                rv[u] = rf[row];
-#pragma unroll
-                for (int c = 0; c < 6; ++c) qv[u][c] = Q[row * 6 + c];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (r0 + 32 * u < rows) {
-#pragma unroll
-                for (int c = 0; c < 6; ++c) acc[c] += qv[u][c] * rv[u];
-            }
-    }
+template <int BS>
+__global__ void __launch_bounds__(32 * kRestrictWarps)
+    k_restrict(const int32_t* __restrict__ t_ptr, const int32_t* __restrict__ t_row, const double2* __restrict__ t_val,
+               const double* __restrict__ rf, double* __restrict__ bc, CoarseStart cs) {
+    __shared__ double sh[kRestrictWarps][6];
+    const int a = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double t[6];
+    restrict_agg<BS, false>(t_row, t_val, rf, t_ptr[a], t_ptr[a + 1], w, lane, t);
+    if (lane == 0)
 #pragma unroll
-    for (int c = 0; c < 6; ++c) t[c] = warp_sum(acc[c]);  // every lane holds the sums
-    if (lane < 6) {
-        const int64_t o = (int64_t)a * 6 + lane;
-        double tk = t[0];
+        for (int c = 0; c < 6; ++c) sh[w][c] = t[c];
+    __syncthreads();
+    if (threadIdx.x >= 6) return;
 #pragma unroll
-        for (int c = 1; c < 6; ++c)
-            if (lane == c) tk = t[c];
-        bc[o] = tk;
-        if (cs.dinv) {
-            const double* Di = cs.dinv + (int64_t)a * 36 + lane * 6;
-            double v = 0.0;
+    for (int c = 0; c < 6; ++c) {
+        t[c] = sh[0][c];
 #pragma unroll
-            for (int j = 0; j < 6; ++j) v += Di[j] * t[j];
-            v *= cs.c2;
-            cs.d[o] = v;
-            cs.xs[o] = v;
-            cs.r[o] = tk;
-        }
+        for (int k = 1; k < kRestrictWarps; ++k) t[c] += sh[k][c];
+    }
+    const int64_t o = (int64_t)a * 6 + lane;
+    double tk = t[0];
+#pragma unroll
+    for (int c = 1; c < 6; ++c)
+        if (lane == c) tk = t[c];
+    bc[o] = tk;
+    if (cs.dinv) {
+        const double* Di = cs.dinv + (int64_t)a * 36 + lane * 6;
+        double v = 0.0;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) v += Di[j] * t[j];
+        v *= cs.c2;
+        cs.d[o] = v;
+        cs.xs[o] = v;
+        cs.r[o] = tk;
     }
 }
 
-__global__ void k_prolong(int ndof, int bs, const int32_t* __restrict__ agg, const double* __restrict__ Q,
-                          const double* __restrict__ xc, double* __restrict__ xf, double alpha) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= ndof) return;
-    int j = k / bs;
-    const double* q = Q + (int64_t)k * 6;
-    const double* x = xc + (int64_t)agg[j] * 6;
-    double t = 0.0;
-    for (int c = 0; c < 6; ++c) t += q[c] * x[c];
-    xf[k] += alpha * t;
+// x_f += alpha P x_c; x4 != null (3x3 levels): the FP32 copy of the new x_f for the smoother's
+// gathers, scaled by sqrt(a_ii) where sq4 is given. A CTA takes kProlongRows<BS> rows: a thread per
+// entry (2-8 entries a row at the 3x3 levels, up to ~27 above) forms the entry's BS products into
+// shared memory, then a thread per DOF adds its row's in order.
+template <int BS>
+constexpr int kProlongRows = BS == 3 ? 64 : 16;
+template <int BS>
+__global__ void __launch_bounds__(256) k_prolong(int n, const int32_t* __restrict__ p_ptr,
+                                                 const int32_t* __restrict__ p_col, const double2* __restrict__ p_val,
+                                                 const double* __restrict__ xc, double* __restrict__ xf, double alpha,
+                                                 float* __restrict__ x4, const float4* __restrict__ sq4) {
+    constexpr int ST = BS | 1;  // odd stride: no bank conflicts
+    __shared__ double sh[256 * ST];
+    const int r0 = blockIdx.x * kProlongRows<BS>, r1 = min(r0 + kProlongRows<BS>, n);
+    const int e0 = p_ptr[r0], e1 = p_ptr[r1];
+    const int j = r0 + (int)threadIdx.x / BS, c = (int)threadIdx.x % BS;
+    const bool own = (int)threadIdx.x < kProlongRows<BS> * BS && j < r1;
+    const int64_t k = (int64_t)j * BS + c;
+    int p0 = 0, p1 = 0;
+    double x0 = 0.0, q = 1.0, t = 0.0;
+    if (own) {
+        p0 = p_ptr[j];
+        p1 = p_ptr[j + 1];
+        x0 = xf[k];
+        if (BS == 3 && x4 && sq4) q = (double)reinterpret_cast<const float*>(sq4)[4 * (int64_t)j + c];
+    }
+    for (int tile = e0; tile < e1; tile += 256) {  // CTA-uniform
+        const int e = tile + (int)threadIdx.x;
+        if (e < e1) {
+            double2 v[3 * BS], w[3];
+#pragma unroll
+            for (int u = 0; u < 3 * BS; ++u) v[u] = __ldg(p_val + p32<BS>(e, u));
+            const double2* x = reinterpret_cast<const double2*>(xc + (int64_t)p_col[e] * 6);
+#pragma unroll
+            for (int h = 0; h < 3; ++h) w[h] = x[h];
+#pragma unroll
+            for (int u = 0; u < BS; ++u) sh[threadIdx.x * ST + u] = entry_dot(v + 3 * u, w);
+        }
+        __syncthreads();
+        for (int p = max(p0, tile); p < min(p1, tile + 256); ++p) t = __dadd_rn(t, sh[(p - tile) * ST + c]);
+        __syncthreads();
+    }
+    if (!own) return;
+    const double v = x0 + alpha * t;
+    xf[k] = v;
+    if (BS == 3 && x4) x4[4 * (int64_t)j + c] = (float)(v * q);
 }
 
 // ------------------------------------------------------------------ coarsest level
@@ -520,27 +445,39 @@ constexpr double kSingularPivot = 1e-12;
 
 // P = inverse of the pivot block that the 256 threads hold (thread (ty, tx): entries (ty + 8 u, tx)),
 // b pivots from k0, the rest the identity; *singular |= 1 when a pivot is not above
-// kSingularPivot times its original diagonal. One barrier per pivot: its row and column go
-// through alternating shared buffers, everything else stays in registers.
+// kSingularPivot times its original diagonal. Two pivots per step: their rows and columns go
+// through alternating shared buffers (one barrier a step), everything else stays in registers,
+// and the chain of a step (exchange, reciprocal, update) is paid 16 times instead of 32.
 __device__ __forceinline__ void invert_pivot(double (&a)[4], int k0, int b, const double* __restrict__ diag,
                                              int* __restrict__ singular, double* __restrict__ P) {
-    __shared__ double s_row[2][kPanel], s_col[2][kPanel];
+    __shared__ double s_row[2][2][kPanel], s_col[2][2][kPanel];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int t = 0; t < b; ++t) {
-        const int q = t & 1;
+    for (int t = 0; t < b; t += 2) {  // (b odd: the last step's second pivot is an identity row)
+        const int q = (t >> 1) & 1;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            if (tx == t) s_col[q][ty + 8 * u] = a[u];
-            if (ty + 8 * u == t) s_row[q][tx] = a[u];
+            const int r = ty + 8 * u;
+            if ((tx & ~1) == t) s_col[q][tx & 1][r] = a[u];
+            if ((r & ~1) == t) s_row[q][r & 1][tx] = a[u];
         }
         __syncthreads();
-        const double p = s_row[q][t], ip = 1.0 / p, rt = s_row[q][tx] * ip;
-        if (threadIdx.x == 0 && !(p > kSingularPivot * diag[k0 + t])) *singular = 1;
+        const double p00 = s_row[q][0][t], p01 = s_row[q][0][t + 1], p10 = s_row[q][1][t], p11 = s_row[q][1][t + 1];
+        const double det = p00 * p11 - p01 * p10, id = 1.0 / det;
+        const double i00 = p11 * id, i01 = -p01 * id, i10 = -p10 * id, i11 = p00 * id;
+        if (threadIdx.x == 0 &&
+            (!(p00 > kSingularPivot * diag[k0 + t]) ||
+             (t + 1 < b && !(det > kSingularPivot * diag[k0 + t + 1] * p00))))
+            *singular = 1;
+        const double r0 = s_row[q][0][tx], r1 = s_row[q][1][tx];
+        const bool pc = (tx & ~1) == t;  // a pivot column: the inverse's own entries
+        const double m0 = pc ? ((tx & 1) ? i01 : i00) : i00 * r0 + i01 * r1;
+        const double m1 = pc ? ((tx & 1) ? i11 : i10) : i10 * r0 + i11 * r1;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const double f = s_col[q][ty + 8 * u];
-            if (ty + 8 * u == t) a[u] = tx == t ? ip : rt;
-            else a[u] = tx == t ? -f * ip : a[u] - f * rt;
+            const int r = ty + 8 * u;
+            const double f0 = s_col[q][0][r], f1 = s_col[q][1][r];
+            if ((r & ~1) == t) a[u] = (r & 1) ? m1 : m0;
+            else a[u] = (pc ? 0.0 : a[u]) - f0 * m0 - f1 * m1;
         }
     }
 #pragma unroll
@@ -1233,7 +1170,7 @@ struct LnOp {
     int n;
     const int32_t* row_ptr;
     const int32_t* cols;
-    const double* vals;
+    const double2* vals;
     const double* v;
     const double* b;
     double* y;
@@ -1379,22 +1316,48 @@ __global__ void k_l0_cheb_start(int n, const double* __restrict__ dinv, const do
         for (int c = 0; c < 3; ++c) d[o3 + c] = t[c];
 }
 
-// fine level: x += Q xc (3 rows per node) and the FP32 copy of x for the smoother gathers
-__global__ void k_prolong0(int n, const int32_t* __restrict__ agg, const double* __restrict__ Q,
-                           const double* __restrict__ xc, double* __restrict__ xf, float4* __restrict__ x4,
-                           double alpha, const float4* __restrict__ sq4) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double* x = xc + (int64_t)agg[i] * 6;
-    double out[3];
-    for (int k = 0; k < 3; ++k) {
-        const double* q = Q + (3 * (int64_t)i + k) * 6;
-        double t = 0.0;
-        for (int c = 0; c < 6; ++c) t += q[c] * x[c];
-        out[k] = xf[3 * (int64_t)i + k] + alpha * t;
-        xf[3 * (int64_t)i + k] = out[k];
+// b = P^T r of the corner level (a group of lanes per corner) fused with the level's first
+// pre-smoothing step from x = 0, as k_l0_cheb_start (hs: the V-cycle's scale of FP16 directions,
+// already published)
+__global__ void __launch_bounds__(256) k_corner_restrict(CornerView V, const double* __restrict__ rf,
+                                                         double* __restrict__ b, const double* __restrict__ dinv,
+                                                         double* __restrict__ r, double* __restrict__ x,
+                                                         double* __restrict__ d, float4* __restrict__ d4, double c2,
+                                                         const float4* __restrict__ sq4,
+                                                         const float* __restrict__ hs) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / kCornerLanes, sub = t % kCornerLanes;
+    double v[3];
+    corner_restrict_row<false>(V, rf, i < V.n ? i : -1, sub, v);
+    if (i >= V.n || sub != 0) return;
+    const int64_t o3 = 3 * (int64_t)i;
+    const double* D = dinv + 9 * (int64_t)i;
+    double u[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        u[c] = c2 * (D[3 * c] * v[0] + D[3 * c + 1] * v[1] + D[3 * c + 2] * v[2]);
+        b[o3 + c] = v[c];
+        r[o3 + c] = v[c];
+        x[o3 + c] = u[c];
     }
-    x4[i] = scaled4(out, sq4, i);
+    if (d4) store_dir4(d4, i, u, sq4, hs ? hs[0] : 1.0f);
+    else
+        for (int c = 0; c < 3; ++c) d[o3 + c] = u[c];
+}
+
+// x += alpha P x_c from the corner level, and the FP32 copy of x for the smoother's gathers
+__global__ void __launch_bounds__(256) k_corner_prolong(CornerView V, const double* __restrict__ xc,
+                                                        double* __restrict__ xf, double alpha,
+                                                        float4* __restrict__ x4, const float4* __restrict__ sq4) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= V.n_fine) return;
+    double u[3];
+    corner_prolong_node<false>(V, xc, j, u);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        u[k] = xf[3 * (int64_t)j + k] + alpha * u[k];
+        xf[3 * (int64_t)j + k] = u[k];
+    }
+    if (x4) x4[j] = scaled4(u, sq4, j);
 }
 
 // The CG update fused with the first step of the V-cycle that follows it:
@@ -1566,6 +1529,16 @@ static L0Op<VT> l0_op(const AmgLevel& l, const VT* vals) {
     return o;
 }
 
+static LnOp ln_op(const AmgLevel& l) {
+    LnOp o{};
+    o.n = l.n;
+    o.row_ptr = l.row_ptr.ptr;
+    o.cols = l.cols.ptr;
+    o.vals = l.pvals.ptr;
+    o.dinv = l.dinv.ptr;
+    return o;
+}
+
 static void level_spmv(const AmgLevel& l, const double* x, const double* b, double* y, cudaStream_t s) {
     if (l.S0) {
         L0Op<double> o = l0_op<double>(l, l.vals0);
@@ -1574,8 +1547,11 @@ static void level_spmv(const AmgLevel& l, const double* x, const double* b, doub
         o.y = y;
         FX_LAUNCH((k_l0_op<double, kL0Resid>), l0_grid(l.n), 256, 0, s, o);
     } else {
-        FX_LAUNCH(k_ln_spmv, grid_for((int64_t)l.n * 32), 256, 0, s, l.n, l.row_ptr.ptr, l.cols.ptr, l.vals.ptr, x, b,
-                  y);
+        LnOp o = ln_op(l);
+        o.v = x;
+        o.b = b;
+        o.y = y;
+        FX_LAUNCH(k_ln_op<kL0Resid>, grid_for((int64_t)l.n * 32, kLnThreads), kLnThreads, 0, s, o);
     }
 }
 
@@ -1589,12 +1565,14 @@ static void dot_dev(const double* a, const double* b, int64_t n, DBuf<double>& r
 
 // Largest eigenvalue of D^-1 A by 12 power iterations from a fixed hashed start
 // vector, normalised on the device; one host read at the end.
-// (level 0: with vals16 / sq4 the products come from the FP16 scaled matrix the smoother
+// (planar levels: with vals16 / sq4 the products come from the FP16 scaled matrix the smoother
 // reads, through float4 copies of x in l.x4; else from vals32, an FP32 copy, when given)
 // warm: start from the vector the previous estimate on this level ended with (a
 // refresh after a small change of the matrix) and iterate 4 times instead of 12.
-static void estimate_lmax(AmgLevel& l, DBuf<double>& red, cudaStream_t s, const float* vals32, bool warm,
-                          const __half* vals16 = nullptr, const float4* sq4 = nullptr) {
+static void estimate_lmax(AmgLevel& l, DBuf<double>& red, cudaStream_t s, bool warm) {
+    const float* vals32 = l.vals32;
+    const __half* vals16 = kAmgEstF16 ? l.vals16 : nullptr;
+    const float4* sq4 = l.sq4;
     const int64_t nd = (int64_t)l.n * l.bs;
     const int nb = 296;
     const bool from_ev = warm && l.ev.n == (size_t)nd;
@@ -1632,14 +1610,16 @@ static void estimate_lmax(AmgLevel& l, DBuf<double>& red, cudaStream_t s, const 
     double nd2 = 0.0;
     FX_CUDA_CHECK(cudaMemcpyAsync(&nd2, red.ptr + nb, sizeof(double), cudaMemcpyDeviceToHost, s));
     stream_wait(s, "amg eigenvalue estimate");
-    l.lmax = 1.1 * (nd2 > 0.0 ? std::sqrt(nd2) : 1.0);
+    l.lmax = kLmaxMargin * (nd2 > 0.0 ? std::sqrt(nd2) : 1.0);
 }
 
-// The fine level of a Galerkin product as the kernels read it: the planar BSR3
-// at level 0, row-major 6x6 block CSR (with each block's row) above.
+// A level's matrix as the transfer kernels read it: the planar BSR3 at level 0,
+// row-major 6x6 block CSR (with each block's row) above.
 static FineView fine_view(const AmgLevel& l) {
     FineView F{};
     F.bs = l.bs;
+    F.n = l.n;
+    F.nblocks = l.nblocks;
     if (l.S0) {
         F.blk_row = l.S0->blk_row.ptr;
         F.vals = l.vals0;
@@ -1647,23 +1627,12 @@ static FineView fine_view(const AmgLevel& l) {
         F.goff = l.S0->goff.ptr;
         F.cols4 = l.S0->cols.ptr;
     } else {
-        F.blk_row = l.gal_rows.ptr;
+        F.blk_row = l.blk_row.ptr;
         F.blk_col = l.cols.ptr;
         F.vals = l.vals.ptr;
+        F.row_ptr = l.row_ptr.ptr;
     }
     return F;
-}
-
-// c.vals = Q^T A Q over lf's Galerkin map (fixed-order sums per coarse block)
-static void galerkin(const AmgLevel& lf, AmgLevel& c, cudaStream_t s) {
-    const FineView F = fine_view(lf);
-    const int64_t ncb = c.nblocks;
-    if (F.bs == 3)
-        FX_LAUNCH(k_galerkin<3>, grid_for(ncb * 32, 128), 128, 0, s, ncb, lf.gal_seg.ptr, lf.gal_blk.ptr, F, lf.Q.ptr,
-                  c.vals.ptr);
-    else
-        FX_LAUNCH(k_galerkin<6>, grid_for(ncb * 32, 128), 128, 0, s, ncb, lf.gal_seg.ptr, lf.gal_blk.ptr, F, lf.Q.ptr,
-                  c.vals.ptr);
 }
 
 // Dense inverse of the coarsest level's matrix (blocked Gauss-Jordan); fails
@@ -1702,155 +1671,192 @@ void Amg::coarsest_inverse(AmgLevel& l, cudaStream_t s) {
                            "positive definite). Check for rigid body modes!");
 }
 
-void Amg::setup(const BsrStructure& S0, const double* vals0, const double* dinv0, const double* xyz, int n_nodes,
-                double cell0, cudaStream_t s, AmgStats* st) {
+// The grid of cells with edges near `cell` over a box of these extents.
+static CellGrid cell_grid(const double extent[3], double cell) {
+    CellGrid g{};
+    for (int d = 0; d < 3; ++d) {
+        const double parts = extent[d] > 0.0 && cell > 0.0 ? extent[d] / cell : 1.0;
+        g.k[d] = (int)std::min(1048576.0, std::max(1.0, std::floor(parts + 0.5)));
+        g.inv[d] = extent[d] > 0.0 ? g.k[d] / extent[d] : 0.0;
+    }
+    return g;
+}
+
+// Edge of the aggregation cells of a level when the caller leaves it open: `extent` of the level's
+// points, lo .. hi the edges that pay and mid the usual one. A level whose cells fit the dense
+// coarsest solve ends the hierarchy, which saves the six launches per V-cycle of a level between
+// (~2.5 us each on a small system), so the smallest such edge is taken while it is at most hi
+// (with larger cells the CG needs more iterations than the launches are worth); otherwise mid.
+// The cell count is that of a box of these extents, an upper bound for other shapes.
+static double pick_cell(const double extent[3], double lo, double mid, double hi) {
+    auto fits = [&](double c) {
+        const CellGrid g = cell_grid(extent, c);
+        return (double)g.k[0] * g.k[1] * g.k[2] * 6.0 <= kCoarseMaxDof;
+    };
+    if (!fits(hi)) return mid;
+    if (fits(lo)) return lo;
+    double a = lo, b = hi;
+    for (int k = 0; k < 30; ++k) {
+        const double m = 0.5 * (a + b);
+        (fits(m) ? b : a) = m;
+    }
+    return b;
+}
+
+static void planar_values(AmgLevel& l, cudaStream_t s) {
+    l.pvals.alloc((size_t)l.nblocks * 18, s);
+    FX_LAUNCH(k_planar6, grid_for((int64_t)l.n * 32, 128), 128, 0, s, l.n, l.row_ptr.ptr, l.vals.ptr, l.pvals.ptr);
+}
+
+static void set_planar(AmgLevel& l, const PlanarIn& in) {
+    l.n = in.S->n_rows;
+    l.bs = 3;
+    l.S0 = in.S;
+    l.nblocks = in.S->n_blocks;
+    l.vals0 = in.vals;
+    l.dinv0 = in.dinv;
+    l.vals32 = in.vals32;
+    l.vals16 = in.vals16;
+    l.sq4 = in.sq4;
+}
+
+static void planar_work(AmgLevel& l, bool result, cudaStream_t s) {
+    const int64_t nd = 3 * (int64_t)l.n;
+    for (DBuf<double>* v : {&l.x, &l.b, &l.r, &l.d, &l.t}) v->alloc(nd, s);
+    if (result) l.xs.alloc(nd, s);
+    for (DBuf<float>* v : {&l.d4a, &l.d4b, &l.x4}) {
+        v->alloc(4 * (size_t)l.n, s);
+        v->zero(s);  // the fourth component stays 0
+    }
+}
+
+void Amg::setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz, double cell0, double node_volume,
+                cudaStream_t s, AmgStats* st) {
     EventTimer timer;
     timer.start(s);
     L.clear();
-    L.reserve(kMaxLevels);
-    L.emplace_back();
-    {
-        AmgLevel& l0 = L[0];
-        l0.n = n_nodes;
-        l0.bs = 3;
-        l0.S0 = &S0;
-        l0.vals0 = vals0;
-        l0.dinv0 = dinv0;
-        l0.nblocks = S0.n_blocks;
+    L.reserve(kMaxLevels + 1);
+    planar_ = corner ? 2 : 1;
+    corner_ = corner ? corner_view(*corner) : CornerView{};
+    for (int m = 0; m < planar_; ++m) {
+        L.emplace_back();
+        set_planar(L[m], in[m]);
+        planar_work(L[m], m > 0, s);
+        if (m + 1 < planar_) {
+            L[m].corner_next = true;
+            L[m].pscale = 1.0 / kAmgOvercorrect;
+            estimate_lmax(L[m], red_, s, false);
+        }
     }
-    // the level-0 points and their origin (cell keys of every level are taken from it)
-    DBuf<double> coords, cent, Rprev, Rnext, org;
-    coords.alloc(3 * (size_t)n_nodes, s);
-    FX_CUDA_CHECK(cudaMemcpyAsync(coords.ptr, xyz, 3 * (size_t)n_nodes * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    org.alloc(3, s);
-    FX_LAUNCH(k_min3, 1, 1024, 0, s, n_nodes, coords.ptr, org.ptr);
-    double cell = cell0;
-    for (int lev = 0;; ++lev) {
+    // the points of the last planar level and their bounding box (cell keys of every level are
+    // taken from its lower corner)
+    DBuf<double> coords, cent, Rprev, Rnext;
+    DBuf<unsigned long long> box;
+    const int n_points = L.back().n;
+    coords.alloc(3 * (size_t)n_points, s);
+    FX_CUDA_CHECK(cudaMemcpyAsync(coords.ptr, xyz, 3 * (size_t)n_points * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    box.alloc(6, s);
+    FX_CUDA_CHECK(cudaMemsetAsync(box.ptr, 0xff, 3 * sizeof(unsigned long long), s));
+    FX_CUDA_CHECK(cudaMemsetAsync(box.ptr + 3, 0, 3 * sizeof(unsigned long long), s));
+    FX_LAUNCH(k_box, std::min(148u, grid_for(n_points)), 256, 0, s, n_points, coords.ptr, box.ptr);
+    unsigned long long hbox[6];
+    FX_CUDA_CHECK(cudaMemcpyAsync(hbox, box.ptr, sizeof(hbox), cudaMemcpyDeviceToHost, s));
+    double cell = cell0, extent[3] = {0.0, 0.0, 0.0};
+    for (int lev = planar_ - 1;; ++lev) {
         AmgLevel& l = L[lev];
         const int64_t nd = (int64_t)l.n * l.bs;
-        for (DBuf<double>* v : {&l.x, &l.b, &l.r, &l.d, &l.t}) v->alloc(nd, s);
-        if (lev > 0) l.xs.alloc(nd, s);
-        if (lev == 0)
-            for (DBuf<float>* v : {&l.d4a, &l.d4b, &l.x4}) {
-                v->alloc(4 * (size_t)l.n, s);
-                v->zero(s);  // the fourth component stays 0
-            }
-        if (lev > 0) {
+        if (!l.S0) {
+            for (DBuf<double>* v : {&l.x, &l.b, &l.r, &l.d, &l.t, &l.xs}) v->alloc(nd, s);
             l.dinv.alloc((size_t)l.n * 36, s);
             FX_LAUNCH(k_block_inv6, grid_for(l.n, 128), 128, 0, s, l.n, l.row_ptr.ptr, l.cols.ptr, l.vals.ptr,
                       l.dinv.ptr);
         }
-        if (lev > 0 && (nd <= kCoarseMaxDof || lev + 1 >= kMaxLevels)) {
+        if (!l.S0 && (nd <= kCoarseMaxDof || lev + 1 >= kMaxLevels)) {
             l.coarsest = true;
             coarsest_inverse(l, s);
             break;
         }
-        estimate_lmax(l, red_, s, lev == 0 ? vals0_f32_ : nullptr, false,
-                      lev == 0 && kAmgEstF16 ? vals0_f16_ : nullptr, sq4_);
+        if (!l.S0) planar_values(l, s);
+        estimate_lmax(l, red_, s, false);  // (its host wait also covers the bounding box)
+        if (lev == planar_ - 1)
+            for (int d = 0; d < 3; ++d) {
+                double lohi[2];
+                for (int k = 0; k < 2; ++k) {
+                    const unsigned long long u = unordered_bits(hbox[3 * k + d]);
+                    std::memcpy(&lohi[k], &u, sizeof(double));
+                }
+                extent[d] = std::isfinite(lohi[1] - lohi[0]) ? std::max(0.0, lohi[1] - lohi[0]) : 0.0;
+            }
+        if (cell0 <= 0.0) {
+            // 20 to 80 nodes per cell, else 27 (three per direction on a regular mesh); above, cells of
+            // twice to 3.5 times the edge of the level before, else three times
+            const double h = std::cbrt(node_volume);
+            cell = lev == planar_ - 1 ? pick_cell(extent, std::cbrt(20.0) * h, 3.0 * h, std::cbrt(80.0) * h)
+                                      : pick_cell(extent, 2.0 * cell, 3.0 * cell, 3.5 * cell);
+        }
         // ---- aggregation by cells
         DBuf<uint64_t> keys, keys_s;
         DBuf<int32_t> ids, ids_s, head, rank1;
-        keys.alloc(l.n, s);
-        keys_s.alloc(l.n, s);
-        ids.alloc(l.n, s);
-        ids_s.alloc(l.n, s);
-        FX_LAUNCH(k_cell_keys, grid_for(l.n), 256, 0, s, l.n, coords.ptr, org.ptr, 1.0 / cell, keys.ptr,
-                  ids.ptr);
-        cub_call([&](void* t, size_t& b) {
-            return cub::DeviceRadixSort::SortPairs(t, b, keys.ptr, keys_s.ptr, ids.ptr, ids_s.ptr, l.n, 0, 63, s);
-        }, tmp_, s);
-        head.alloc(l.n, s);
-        rank1.alloc(l.n, s);
-        FX_LAUNCH(k_heads64, grid_for(l.n), 256, 0, s, l.n, keys_s.ptr, head.ptr);
-        cub_call([&](void* t, size_t& b) { return cub::DeviceScan::InclusiveSum(t, b, head.ptr, rank1.ptr, l.n, s); },
-                 tmp_, s);
         int na = 0;
-        FX_CUDA_CHECK(cudaMemcpyAsync(&na, rank1.ptr + l.n - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-        stream_wait(s, "amg aggregates");
-        if (na >= l.n) {  // cells too small to aggregate: grow and retry this level
+        while (true) {
+            keys.alloc(l.n, s);
+            keys_s.alloc(l.n, s);
+            ids.alloc(l.n, s);
+            ids_s.alloc(l.n, s);
+            const CellGrid grid = cell_grid(extent, cell);
+            int bits = 1;
+            while (bits < 63 && std::ldexp(1.0, bits) < (double)grid.k[0] * grid.k[1] * grid.k[2]) ++bits;
+            FX_LAUNCH(k_cell_keys, grid_for(l.n), 256, 0, s, l.n, coords.ptr, box.ptr, grid, keys.ptr, ids.ptr);
+            cub_call([&](void* t, size_t& b) {
+                return cub::DeviceRadixSort::SortPairs(t, b, keys.ptr, keys_s.ptr, ids.ptr, ids_s.ptr, l.n, 0, bits, s);
+            }, tmp_, s);
+            head.alloc(l.n, s);
+            rank1.alloc(l.n, s);
+            FX_LAUNCH(k_heads64, grid_for(l.n), 256, 0, s, l.n, keys_s.ptr, head.ptr);
+            cub_call([&](void* t, size_t& b) { return cub::DeviceScan::InclusiveSum(t, b, head.ptr, rank1.ptr, l.n, s); },
+                     tmp_, s);
+            FX_CUDA_CHECK(cudaMemcpyAsync(&na, rank1.ptr + l.n - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+            stream_wait(s, "amg aggregates");
+            if (na < l.n) break;
+            // cells too small to aggregate: grow and retry (a single cell in the end)
             if (l.n <= 1) fail(FX_GENERIC, "multigrid: a single block row cannot be coarsened");
             cell *= 1.5;
-            --lev;
-            continue;
         }
-        l.n_agg = na;
-        l.agg.alloc(l.n, s);
-        l.agg_ptr.alloc(na + 1, s);
-        FX_LAUNCH(k_agg_assign, grid_for(l.n), 256, 0, s, l.n, rank1.ptr, head.ptr, ids_s.ptr, l.agg.ptr,
-                  l.agg_ptr.ptr);
-        FX_CUDA_CHECK(cudaMemcpyAsync(l.agg_ptr.ptr + na, &l.n, sizeof(int), cudaMemcpyHostToDevice, s));
-        l.agg_nodes = std::move(ids_s);
+        DBuf<int32_t> agg, agg_ptr;
+        agg.alloc(l.n, s);
+        agg_ptr.alloc(na + 1, s);
+        FX_LAUNCH(k_agg_assign, grid_for(l.n), 256, 0, s, l.n, rank1.ptr, head.ptr, ids_s.ptr, agg.ptr, agg_ptr.ptr);
+        FX_CUDA_CHECK(cudaMemcpyAsync(agg_ptr.ptr + na, &l.n, sizeof(int), cudaMemcpyHostToDevice, s));
         cent.alloc((size_t)na * 3, s);
-        FX_LAUNCH(k_agg_centroid, grid_for(na), 256, 0, s, na, l.agg_ptr.ptr, l.agg_nodes.ptr, coords.ptr, cent.ptr);
+        FX_LAUNCH(k_agg_centroid, grid_for(na), 256, 0, s, na, agg_ptr.ptr, ids_s.ptr, coords.ptr, cent.ptr);
         // ---- tentative prolongator
-        l.Q.alloc((size_t)nd * 6, s);
+        DBuf<double> Q;
+        Q.alloc((size_t)nd * 6, s);
         Rnext.alloc((size_t)na * 36, s);
-        FX_LAUNCH(k_agg_qr, grid_for((int64_t)na * 32), 256, 0, s, na, l.agg_ptr.ptr, l.agg_nodes.ptr, l.bs,
-                  coords.ptr, cent.ptr, Rprev.ptr, l.Q.ptr, Rnext.ptr);
-        // ---- Galerkin coarse matrix
+        FX_LAUNCH(k_agg_qr, grid_for(na, kQrWarps), 32 * kQrWarps, 0, s, na, agg_ptr.ptr, ids_s.ptr, l.bs, coords.ptr,
+                  cent.ptr, Rprev.ptr, Q.ptr, Rnext.ptr);
+        // ---- smoothed prolongator, coarse pattern and Galerkin coarse matrix
         if (!l.S0) {
-            l.gal_rows.alloc(l.nblocks, s);
-            FX_LAUNCH(k_expand_rows, grid_for(l.n), 256, 0, s, l.n, l.row_ptr.ptr, l.gal_rows.ptr);
+            l.blk_row.alloc(l.nblocks, s);
+            FX_LAUNCH(k_expand_rows, grid_for(l.n), 256, 0, s, l.n, l.row_ptr.ptr, l.blk_row.ptr);
         }
-        const FineView F = fine_view(l);
-        const int nbits = bits_for(na > 1 ? na : 2);
-        DBuf<uint64_t> ck, ck_s;
-        DBuf<int64_t> cb, cb_s;
-        ck.alloc(l.nblocks, s);
-        ck_s.alloc(l.nblocks, s);
-        cb.alloc(l.nblocks, s);
-        cb_s.alloc(l.nblocks, s);
-        FX_LAUNCH(k_coarse_keys, grid_for(l.nblocks), 256, 0, s, l.nblocks, F, l.agg.ptr, nbits, ck.ptr, cb.ptr);
-        cub_call([&](void* t, size_t& b) {
-            return cub::DeviceRadixSort::SortPairs(t, b, ck.ptr, ck_s.ptr, cb.ptr, cb_s.ptr, l.nblocks, 0, 2 * nbits,
-                                                   s);
-        }, tmp_, s);
-        ck.release();
-        cb.release();
-        DBuf<int32_t> chead, cbid;
-        chead.alloc(l.nblocks, s);
-        cbid.alloc(l.nblocks, s);
-        FX_LAUNCH(k_heads_u64, grid_for(l.nblocks), 256, 0, s, l.nblocks, ck_s.ptr, chead.ptr);
-        cub_call([&](void* t, size_t& b) {
-            return cub::DeviceScan::InclusiveSum(t, b, chead.ptr, cbid.ptr, l.nblocks, s);
-        }, tmp_, s);
-        int ncb = 0;
-        FX_CUDA_CHECK(cudaMemcpyAsync(&ncb, cbid.ptr + l.nblocks - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-        stream_wait(s, "amg coarse blocks");
         L.emplace_back();
         AmgLevel& c = L.back();
         AmgLevel& lf = L[L.size() - 2];
+        const bool smoothed = build_transfer(fine_view(lf), na, agg.ptr, Q.ptr, lf.dinv_ptr(), kSmoothOmega / lf.lmax,
+                                             lf.tr, c.row_ptr, c.cols, &c.nblocks, tmp_, s);
+        lf.pscale = smoothed ? 1.0 / kAmgOvercorrect : 1.0;
         c.n = na;
         c.bs = 6;
-        c.nblocks = ncb;
-        DBuf<int64_t> seg;
-        DBuf<int32_t> crow, cnt;
-        seg.alloc(ncb + 1, s);
-        crow.alloc(ncb, s);
-        c.cols.alloc(ncb, s);
-        cnt.alloc(na, s);
-        cnt.zero(s);
-        FX_LAUNCH(k_coarse_blocks, grid_for(lf.nblocks), 256, 0, s, lf.nblocks, ck_s.ptr, cbid.ptr, nbits, seg.ptr,
-                  crow.ptr, c.cols.ptr, cnt.ptr);
-        const int64_t nbf = lf.nblocks;
-        FX_CUDA_CHECK(cudaMemcpyAsync(seg.ptr + ncb, &nbf, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-        c.row_ptr.alloc(na + 1, s);
-        FX_CUDA_CHECK(cudaMemsetAsync(c.row_ptr.ptr, 0, sizeof(int32_t), s));
-        cub_call([&](void* t, size_t& b) {
-            return cub::DeviceScan::InclusiveSum(t, b, cnt.ptr, c.row_ptr.ptr + 1, na, s);
-        }, tmp_, s);
-        c.vals.alloc((size_t)ncb * 36, s);
-        lf.gal_seg = std::move(seg);  // kept for refresh()
-        lf.gal_blk = std::move(cb_s);
-        galerkin(lf, c, s);
-        stream_wait(s, "amg galerkin");
+        c.vals.alloc((size_t)c.nblocks * 36, s);
+        galerkin_product(fine_view(lf), lf.tr, c.vals.ptr, s);
         // next level points and near-null-space
         coords = std::move(cent);
         Rprev = std::move(Rnext);
-        cell *= 2.0;
+        if (cell0 > 0.0) cell *= 2.0;
     }
-    if (L.size() > 2) {  // K-cycle work vectors on the first coarse level
-        AmgLevel& l1 = L[1];
+    if ((int)L.size() > planar_ + 1) {  // K-cycle work vectors on the first 6x6 level
+        AmgLevel& l1 = L[planar_];
         const int64_t nd1 = (int64_t)l1.n * l1.bs;
         for (auto& v : l1.kc) v.alloc(nd1, s);
         l1.kcs.alloc(8, s);
@@ -1864,23 +1870,22 @@ void Amg::setup(const BsrStructure& S0, const double* vals0, const double* dinv0
     }
 }
 
-void Amg::refresh(const double* vals0, const double* dinv0, cudaStream_t s, AmgStats* st) {
+void Amg::refresh(const PlanarIn* in, cudaStream_t s, AmgStats* st) {
     EventTimer timer;
     timer.start(s);
-    L[0].vals0 = vals0;
-    L[0].dinv0 = dinv0;
+    for (int m = 0; m < planar_; ++m) set_planar(L[m], in[m]);
     for (size_t lev = 0; lev < L.size(); ++lev) {  // the numeric steps of setup(), in its order
         AmgLevel& l = L[lev];
-        if (lev > 0)
+        if (!l.S0)
             FX_LAUNCH(k_block_inv6, grid_for(l.n, 128), 128, 0, s, l.n, l.row_ptr.ptr, l.cols.ptr, l.vals.ptr,
                       l.dinv.ptr);
         if (l.coarsest) {
             coarsest_inverse(l, s);
             break;
         }
-        estimate_lmax(l, red_, s, lev == 0 ? vals0_f32_ : nullptr, true,
-                      lev == 0 && kAmgEstF16 ? vals0_f16_ : nullptr, sq4_);
-        galerkin(l, L[lev + 1], s);
+        if (!l.S0) planar_values(l, s);
+        estimate_lmax(l, red_, s, true);
+        if (!l.corner_next) galerkin_product(fine_view(l), l.tr, L[lev + 1].vals.ptr, s);
     }
     if (st) {
         st->levels = (int)L.size();
@@ -1928,16 +1933,6 @@ static ChebCoef cheb_coef(double lmax, int degree, int kind, double ratio) {
     return k;
 }
 
-static LnOp ln_op(const AmgLevel& l) {
-    LnOp o{};
-    o.n = l.n;
-    o.row_ptr = l.row_ptr.ptr;
-    o.cols = l.cols.ptr;
-    o.vals = l.vals.ptr;
-    o.dinv = l.dinv.ptr;
-    return o;
-}
-
 // Cycle at a coarse level (6x6 blocks) for A x = b (b and x of that level's size):
 // Chebyshev pre-smoothing from x = 0 into the scratch iterate xs (start kernel,
 // then SpMVs fused with the updates), the residual, the coarse correction added
@@ -1945,7 +1940,7 @@ static LnOp ln_op(const AmgLevel& l) {
 CoarseStart Amg::coarse_start(int m) const {
     CoarseStart cs{};
     const AmgLevel& c = L[m];
-    if (c.coarsest || (kcycle_ && m == 1)) return cs;  // dense solve; K-cycle calls the cycle on other vectors
+    if (c.coarsest || (kcycle_ && m == planar_)) return cs;  // dense solve; K-cycle calls the cycle on other vectors
     cs.dinv = c.dinv.ptr;
     cs.r = c.r.ptr;
     cs.d = c.d.ptr;
@@ -1962,8 +1957,8 @@ void Amg::cycle(int lev, const double* b, double* x, cudaStream_t s, bool starte
         return;
     }
     AmgLevel& c = L[lev + 1];
-    // coarse_row6 reads the 6x6 blocks and the gathered 6-vectors as 16-byte pairs
-    if ((reinterpret_cast<uintptr_t>(l.vals.ptr) | reinterpret_cast<uintptr_t>(l.d.ptr) |
+    // coarse_row6 reads the gathered 6-vectors as 16-byte pairs
+    if ((reinterpret_cast<uintptr_t>(l.d.ptr) |
          reinterpret_cast<uintptr_t>(l.t.ptr) | reinterpret_cast<uintptr_t>(l.xs.ptr)) & 15)
         fail(FX_GENERIC, "multigrid: coarse-level buffers not 16-byte aligned");
     const ChebCoef k = cheb_coef(l.lmax, degree_, cheb_kind_, cheb_ratio_);
@@ -1990,10 +1985,12 @@ void Amg::cycle(int lev, const double* b, double* x, cudaStream_t s, bool starte
         o.r = l.r.ptr;
         FX_LAUNCH(k_ln_op<kL0RUpd>, grid, kLnThreads, 0, s, o);  // r = b - A xs
     }
-    FX_LAUNCH(k_restrict, grid_for((int64_t)l.n_agg * 32, kLnThreads), kLnThreads, 0, s, l.n_agg, l.agg_ptr.ptr, l.agg_nodes.ptr, l.bs,
-              l.Q.ptr, l.r.ptr, c.b.ptr, coarse_start(lev + 1));
+    FX_LAUNCH(k_restrict<6>, (unsigned)l.tr.na, 32 * kRestrictWarps, 0, s, l.tr.t_ptr.ptr, l.tr.t_row.ptr,
+              l.tr.t_val32.ptr, l.r.ptr, c.b.ptr, coarse_start(lev + 1));
     coarse(lev + 1, s);
-    FX_LAUNCH(k_prolong, grid_for(nd), 256, 0, s, (int)nd, l.bs, l.agg.ptr, l.Q.ptr, c.x.ptr, xs, alpha_);
+    FX_LAUNCH(k_prolong<6>, grid_for(l.n, kProlongRows<6>), 256, 0, s, l.n, l.tr.ptr.ptr, l.tr.col.ptr,
+              l.tr.val32.ptr, c.x.ptr, xs,
+              alpha_ * l.pscale, nullptr, nullptr);
     {
         LnOp o = ln_op(l);
         o.v = xs;
@@ -2017,11 +2014,11 @@ void Amg::cycle(int lev, const double* b, double* x, cudaStream_t s, bool starte
     }
 }
 
-// Coarse correction at level m: L[m].x ~ A_m^-1 L[m].b, by a K-cycle at the first
-// coarse level (when it is not the coarsest) and V-cycles below.
+// Coarse correction at 6x6 level m: L[m].x ~ A_m^-1 L[m].b, by a K-cycle at the first
+// such level (when it is not the coarsest) and V-cycles below.
 void Amg::coarse(int m, cudaStream_t s) {
     AmgLevel& l = L[m];
-    if (!(kcycle_ && m == 1 && !l.coarsest)) {
+    if (!(kcycle_ && m == planar_ && !l.coarsest)) {
         cycle(m, l.b.ptr, l.x.ptr, s, coarse_start(m).dinv != nullptr);
         return;
     }
@@ -2035,16 +2032,35 @@ void Amg::coarse(int m, cudaStream_t s) {
     FX_LAUNCH(k_kcycle2, 1, 1024, 0, s, nd, z1, v1, z2, v2, r, l.x.ptr, l.kcs.ptr);
 }
 
-// Level 0 with the fused operators: pre-smoothing from x = 0 (one elementwise
+// The first 6x6 level's correction of the last planar level: restriction of its residual, the
+// coarse cycle, prolongation into its iterate (and the FP32 copy for the smoother's gathers).
+void Amg::first_coarse(cudaStream_t s) {
+    AmgLevel& l = L[planar_ - 1];
+    AmgLevel& c = L[planar_];
+    const bool g32 = l.vals32 || l.vals16;
+    if (fused_coarse_ && !kcycle_ && desc_.ptr) {  // one launch
+        launch_coarse_grid(desc_.ptr, gbar_.ptr, gflag_, g32, degree_, alpha_, s);
+        return;
+    }
+    FX_LAUNCH(k_restrict<3>, (unsigned)l.tr.na, 32 * kRestrictWarps, 0, s, l.tr.t_ptr.ptr, l.tr.t_row.ptr,
+              l.tr.t_val32.ptr, l.r.ptr, c.b.ptr, coarse_start(planar_));
+    coarse(planar_, s);
+    FX_LAUNCH(k_prolong<3>, grid_for(l.n, kProlongRows<3>), 256, 0, s, l.n, l.tr.ptr.ptr, l.tr.col.ptr,
+              l.tr.val32.ptr, c.x.ptr, l.x.ptr, alpha_ * l.pscale, g32 ? l.x4.ptr : nullptr, l.sq4);
+}
+
+// A planar level with the fused operators: pre-smoothing from x = 0 (one elementwise
 // start, degree-1 fused steps, one fused residual update), coarse correction,
-// post-smoothing written straight into z. With S != null the last step also
+// post-smoothing written straight into z. With S != null (level 0) the last step also
 // reduces r.z and beta for the outer CG.
 template <typename VT>
-void Amg::vcycle0(const VT* vals, const double* b, double* z, double* S, double* part, int* counter,
-                  const double* zold, cudaStream_t s, bool started) {
-    AmgLevel& l = L[0];
-    AmgLevel& c = L[1];
-    const int64_t nd = (int64_t)l.n * 3;
+void Amg::vcycle(int m, const double* b, double* z, double* S, double* part, int* counter, const double* zold,
+                 cudaStream_t s, bool started) {
+    AmgLevel& l = L[m];
+    const VT* vals;
+    if constexpr (std::is_same<VT, __half>::value) vals = l.vals16;
+    else if constexpr (std::is_same<VT, float>::value) vals = l.vals32;
+    else vals = l.vals0;
     const ChebCoef k = cheb_coef(l.lmax, degree_, cheb_kind_, cheb_ratio_);
     const unsigned grid = l0_grid(l.n, std::is_same<VT, __half>::value);
     // FP32 or FP16 values: the smoother's gathered vectors are FP32 (float4 per node),
@@ -2058,10 +2074,10 @@ void Amg::vcycle0(const VT* vals, const double* b, double* z, double* S, double*
     float4* x4 = reinterpret_cast<float4*>(l.x4.ptr);
     if (!started)
         FX_LAUNCH(k_l0_cheb_start, grid_for(l.n), 256, 0, s, l.n, l.dinv0, b, l.r.ptr, dA, g32 ? dA4 : nullptr,
-                  l.x.ptr, k.c2_start, sq4_, rdr_, hs);
+                  l.x.ptr, k.c2_start, l.sq4, rdr_, hs);
     auto op = [&]() {
         L0Op<VT> o = l0_op<VT>(l, vals);
-        o.sq4 = sq4_;
+        o.sq4 = l.sq4;
         o.hs = hs;
         return o;
     };
@@ -2086,16 +2102,16 @@ void Amg::vcycle0(const VT* vals, const double* b, double* z, double* S, double*
         o.r = l.r.ptr;
         FX_LAUNCH((k_l0_op<VT, kL0RUpd, g32>), grid, 256, 0, s, o);  // r = b - A x
     }
-    if (fused_coarse_ && !kcycle_ && desc_.ptr) {  // restriction, coarse levels, prolongation: one launch
-        launch_coarse_grid(desc_.ptr, gbar_.ptr, gflag_, g32, degree_, alpha_, s);
+    if (l.corner_next) {
+        AmgLevel& c = L[m + 1];
+        const Start0 c0 = start_of(c);
+        FX_LAUNCH(k_corner_restrict, grid_for((int64_t)c.n * kCornerLanes), 256, 0, s, corner_, l.r.ptr, c.b.ptr,
+                  c.dinv0, c0.r, c0.x, c0.d, c0.d4, c0.c2, c0.sq4, c0.hs);
+        vcycle<VT>(m + 1, c.b.ptr, c.xs.ptr, nullptr, nullptr, nullptr, nullptr, s, true);
+        FX_LAUNCH(k_corner_prolong, grid_for(l.n), 256, 0, s, corner_, c.result(), l.x.ptr, alpha_ * l.pscale,
+                  g32 ? x4 : nullptr, l.sq4);
     } else {
-        FX_LAUNCH(k_restrict, grid_for((int64_t)l.n_agg * 32, kLnThreads), kLnThreads, 0, s, l.n_agg, l.agg_ptr.ptr, l.agg_nodes.ptr, 3,
-                  l.Q.ptr, l.r.ptr, c.b.ptr, coarse_start(1));
-        coarse(1, s);
-        if (g32)
-            FX_LAUNCH(k_prolong0, grid_for(l.n), 256, 0, s, l.n, l.agg.ptr, l.Q.ptr, c.x.ptr, l.x.ptr, x4, alpha_,
-                      sq4_);
-        else FX_LAUNCH(k_prolong, grid_for(nd), 256, 0, s, (int)nd, 3, l.agg.ptr, l.Q.ptr, c.x.ptr, l.x.ptr, alpha_);
+        first_coarse(s);
     }
     for (int st = 0; st < degree_; ++st) {
         L0Op<VT> o = op();
@@ -2136,21 +2152,20 @@ void Amg::vcycle0(const VT* vals, const double* b, double* z, double* S, double*
 
 void Amg::apply(const double* r, double* z, double* S, double* part, int* counter, const double* zold,
                 cudaStream_t s, bool started) {
-    if (vals0_f16_) vcycle0<__half>(vals0_f16_, r, z, S, part, counter, zold, s, started);
-    else if (vals0_f32_) vcycle0<float>(vals0_f32_, r, z, S, part, counter, zold, s, started);
-    else vcycle0<double>(L[0].vals0, r, z, S, part, counter, zold, s, started);
+    if (L[0].vals16) vcycle<__half>(0, r, z, S, part, counter, zold, s, started);
+    else if (L[0].vals32) vcycle<float>(0, r, z, S, part, counter, zold, s, started);
+    else vcycle<double>(0, r, z, S, part, counter, zold, s, started);
 }
 
-Amg::Start0 Amg::start0() const {
-    const AmgLevel& l = L[0];
+Amg::Start0 Amg::start_of(const AmgLevel& l) const {
     Start0 o{};
     o.r = l.r.ptr;
     o.x = l.x.ptr;
     o.d = l.d.ptr;
-    o.d4 = vals0_f32_ || vals0_f16_ ? reinterpret_cast<float4*>(l.d4a.ptr) : nullptr;
+    o.d4 = l.vals32 || l.vals16 ? reinterpret_cast<float4*>(l.d4a.ptr) : nullptr;
     o.c2 = cheb_coef(l.lmax, degree_, cheb_kind_, cheb_ratio_).c2_start;
-    o.sq4 = sq4_;
-    o.hs = vals0_f16_ ? h16_scale_slot() : nullptr;
+    o.sq4 = l.sq4;
+    o.hs = l.vals16 ? h16_scale_slot() : nullptr;
     return o;
 }
 
@@ -2247,49 +2262,55 @@ double profile_smoother_op(const BsrStructure& S, const double* vals64, const do
     return ms;
 }
 
+static ClTransfer cl_transfer(const AmgLevel& l) {
+    const Transfer& t = l.tr;
+    return ClTransfer{t.na, t.ptr.ptr, t.col.ptr, t.t_ptr.ptr, t.t_row.ptr, t.val32.ptr, t.t_val32.ptr, l.pscale};
+}
+
 void Amg::describe(ClInst& o) const {
-    const AmgLevel& l0 = L[0];
-    o.n = l0.n;
+    o.n = L[0].n;
     o.levels = (int)L.size();
-    o.goff = l0.S0->goff.ptr;
-    o.cols = l0.S0->cols.ptr;
-    o.vals64 = l0.vals0;
-    o.vals32 = vals0_f32_;
-    o.dinv0 = l0.dinv0;
-    o.sq4 = sq4_;
-    o.agg = l0.agg.ptr;
-    o.agg_ptr = l0.agg_ptr.ptr;
-    o.agg_nodes = l0.agg_nodes.ptr;
-    o.Q = l0.Q.ptr;
-    o.n_agg = l0.n_agg;
-    o.lr = l0.r.ptr;
-    o.lx = l0.x.ptr;
-    o.ld = l0.d.ptr;
-    o.lt = l0.t.ptr;
-    o.d4a = l0.d4a.ptr;
-    o.d4b = l0.d4b.ptr;
-    o.x4 = l0.x4.ptr;
-    const ChebCoef k0 = cheb_coef(l0.lmax, degree_, cheb_kind_, cheb_ratio_);
-    o.c2_start = k0.c2_start;
-    for (int i = 0; i < 8; ++i) {
-        o.c1[i] = k0.c1[i];
-        o.c2[i] = k0.c2[i];
+    o.planar = planar_;
+    for (int m = 0; m < planar_; ++m) {
+        const AmgLevel& l = L[m];
+        ClPlanar& p = o.pl[m];
+        p.n = l.n;
+        p.goff = l.S0->goff.ptr;
+        p.cols = l.S0->cols.ptr;
+        p.vals64 = l.vals0;
+        p.vals32 = l.vals32;
+        p.dinv0 = l.dinv0;
+        p.sq4 = l.sq4;
+        p.lr = l.r.ptr;
+        p.lx = l.x.ptr;
+        p.ld = l.d.ptr;
+        p.lt = l.t.ptr;
+        p.b = l.b.ptr;
+        p.z = l.xs.ptr;
+        p.d4a = l.d4a.ptr;
+        p.d4b = l.d4b.ptr;
+        p.x4 = l.x4.ptr;
+        const ChebCoef k = cheb_coef(l.lmax, degree_, cheb_kind_, cheb_ratio_);
+        p.c2_start = k.c2_start;
+        for (int i = 0; i < 8; ++i) {
+            p.c1[i] = k.c1[i];
+            p.c2[i] = k.c2[i];
+        }
     }
-    for (size_t m = 1; m < L.size() && m < (size_t)kClMaxLevels; ++m) {
+    o.corner = corner_;
+    o.corner_scale = L[0].pscale;
+    o.tr = cl_transfer(L[planar_ - 1]);
+    for (size_t m = planar_; m < L.size() && m < (size_t)kClMaxLevels; ++m) {
         const AmgLevel& l = L[m];
         ClLevel& c = o.lev[m];
         c.n = l.n;
         c.coarsest = l.coarsest ? 1 : 0;
-        c.n_agg = l.n_agg;
         c.row_ptr = l.row_ptr.ptr;
         c.cols = l.cols.ptr;
-        c.vals = l.vals.ptr;
+        c.vals = l.pvals.ptr;
         c.dinv = l.dinv.ptr;
         c.dense_inv = l.dense_inv.ptr;
-        c.agg = l.agg.ptr;
-        c.agg_ptr = l.agg_ptr.ptr;
-        c.agg_nodes = l.agg_nodes.ptr;
-        c.Q = l.Q.ptr;
+        c.tr = cl_transfer(l);
         c.x = l.x.ptr;
         c.b = l.b.ptr;
         c.r = l.r.ptr;
@@ -2312,34 +2333,48 @@ void Amg::describe(ClInst& o) const {
 }
 
 void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* dinv64, const double* xyz,
-                     double cell0, const PcgOptions& opt, cudaStream_t s, AmgStats* st, bool reuse, bool persistent) {
+                     const CornerLevel* corner, double cell0, double node_volume, const PcgOptions& opt,
+                     cudaStream_t s, AmgStats* st, bool reuse, bool persistent) {
     const int n = S.n_rows;
     const int64_t nd = 3 * (int64_t)n;
     if (opt.amg_degree < 1 || opt.amg_degree > 8) fail(FX_INVALID_ARGUMENT, "multigrid smoother degree must be 1..8");
-    const float* v32 = nullptr;
+    PlanarIn in[2];
+    in[0].S = &S;
+    in[0].vals = vals64;
+    in[0].dinv = dinv64;
+    if (corner) {
+        in[1].S = &corner->S;
+        in[1].vals = corner->vals.ptr;
+        in[1].dinv = corner->minv.ptr;
+    }
     const bool f16 = opt.amg_fp32 && opt.amg_fp16 && !persistent;
-    if (f16) {  // FP16 values of S A S and the scales
-        sq4_.alloc((size_t)n, s);
-        FX_LAUNCH(k_diag_sqrt, grid_for(n), 256, 0, s, n, S.goff.ptr, S.diag_k.ptr, vals64, sq4_.ptr);
-        vals16_.alloc((size_t)S.n_groups * 36, s);
-        FX_LAUNCH(k_vals_to_f16, grid_for((int64_t)n * 32), 256, 0, s, n, S.goff.ptr, S.cols.ptr, vals64, sq4_.ptr,
-                  vals16_.ptr);
+    for (int m = 0; m < (corner ? 2 : 1); ++m) {
+        const BsrStructure& Sm = *in[m].S;
+        if (f16) {  // FP16 values of S A S and the scales
+            sq4_[m].alloc((size_t)Sm.n_rows, s);
+            FX_LAUNCH(k_diag_sqrt, grid_for(Sm.n_rows), 256, 0, s, Sm.n_rows, Sm.goff.ptr, Sm.diag_k.ptr, in[m].vals,
+                      sq4_[m].ptr);
+            vals16_[m].alloc((size_t)Sm.n_groups * 36, s);
+            FX_LAUNCH(k_vals_to_f16, grid_for((int64_t)Sm.n_rows * 32), 256, 0, s, Sm.n_rows, Sm.goff.ptr, Sm.cols.ptr,
+                      in[m].vals, sq4_[m].ptr, vals16_[m].ptr);
+            in[m].vals16 = vals16_[m].ptr;
+            in[m].sq4 = sq4_[m].ptr;
+        }
+        // FP32 values: the FP32 smoother's; with the FP16 smoother only when the eigenvalue
+        // estimate reads them (kAmgEstF16 off) instead of the FP16 values
+        if (opt.amg_fp32 && (!f16 || !kAmgEstF16)) {
+            const int64_t nv = (int64_t)Sm.n_groups * 36;
+            vals32_[m].alloc(nv, s);
+            FX_LAUNCH(k_f64_to_f32, 148 * 8, 256, 0, s, nv, in[m].vals, vals32_[m].ptr);
+            in[m].vals32 = vals32_[m].ptr;
+        }
     }
-    // FP32 values: the FP32 smoother's; with the FP16 smoother only when the level-0
-    // eigenvalue estimate reads them (kAmgEstF16 off) instead of the FP16 values
-    if (opt.amg_fp32 && (!f16 || !kAmgEstF16)) {
-        const int64_t nv = (int64_t)S.n_groups * 36;
-        vals32_.alloc(nv, s);
-        FX_LAUNCH(k_f64_to_f32, 148 * 8, 256, 0, s, nv, vals64, vals32_.ptr);
-        v32 = vals32_.ptr;
-    }
-    amg.set_smoother(opt.amg_degree, v32);  // before setup: its eigenvalue estimate uses v32
-    if (f16) amg.set_smoother_f16(vals16_.ptr, sq4_.ptr);
-    if (reuse && amg.built_for == S.id && !amg.L.empty() && amg.L[0].n == n) {
-        amg.refresh(vals64, dinv64, s, st);
+    amg.set_degree(opt.amg_degree);
+    if (reuse && amg.built_for == S.id && !amg.L.empty() && amg.L[0].n == n && amg.planar() == (corner ? 2 : 1)) {
+        amg.refresh(in, s, st);
     } else {
         amg.built_for = 0;  // (a failed setup leaves nothing to reuse)
-        amg.setup(S, vals64, dinv64, xyz, n, cell0, s, st);
+        amg.setup(in, corner, corner ? corner->xyz.ptr : xyz, cell0, node_volume, s, st);
         amg.built_for = S.id;
     }
     amg.set_cycle(opt.amg_kcycle);
@@ -2404,11 +2439,11 @@ double AmgPcg::true_relres(const double* b, const double* x, cudaStream_t s) {
 }
 
 int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* dinv64, const double* xyz,
-                  double cell0, const double* b, double* x, const PcgOptions& opt, cudaStream_t s,
+                  const CornerLevel* corner, double cell0, double node_volume, const double* b, double* x, const PcgOptions& opt, cudaStream_t s,
                   int64_t* launches, long long* iters, double* relres, AmgStats* st, bool reuse) {
     const int n = S.n_rows;
     const int64_t nd = 3 * (int64_t)n;
-    prepare(S, vals64, dinv64, xyz, cell0, opt, s, st, reuse);
+    prepare(S, vals64, dinv64, xyz, corner, cell0, node_volume, opt, s, st, reuse);
     const int nb = 296;
     const unsigned g0 = l0_grid(n, false, true);  // q = K p
     if (2 * (int64_t)g0 > (int64_t)part_.n) fail(FX_GENERIC, "multigrid: partial-sum buffer smaller than the CG grid");

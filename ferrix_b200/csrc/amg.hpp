@@ -2,17 +2,19 @@
 // node), used inside PCG in place of the 3x3 block-Jacobi preconditioner.
 //
 // Hierarchy (setup, all on the GPU, deterministic):
+//   * C3D20 meshes: the first coarse level is the corner level (corner.hpp), a planar BSR3
+//     matrix like the fine one (417k-DOF box to 1e-10: 116 CG iterations without it and with
+//     unsmoothed aggregation, 36 with both, 59.2 -> 25.4 ms a solve);
 //   * aggregation by spatial binning of the level's points (nodes, then
 //     aggregate centroids) into cubic cells;
 //   * tentative prolongator from the six rigid-body modes (three translations,
 //     three rotations about the aggregate centroid): per aggregate a QR of the
 //     stacked near-null-space rows (one warp per aggregate, modified
-//     Gram-Schmidt applied twice); Q gives the prolongator rows, R the next
-//     level's near-null-space (Vanek, Mandel & Brezina 1996, without the
-//     prolongator smoothing step);
-//   * Galerkin coarse matrix A_c = Q^T A Q: fine blocks are sorted by their
-//     (aggregate, aggregate) key and every coarse 6x6 block sums Q_i^T A_ij Q_j
-//     over its fine blocks in a fixed order (no atomics);
+//     Gram-Schmidt applied twice); Q gives the tentative rows, R the next
+//     level's near-null-space (Vanek, Mandel & Brezina 1996);
+//   * smoothed prolongator P = (I - omega D^-1 A) Q and Galerkin coarse matrix
+//     A_c = P^T A P (amg_transfer.hpp). Without the smoothing step the CG needs about twice
+//     the iterations (C3D4, 205k DOF to 1e-10: 64 against 36, 14.3 -> 13.8 ms a solve);
 //   * Chebyshev smoothing of degree 2 on D^-1 A (D = block diagonal) with the
 //     largest eigenvalue from power iteration; dense inverse at the coarsest
 //     level.
@@ -23,6 +25,8 @@
 
 #include <vector>
 
+#include "amg_transfer.hpp"
+#include "corner.hpp"
 #include "kernels.hpp"
 #include "pcg.hpp"
 
@@ -39,34 +43,38 @@ struct ClInst;
 struct AmgLevel {
     int n = 0;   // block rows (nodes at level 0, aggregates above)
     int bs = 3;  // block size
-    // level 0 matrix: the planar BSR3 of the fine system
+    // planar levels (the fine system, and the corner level of C3D20 meshes): BSR3 matrix, 3x3 block
+    // inverses of its diagonal, and the smoother's copies of the values: FP32, or FP16 of the
+    // scaled matrix S A S (S = diag(a_ii)^-1/2) with sqrt(a_ii) per node (null: FP64 smoothing)
     const BsrStructure* S0 = nullptr;
     const double* vals0 = nullptr;
-    const double* dinv0 = nullptr;  // 3x3 block inverses of the fine diagonal (block-Jacobi)
+    const double* dinv0 = nullptr;
+    const float* vals32 = nullptr;
+    const __half* vals16 = nullptr;
+    const float4* sq4 = nullptr;
     // coarse levels: row-major block CSR, blocks of bs x bs
     DBuf<int32_t> row_ptr, cols;
     DBuf<double> vals, dinv;
+    DBuf<double2> pvals;  // the cycle's copy of vals (coarse_row6)
     int64_t nblocks = 0;
     double lmax = 0.0;
-    // transfer to the next level
-    DBuf<int32_t> agg;                 // aggregate of each block row
-    DBuf<double> Q;                    // n * bs * 6 prolongator rows
-    DBuf<int32_t> agg_ptr, agg_nodes;  // members of each aggregate
-    int n_agg = 0;
-    // work vectors (n * bs); xs: pre-smoothed iterate of the coarse-level cycle
+    // transfer to the next level (its pair lists are kept for refresh) and the scale of its
+    // coarse corrections relative to Amg::overcorrect()
+    Transfer tr;
+    double pscale = 1.0;
+    bool corner_next = false;  // the next level is the corner level (transfer corner.hpp instead of tr)
+    // work vectors (n * bs); xs: at 6x6 levels the pre-smoothed iterate (the cycle's result goes to
+    // x), at the corner level the cycle's result
     DBuf<double> x, b, r, d, t, xs;
-    // fine level with FP32 smoother values: directions and the iterate as float4 per node
+    const double* result() const { return S0 ? xs.ptr : x.ptr; }
+    // planar levels with FP32 smoother values: directions and the iterate as float4 per node
     DBuf<float> d4a, d4b, x4;
     // coarsest level: dense inverse (n*bs)^2
     bool coarsest = false;
     DBuf<double> dense_inv;
     // K-cycle work vectors (first coarse level): z1, v1, r, z2, v2 and scalars
     DBuf<double> kc[5], kcs;
-    // Galerkin map to the next level (kept for refresh): the fine blocks sorted by
-    // coarse block, each coarse block's segment of them, and (levels > 0) the row
-    // of every fine block
-    DBuf<int64_t> gal_seg, gal_blk;
-    DBuf<int32_t> gal_rows;
+    DBuf<int32_t> blk_row;  // levels > 0: the row of every block
     // last power-iteration vector of the eigenvalue estimate (start of the next refresh's)
     DBuf<double> ev;
     const double* dinv_ptr() const { return S0 ? dinv0 : dinv.ptr; }
@@ -78,6 +86,15 @@ struct AmgStats {
     double setup_ms = 0.0;
 };
 
+// A planar level's matrix as setup() and refresh() take it (AmgLevel's fields of the same names).
+struct PlanarIn {
+    const BsrStructure* S = nullptr;
+    const double *vals = nullptr, *dinv = nullptr;
+    const float* vals32 = nullptr;
+    const __half* vals16 = nullptr;
+    const float4* sq4 = nullptr;
+};
+
 // First smoothing step of a coarse level, done by the restriction kernel into it.
 struct CoarseStart {
     const double* dinv;  // 6x6 block inverses of the coarse level
@@ -87,28 +104,19 @@ struct CoarseStart {
 
 class Amg {
    public:
-    // xyz: FP64 node coordinates (device, 3 per node); dinv0: fine 3x3 block inverses.
-    void setup(const BsrStructure& S0, const double* vals0, const double* dinv0, const double* xyz, int n_nodes,
-               double cell0, cudaStream_t s, AmgStats* st);
-    // New matrix values on the structure of the last setup: aggregates, prolongators
-    // and coarse patterns are kept; coarse values, block inverses, eigenvalue
+    // in: the fine matrix and, with a corner level (corner != null), that level's. xyz: FP64
+    // coordinates (device, 3 per node) of the last planar level's nodes. cell0: edge of the first
+    // aggregates' cells, 0 = chosen from the mesh (pick_cell; node_volume: volume per such node).
+    void setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz, double cell0, double node_volume,
+               cudaStream_t s, AmgStats* st);
+    // New matrix values on the structure of the last setup: aggregates, prolongators (values
+    // included) and coarse patterns are kept; coarse values, block inverses, eigenvalue
     // estimates and the coarsest inverse are recomputed.
-    void refresh(const double* vals0, const double* dinv0, cudaStream_t s, AmgStats* st);
+    void refresh(const PlanarIn* in, cudaStream_t s, AmgStats* st);
+    int planar() const { return planar_; }  // planar levels: 1, or 2 with a corner level
     uint64_t built_for = 0;  // BsrStructure::id of the last setup (0: none)
-    // Smoother settings: Chebyshev degree (1..8) and, when vals_f32 is not null,
-    // FP32 values of the fine matrix for the level-0 smoothing (FP64 vectors).
-    void set_smoother(int degree, const float* vals_f32) {
-        degree_ = degree;
-        vals0_f32_ = vals_f32;
-        vals0_f16_ = nullptr;
-        sq4_ = nullptr;
-    }
-    // FP16 values of the scaled fine matrix S A S (S = diag(a_ii)^-1/2) and sqrt(a_ii) per
-    // node for the level-0 smoothing steps, in place of FP32 values (null: off)
-    void set_smoother_f16(const __half* vals16, const float4* sq4) {
-        vals0_f16_ = vals16;
-        sq4_ = sq4;
-    }
+    // Chebyshev degree (1..8)
+    void set_degree(int degree) { degree_ = degree; }
     // FP16 smoother directions: where the V-cycle started from x = 0 finds r.D^-1 r of its
     // right-hand side (rdr) and the two floats where each V-cycle publishes its power-of-two
     // scale of the stored directions (hs); null: unscaled
@@ -141,7 +149,8 @@ class Amg {
         const float4* sq4;  // FP16 smoother: the float4 direction is written scaled by sqrt(a_ii)
         float* hs;          // FP16 directions: where the start publishes the V-cycle's scale (else null)
     };
-    Start0 start0() const;
+    Start0 start0() const { return start_of(L[0]); }
+    Start0 start_of(const AmgLevel& l) const;
     // the hierarchy, smoother coefficients and work vectors, for the persistent solve
     void describe(ClInst& out) const;
     // The coarse part of each V-cycle as one cooperative launch (on: after every setup /
@@ -163,17 +172,18 @@ class Amg {
     CoarseStart coarse_start(int m) const;
     void coarse(int m, cudaStream_t s);
     void coarsest_inverse(AmgLevel& l, cudaStream_t s);
+    // V-cycle from planar level m, whose smoother values are VT
     template <typename VT>
-    void vcycle0(const VT* vals, const double* b, double* z, double* S, double* part, int* counter,
-                 const double* zold, cudaStream_t s, bool started);
+    void vcycle(int m, const double* b, double* z, double* S, double* part, int* counter, const double* zold,
+                cudaStream_t s, bool started);
+    void first_coarse(cudaStream_t s);  // from the last planar level's residual into its iterate
+    int planar_ = 1;
+    CornerView corner_;
     bool kcycle_ = false;
     int64_t part_slots_ = 0;
     int cheb_kind_ = 0;
     double alpha_ = 1.0, cheb_ratio_ = 30.0;
     int degree_ = 2;
-    const float* vals0_f32_ = nullptr;
-    const __half* vals0_f16_ = nullptr;
-    const float4* sq4_ = nullptr;
     const double* rdr_ = nullptr;
     float* hs_ = nullptr;
     float* h16_scale_slot() const;
@@ -194,30 +204,43 @@ class Amg {
 // arithmetic does not depend on the others, so it is the same alone and in a batch.
 constexpr int kClMaxLevels = 8;
 
+struct ClTransfer {  // transfer.cuh
+    int na = 0;
+    const int32_t *ptr = nullptr, *col = nullptr, *t_ptr = nullptr, *t_row = nullptr;
+    const double2 *val = nullptr, *t_val = nullptr;
+    double pscale = 1.0;
+};
+
 struct ClLevel {  // coarse level m >= 1 (6x6 blocks) and its transfer to level m + 1
-    int n = 0, coarsest = 0, n_agg = 0;
+    int n = 0, coarsest = 0;
     const int32_t *row_ptr = nullptr, *cols = nullptr;
-    const double *vals = nullptr, *dinv = nullptr, *dense_inv = nullptr;
-    const int32_t *agg = nullptr, *agg_ptr = nullptr, *agg_nodes = nullptr;
-    const double* Q = nullptr;
+    const double2* vals = nullptr;
+    const double *dinv = nullptr, *dense_inv = nullptr;
+    ClTransfer tr;
     double *x = nullptr, *b = nullptr, *r = nullptr, *d = nullptr, *t = nullptr, *xs = nullptr;
     double c2_start = 0.0, c1[8] = {}, c2[8] = {};
 };
 
-struct ClInst {
-    int n = 0, levels = 0;
-    // level 0: planar BSR3 (FP64 values; FP32 copy for the smoother or null), 3x3 block inverses
+// A planar level: BSR3 (FP64 values; FP32 copy for the smoother or null), 3x3 block inverses
+struct ClPlanar {
+    int n = 0;
     const int32_t *goff = nullptr, *cols = nullptr;
     const double* vals64 = nullptr;
     const float* vals32 = nullptr;
     const double* dinv0 = nullptr;
     const float4* sq4 = nullptr;  // FP16 smoother: the FP32 iterate copy is scaled by sqrt(a_ii)
-    const int32_t *agg = nullptr, *agg_ptr = nullptr, *agg_nodes = nullptr;
-    const double* Q = nullptr;
-    int n_agg = 0;
     double *lr = nullptr, *lx = nullptr, *ld = nullptr, *lt = nullptr;
+    double *b = nullptr, *z = nullptr;  // the corner level's right-hand side and result
     float *d4a = nullptr, *d4b = nullptr, *x4 = nullptr;
     double c2_start = 0.0, c1[8] = {}, c2[8] = {};
+};
+
+struct ClInst {
+    int n = 0, levels = 0, planar = 1;  // lev[m] is used from m = planar on
+    ClPlanar pl[2];
+    CornerView corner;     // with two planar levels: the transfer between them
+    double corner_scale = 1.0;  // of its corrections, relative to the overcorrection factor
+    ClTransfer tr;         // last planar level to the first 6x6 level
     // the CG: right-hand side, iterate and work vectors (3n each)
     const double* b = nullptr;
     double *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr;
@@ -248,6 +271,9 @@ void launch_coarse_grid(const ClInst* inst, GridBarState* st, double* flag, bool
 // took 243-324 ms against 183 ms for the multi-launch path on every stream (B200).
 constexpr int64_t kClDefaultMaxDof = 2000;
 
+// The default of the option amg_aggregate_nodes: with it the hierarchy chooses its cells (pick_cell).
+constexpr int kAmgAggregateNodes = 40;
+
 // CG on the FP64 BSR3 system preconditioned by one V-cycle per iteration.
 // CUDA-event time (ms per launch) of the fused fine-level Chebyshev step (SpMV +
 // smoother update) on the given FP64 system, with FP32 values when fp32; bytes =
@@ -260,15 +286,17 @@ class AmgPcg {
    public:
     // For the persistent solve: set up (or refresh) the hierarchy for the system and
     // allocate the CG vectors, without iterating; then describe it for the kernel.
-    void prepare(const BsrStructure& S, const double* vals64, const double* dinv64, const double* xyz, double cell0,
-                 const PcgOptions& opt, cudaStream_t s, AmgStats* st, bool reuse, bool persistent = false);
+    // corner: the corner level with its matrix, or null; cell0, node_volume: Amg::setup
+    void prepare(const BsrStructure& S, const double* vals64, const double* dinv64, const double* xyz,
+                 const CornerLevel* corner, double cell0, double node_volume, const PcgOptions& opt, cudaStream_t s,
+                 AmgStats* st, bool reuse, bool persistent = false);
     ClInst describe(const double* b, double* x) const;
     // ||b - A x||_D / ||b||_D of the assembled FP64 system after a persistent solve
     double true_relres(const double* b, const double* x, cudaStream_t s);
     // reuse: keep the hierarchy's aggregates, prolongators and coarse patterns when
     // the last setup was on the same structure S (only the values are refreshed)
-    int solve(const BsrStructure& S, const double* vals64, const double* dinv64, const double* xyz, double cell0,
-              const double* b, double* x, const PcgOptions& opt, cudaStream_t s, int64_t* launches, long long* iters,
+    int solve(const BsrStructure& S, const double* vals64, const double* dinv64, const double* xyz,
+              const CornerLevel* corner, double cell0, double node_volume, const double* b, double* x, const PcgOptions& opt, cudaStream_t s, int64_t* launches, long long* iters,
               double* relres, AmgStats* st, bool reuse = false);
     Amg amg;
 
@@ -277,9 +305,9 @@ class AmgPcg {
     const double* vals64_ = nullptr;
     const double* dinv64_ = nullptr;
     DBuf<double> r_, z_, z2_, p_, q_, part_, sc_;
-    DBuf<float> vals32_;
-    DBuf<__half> vals16_;
-    DBuf<float4> sq4_;
+    DBuf<float> vals32_[2];  // per planar level
+    DBuf<__half> vals16_[2];
+    DBuf<float4> sq4_[2];
     DBuf<float> hs_;  // FP16 smoother directions: the current V-cycle's {2^k, 2^-k}
     DBuf<int> counter_;
 };

@@ -24,6 +24,8 @@
 
 #include "amg.hpp"
 #include "coarse_row.cuh"
+#include "corner.cuh"
+#include "transfer.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -99,7 +101,7 @@ __device__ __forceinline__ void ld4g<double>(const double* p, double o[4]) {
     o[3] = b.y;
 }
 
-// Level-0 operator over the planar BSR3 (8 lanes per block row, 4 rows per warp,
+// Operator of a planar level's BSR3 matrix (8 lanes per block row, 4 rows per warp,
 // uniform trip count per warp), as the multi-kernel path's fine-level operator:
 //   kOpApply  y = A v, dsum += v.y
 //   kOpRUpd   r -= A v
@@ -108,7 +110,7 @@ __device__ __forceinline__ void ld4g<double>(const double* p, double o[4]) {
 // G32: gathers from v4 (FP32, float4 per node) and writes the direction into d4;
 // the row's own FP64 component comes from v where the mode needs the iterate (Cheb0).
 template <typename VT, int MODE, bool G32>
-__device__ __noinline__ void l0_op(const ClInst& I, Vg g, const VT* __restrict__ vals, const double* v, const float4* v4,
+__device__ __noinline__ void l0_op(const ClPlanar& I, Vg g, const VT* __restrict__ vals, const double* v, const float4* v4,
                       const double* b, double* y, double* r, double* d_out, float* d4_out, double* xo, double c1,
                       double c2, bool dot, double& dsum) {
     const int sub = g.t & 7;
@@ -260,39 +262,22 @@ __device__ __noinline__ void ln_op(const ClLevel& L, Vg g, const double* v, cons
     }
 }
 
-// b_c = Q^T r_f per aggregate (warp per aggregate); with a coarse start (dinv != null)
-// also the coarse level's first smoothing step from x = 0: d = xs = c2 D^-1 b_c, r = b_c.
-__device__ __noinline__ void restrict_op(Vg g, int na, const int32_t* ptr, const int32_t* nodes, int bs, const double* Q,
-                            const double* rf, double* bc, const double* dinv, double* cr, double* cd, double* cxs,
-                            double c2) {
+// b_c = P^T r_f (warp per aggregate); with a coarse start (dinv != null) also the
+// coarse level's first smoothing step from x = 0: d = xs = c2 D^-1 b_c, r = b_c.
+template <int BS>
+__device__ __noinline__ void restrict_op(Vg g, const ClTransfer& T, const double* rf, double* bc, const double* dinv,
+                                         double* cr, double* cd, double* cxs, double c2) {
     const int lane = g.t & 31;
-    for (int a = g.t >> 5; a < na; a += g.nt >> 5) {
-        const int p0 = __ldg(ptr + a), rows = (__ldg(ptr + a + 1) - p0) * bs;
-        double acc[6] = {0, 0, 0, 0, 0, 0};
-        for (int r0 = lane; r0 < rows; r0 += 128) {
-            double rv[4], qv[4][6];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int rr = r0 + 32 * u;
-                rv[u] = 0.0;
-                if (rr < rows) {
-                    const int j = __ldg(nodes + p0 + rr / bs);
-                    const int64_t row = (int64_t)j * bs + rr % bs;
-                    rv[u] = ldv(rf + row);
-#pragma unroll
-                    for (int c = 0; c < 6; ++c) qv[u][c] = __ldg(Q + row * 6 + c);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (r0 + 32 * u < rows) {
-#pragma unroll
-                    for (int c = 0; c < 6; ++c) acc[c] += qv[u][c] * rv[u];
-                }
-        }
+    for (int a = g.t >> 5; a < T.na; a += g.nt >> 5) {
+        const int p0 = __ldg(T.t_ptr + a), p1 = __ldg(T.t_ptr + a + 1);
         double t[6];
+        restrict_agg<BS, true>(T.t_row, T.t_val, rf, p0, p1, 0, lane, t);
+        for (int v = 1; v < kRestrictWarps; ++v) {
+            double u[6];
+            restrict_agg<BS, true>(T.t_row, T.t_val, rf, p0, p1, v, lane, u);
 #pragma unroll
-        for (int c = 0; c < 6; ++c) t[c] = warp_sum(acc[c]);
+            for (int c = 0; c < 6; ++c) t[c] += u[c];
+        }
         if (lane < 6) {
             const int64_t o = (int64_t)a * 6 + lane;
             double tk = t[0];
@@ -314,35 +299,19 @@ __device__ __noinline__ void restrict_op(Vg g, int na, const int32_t* ptr, const
     }
 }
 
-// x_f += alpha Q x_c over the fine level's dofs (bs per block row)
-__device__ __noinline__ void prolong_op(Vg g, int ndof, int bs, const int32_t* agg, const double* Q, const double* xc, double* xf,
-                           double alpha) {
-    for (int k = g.t; k < ndof; k += g.nt) {
-        const int j = k / bs;
-        const double* q = Q + (int64_t)k * 6;
-        const double* x = xc + (int64_t)__ldg(agg + j) * 6;
-        double t = 0.0;
-        for (int c = 0; c < 6; ++c) t += __ldg(q + c) * ldv(x + c);
-        xf[k] += alpha * t;
-    }
-}
-
-// fine level: x += alpha Q x_c and the FP32 copy of x for the smoother's gathers
-__device__ __noinline__ void prolong0_op(Vg g, const ClInst& I, const double* xc, double alpha) {
-    for (int i = g.t; i < I.n; i += g.nt) {
-        const double* x = xc + (int64_t)__ldg(I.agg + i) * 6;
-        double out[3];
-        for (int k = 0; k < 3; ++k) {
-            const double* q = I.Q + (3 * (int64_t)i + k) * 6;
-            double t = 0.0;
-            for (int c = 0; c < 6; ++c) t += __ldg(q + c) * ldv(x + c);
-            out[k] = ldv(I.lx + 3 * (int64_t)i + k) + alpha * t;
-            I.lx[3 * (int64_t)i + k] = out[k];
+// x_f += alpha P x_c over the fine level's DOFs; x4 != null (3x3 levels): the FP32 copy of the
+// new x_f for the smoother's gathers, scaled by sqrt(a_ii) where sq4 is given
+template <int BS>
+__device__ __noinline__ void prolong_op(Vg g, int n, const ClTransfer& T, const double* xc, double* xf, double alpha,
+                                        float* x4, const float4* sq4) {
+    for (int k = g.t; k < n * BS; k += g.nt) {
+        const int j = k / BS, c = k - j * BS;
+        const double v = ldv(xf + k) + alpha * prolong_dof<BS>(T.ptr, T.col, T.val, xc, j, c);
+        xf[k] = v;
+        if (BS == 3 && x4) {
+            const double q = sq4 ? (double)__ldg(reinterpret_cast<const float*>(sq4) + 4 * (int64_t)j + c) : 1.0;
+            x4[4 * (int64_t)j + c] = (float)(v * q);
         }
-        float4 q = make_float4(1.f, 1.f, 1.f, 0.f);
-        if (I.sq4) q = __ldg(I.sq4 + i);  // FP16 smoother: the gathered copy is scaled by sqrt(a_ii)
-        reinterpret_cast<float4*>(I.x4)[i] = make_float4((float)(out[0] * (double)q.x), (float)(out[1] * (double)q.y),
-                                                         (float)(out[2] * (double)q.z), 0.0f);
     }
 }
 
@@ -355,10 +324,11 @@ __device__ __noinline__ void dense_op(Vg g, int nd, const double* A, const doubl
 }
 
 // Level-0 start of the V-cycle from x = 0 with right-hand side rhs: r0 = rhs,
-// x0 = d = c2 D^-1 rhs. With alpha != 0 first the CG update x += alpha p,
-// r -= alpha q (rhs = r). Returns this thread's part of rhs.D^-1 rhs.
+// x0 = d = c2 D^-1 rhs. With update first the CG update x += alpha p, r -= alpha q
+// (rhs = r). Returns this thread's part of rhs.D^-1 rhs.
 template <bool G32>
 __device__ __noinline__ double start0_op(Vg g, const ClInst& I, double alpha, bool update) {
+    const ClPlanar& P = I.pl[0];
     double acc = 0.0;
     for (int i = g.t; i < I.n; i += g.nt) {
         const int64_t o3 = 3 * (int64_t)i;
@@ -371,21 +341,67 @@ __device__ __noinline__ double start0_op(Vg g, const ClInst& I, double alpha, bo
             } else {
                 rv[c] = ldv(I.r + o3 + c);
             }
-            I.lr[o3 + c] = rv[c];
+            P.lr[o3 + c] = rv[c];
         }
-        const double* D = I.dinv0 + 9 * (int64_t)i;
+        const double* D = P.dinv0 + 9 * (int64_t)i;
         double t[3];
         for (int c = 0; c < 3; ++c) {
             const double dr = __ldg(D + 3 * c) * rv[0] + __ldg(D + 3 * c + 1) * rv[1] + __ldg(D + 3 * c + 2) * rv[2];
             acc += rv[c] * dr;
-            t[c] = I.c2_start * dr;
-            I.lx[o3 + c] = t[c];
+            t[c] = P.c2_start * dr;
+            P.lx[o3 + c] = t[c];
         }
-        if (G32) reinterpret_cast<float4*>(I.d4a)[i] = make_float4((float)t[0], (float)t[1], (float)t[2], 0.0f);
+        if (G32) reinterpret_cast<float4*>(P.d4a)[i] = make_float4((float)t[0], (float)t[1], (float)t[2], 0.0f);
         else
-            for (int c = 0; c < 3; ++c) I.ld[o3 + c] = t[c];
+            for (int c = 0; c < 3; ++c) P.ld[o3 + c] = t[c];
     }
     return acc;
+}
+
+// Restriction to the corner level with its first smoothing step from x = 0
+template <bool G32>
+__device__ __noinline__ void corner_restrict_op(Vg g, const ClInst& I) {
+    const ClPlanar& P = I.pl[1];
+    const int sub = g.t % kCornerLanes;
+    constexpr int R = 32 / kCornerLanes;
+    const int rows = (P.n + R - 1) / R * R;  // uniform trip count per warp
+    for (int i = g.t / kCornerLanes; i < rows; i += g.nt / kCornerLanes) {
+        double v[3];
+        corner_restrict_row<true>(I.corner, I.pl[0].lr, i < P.n ? i : -1, sub, v);
+        if (i >= P.n || sub != 0) continue;
+        const int64_t o3 = 3 * (int64_t)i;
+        const double* D = P.dinv0 + 9 * (int64_t)i;
+        double t[3];
+        for (int c = 0; c < 3; ++c) {
+            t[c] = P.c2_start * (__ldg(D + 3 * c) * v[0] + __ldg(D + 3 * c + 1) * v[1] + __ldg(D + 3 * c + 2) * v[2]);
+            P.b[o3 + c] = v[c];
+            P.lr[o3 + c] = v[c];
+            P.lx[o3 + c] = t[c];
+        }
+        if (G32) reinterpret_cast<float4*>(P.d4a)[i] = make_float4((float)t[0], (float)t[1], (float)t[2], 0.0f);
+        else
+            for (int c = 0; c < 3; ++c) P.ld[o3 + c] = t[c];
+    }
+}
+
+// x0 += alpha P z1 from the corner level's result (and the FP32 copy of x0)
+template <bool G32>
+__device__ __noinline__ void corner_prolong_op(Vg g, const ClInst& I, double alpha) {
+    const ClPlanar& P = I.pl[0];
+    for (int j = g.t; j < P.n; j += g.nt) {
+        double u[3];
+        corner_prolong_node<true>(I.corner, I.pl[1].z, j, u);
+        for (int k = 0; k < 3; ++k) {
+            u[k] = ldv(P.lx + 3 * (int64_t)j + k) + alpha * u[k];
+            P.lx[3 * (int64_t)j + k] = u[k];
+        }
+        if (G32) {
+            float4 q = make_float4(1.f, 1.f, 1.f, 0.f);
+            if (P.sq4) q = __ldg(P.sq4 + j);
+            reinterpret_cast<float4*>(P.x4)[j] = make_float4((float)(u[0] * (double)q.x), (float)(u[1] * (double)q.y),
+                                                             (float)(u[2] * (double)q.z), 0.0f);
+        }
+    }
 }
 
 // One V-cycle for the right-hand side I.r (level-0 start already done by start0_op):
@@ -437,22 +453,21 @@ struct GridBar {
     }
 };
 
-// The coarse part of one V-cycle, from the level-0 residual I.lr: restriction into
-// level 1 (with its first smoothing step unless it is the coarsest), the coarse
+// The coarse part of one V-cycle, from the last planar level's residual: restriction into
+// the first 6x6 level (with its first smoothing step unless it is the coarsest), these
 // levels down to the dense coarsest solve and back up, and the prolongation of the
-// correction into the level-0 iterate (I.lx, and I.x4 with FP32 smoother vectors).
+// correction into the planar level's iterate (lx, and x4 with FP32 smoother vectors).
 // Returns false when a barrier wait ran out (the caller stops).
 template <bool G32, typename Bar>
 __device__ bool coarse_cycle(const ClInst& I, Vg g, int degree, double alpha, Bar& bar) {
-    // restriction into level 1 (with its first smoothing step unless it is the coarsest)
+    const ClPlanar& P = I.pl[I.planar - 1];
     {
-        const ClLevel& c = I.lev[1];
-        restrict_op(g, I.n_agg, I.agg_ptr, I.agg_nodes, 3, I.Q, I.lr, c.b, c.coarsest ? nullptr : c.dinv, c.r, c.d,
-                    c.xs, c.c2_start);
+        const ClLevel& c = I.lev[I.planar];
+        restrict_op<3>(g, I.tr, P.lr, c.b, c.coarsest ? nullptr : c.dinv, c.r, c.d, c.xs, c.c2_start);
         if (!bar.sync()) return false;
     }
     // coarse levels: down to the coarsest, dense solve, back up
-    int m = 1;
+    int m = I.planar;
     const int last = min(I.levels, kClMaxLevels) - 1;  // the coarsest level (setup always ends with one)
     for (; m < last && !I.lev[m].coarsest; ++m) {
         const ClLevel& l = I.lev[m];
@@ -468,8 +483,7 @@ __device__ bool coarse_cycle(const ClInst& I, Vg g, int degree, double alpha, Ba
         ln_op<kOpRUpd>(l, g, cA, nullptr, l.r, nullptr, nullptr, 0.0, 0.0);
         if (!bar.sync()) return false;
         const ClLevel& c = I.lev[m + 1];
-        restrict_op(g, l.n_agg, l.agg_ptr, l.agg_nodes, 6, l.Q, l.r, c.b, c.coarsest ? nullptr : c.dinv, c.r, c.d,
-                    c.xs, c.c2_start);
+        restrict_op<6>(g, l.tr, l.r, c.b, c.coarsest ? nullptr : c.dinv, c.r, c.d, c.xs, c.c2_start);
         if (!bar.sync()) return false;
     }
     {
@@ -477,10 +491,10 @@ __device__ bool coarse_cycle(const ClInst& I, Vg g, int degree, double alpha, Ba
         dense_op(g, 6 * l.n, l.dense_inv, l.b, l.x);
         if (!bar.sync()) return false;
     }
-    for (--m; m >= 1; --m) {
+    for (--m; m >= I.planar; --m) {
         const ClLevel& l = I.lev[m];
         const ClLevel& c = I.lev[m + 1];
-        prolong_op(g, 6 * l.n, 6, l.agg, l.Q, c.x, l.xs, alpha);
+        prolong_op<6>(g, l.n, l.tr, c.x, l.xs, alpha * l.tr.pscale, nullptr, nullptr);
         if (!bar.sync()) return false;
         double* cA = l.d;
         double* cB = l.t;
@@ -494,22 +508,28 @@ __device__ bool coarse_cycle(const ClInst& I, Vg g, int degree, double alpha, Ba
             cB = t;
         }
     }
-    if (G32) prolong0_op(g, I, I.lev[1].x, alpha);
-    else prolong_op(g, 3 * I.n, 3, I.agg, I.Q, I.lev[1].x, I.lx, alpha);
+    prolong_op<3>(g, P.n, I.tr, I.lev[I.planar].x, P.lx, alpha * I.tr.pscale, G32 ? P.x4 : nullptr, P.sq4);
     return bar.sync();
 }
 
 template <typename VT, bool G32>
-__device__ double vcycle(const ClInst& I, Vg g, const VT* vals, int degree, double alpha, cg::cluster_group& cl) {
+__device__ __forceinline__ const VT* planar_vals(const ClPlanar& P) {
+    return G32 ? reinterpret_cast<const VT*>(P.vals32) : reinterpret_cast<const VT*>(P.vals64);
+}
+
+// Pre-smoothing of a planar level after its start, up to the residual r = b - A x; the directions
+// alternate between (ld, d4a) and (lt, d4b) and end in (dA, dA4)
+template <typename VT, bool G32>
+__device__ void planar_down(const ClPlanar& P, Vg g, int degree, cg::cluster_group& cl, double*& dA, double*& dB,
+                            float*& dA4, float*& dB4) {
     double dummy = 0.0;
-    // level-0 pre-smoothing: directions alternate between (ld, d4a) and (lt, d4b)
-    double* dA = I.ld;
-    double* dB = I.lt;
-    float* dA4 = I.d4a;
-    float* dB4 = I.d4b;
+    dA = P.ld;
+    dB = P.lt;
+    dA4 = P.d4a;
+    dB4 = P.d4b;
     for (int st = 1; st < degree; ++st) {
-        l0_op<VT, kOpChebK, G32>(I, g, vals, dA, reinterpret_cast<const float4*>(dA4), nullptr, nullptr, I.lr, dB,
-                                 dB4, I.lx, I.c1[st], I.c2[st], false, dummy);
+        l0_op<VT, kOpChebK, G32>(P, g, planar_vals<VT, G32>(P), dA, reinterpret_cast<const float4*>(dA4), nullptr,
+                                 nullptr, P.lr, dB, dB4, P.lx, P.c1[st], P.c2[st], false, dummy);
         cl.sync();
         double* t = dA;
         dA = dB;
@@ -518,19 +538,22 @@ __device__ double vcycle(const ClInst& I, Vg g, const VT* vals, int degree, doub
         dA4 = dB4;
         dB4 = t4;
     }
-    l0_op<VT, kOpRUpd, G32>(I, g, vals, dA, reinterpret_cast<const float4*>(dA4), nullptr, nullptr, I.lr, nullptr,
-                            nullptr, nullptr, 0.0, 0.0, false, dummy);  // r = b - A x
+    l0_op<VT, kOpRUpd, G32>(P, g, planar_vals<VT, G32>(P), dA, reinterpret_cast<const float4*>(dA4), nullptr, nullptr,
+                            P.lr, nullptr, nullptr, nullptr, 0.0, 0.0, false, dummy);  // r = b - A x
     cl.sync();
-    ClusterBar bar{cl};
-    coarse_cycle<G32>(I, g, degree, alpha, bar);
-    // post-smoothing into z (the last step reduces r.z)
+}
+
+// Post-smoothing of a planar level from its iterate into z; dot: returns this thread's part of b.z
+template <typename VT, bool G32>
+__device__ double planar_up(const ClPlanar& P, Vg g, const double* b, double* z, int degree, bool dot,
+                            cg::cluster_group& cl, double* dA, double* dB, float* dA4, float* dB4) {
     double dsum = 0.0;
-    l0_op<VT, kOpCheb0, G32>(I, g, vals, I.lx, reinterpret_cast<const float4*>(I.x4), I.r, nullptr, I.lr, dA, dA4,
-                             I.z, 0.0, I.c2_start, degree == 1, dsum);
+    l0_op<VT, kOpCheb0, G32>(P, g, planar_vals<VT, G32>(P), P.lx, reinterpret_cast<const float4*>(P.x4), b, nullptr,
+                             P.lr, dA, dA4, z, 0.0, P.c2_start, dot && degree == 1, dsum);
     cl.sync();
     for (int st = 1; st < degree; ++st) {
-        l0_op<VT, kOpChebK, G32>(I, g, vals, dA, reinterpret_cast<const float4*>(dA4), I.r, nullptr, I.lr, dB, dB4,
-                                 I.z, I.c1[st], I.c2[st], st == degree - 1, dsum);
+        l0_op<VT, kOpChebK, G32>(P, g, planar_vals<VT, G32>(P), dA, reinterpret_cast<const float4*>(dA4), b, nullptr,
+                                 P.lr, dB, dB4, z, P.c1[st], P.c2[st], dot && st == degree - 1, dsum);
         cl.sync();
         double* t = dA;
         dA = dB;
@@ -540,6 +563,26 @@ __device__ double vcycle(const ClInst& I, Vg g, const VT* vals, int degree, doub
         dB4 = t4;
     }
     return dsum;
+}
+
+template <typename VT, bool G32>
+__device__ double vcycle(const ClInst& I, Vg g, int degree, double alpha, cg::cluster_group& cl) {
+    double *dA, *dB, *eA, *eB;
+    float *dA4, *dB4, *eA4, *eB4;
+    ClusterBar bar{cl};
+    planar_down<VT, G32>(I.pl[0], g, degree, cl, dA, dB, dA4, dB4);
+    if (I.planar == 2) {
+        corner_restrict_op<G32>(g, I);
+        cl.sync();
+        planar_down<VT, G32>(I.pl[1], g, degree, cl, eA, eB, eA4, eB4);
+        coarse_cycle<G32>(I, g, degree, alpha, bar);
+        planar_up<VT, G32>(I.pl[1], g, I.pl[1].b, I.pl[1].z, degree, false, cl, eA, eB, eA4, eB4);
+        corner_prolong_op<G32>(g, I, alpha * I.corner_scale);
+        cl.sync();
+    } else {
+        coarse_cycle<G32>(I, g, degree, alpha, bar);
+    }
+    return planar_up<VT, G32>(I.pl[0], g, I.r, I.z, degree, true, cl, dA, dB, dA4, dB4);
 }
 
 template <typename VT, bool G32>
@@ -553,7 +596,6 @@ __global__ void __launch_bounds__(kClThreads, 2)
     __syncthreads();
     if (inst >= n_inst) return;  // whole clusters only: the grid is n_inst * kClCtas
     const ClInst& I = insts[inst];
-    const VT* vals = G32 ? reinterpret_cast<const VT*>(I.vals32) : reinterpret_cast<const VT*>(I.vals64);
     const Vg g{(int)cl.block_rank() * kClThreads + (int)threadIdx.x, (int)cl.num_blocks() * kClThreads};
     const int64_t nd = 3 * (int64_t)I.n;
     // x = 0, r = b
@@ -568,7 +610,7 @@ __global__ void __launch_bounds__(kClThreads, 2)
     cluster_sum<1>(v1, sh, cl);
     const double bd = v1[0];
     double rzd = bd;
-    double rz1[1] = {vcycle<VT, G32>(I, g, vals, degree, alpha, cl)};
+    double rz1[1] = {vcycle<VT, G32>(I, g, degree, alpha, cl)};
     cluster_sum<1>(rz1, sh, cl);
     double rz = rz1[0];
     for (int64_t i = g.t; i < nd; i += g.nt) I.p[i] = ldv(I.z + i);
@@ -583,7 +625,7 @@ __global__ void __launch_bounds__(kClThreads, 2)
         }
         // q = A p, alpha = r.z / p.q
         double pq[1] = {0.0};
-        l0_op<double, kOpApply, false>(I, g, I.vals64, I.p, nullptr, nullptr, I.q, nullptr, nullptr, nullptr,
+        l0_op<double, kOpApply, false>(I.pl[0], g, I.pl[0].vals64, I.p, nullptr, nullptr, I.q, nullptr, nullptr, nullptr,
                                        nullptr, 0.0, 0.0, false, pq[0]);
         cl.sync();
         cluster_sum<1>(pq, sh, cl);
@@ -599,7 +641,7 @@ __global__ void __launch_bounds__(kClThreads, 2)
         rzd = rd[0];
         ++it;
         if (rzd <= rtol2 * bd) break;
-        double rzn[1] = {vcycle<VT, G32>(I, g, vals, degree, alpha, cl)};
+        double rzn[1] = {vcycle<VT, G32>(I, g, degree, alpha, cl)};
         cluster_sum<1>(rzn, sh, cl);
         const double beta = rz > 0.0 ? rzn[0] / rz : 0.0;
         rz = rzn[0];

@@ -101,8 +101,8 @@ int preload_kernels(int device) {
                         cudaSuccess && p_load;
     if (ok) {
         loaded = 0;
-        for (const void* anchor : {kernels_anchor_amg(), kernels_anchor_amg_cluster(), kernels_anchor_assembly(),
-                                   kernels_anchor_csr_solve(),
+        for (const void* anchor : {kernels_anchor_amg(), kernels_anchor_amg_cluster(), kernels_anchor_amg_transfer(),
+                                   kernels_anchor_assembly(), kernels_anchor_corner(), kernels_anchor_csr_solve(),
                                    kernels_anchor_elements(), kernels_anchor_noalloc(), kernels_anchor_pcg(),
                                    kernels_anchor_pcg_csr(), kernels_anchor_vectors()}) {
             cudaFunction_t f = nullptr;
@@ -487,6 +487,7 @@ int fx_model_drop_cache(fx_model* m) {
         ModelDev& d = m->dev;
         d.have_structure = false;
         d.S = BsrStructure();
+        d.corner = CornerLevel();
         d.ebuf32.release();
         d.vals32.release();
         d.minv32.release();

@@ -116,13 +116,15 @@ static void exclusive_scan_i32(const int32_t* in, int32_t* out, int n, DBuf<uint
     cub_call([&](void* t, size_t& b) { return cub::DeviceScan::InclusiveSum(t, b, in, out + 1, n, s); }, tmp, s);
 }
 
-void build_bsr_structure(const ElemView& g4, const ElemView& g20, int n_nodes, BsrStructure& S, cudaStream_t s) {
+void build_bsr_structure(const ElemView& g4, const ElemView& g20, int n_nodes, BsrStructure& S, cudaStream_t s,
+                         int npe) {
+    const int pairs = npe * (npe + 1) / 2;
     static std::atomic<uint64_t> next_id{1};
     S.id = next_id.fetch_add(1);
     S.n_rows = n_nodes;
-    const int64_t p4 = (int64_t)g4.n * 16, p20 = (int64_t)g20.n * 400;
+    const int64_t p4 = (int64_t)g4.n * 16, p20 = (int64_t)g20.n * npe * npe;
     const int64_t P = p4 + p20;
-    if ((int64_t)g4.n * kPairs4 + (int64_t)g20.n * kPairs20 >= (int64_t(1) << 31))
+    if ((int64_t)g4.n * kPairs4 + (int64_t)g20.n * pairs >= (int64_t(1) << 31))
         fail(FX_INVALID_ARGUMENT, "mesh too large for 31-bit element-pair slots");
     // the sort items (ordered node pairs of every element) are counted, scanned and
     // indexed in 32 bits: about twice the slots, so this bound is the tighter one
@@ -141,8 +143,8 @@ void build_bsr_structure(const ElemView& g4, const ElemView& g20, int n_nodes, B
         FX_LAUNCH(k_pair_keys, (unsigned)((p4 + T - 1) / T), T, 0, s, g4.n, 4, g4.conn, nb, 0u, kPairs4, keys.ptr,
                   vals.ptr, (int64_t)0);
     if (g20.n)
-        FX_LAUNCH(k_pair_keys, (unsigned)((p20 + T - 1) / T), T, 0, s, g20.n, 20, g20.conn, nb,
-                  (uint32_t)(g4.n * kPairs4), kPairs20, keys.ptr, vals.ptr, p4);
+        FX_LAUNCH(k_pair_keys, (unsigned)((p20 + T - 1) / T), T, 0, s, g20.n, npe, g20.conn, nb,
+                  (uint32_t)(g4.n * kPairs4), pairs, keys.ptr, vals.ptr, p4);
     const int end_bit = 2 * nb;
     cub_call([&](void* t, size_t& b) {
         return cub::DeviceRadixSort::SortPairs(t, b, keys.ptr, keys_s.ptr, vals.ptr, S.slot_sorted.ptr, P, 0,
@@ -189,6 +191,7 @@ void build_bsr_structure(const ElemView& g4, const ElemView& g20, int n_nodes, B
     FX_LAUNCH(k_fill_cols_pad, (n_nodes + T - 1) / T, T, 0, s, n_nodes, S.goff.ptr, S.cols.ptr);
     FX_LAUNCH(k_place_cols, (unsigned)((nblk + T - 1) / T), T, 0, s, (int64_t)nblk, S.blk_row.ptr, blk_col.ptr,
               S.row_ptr.ptr, S.goff.ptr, S.cols.ptr, S.diag_k.ptr);
+    if (npe != 20) return;
     // node -> element-node slots (fixed order: group, element, local node)
     const int64_t q4 = (int64_t)g4.n * 4, q20 = (int64_t)g20.n * 20, Q = q4 + q20;
     DBuf<int32_t> nk, nv, nks;

@@ -1,9 +1,12 @@
-// One warp's sums of a coarse-level block row (row-major 6x6 block CSR): lane l
+// One warp's sums of a coarse-level block row (6x6 block CSR): lane l
 // handles the row's blocks l, l + 32, ..., each whole (its 36 values, its column id
 // and the 6 gathered source values), and the six row sums are reduced over the warp
 // by a fixed xor tree, so that every lane ends with the same six sums. Per row, the
 // loads form three dependent steps (row pointer; column ids and values; gathered
-// sources) whatever the row's length up to 32 blocks. Shared by the per-step coarse
+// sources) whatever the row's length up to 32 blocks. The values of a block row are stored as 18
+// planes of 16-byte pairs (pair q of block k at (b0 * 18 + q * blocks of the row + k)), so that the
+// lanes' loads are consecutive; block after block they were 288 bytes apart and each load
+// touched 32 lines. Shared by the per-step coarse
 // kernels and the persistent / cooperative coarse kernels, which must produce the
 // same sums.
 #pragma once
@@ -25,17 +28,17 @@ __device__ __forceinline__ double2 coarse_ld2(const double* p) {
 // are added by xor shuffles over 16, 8, 4, 2, 1 (both partners add the same two values,
 // so all lanes hold identical bits).
 template <bool CG>
-__device__ __forceinline__ void coarse_row6(const int32_t* __restrict__ cols, const double* __restrict__ vals,
+__device__ __forceinline__ void coarse_row6(const int32_t* __restrict__ cols, const double2* __restrict__ vals,
                                             const double* v, int b0, int nblk, int lane, double (&acc)[6]) {
 #pragma unroll
     for (int r = 0; r < 6; ++r) acc[r] = 0.0;
     for (int j = lane; j < nblk; j += 32) {
         const int64_t blk = b0 + j;
         const int col = __ldg(cols + blk);
-        const double2* a = reinterpret_cast<const double2*>(vals + blk * 36);
+        const double2* a = vals + (int64_t)b0 * 18 + j;
         double2 m[18];
 #pragma unroll
-        for (int k = 0; k < 18; ++k) m[k] = __ldg(a + k);
+        for (int k = 0; k < 18; ++k) m[k] = __ldg(a + (int64_t)k * nblk);
         const double* xs = v + 6 * (int64_t)col;
         const double2 x0 = coarse_ld2<CG>(xs), x1 = coarse_ld2<CG>(xs + 2), x2 = coarse_ld2<CG>(xs + 4);
 #pragma unroll

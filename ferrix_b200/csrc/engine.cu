@@ -78,8 +78,10 @@ static void upload_mats(const MatTableHost& h, MatTableDev& d, cudaStream_t s) {
 double model_footprint(const DenseModel& D) {
     const double e20 = (double)D.g20.size(), e4 = (double)D.g4.size(), n = (double)D.n_nodes;
     const double blocks = 240.0 * e20 + 2.8 * e4;
-    // per 3x3 block: FP64, FP32 and FP16 values (126 B), column ids and group padding
-    return e20 * 32.0e3 + e4 * 1.6e3 + blocks * 136.0 + n * 1.0e3 + 64.0e6;
+    // per 3x3 block: FP64, FP32 and FP16 values (126 B), column ids and group padding. Per element
+    // besides the sort: the multigrid's transfer (C3D4: ~3 operand pairs per block, 40 B each while
+    // sorted, its entries and the product's values) or corner level (C3D20)
+    return e20 * 40.0e3 + e4 * 2.6e3 + blocks * 136.0 + n * 1.0e3 + 64.0e6;
 }
 
 // Spare pool memory to hold before a model's work is queued: 50 % over the
@@ -312,7 +314,7 @@ struct StepRunner {
     double csr_relres = 0.0;
     // aggregation-multigrid preconditioned FP64 CG (FX_PRECOND_AMG)
     bool amg = false;
-    double amg_cell = 0.0;
+    double amg_cell = 0.0, amg_node_volume = 0.0;
     DBuf<double> amg_xyz;
 
     void begin(fx_model* mm, int kk, const fx_solve_opts& oo) {
@@ -330,10 +332,17 @@ struct StepRunner {
         csr = o.precision == FX_PREC_FP64_CSR || csr_reference;
         amg = !csr && o.preconditioner == FX_PRECOND_AMG;
         fp64 = o.precision == FX_PREC_FP64 || csr || amg;
-        if (amg) {  // aggregate cells holding amg_aggregate_nodes nodes on average
+        if (amg) {
+            ModelDev& d = m->dev;
+            if (d.corner.built_for != d.S.id)
+                build_corner_level(d.g4(), d.g20(), (int)m->dense.n_nodes, d.S.id, d.corner, m->ctx->stream);
+            // volume per node of the level that is aggregated; aggregate cells holding the asked
+            // number of its nodes on average, or (the default) chosen by the hierarchy
             const double vol = m->dense.volume > 0.0 ? m->dense.volume : 1.0;
-            const double per = o.amg_aggregate_nodes > 0 ? (double)o.amg_aggregate_nodes : 40.0;
-            amg_cell = std::cbrt(per * vol / (double)std::max<int64_t>(1, m->dense.n_nodes));
+            const int64_t nodes = d.corner.usable ? d.corner.n : m->dense.n_nodes;
+            amg_node_volume = vol / (double)std::max<int64_t>(1, nodes);
+            const bool chosen = o.amg_aggregate_nodes > 0 && o.amg_aggregate_nodes != kAmgAggregateNodes;
+            amg_cell = chosen ? std::cbrt((double)o.amg_aggregate_nodes * amg_node_volume) : 0.0;
         }
         cudaStream_t s = m->ctx->stream;
         ModelDev& d = m->dev;
@@ -496,6 +505,10 @@ struct StepRunner {
             // aggregation and rigid-body modes on the configuration the tangent is taken at
             launch_axpby(3 * nn, 1.0, d.xyz.ptr, step->nlgeom ? 1.0 : 0.0, step->nlgeom ? ucur.ptr : nullptr,
                          amg_xyz.ptr, s);
+            if (d.corner.usable) {  // (a reused hierarchy keeps its interpolation weights)
+                if (!(step->nlgeom && it > 0) || !d.corner.wgt.ptr) corner_weights(d.corner, amg_xyz.ptr, s);
+                corner_matrix(d.corner, d.g4(), d.g20(), d.ebuf64.ptr, bcv, d.maxdiag.ptr, s);
+            }
         } else if (fp64) {
             launch_penalty<double>(d.S, d.vals64.ptr, bcv, d.maxdiag.ptr, d.R.ptr, ucur.ptr, s);
             d.minv64.alloc((size_t)nn * 9, s);
@@ -684,20 +697,22 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
                 const bool reuse = r.step->nlgeom && r.it > 0;
                 ModelDev& d = r.m->dev;
                 if (!d.amg) d.amg = std::make_unique<AmgPcg>();
+                const CornerLevel* corner = d.corner.usable ? &d.corner : nullptr;
                 const int64_t ndof = 3 * r.m->dense.n_nodes;
                 if (!po.amg_kcycle && po.amg_persistent_max_dof > 0 && ndof <= po.amg_persistent_max_dof) {
                     // small system: hierarchy now, its whole CG in the round's persistent launch below
                     guard(i, [&] {
-                        d.amg->prepare(d.S, d.vals64.ptr, d.minv64.ptr, r.amg_xyz.ptr, r.amg_cell, po, s, &ast,
-                                       reuse, true);
+                        d.amg->prepare(d.S, d.vals64.ptr, d.minv64.ptr, r.amg_xyz.ptr, corner, r.amg_cell,
+                                       r.amg_node_volume, po, s, &ast, reuse, true);
                         r.S.amg_levels = ast.levels;
                         r.S.amg_setup_ms += ast.setup_ms;
                         cluster_ids.push_back(i);
                     });
                     continue;
                 }
-                r.csr_status = d.amg->solve(d.S, d.vals64.ptr, d.minv64.ptr, r.amg_xyz.ptr, r.amg_cell, d.R.ptr,
-                                            d.du.ptr, po, s, &ctx->launches, &r.csr_iters, &r.csr_relres, &ast, reuse);
+                r.csr_status = d.amg->solve(d.S, d.vals64.ptr, d.minv64.ptr, r.amg_xyz.ptr, corner, r.amg_cell,
+                                            r.amg_node_volume, d.R.ptr, d.du.ptr, po, s, &ctx->launches, &r.csr_iters,
+                                            &r.csr_relres, &ast, reuse);
                 r.S.amg_levels = ast.levels;
                 r.S.amg_setup_ms += ast.setup_ms;
                 continue;

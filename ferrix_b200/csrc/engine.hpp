@@ -12,6 +12,7 @@
 #include "pcg.hpp"
 #include "pcg_csr.hpp"
 #include "amg.hpp"
+#include "corner.hpp"
 
 struct fx_ctx {
     int device = 0;
@@ -70,6 +71,7 @@ struct ModelDev {
     // the model's multigrid hierarchy and CG workspace (kept between Newton iterations,
     // whose values are refreshed on it, and across steps until the structure changes)
     std::unique_ptr<AmgPcg> amg;
+    CornerLevel corner;  // the multigrid's corner level of C3D20 meshes
     ElemView g4() const { return ElemView{(int)conn4.n / 4, conn4.ptr, mat4.ptr}; }
     ElemView g20() const { return ElemView{(int)conn20.n / 20, conn20.ptr, mat20.ptr}; }
 };
@@ -126,7 +128,9 @@ void ensure_dense(fx_model* m);
 // running on other streams.
 const void* kernels_anchor_amg();
 const void* kernels_anchor_amg_cluster();
+const void* kernels_anchor_amg_transfer();
 const void* kernels_anchor_assembly();
+const void* kernels_anchor_corner();
 const void* kernels_anchor_csr_solve();
 const void* kernels_anchor_elements();
 const void* kernels_anchor_noalloc();

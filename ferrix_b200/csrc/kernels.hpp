@@ -59,7 +59,10 @@ struct BsrStructure {
     DBuf<int32_t> node_ptr, node_slots;
 };
 
-void build_bsr_structure(const ElemView& g4, const ElemView& g20, int n_nodes, BsrStructure& S, cudaStream_t s);
+// g20's elements have npe nodes each: 20, or 8 for the corner level's hexahedra (which has no node
+// slots: node_ptr and node_slots stay empty).
+void build_bsr_structure(const ElemView& g4, const ElemView& g20, int n_nodes, BsrStructure& S, cudaStream_t s,
+                         int npe = 20);
 
 template <typename T>
 void launch_bsr_gather(const BsrStructure& S, const T* ebuf, T* vals, cudaStream_t s);

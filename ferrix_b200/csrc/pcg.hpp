@@ -85,7 +85,8 @@ struct PcgSystem {
 // Multigrid defaults, from a sweep on the 417k-DOF C3D20 box (136 -> 100 CG
 // iterations) and a population of C3D4 / C3D20 boxes (13 % less time):
 // coarse corrections scaled by 1.7 (aggregation without prolongator smoothing
-// under-corrects), first-kind Chebyshev on [lmax / 12, lmax].
+// under-corrects; a smoothed transfer, which does not, scales its corrections by the
+// option's value over 1.7, so by 1 by default), first-kind Chebyshev on [lmax / 12, lmax].
 constexpr double kAmgOvercorrect = 1.7;
 constexpr double kAmgChebRatio = 12.0;
 

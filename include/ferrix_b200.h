@@ -85,14 +85,17 @@ typedef struct {
     int reference_iterative; /* SOLVER=ITERATIVE steps: reference semantics (Jacobi PCG, absolute
                                 sqrt(r.z) < 1e-8, at most 1000 iterations; iterative.rs:26-136) */
     int preconditioner;     /* fx_preconditioner */
-    int amg_aggregate_nodes; /* FX_PRECOND_AMG: mean nodes per fine aggregate (cell size); 0 = 40 */
+    int amg_aggregate_nodes; /* FX_PRECOND_AMG: mean nodes per aggregate of the first aggregated level (cell
+                                size; C3D20 meshes: of element corners); 0 or 40 (the default) = chosen from
+                                the mesh, 20 to 80 */
     int amg_smoother_degree; /* FX_PRECOND_AMG: Chebyshev steps per pre/post smoothing, 1..8; 0 = 2 */
     int amg_cycle;           /* FX_PRECOND_AMG: 0 = V-cycle, 1 = K-cycle at the first coarse level (two
                                 flexible-CG steps per coarse correction; the outer CG is then flexible) */
     int amg_smoother;        /* FX_PRECOND_AMG: 0 = Chebyshev of the first kind on [lmax/ratio, lmax],
                                 1 = Chebyshev of the fourth kind (Lottes 2023) */
-    double amg_overcorrect;  /* FX_PRECOND_AMG: coarse corrections are scaled by this factor, in (0, 2);
-                                0 = 1.7 */
+    double amg_overcorrect;  /* FX_PRECOND_AMG: coarse corrections are scaled by this factor, in (0, 2), through
+                                an unsmoothed transfer, and by the factor over 1.7 through a smoothed one or the
+                                corner level's (which do not under-correct); 0 = 1.7 */
     double amg_cheb_ratio;   /* FX_PRECOND_AMG: lmax / lmin of the first-kind Chebyshev interval; 0 = 12 */
     int amg_persistent_max_dof; /* FX_PRECOND_AMG, V-cycle: systems of at most this many DOF run their
                                    whole CG in one persistent launch, one thread-block cluster per system
@@ -111,7 +114,8 @@ typedef struct {
 /* Preconditioner of the BSR3 PCG. */
 typedef enum {
     FX_PRECOND_BLOCK_JACOBI = 0, /* 3x3 block-Jacobi */
-    FX_PRECOND_AMG = 1           /* aggregation multigrid V-cycle (rigid-body near-null-space), FP64 CG;
+    FX_PRECOND_AMG = 1           /* smoothed-aggregation multigrid V-cycle (rigid-body near-null-space; C3D20
+                                    meshes: below a level of the element corners), FP64 CG;
                                     with FX_PREC_MIXED the fine-level smoother reads FP32 matrix values */
 } fx_preconditioner;
 
@@ -131,8 +135,8 @@ typedef struct {
 } fx_step_stats;
 
 /* Defaults: FX_PREC_MIXED, FX_PRECOND_AMG, rtol 1e-8, max_iter 50000, poll 32,
- * reliable_delta 1e-2, graphs on, 40 nodes per aggregate, Chebyshev degree 2 on
- * [lmax/12, lmax], coarse corrections scaled by 1.7.
+ * reliable_delta 1e-2, graphs on, aggregates chosen from the mesh, Chebyshev degree 2 on
+ * [lmax/12, lmax], coarse corrections scaled by 1.7 (smoothed transfers: 1).
  * fx_solve_csr has no node coordinates and always uses block-Jacobi. */
 void fx_default_solve_opts(fx_solve_opts* opts);
 

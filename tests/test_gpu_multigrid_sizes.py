@@ -1,7 +1,12 @@
-"""The multigrid's coarsest-level inverse at the sizes where its panels and tiles end: one
-aggregate (6 DOF, a partial panel), just below and above one 32-pivot panel, partial last
-panels, sizes on both sides of a 64-row tile, up to the largest dense level. The size follows
-from the aggregate size asked for; the solve must meet the oracle's FP64 direct solution.
+"""The multigrid's kernels at the sizes where they can go wrong.
+
+Coarsest-level inverse, transfers and aggregate factorisation: the aggregate size asked for sets
+the coarsest size (one aggregate: 6 DOF, a partial panel; both sides of a 32-pivot panel and of
+a 64-row tile; up to the largest dense level), the entries per transfer row and the rows per
+aggregate (beyond 256 its factorisation leaves shared memory). Corner level: C3D20 decks down to
+one element, with distorted mid nodes, beside C3D4 elements on the same corners, and with
+a C3D4 element on a mid node (where the hierarchy does without the corner level).
+Every solve must meet the oracle's FP64 direct solution.
 
 Tolerance: the FP64 solver's bound of the other parity tests, 1e-10 relative in the 2-norm, with the
 residual target tightened to 1e-11 so that the bound does not depend on the stopping point."""
@@ -39,3 +44,61 @@ def test_coarsest_inverse_sizes(ctx, deck, nodes):
     err = float(np.linalg.norm(st.displacements - ref) / np.linalg.norm(ref))
     p.close()
     assert err <= 1e-10, err
+
+
+def _solve(ctx, text, **kw):
+    p = fx.Project.from_inp_text(text, ctx)
+    st = fx.SolutionState(p.num_dofs, p.num_nodes)
+    st.initialize(p)
+    stats = p.steps[0].solve(1, p, st, opts=fx.solve_opts(rtol=1e-11, **kw))
+    u = st.displacements
+    p.close()
+    return u, stats
+
+
+def _with_tets(nodes_of_face):
+    """A C3D20 box with C3D4 elements on its top: apex nodes above triples of its nodes."""
+    spec = decks.c3d20_box_spec(2, 2, 4, lengths=(2.0, 2.0, 4.0))
+    m = spec.mesh
+    lines, extra, nid, eid = decks.write_deck(spec).split("\n"), [], len(m.xyz) + 1, len(m.conn) + 1
+    nodes = []
+    for tri in nodes_of_face(m):
+        c = m.xyz[list(tri)].mean(axis=0) + [0.0, 0.0, 0.6]
+        nodes.append(f"{nid}, {c[0]!r}, {c[1]!r}, {c[2]!r}".replace("np.float64(", "").replace(")", ""))
+        extra.append(f"{eid}, " + ", ".join(str(int(i) + 1) for i in tri) + f", {nid}")
+        nid, eid = nid + 1, eid + 1
+    at = next(i for i, line in enumerate(lines) if line.startswith("*Element"))
+    lines[at:at] = nodes
+    at = next(i for i, line in enumerate(lines) if line.startswith("*Nset"))
+    return "\n".join(lines[:at] + ["*Element, Type=C3D4, Elset=Solid"] + extra + lines[at:])
+
+
+def _corner_tris(m):  # two triangles of the top face's first quad, corners only
+    c = m.conn[-1]
+    return [(c[4], c[5], c[6]), (c[4], c[6], c[7])]
+
+
+def _mid_tri(m):  # a triangle with a mid-edge node of the top face
+    c = m.conn[-1]
+    return [(c[4], c[5], c[14])]
+
+
+CORNER = {
+    "one_element": lambda: decks.c3d20_box(1, 1, 1, lengths=(1.0, 1.0, 1.0)),
+    "column": lambda: decks.c3d20_box(1, 1, 9, lengths=(1.0, 1.0, 9.0)),
+    "slender": lambda: decks.c3d20_box(2, 3, 33, lengths=(2.0, 3.0, 33.0)),
+    "block": lambda: decks.c3d20_box(5, 6, 7, lengths=(5.0, 6.0, 7.0)),
+    "with_tets": lambda: _with_tets(_corner_tris),
+    "tet_on_mid_node": lambda: _with_tets(_mid_tri),
+}
+
+
+@pytest.mark.parametrize("prec", [fx.PREC_FP64, fx.PREC_MIXED])
+@pytest.mark.parametrize("case", list(CORNER))
+def test_corner_level(ctx, case, prec):
+    text = CORNER[case]()
+    ref = static_step.Runner(inp.parse_inp_text(text)).run().displacements
+    per_step, s1 = _solve(ctx, text, precision=prec, amg_persistent_max_dof=-1)
+    cluster, s2 = _solve(ctx, text, precision=prec, amg_persistent_max_dof=100000)
+    for u in (per_step, cluster):
+        assert float(np.linalg.norm(u - ref) / np.linalg.norm(ref)) <= 1e-10, (s1, s2)
