@@ -283,22 +283,6 @@ __global__ void __launch_bounds__(128) k_planar6(int n, const int32_t* __restric
     }
 }
 
-// Chebyshev start: d = D^-1 r / theta; x = (zero ? 0 : x) + d
-__global__ void k_cheb_init(int n, int bs, const double* __restrict__ dinv, const double* __restrict__ r,
-                            double* __restrict__ d, double* __restrict__ x, double inv_theta, int zero) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double* Di = dinv + (int64_t)i * bs * bs;
-    const double* ri = r + (int64_t)i * bs;
-    for (int k = 0; k < bs; ++k) {
-        double t = 0.0;
-        for (int c = 0; c < bs; ++c) t += Di[k * bs + c] * ri[c];
-        t *= inv_theta;
-        d[(int64_t)i * bs + k] = t;
-        x[(int64_t)i * bs + k] = zero ? t : x[(int64_t)i * bs + k] + t;
-    }
-}
-
 // b_c = P^T r_f: a CTA of kRestrictWarps warps per aggregate (restrict_agg).
 // Coarse Chebyshev start fused into the restriction (cs.dinv != null): with
 // b = P^T r the first pre-smoothing step of the coarse level from x = 0 is
@@ -613,15 +597,38 @@ __global__ void k_dot_part(int64_t n, const double* __restrict__ a, const double
     }
 }
 
-__global__ void k_sum_part(int nb, const double* __restrict__ part, double* __restrict__ out) {
-    double t = 0.0;
-    for (int k = threadIdx.x; k < nb; k += 32) t += part[k];
+// |a|^2 and |b|^2 in two launches (fixed order): partials of a in part[0 .. nb), of b in part[nb .. 2 nb)
+__global__ void __launch_bounds__(256) k_norm2_part(int64_t n, const double* __restrict__ a,
+                                                    const double* __restrict__ b, double* __restrict__ part, int nb) {
+    __shared__ double sh[2][8];
+    double t = 0.0, u = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        t += a[i] * a[i];
+        u += b[i] * b[i];
+    }
     t = warp_sum(t);
-    if (threadIdx.x == 0) *out = t;
+    u = warp_sum(u);
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][threadIdx.x >> 5] = t;
+        sh[1][threadIdx.x >> 5] = u;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double v = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += sh[threadIdx.x][w];
+        part[threadIdx.x * nb + blockIdx.x] = v;
+    }
+}
+
+__global__ void k_norm2_sum(int nb, const double* __restrict__ part, double* __restrict__ out) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;  // a warp per norm
+    double t = 0.0;
+    for (int k = lane; k < nb; k += 32) t += part[w * nb + k];
+    t = warp_sum(t);
+    if (lane == 0) out[w] = t;
 }
 
 // x = d / sqrt(*nrm2), the norm read on the device
-// x = d / |d| (x may be d itself)
 __global__ void k_normalize(int64_t n, const double* __restrict__ nrm2, const double* d, double* x) {
     const double v = *nrm2;
     const double inv = v > 0.0 ? 1.0 / sqrt(v) : 1.0;
@@ -700,10 +707,11 @@ __global__ void k_xpby(int64_t n, const double* __restrict__ z, const double* __
 //   kL0Cheb0  r = b - A v; d = c2 D^-1 r; xo = v + d             (first Chebyshev step from v = x)
 //   kL0ChebK  r -= A v; d = c1 v + c2 D^-1 r; xo += d            (later steps, v = previous direction)
 //   kL0Apply  y = A v
+//   kL0Power  d = c2 D^-1 A v                                    (a step of the power iteration)
 // With dot = 1 the CTA partials of v.y give alpha = r.z / p.q; with dot = 2 the
 // partials of b.xo give r.z and beta (the last V-cycle step of the outer CG).
 // The last CTA to finish sums the partials in a fixed order.
-enum : int { kL0Resid = 0, kL0RUpd = 1, kL0Cheb0 = 2, kL0ChebK = 3, kL0Apply = 4 };
+enum : int { kL0Resid = 0, kL0RUpd = 1, kL0Cheb0 = 2, kL0ChebK = 3, kL0Apply = 4, kL0Power = 5 };
 
 template <typename VT>
 struct L0Op {
@@ -966,6 +974,9 @@ __global__ void __launch_bounds__(256, std::is_same<VT, __half>::value ? kL0MinB
                 if (o.dot && o.zold) zoc = o.zold[o3 + c];
             } else if (MODE == kL0Apply) {
                 vc = v[o3 + c];
+            } else if (MODE == kL0Power) {
+#pragma unroll
+                for (int kk = 0; kk < 3; ++kk) Dr[kk] = o.dinv[9 * (int64_t)row + 3 * c + kk];
             } else if (MODE == kL0Resid) {
                 bc = o.b ? o.b[o3 + c] : 0.0;
             } else {
@@ -1058,6 +1069,11 @@ __global__ void __launch_bounds__(256, std::is_same<VT, __half>::value ? kL0MinB
         } else if (MODE == kL0Apply) {
             o.y[o3 + c] = axc;
             dsum += vc * axc;
+        } else if (MODE == kL0Power) {
+            const double z = o.c2 * (Dr[0] * acc[0] + Dr[1] * acc[1] + Dr[2] * acc[2]);
+            if (G32) o.d4_out[4 * (int64_t)row + c] =
+                (float)(H ? z * (double)(c == 0 ? sqi.x : (c == 1 ? sqi.y : sqi.z)) : z);
+            if (!G32 || o.d_out) o.d_out[o3 + c] = z;
         } else {  // Chebyshev steps
             const double rr[3] = {src3[0] - acc[0], src3[1] - acc[1], src3[2] - acc[2]};
             const double z = Dr[0] * rr[0] + Dr[1] * rr[1] + Dr[2] * rr[2];
@@ -1200,6 +1216,9 @@ __global__ void __launch_bounds__(kLnThreads, kLnMinBlocks) k_ln_op(LnOp o) {
             }
             vc = o.v[o6 + c];
             if (MODE == kL0ChebK) xoc = o.xo[o6 + c];
+        } else if (MODE == kL0Power) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) Dr[k] = o.dinv[36 * (int64_t)row + 6 * c + k];
         } else if (MODE == kL0Resid) {
             bc = o.b ? o.b[o6 + c] : 0.0;
         } else {
@@ -1223,6 +1242,11 @@ __global__ void __launch_bounds__(kLnThreads, kLnMinBlocks) k_ln_op(LnOp o) {
         o.y[o6 + c] = o.b ? bc - axc : axc;
     } else if (MODE == kL0RUpd) {
         o.r[o6 + c] = src6[0] - axc;
+    } else if (MODE == kL0Power) {
+        double z = 0.0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) z += Dr[k] * acc[k];
+        o.d_out[o6 + c] = o.c2 * z;
     } else {
         double z = 0.0, rc = 0.0;
 #pragma unroll
@@ -1555,62 +1579,71 @@ static void level_spmv(const AmgLevel& l, const double* x, const double* b, doub
     }
 }
 
-// red[nb] = a . b (deterministic, stays on the device)
-static void dot_dev(const double* a, const double* b, int64_t n, DBuf<double>& red, cudaStream_t s) {
-    const int nb = 296;
-    if (red.n < (size_t)nb + 1) red.alloc(nb + 1, s);
-    FX_LAUNCH(k_dot_part, nb, 256, 0, s, n, a, b, red.ptr);
-    FX_LAUNCH(k_sum_part, 1, 32, 0, s, nb, red.ptr, red.ptr + nb);
-}
-
-// Largest eigenvalue of D^-1 A by 12 power iterations from a fixed hashed start
-// vector, normalised on the device; one host read at the end.
-// (planar levels: with vals16 / sq4 the products come from the FP16 scaled matrix the smoother
-// reads, through float4 copies of x in l.x4; else from vals32, an FP32 copy, when given)
+// Largest eigenvalue of D^-1 A by 12 power iterations from a fixed hashed start vector, one launch
+// each: a step is x <- c2 D^-1 A x without a normalisation (c2 = 1/4 keeps 12 steps of a spectrum
+// up to ~5,000 within FP32's range), and the eigenvalue is the ratio of the last two vectors' norms.
+// (Normalised after every step, an iteration was six launches, ~18 us on a small level.)
+// Planar levels: the products come from the FP16 scaled matrix that the smoother reads, through
+// float4 vectors, or from the FP32 copy or the FP64 values with FP64 vectors.
 // warm: start from the vector the previous estimate on this level ended with (a
 // refresh after a small change of the matrix) and iterate 4 times instead of 12.
 static void estimate_lmax(AmgLevel& l, DBuf<double>& red, cudaStream_t s, bool warm) {
-    const float* vals32 = l.vals32;
-    const __half* vals16 = kAmgEstF16 ? l.vals16 : nullptr;
-    const float4* sq4 = l.sq4;
+    constexpr double kStep = 0.25;
+    const bool h16 = l.S0 && kAmgEstF16 && l.vals16 && l.sq4;
     const int64_t nd = (int64_t)l.n * l.bs;
     const int nb = 296;
     const bool from_ev = warm && l.ev.n == (size_t)nd;
-    if (from_ev)
-        FX_CUDA_CHECK(cudaMemcpyAsync(l.x.ptr, l.ev.ptr, nd * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    else
-        FX_LAUNCH(k_fill_hash, grid_for(nd), 256, 0, s, nd, l.x.ptr);
-    dot_dev(l.x.ptr, l.x.ptr, nd, red, s);
-    FX_LAUNCH(k_normalize, grid_for(nd), 256, 0, s, nd, red.ptr + nb, l.x.ptr, l.x.ptr);
     const int iters = from_ev ? 4 : 12;
+    const double* x = from_ev ? l.ev.ptr : l.x.ptr;
+    if (!from_ev) FX_LAUNCH(k_fill_hash, grid_for(nd), 256, 0, s, nd, l.x.ptr);
+    float4* xa = reinterpret_cast<float4*>(l.x4.ptr);
+    float4* xb = reinterpret_cast<float4*>(l.d4a.ptr);
+    if (h16) FX_LAUNCH(k_scaled4, grid_for(l.n), 256, 0, s, l.n, x, l.sq4, xa);
+    double* out[2] = {l.d.ptr, l.t.ptr};
     for (int it = 0; it < iters; ++it) {
-        if (l.S0 && vals16 && sq4) {  // t = A x, |x| = 1, from the FP16 scaled matrix
-            float4* x4 = reinterpret_cast<float4*>(l.x4.ptr);
-            FX_LAUNCH(k_scaled4, grid_for(l.n), 256, 0, s, l.n, l.x.ptr, sq4, x4);
-            L0Op<__half> o = l0_op<__half>(l, vals16);
-            o.v4 = x4;
-            o.y = l.t.ptr;
-            o.sq4 = sq4;
-            FX_LAUNCH((k_l0_op<__half, kL0Resid, true>), l0_grid(l.n, true), 256, 0, s, o);
-        } else if (l.S0 && vals32) {  // t = A x, |x| = 1
-            L0Op<float> o = l0_op<float>(l, vals32);
-            o.v = l.x.ptr;
-            o.y = l.t.ptr;
-            FX_LAUNCH((k_l0_op<float, kL0Resid>), l0_grid(l.n), 256, 0, s, o);
+        double* y = out[it & 1];
+        if (h16) {
+            L0Op<__half> o = l0_op<__half>(l, l.vals16);
+            o.v4 = xa;
+            o.d4_out = reinterpret_cast<float*>(xb);
+            o.d_out = it >= iters - 2 ? y : nullptr;
+            o.sq4 = l.sq4;
+            o.c2 = kStep;
+            FX_LAUNCH((k_l0_op<__half, kL0Power, true>), l0_grid(l.n, true), 256, 0, s, o);
+            std::swap(xa, xb);
+        } else if (l.S0 && l.vals32) {
+            L0Op<float> o = l0_op<float>(l, l.vals32);
+            o.v = x;
+            o.d_out = y;
+            o.c2 = kStep;
+            FX_LAUNCH((k_l0_op<float, kL0Power>), l0_grid(l.n), 256, 0, s, o);
+        } else if (l.S0) {
+            L0Op<double> o = l0_op<double>(l, l.vals0);
+            o.v = x;
+            o.d_out = y;
+            o.c2 = kStep;
+            FX_LAUNCH((k_l0_op<double, kL0Power>), l0_grid(l.n), 256, 0, s, o);
         } else {
-            level_spmv(l, l.x.ptr, nullptr, l.t.ptr, s);
+            LnOp o = ln_op(l);
+            o.v = x;
+            o.d_out = y;
+            o.c2 = kStep;
+            FX_LAUNCH(k_ln_op<kL0Power>, grid_for((int64_t)l.n * 32, kLnThreads), kLnThreads, 0, s, o);
         }
-        FX_LAUNCH(k_cheb_init, grid_for(l.n), 256, 0, s, l.n, l.bs, l.dinv_ptr(), l.t.ptr, l.d.ptr, l.r.ptr, 1.0,
-                  1);  // d = D^-1 A x
-        dot_dev(l.d.ptr, l.d.ptr, nd, red, s);
-        FX_LAUNCH(k_normalize, grid_for(nd), 256, 0, s, nd, red.ptr + nb, l.d.ptr, l.x.ptr);
+        x = y;
     }
+    // |last|^2 and |last but one|^2
+    if (red.n < 2 * (size_t)(nb + 1)) red.alloc(2 * (nb + 1), s);
+    double* last = out[(iters - 1) & 1];
+    FX_LAUNCH(k_norm2_part, nb, 256, 0, s, nd, last, out[iters & 1], red.ptr, nb);
+    FX_LAUNCH(k_norm2_sum, 1, 64, 0, s, nb, red.ptr, red.ptr + 2 * nb);
     l.ev.alloc(nd, s);
-    FX_CUDA_CHECK(cudaMemcpyAsync(l.ev.ptr, l.x.ptr, nd * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    double nd2 = 0.0;
-    FX_CUDA_CHECK(cudaMemcpyAsync(&nd2, red.ptr + nb, sizeof(double), cudaMemcpyDeviceToHost, s));
+    FX_LAUNCH(k_normalize, grid_for(nd), 256, 0, s, nd, red.ptr + 2 * nb, last, l.ev.ptr);
+    double h[2] = {0.0, 0.0};
+    FX_CUDA_CHECK(cudaMemcpyAsync(h, red.ptr + 2 * nb, sizeof(h), cudaMemcpyDeviceToHost, s));
     stream_wait(s, "amg eigenvalue estimate");
-    l.lmax = kLmaxMargin * (nd2 > 0.0 ? std::sqrt(nd2) : 1.0);
+    const double q = h[0] / h[1] / (kStep * kStep);
+    l.lmax = kLmaxMargin * (q > 0.0 && std::isfinite(q) ? std::sqrt(q) : 1.0);
 }
 
 // A level's matrix as the transfer kernels read it: the planar BSR3 at level 0,
@@ -1892,6 +1925,16 @@ void Amg::refresh(const PlanarIn* in, cudaStream_t s, AmgStats* st) {
         st->sizes.clear();
         for (auto& l : L) st->sizes.push_back(l.n * l.bs);
         st->setup_ms = timer.stop_ms(s);
+    }
+}
+
+void Amg::keep(const PlanarIn& fine, AmgStats* st) {
+    set_planar(L[0], fine);
+    if (st) {
+        st->levels = (int)L.size();
+        st->sizes.clear();
+        for (auto& l : L) st->sizes.push_back(l.n * l.bs);
+        st->setup_ms = 0.0;
     }
 }
 
@@ -2348,7 +2391,8 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
         in[1].dinv = corner->minv.ptr;
     }
     const bool f16 = opt.amg_fp32 && opt.amg_fp16 && !persistent;
-    for (int m = 0; m < (corner ? 2 : 1); ++m) {
+    const bool keep = keeps(S, reuse) && amg.planar() == (corner ? 2 : 1);
+    for (int m = 0; m < (corner && !keep ? 2 : 1); ++m) {
         const BsrStructure& Sm = *in[m].S;
         if (f16) {  // FP16 values of S A S and the scales
             sq4_[m].alloc((size_t)Sm.n_rows, s);
@@ -2370,12 +2414,20 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
         }
     }
     amg.set_degree(opt.amg_degree);
-    if (reuse && amg.built_for == S.id && !amg.L.empty() && amg.L[0].n == n && amg.planar() == (corner ? 2 : 1)) {
+    if (keep) {
+        amg.keep(in[0], st);
+    } else if (reuse && amg.built_for == S.id && !amg.L.empty() && amg.L[0].n == n && amg.planar() == (corner ? 2 : 1)) {
+        drop_graph();
         amg.refresh(in, s, st);
+        fresh_ = true;
+        stale_ = false;
     } else {
+        drop_graph();
         amg.built_for = 0;  // (a failed setup leaves nothing to reuse)
         amg.setup(in, corner, corner ? corner->xyz.ptr : xyz, cell0, node_volume, s, st);
         amg.built_for = S.id;
+        fresh_ = true;
+        stale_ = false;
     }
     amg.set_cycle(opt.amg_kcycle);
     amg.set_smoother_kind(opt.amg_cheb_kind);
@@ -2402,6 +2454,11 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
     // a barrier timeout sets S[7]
     amg.set_fused_coarse(opt.amg_fused_coarse && !opt.amg_kcycle, sc_.ptr + 7);
     if (opt.amg_fused_coarse && !opt.amg_kcycle) amg.upload_descriptor(s);
+}
+
+void AmgPcg::drop_graph() {
+    if (gexec_) cudaGraphExecDestroy(gexec_);
+    gexec_ = nullptr;
 }
 
 void Amg::upload_descriptor(cudaStream_t s) {
@@ -2488,9 +2545,10 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
     // as a WHILE graph node, one or four iterations per body, measured 1-7 %
     // slower per iteration on B200 than these host-polled replays.)
     const int per_poll = 4;
-    cudaGraphExec_t gexec = nullptr;
-    int64_t per_iter_launches = 0;
-    if (opt.graphs && !debug_sync()) {
+    const bool graphs = opt.graphs && !debug_sync();
+    const void* key[4] = {x, vals64, dinv64, r_.ptr};
+    if (gexec_ && (!graphs || !std::equal(key, key + 4, graph_key_))) drop_graph();
+    if (graphs && !gexec_) {
         cudaGraph_t g;
         int64_t count = 0;
         int64_t* saved = g_launch_counter;
@@ -2500,9 +2558,12 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
         const cudaError_t ce = cudaStreamEndCapture(s, &g);
         g_launch_counter = saved;
         FX_CUDA_CHECK(ce);
-        per_iter_launches = count;
-        FX_CUDA_CHECK(cudaGraphInstantiate(&gexec, g, 0));
+        graph_launches_ = count;
+        const cudaError_t ci = cudaGraphInstantiate(&gexec_, g, 0);
         cudaGraphDestroy(g);
+        if (ci != cudaSuccess) gexec_ = nullptr;
+        FX_CUDA_CHECK(ci);
+        std::copy(key, key + 4, graph_key_);
     }
     double h[8];
     long long it = 0;
@@ -2521,15 +2582,15 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
             rc = FX_CONVERGENCE;
             break;
         }
-        if (gexec) {
-            FX_CUDA_CHECK(cudaGraphLaunch(gexec, s));
-            if (launches) *launches += per_iter_launches;
+        if (gexec_) {
+            FX_CUDA_CHECK(cudaGraphLaunch(gexec_, s));
+            if (launches) *launches += graph_launches_;
         } else {
             for (int k = 0; k < per_poll; ++k) iteration();
         }
         it += per_poll;
     }
-    if (gexec) cudaGraphExecDestroy(gexec);
+    solved(it);
     // true residual of the assembled FP64 system in the block-Jacobi norm
     level_spmv(l0, x, b, q_.ptr, s);
     FX_LAUNCH(k_rdr_part, nb, 256, 0, s, n, q_.ptr, dinv64, part_.ptr);

@@ -113,6 +113,9 @@ class Amg {
     // included) and coarse patterns are kept; coarse values, block inverses, eigenvalue
     // estimates and the coarsest inverse are recomputed.
     void refresh(const PlanarIn* in, cudaStream_t s, AmgStats* st);
+    // New fine matrix values only: the smoother works on them, everything below and the eigenvalue
+    // estimates stay as they are.
+    void keep(const PlanarIn& fine, AmgStats* st);
     int planar() const { return planar_; }  // planar levels: 1, or 2 with a corner level
     uint64_t built_for = 0;  // BsrStructure::id of the last setup (0: none)
     // Chebyshev degree (1..8)
@@ -284,6 +287,25 @@ double profile_smoother_op(const BsrStructure& S, const double* vals64, const do
 
 class AmgPcg {
    public:
+    AmgPcg() = default;
+    AmgPcg(const AmgPcg&) = delete;
+    AmgPcg& operator=(const AmgPcg&) = delete;
+    ~AmgPcg() { drop_graph(); }
+    // Whether the next solve on this structure keeps the hierarchy below the fine level as it is
+    // (reuse: the caller allows it, the matrix being a later Newton tangent of the same increment).
+    // A V-cycle with a lagged coarse operator is still symmetric positive definite and the CG tests
+    // the true system, so only its iteration count can suffer: once a solve on the kept hierarchy takes
+    // a quarter (and more than 4 iterations) longer than the first one did, the next one
+    // recomputes it. (NLGEOM beam, 16k DOF: setups 80 of 215 ms with every tangent's recomputed.)
+    bool keeps(const BsrStructure& S, bool reuse) const {
+        return reuse && amg.built_for == S.id && !amg.L.empty() && amg.L[0].n == S.n_rows && !stale_;
+    }
+    // iterations of the solve that prepare() was called for (solve() calls it itself)
+    void solved(long long iterations) {
+        if (fresh_) first_iters_ = iterations;
+        else if (iterations > first_iters_ + first_iters_ / 4 + 4) stale_ = true;
+        fresh_ = false;
+    }
     // For the persistent solve: set up (or refresh) the hierarchy for the system and
     // allocate the CG vectors, without iterating; then describe it for the kernel.
     // corner: the corner level with its matrix, or null; cell0, node_volume: Amg::setup
@@ -293,8 +315,8 @@ class AmgPcg {
     ClInst describe(const double* b, double* x) const;
     // ||b - A x||_D / ||b||_D of the assembled FP64 system after a persistent solve
     double true_relres(const double* b, const double* x, cudaStream_t s);
-    // reuse: keep the hierarchy's aggregates, prolongators and coarse patterns when
-    // the last setup was on the same structure S (only the values are refreshed)
+    // reuse: keep the hierarchy (keeps()), or else at least its aggregates, prolongators and coarse
+    // patterns when the last setup was on the same structure S (the values are refreshed)
     int solve(const BsrStructure& S, const double* vals64, const double* dinv64, const double* xyz,
               const CornerLevel* corner, double cell0, double node_volume, const double* b, double* x, const PcgOptions& opt, cudaStream_t s, int64_t* launches, long long* iters,
               double* relres, AmgStats* st, bool reuse = false);
@@ -310,6 +332,13 @@ class AmgPcg {
     DBuf<float4> sq4_[2];
     DBuf<float> hs_;  // FP16 smoother directions: the current V-cycle's {2^k, 2^-k}
     DBuf<int> counter_;
+    bool fresh_ = false, stale_ = false;  // the hierarchy was (re)computed for this solve; should be for the next
+    long long first_iters_ = 0;
+    // the captured iterations, kept while the hierarchy is: what they were captured with
+    void drop_graph();
+    cudaGraphExec_t gexec_ = nullptr;
+    int64_t graph_launches_ = 0;
+    const void* graph_key_[4] = {nullptr, nullptr, nullptr, nullptr};
 };
 
 }  // namespace fx

@@ -480,6 +480,10 @@ struct StepRunner {
         }
     }
 
+    // NLGEOM: the Newton iterations after the first of an increment may go on with the multigrid
+    // hierarchy built at the increment's first tangent (AmgPcg::keeps)
+    bool reuse_hierarchy() const { return step->nlgeom && it > 0; }
+
     // tangent, penalty, block-Jacobi (static_step.rs:173-199)
     void prepare_solve() {
         ModelDev& d = m->dev;
@@ -505,8 +509,9 @@ struct StepRunner {
             // aggregation and rigid-body modes on the configuration the tangent is taken at
             launch_axpby(3 * nn, 1.0, d.xyz.ptr, step->nlgeom ? 1.0 : 0.0, step->nlgeom ? ucur.ptr : nullptr,
                          amg_xyz.ptr, s);
-            if (d.corner.usable) {  // (a reused hierarchy keeps its interpolation weights)
-                if (!(step->nlgeom && it > 0) || !d.corner.wgt.ptr) corner_weights(d.corner, amg_xyz.ptr, s);
+            const bool reuse = reuse_hierarchy();
+            if (d.corner.usable && !(d.amg && d.amg->keeps(d.S, reuse))) {
+                if (!reuse || !d.corner.wgt.ptr) corner_weights(d.corner, amg_xyz.ptr, s);  // (a refresh keeps them)
                 corner_matrix(d.corner, d.g4(), d.g20(), d.ebuf64.ptr, bcv, d.maxdiag.ptr, s);
             }
         } else if (fp64) {
@@ -691,10 +696,7 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
             StepRunner& r = *rs[i];
             if (r.amg) {
                 AmgStats ast;
-                // NLGEOM: the Newton iterations after the first of an increment keep the
-                // hierarchy built at the increment's first tangent (aggregates and
-                // rigid-body prolongators of that configuration) and refresh its values
-                const bool reuse = r.step->nlgeom && r.it > 0;
+                const bool reuse = r.reuse_hierarchy();
                 ModelDev& d = r.m->dev;
                 if (!d.amg) d.amg = std::make_unique<AmgPcg>();
                 const CornerLevel* corner = d.corner.usable ? &d.corner : nullptr;
@@ -744,6 +746,7 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
                 StepRunner& r = *rs[cluster_ids[k]];
                 r.csr_status = res[k].status;
                 r.csr_iters = res[k].iterations;
+                r.m->dev.amg->solved(r.csr_iters);
                 guard(cluster_ids[k], [&] {
                     r.csr_relres = r.m->dev.amg->true_relres(r.m->dev.R.ptr, r.m->dev.du.ptr, s);
                 });

@@ -102,3 +102,21 @@ def test_corner_level(ctx, case, prec):
     cluster, s2 = _solve(ctx, text, precision=prec, amg_persistent_max_dof=100000)
     for u in (per_step, cluster):
         assert float(np.linalg.norm(u - ref) / np.linalg.norm(ref)) <= 1e-10, (s1, s2)
+
+
+@pytest.mark.parametrize("persistent", [-1, 100000])
+@pytest.mark.parametrize("npe", [4, 20])
+def test_kept_hierarchy_over_newton_iterations(ctx, npe, persistent):
+    """An NLGEOM step with displacements of up to a seventh of the beam's length (the C3D20 beam, which
+    is softer, at a load for which the reference's Newton iteration converges): the hierarchy kept from
+    an increment's first tangent preconditions ever different ones; the increments must end where the
+    oracle's do (the NLGEOM bound of the other parity tests, 1e-8)."""
+    spec = decks.c3d4_nlgeom_beam_spec(10, 2, 2, tip_load=6.0e4 if npe == 4 else 1.5e4, increments=3)
+    if npe == 20:
+        spec.mesh = decks.hex20_box(6, 1, 1, 50.0, 10.0, 10.0, jitter=0.05, seed=3)
+        spec.init_temp = 20.0 + 200.0 * spec.mesh.xyz[:, 0] / 50.0
+    text = decks.write_deck(spec)
+    ref = static_step.Runner(inp.parse_inp_text(text)).run().displacements
+    u, stats = _solve(ctx, text, amg_persistent_max_dof=persistent)
+    assert stats["linear_solves"] > 2 * stats["increments"]
+    assert float(np.linalg.norm(u - ref) / np.linalg.norm(ref)) <= 1e-8, stats
