@@ -412,11 +412,16 @@ __global__ void __launch_bounds__(1024) k_dense_decouple(int nd, double* __restr
     __syncthreads();
     double dmax = 0.0;
     for (int w = 0; w < nw; ++w) dmax = fmax(dmax, s_red[w]);
-    for (int k = threadIdx.x; k < nd; k += blockDim.x) dead[k] = !(fabs(A[(int64_t)k * nd + k]) > 1e-12 * dmax);
-    __syncthreads();
-    for (int r = warp; r < nd; r += nw)
-        for (int c = lane; c < nd; c += 32)
-            if (dead[r] || dead[c]) A[(int64_t)r * nd + c] = (r == c) ? 1.0 : 0.0;
+    int any = 0;
+    for (int k = threadIdx.x; k < nd; k += blockDim.x) {
+        dead[k] = !(fabs(A[(int64_t)k * nd + k]) > 1e-12 * dmax);
+        any |= dead[k];
+    }
+    if (__syncthreads_or(any)) {  // (rank-deficient aggregates only: the pass over A takes ~50 us at 700 DOF)
+        for (int r = warp; r < nd; r += nw)
+            for (int c = lane; c < nd; c += 32)
+                if (dead[r] || dead[c]) A[(int64_t)r * nd + c] = (r == c) ? 1.0 : 0.0;
+    }
     __syncthreads();
     for (int k = threadIdx.x; k < nd; k += blockDim.x) diag[k] = A[(int64_t)k * nd + k];  // before elimination
 }
@@ -647,29 +652,39 @@ __global__ void k_fill_hash(int64_t n, double* __restrict__ v) {
 
 unsigned grid_for(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
-// ---- outer PCG scalars: S[0] r.z, S[1] p.q, S[2] r.D^-1 r, S[3] b.D^-1 b, S[4] beta, S[5] alpha, S[6] breakdown
+// ---- outer PCG scalars: S[0] r.z of the last beta, S[2] r.D^-1 r, S[3] b.D^-1 b, S[6] breakdown, S[7] barrier
+// timeout, S[8] r.z. The sums p.q, r.z and r.D^-1 r are left as partial sums by the launch that forms
+// their terms and added by every CTA of the launch that needs them, in the same fixed order
+// (cta_total): reducing them in the producing launch's last CTA (fence, counter, second read of
+// the partials) ended three launches of every iteration with ~3 us of one CTA's latency.
 __global__ void k_fin(int nb, const double* __restrict__ part, double* __restrict__ S, int what) {
     double t = 0.0;  // fixed lane assignment and tree: deterministic
     for (int k = threadIdx.x; k < nb; k += 32) t += part[k];
     t = warp_sum(t);
     if (threadIdx.x != 0) return;
-    if (what == 0) {  // p.q -> alpha
-        S[1] = t;
-        if (!(t > 0.0) || !isfinite(t)) {
-            S[6] = 1.0;
-            S[5] = 0.0;
-        } else {
-            S[5] = S[0] / t;
-        }
-    } else if (what == 1) {  // r.D^-1 r
+    if (what == 1) {  // r.D^-1 r
         S[2] = t;
-    } else if (what == 2) {  // r.z -> beta
-        S[4] = S[0] > 0.0 ? t / S[0] : 0.0;
+    } else if (what == 3) {  // initial r.z
         S[0] = t;
-    } else if (what == 3) {  // initial: r.z and b.D^-1 b
-        S[0] = t;
-        S[4] = 0.0;
+        S[8] = t;
     }
+}
+
+// Sum of n partial sums (entries of `stride` doubles; minus the second double of each with diff), in
+// every thread of a CTA of 256.
+__device__ __forceinline__ double cta_total(const double* __restrict__ part, int n, int stride, bool diff) {
+    __shared__ double s_tot[8];
+    double t = 0.0;
+    for (int k = threadIdx.x; k < n; k += 256)
+        t += diff ? part[(int64_t)k * stride] - part[(int64_t)k * stride + 1] : part[(int64_t)k * stride];
+    t = warp_sum(t);
+    if ((threadIdx.x & 31) == 0) s_tot[threadIdx.x >> 5] = t;
+    __syncthreads();
+    t = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += s_tot[w];
+    __syncthreads();  // s_tot may be written again
+    return t;
 }
 
 // partial r . D^-1 r without the update (start of the solve)
@@ -692,12 +707,26 @@ __global__ void k_rdr_part(int n, const double* __restrict__ r, const double* __
     }
 }
 
-__global__ void k_xpby(int64_t n, const double* __restrict__ z, const double* __restrict__ S, double* __restrict__ p) {
-    const double beta = S[4];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        p[i] = z[i] + beta * p[i];
+// p = z + beta p with beta = (r.z - r.z_old) / r.z_prev from the V-cycle's partial sums (pairs; z_old only
+// in the flexible CG), r.z into S[8] and r.D^-1 r from the update's partial sums into S[2]
+__global__ void __launch_bounds__(256) k_xpby(int64_t n, const double* __restrict__ z, double* __restrict__ S,
+                                              const double* __restrict__ rz_part, int n_rz, bool flexible,
+                                              const double* __restrict__ rd_part, int n_rd, double* __restrict__ p) {
+    const double prev = S[0];  // (S[0] is moved on by the next update only)
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const double zv = i < n ? z[i] : 0.0, pv = i < n ? p[i] : 0.0;
+    const double rz = cta_total(rz_part, n_rz, 2, false);
+    const double num = flexible ? cta_total(rz_part, n_rz, 2, true) : rz;
+    const double beta = prev > 0.0 ? num / prev : 0.0;
+    if (i < n) p[i] = zv + beta * pv;
+    if (blockIdx.x == 0) {
+        const double rd = cta_total(rd_part, n_rd, 1, false);
+        if (threadIdx.x == 0) {
+            S[8] = rz;
+            S[2] = rd;
+        }
+    }
 }
-
 
 // ------------------------------------------------------------------ level 0: fused operators
 // One pass over the planar BSR3 matrix (8 lanes per block row, FP64 accumulation,
@@ -708,9 +737,8 @@ __global__ void k_xpby(int64_t n, const double* __restrict__ z, const double* __
 //   kL0ChebK  r -= A v; d = c1 v + c2 D^-1 r; xo += d            (later steps, v = previous direction)
 //   kL0Apply  y = A v
 //   kL0Power  d = c2 D^-1 A v                                    (a step of the power iteration)
-// With dot = 1 the CTA partials of v.y give alpha = r.z / p.q; with dot = 2 the
-// partials of b.xo give r.z and beta (the last V-cycle step of the outer CG).
-// The last CTA to finish sums the partials in a fixed order.
+// With dot = 1 the CTAs leave partial sums of v.y (p.q), with dot = 2 of (b.xo, b.zold) (r.z and, in the
+// flexible CG, r.z_old; the last V-cycle step of the outer CG).
 enum : int { kL0Resid = 0, kL0RUpd = 1, kL0Cheb0 = 2, kL0ChebK = 3, kL0Apply = 4, kL0Power = 5 };
 
 template <typename VT>
@@ -729,9 +757,7 @@ struct L0Op {
     double c1, c2;
     int dot;
     const double* zold;  // dot = 2 with a flexible outer CG: the previous preconditioned residual
-    double* part;
-    int* counter;
-    double* S;
+    double* part;        // partial sums per CTA: one (dot = 1) or two doubles
     // FP32 smoother vectors (mixed precision): the gathered vector as float4 per
     // node (x, y, z, 0) and the new direction written into the same layout; with FP16
     // values and kL0H16Vec the directions are four halves per node (8 bytes) instead
@@ -780,14 +806,9 @@ __device__ __forceinline__ void ld4v(const double* p, double o[4]) {
     o[3] = b.y;
 }
 
-// Fixed-order CTA sums of (v, v2), then the last CTA to arrive reduces all CTA
-// partials and finalises the outer CG scalars: mode 1 alpha = r.z / p.q; mode 2
-// beta = (r.z_new - r.z_old) / r.z_prev (Polak-Ribiere, flexible CG; v2 = 0 for
-// the plain form) and r.z.
-__device__ __forceinline__ void cta_dot_finalize(double v, double v2, int mode, double* part, int* counter,
-                                                 double* S) {
+// Fixed-order sums of (v, v2) over the CTA, left in part (two = false: v alone)
+__device__ __forceinline__ void cta_partials(double v, double v2, bool two, double* part) {
     __shared__ double sh[2][32];
-    __shared__ int s_last;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     v = warp_sum(v);
     v2 = warp_sum(v2);
@@ -796,40 +817,10 @@ __device__ __forceinline__ void cta_dot_finalize(double v, double v2, int mode, 
         sh[1][w] = v2;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0, t2 = 0.0;
-        for (int k = 0; k < nw; ++k) {
-            t += sh[0][k];
-            t2 += sh[1][k];
-        }
-        part[2 * blockIdx.x] = t;
-        part[2 * blockIdx.x + 1] = t2;
-        __threadfence();
-        s_last = atomicAdd(counter, 1) == (int)gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!s_last || w != 0) return;
-    __threadfence();
-    double t = 0.0, t2 = 0.0;
-    for (int k = lane; k < (int)gridDim.x; k += 32) {
-        t += __ldcg(part + 2 * k);
-        t2 += __ldcg(part + 2 * k + 1);
-    }
-    t = warp_sum(t);
-    t2 = warp_sum(t2);
-    if (lane != 0) return;
-    *counter = 0;
-    if (mode == 1) {  // p.q -> alpha
-        S[1] = t;
-        if (!(t > 0.0) || !isfinite(t)) {
-            S[6] = 1.0;
-            S[5] = 0.0;
-        } else {
-            S[5] = S[0] / t;
-        }
-    } else {  // new r.z -> beta
-        S[4] = S[0] > 0.0 ? (t - t2) / S[0] : 0.0;
-        S[0] = t;
+    if (threadIdx.x < (two ? 2u : 1u)) {
+        double t = 0.0;
+        for (int k = 0; k < nw; ++k) t += sh[threadIdx.x][k];
+        part[(two ? 2 : 1) * blockIdx.x + threadIdx.x] = t;
     }
 }
 
@@ -1093,7 +1084,7 @@ __global__ void __launch_bounds__(256, std::is_same<VT, __half>::value ? kL0MinB
             }
         }
     }
-    if (o.dot) cta_dot_finalize(dsum, dsum2, o.dot, o.part, o.counter, o.S);
+    if (o.dot) cta_partials(dsum, dsum2, o.dot == 2, o.part);
 }
 
 // ---- K-cycle on a coarse level (one CTA; the level has at most a few 10k DOF)
@@ -1385,35 +1376,59 @@ __global__ void __launch_bounds__(256) k_corner_prolong(CornerView V, const doub
 }
 
 // The CG update fused with the first step of the V-cycle that follows it:
-// x += alpha p, r -= alpha q, r.D^-1 r reduced by the last CTA into S[2], and
-// with b = the new r: r0 = b, x0 = d = c2 D^-1 b (what k_l0_cheb_start does).
-// hs != null (FP16 directions): the V-cycle's scale comes from S[2] as this launch
-// finds it, the previous residual's r.D^-1 r (the new one is reduced only at the end),
-// and the last CTA publishes it in hs for the V-cycle's later launches.
-__global__ void __launch_bounds__(256) k_amg_update_start(int n, double* __restrict__ S, const double* __restrict__ p,
-                                                          const double* __restrict__ q, double* __restrict__ x,
-                                                          double* __restrict__ r, const double* __restrict__ dinv,
-                                                          double* __restrict__ part, int* __restrict__ counter,
+// alpha = r.z / p.q from the operator's partial sums, x += alpha p, r -= alpha q, partial sums of
+// r.D^-1 r, and with b = the new r: r0 = b, x0 = d = c2 D^-1 b (what k_l0_cheb_start does).
+// hs != null (FP16 directions): the V-cycle's scale comes from S[2], the previous residual's
+// r.D^-1 r (the new one is summed later), and is published in hs for the V-cycle's later launches.
+// A thread per node, the node's operands loaded before the sum of the partials.
+__global__ void __launch_bounds__(256) k_amg_update_start(int n, double* __restrict__ S,
+                                                          const double* __restrict__ pq_part, int n_pq,
+                                                          const double* __restrict__ p, const double* __restrict__ q,
+                                                          double* __restrict__ x, double* __restrict__ r,
+                                                          const double* __restrict__ dinv, double* __restrict__ part,
                                                           double* __restrict__ r0, double* __restrict__ x0,
                                                           double* __restrict__ d0, float4* __restrict__ d4,
                                                           double c2, const float4* __restrict__ sq4,
                                                           float* __restrict__ hs) {
-    __shared__ double sh[32];
-    __shared__ int s_last;
-    const double alpha = S[5];
-    const float2 hsc = hs ? h16_scale(S[2]) : make_float2(1.0f, 1.0f);
-    double acc = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int64_t o3 = 3 * (int64_t)i;
-        double rv[3];
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    const bool own = i < n;
+    const int64_t o3 = 3 * (int64_t)i;
+    double pv[3], qv[3], xv[3], rv[3], D[9];
+    if (own) {
+#pragma unroll
         for (int c = 0; c < 3; ++c) {
-            x[o3 + c] += alpha * p[o3 + c];
-            rv[c] = r[o3 + c] - alpha * q[o3 + c];
+            pv[c] = p[o3 + c];
+            qv[c] = q[o3 + c];
+            xv[c] = x[o3 + c];
+            rv[c] = r[o3 + c];
+        }
+#pragma unroll
+        for (int c = 0; c < 9; ++c) D[c] = dinv[9 * (int64_t)i + c];
+    }
+    const double rz = S[8];
+    const float2 hsc = hs ? h16_scale(S[2]) : make_float2(1.0f, 1.0f);
+    const double pq = cta_total(pq_part, n_pq, 1, false);
+    const bool ok = (pq > 0.0 && isfinite(pq)) || rz == 0.0;  // (rz = 0: the residual is zero, queued iterations idle)
+    const double alpha = ok && rz != 0.0 ? rz / pq : 0.0;
+    if (i == 0) {
+        S[0] = rz;
+        if (!ok) S[6] = 1.0;
+        if (hs) {
+            hs[0] = hsc.x;
+            hs[1] = hsc.y;
+        }
+    }
+    double acc = 0.0;
+    if (own) {
+        double t[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            x[o3 + c] = xv[c] + alpha * pv[c];
+            rv[c] -= alpha * qv[c];
             r[o3 + c] = rv[c];
             r0[o3 + c] = rv[c];
         }
-        const double* D = dinv + 9 * (int64_t)i;
-        double t[3];
+#pragma unroll
         for (int c = 0; c < 3; ++c) {
             const double dr = D[3 * c] * rv[0] + D[3 * c + 1] * rv[1] + D[3 * c + 2] * rv[2];
             acc += rv[c] * dr;
@@ -1424,31 +1439,7 @@ __global__ void __launch_bounds__(256) k_amg_update_start(int n, double* __restr
         else
             for (int c = 0; c < 3; ++c) d0[o3 + c] = t[c];
     }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    acc = warp_sum(acc);
-    if (lane == 0) sh[w] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double tt = 0.0;
-        for (int k = 0; k < nw; ++k) tt += sh[k];
-        part[blockIdx.x] = tt;
-        __threadfence();
-        s_last = atomicAdd(counter, 1) == (int)gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!s_last || w != 0) return;
-    __threadfence();
-    double tt = 0.0;
-    for (int k = lane; k < (int)gridDim.x; k += 32) tt += __ldcg(part + k);
-    tt = warp_sum(tt);
-    if (lane == 0) {
-        S[2] = tt;
-        *counter = 0;
-        if (hs) {
-            hs[0] = hsc.x;
-            hs[1] = hsc.y;
-        }
-    }
+    cta_partials(acc, 0.0, false, part);
 }
 
 // sqrt of the fine matrix's diagonal per DOF (float4 per node; 1 where a node has no
@@ -2094,11 +2085,11 @@ void Amg::first_coarse(cudaStream_t s) {
 
 // A planar level with the fused operators: pre-smoothing from x = 0 (one elementwise
 // start, degree-1 fused steps, one fused residual update), coarse correction,
-// post-smoothing written straight into z. With S != null (level 0) the last step also
-// reduces r.z and beta for the outer CG.
+// post-smoothing written straight into z. With part != null (level 0) the last step also
+// leaves the partial sums of r.z for the outer CG.
 template <typename VT>
-void Amg::vcycle(int m, const double* b, double* z, double* S, double* part, int* counter, const double* zold,
-                 cudaStream_t s, bool started) {
+void Amg::vcycle(int m, const double* b, double* z, double* part, const double* zold, cudaStream_t s,
+                 bool started) {
     AmgLevel& l = L[m];
     const VT* vals;
     if constexpr (std::is_same<VT, __half>::value) vals = l.vals16;
@@ -2150,7 +2141,7 @@ void Amg::vcycle(int m, const double* b, double* z, double* S, double* part, int
         const Start0 c0 = start_of(c);
         FX_LAUNCH(k_corner_restrict, grid_for((int64_t)c.n * kCornerLanes), 256, 0, s, corner_, l.r.ptr, c.b.ptr,
                   c.dinv0, c0.r, c0.x, c0.d, c0.d4, c0.c2, c0.sq4, c0.hs);
-        vcycle<VT>(m + 1, c.b.ptr, c.xs.ptr, nullptr, nullptr, nullptr, nullptr, s, true);
+        vcycle<VT>(m + 1, c.b.ptr, c.xs.ptr, nullptr, nullptr, s, true);
         FX_LAUNCH(k_corner_prolong, grid_for(l.n), 256, 0, s, corner_, c.result(), l.x.ptr, alpha_ * l.pscale,
                   g32 ? x4 : nullptr, l.sq4);
     } else {
@@ -2175,14 +2166,12 @@ void Amg::vcycle(int m, const double* b, double* z, double* S, double* part, int
             o.c1 = k.c1[st];
             o.c2 = k.c2[st];
         }
-        if (st == degree_ - 1 && S) {
+        if (st == degree_ - 1 && part) {
             if (2 * (int64_t)grid > part_slots_)
                 fail(FX_GENERIC, "multigrid: partial-sum buffer smaller than the smoother grid");
             o.dot = 2;
             o.zold = zold;
             o.part = part;
-            o.counter = counter;
-            o.S = S;
         }
         if (st == 0) FX_LAUNCH((k_l0_op<VT, kL0Cheb0, g32>), grid, 256, 0, s, o);
         else {
@@ -2193,12 +2182,13 @@ void Amg::vcycle(int m, const double* b, double* z, double* S, double* part, int
     }
 }
 
-void Amg::apply(const double* r, double* z, double* S, double* part, int* counter, const double* zold,
-                cudaStream_t s, bool started) {
-    if (L[0].vals16) vcycle<__half>(0, r, z, S, part, counter, zold, s, started);
-    else if (L[0].vals32) vcycle<float>(0, r, z, S, part, counter, zold, s, started);
-    else vcycle<double>(0, r, z, S, part, counter, zold, s, started);
+void Amg::apply(const double* r, double* z, double* part, const double* zold, cudaStream_t s, bool started) {
+    if (L[0].vals16) vcycle<__half>(0, r, z, part, zold, s, started);
+    else if (L[0].vals32) vcycle<float>(0, r, z, part, zold, s, started);
+    else vcycle<double>(0, r, z, part, zold, s, started);
 }
+
+unsigned Amg::apply_grid() const { return l0_grid(L[0].n, L[0].vals16 != nullptr); }
 
 Amg::Start0 Amg::start_of(const AmgLevel& l) const {
     Start0 o{};
@@ -2443,12 +2433,11 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
     const int nb = 296;
     part_.alloc(std::max<int64_t>(nb, l0_part_slots(n)), s);
     amg.set_part_slots((int64_t)part_.n);
-    sc_.alloc(8, s);
+    rd_part_.alloc(grid_for(n), s);
+    sc_.alloc(16, s);
     sc_.zero(s);
     hs_.alloc(2, s);
     amg.set_smoother_scale(f16 ? sc_.ptr + 2 : nullptr, f16 ? hs_.ptr : nullptr);  // S[2] = r.D^-1 r
-    counter_.alloc(1, s);
-    counter_.zero(s);
     // the fused coarse cycle reads the hierarchy from a device descriptor, re-uploaded
     // after every setup / refresh (new eigenvalue estimates, new Chebyshev coefficients);
     // a barrier timeout sets S[7]
@@ -2511,17 +2500,14 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
     FX_LAUNCH(k_fin, 1, 32, 0, s, nb, part_.ptr, sc_.ptr, 1);
     FX_CUDA_CHECK(cudaMemcpyAsync(sc_.ptr + 3, sc_.ptr + 2, sizeof(double), cudaMemcpyDeviceToDevice, s));
     z2_.alloc(nd, s);
-    amg.apply(r_.ptr, z_.ptr, nullptr, nullptr, nullptr, nullptr, s);
+    amg.apply(r_.ptr, z_.ptr, nullptr, nullptr, s);
     FX_LAUNCH(k_dot_part, nb, 256, 0, s, nd, r_.ptr, z_.ptr, part_.ptr);
     FX_LAUNCH(k_fin, 1, 32, 0, s, nb, part_.ptr, sc_.ptr, 3);
     FX_CUDA_CHECK(cudaMemcpyAsync(p_.ptr, z_.ptr, nd * sizeof(double), cudaMemcpyDeviceToDevice, s));
     const AmgLevel& l0 = amg.L[0];
     // flexible CG (the K-cycle makes the preconditioner vary slightly between
     // iterations): z alternates between two buffers so that r.z_old is at hand
-    // the CG update and p = z + beta p with a thread per node / entry (all of them in
-    // flight at once), the update's grid within the partial-sum slots it reduces into
-    const unsigned gu = (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_for(n), (int64_t)part_.n));
-    const unsigned gx = (unsigned)std::min<int64_t>(grid_for(nd), 4096);
+    const unsigned gu = grid_for(n), gx = grid_for(nd), gz = amg.apply_grid();
     int parity = 0;
     auto iteration = [&]() {
         double* zn = parity ? z_.ptr : z2_.ptr;
@@ -2532,19 +2518,21 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
         o.y = q_.ptr;
         o.dot = 1;
         o.part = part_.ptr;
-        o.counter = counter_.ptr;
-        o.S = sc_.ptr;
-        FX_LAUNCH((k_l0_op<double, kL0Apply>), g0, 256, 0, s, o);  // q = A p, alpha
+        FX_LAUNCH((k_l0_op<double, kL0Apply>), g0, 256, 0, s, o);  // q = A p, p.q
         const Amg::Start0 s0 = amg.start0();
-        FX_LAUNCH(k_amg_update_start, gu, 256, 0, s, n, sc_.ptr, p_.ptr, q_.ptr, x, r_.ptr, dinv64, part_.ptr,
-                  counter_.ptr, s0.r, s0.x, s0.d, s0.d4, s0.c2, s0.sq4, s0.hs);  // x, r, r.D^-1 r; the V-cycle's first step
-        amg.apply(r_.ptr, zn, sc_.ptr, part_.ptr, counter_.ptr, amg.kcycle() ? zo : nullptr, s, true);  // z, r.z, beta
-        FX_LAUNCH(k_xpby, gx, 256, 0, s, nd, zn, sc_.ptr, p_.ptr);
+        FX_LAUNCH(k_amg_update_start, gu, 256, 0, s, n, sc_.ptr, part_.ptr, (int)g0, p_.ptr, q_.ptr, x, r_.ptr, dinv64,
+                  rd_part_.ptr, s0.r, s0.x, s0.d, s0.d4, s0.c2, s0.sq4, s0.hs);  // x, r; the V-cycle's first step
+        amg.apply(r_.ptr, zn, part_.ptr, amg.kcycle() ? zo : nullptr, s, true);  // z, r.z
+        FX_LAUNCH(k_xpby, gx, 256, 0, s, nd, zn, sc_.ptr, part_.ptr, (int)gz, amg.kcycle(), rd_part_.ptr, (int)gu,
+                  p_.ptr);
     };
-    // Four iterations per graph replay between host checks. (A device-side loop
-    // as a WHILE graph node, one or four iterations per body, measured 1-7 %
-    // slower per iteration on B200 than these host-polled replays.)
-    const int per_poll = 4;
+    // Two iterations per graph (z alternates). Between host checks as many replays are queued as the
+    // residual's fall so far says are surely needed (60 % of the estimate, at most 12 iterations, 4 where
+    // an iteration takes several times the ~14 us that a check idles the GPU for): iterations queued
+    // past the end cost more than checks.
+    // (A device-side loop as a WHILE graph node, one or four iterations per body, measured 1-7 %
+    // slower per iteration on B200 than host-polled replays.)
+    const int per_graph = 2;
     const bool graphs = opt.graphs && !debug_sync();
     const void* key[4] = {x, vals64, dinv64, r_.ptr};
     if (gexec_ && (!graphs || !std::equal(key, key + 4, graph_key_))) drop_graph();
@@ -2554,7 +2542,7 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
         int64_t* saved = g_launch_counter;
         g_launch_counter = &count;
         FX_CUDA_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        for (int k = 0; k < per_poll; ++k) iteration();
+        for (int k = 0; k < per_graph; ++k) iteration();
         const cudaError_t ce = cudaStreamEndCapture(s, &g);
         g_launch_counter = saved;
         FX_CUDA_CHECK(ce);
@@ -2565,10 +2553,12 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
         FX_CUDA_CHECK(ci);
         std::copy(key, key + 4, graph_key_);
     }
-    double h[8];
+    double h[9];
     long long it = 0;
     int rc = FX_OK;
     const double rtol2 = opt.rtol * opt.rtol;
+    double seen = -1.0;  // r.D^-1 r at the check before, and the iterations queued since
+    int queued = 0;
     while (true) {
         FX_CUDA_CHECK(cudaMemcpyAsync(h, sc_.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
         stream_wait(s, "amg pcg poll");
@@ -2582,13 +2572,26 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
             rc = FX_CONVERGENCE;
             break;
         }
-        if (gexec_) {
-            FX_CUDA_CHECK(cudaGraphLaunch(gexec_, s));
-            if (launches) *launches += graph_launches_;
-        } else {
-            for (int k = 0; k < per_poll; ++k) iteration();
+        int next = 4;
+        if (seen > 0.0) {
+            const double fall = std::log(h[2] / seen) / queued;  // per iteration
+            const double left = fall < 0.0 ? std::log(rtol2 * h[3] / h[2]) / fall : 4.0;
+            next = (int)(left < 20.0 ? 0.6 * left : 12.0);
+            if (n > 30000) next = std::min(next, 4);
         }
-        it += per_poll;
+        next = (int)std::min<long long>(std::max(next, 1), std::max<long long>(1, opt.max_iter - it));
+        const int replays = (next + per_graph - 1) / per_graph;
+        for (int k = 0; k < replays; ++k) {
+            if (gexec_) {
+                FX_CUDA_CHECK(cudaGraphLaunch(gexec_, s));
+                if (launches) *launches += graph_launches_;
+            } else {
+                for (int j = 0; j < per_graph; ++j) iteration();
+            }
+        }
+        seen = h[2];
+        queued = replays * per_graph;
+        it += queued;
     }
     solved(it);
     // true residual of the assembled FP64 system in the block-Jacobi norm

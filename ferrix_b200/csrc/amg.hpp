@@ -135,13 +135,13 @@ class Amg {
     void set_overcorrect(double alpha) { alpha_ = alpha; }
     void set_cheb_ratio(double ratio) { cheb_ratio_ = ratio; }
     bool kcycle() const { return kcycle_; }
-    // z = cycle(r), FP64 vectors of 3 * n_nodes. With S != null the last
-    // smoothing step also reduces r.z (and r.zold when zold != null, for the
-    // flexible CG) into the outer CG scalars (S[0], S[4]).
+    // z = cycle(r), FP64 vectors of 3 * n_nodes. With part != null the last smoothing step also
+    // leaves partial sums of (r.z, r.zold) (zold null: 0; for the flexible CG), two doubles for each
+    // of its apply_grid() CTAs.
     // started: the level-0 start (r0 = b, x = d = c2 D^-1 b) was done by the caller, into start0()
-    void apply(const double* r, double* z, double* S, double* part, int* counter, const double* zold,
-               cudaStream_t s, bool started = false);
-    // slots of the `part` buffer apply() reduces into (two per CTA of the reducing launch)
+    void apply(const double* r, double* z, double* part, const double* zold, cudaStream_t s, bool started = false);
+    unsigned apply_grid() const;
+    // slots of the `part` buffer apply() writes
     void set_part_slots(int64_t n) { part_slots_ = n; }
     // where the level-0 start writes: the smoother's residual, iterate and first direction
     // (FP32 float4 per node when the smoother is FP32, else FP64), and its coefficient
@@ -177,8 +177,7 @@ class Amg {
     void coarsest_inverse(AmgLevel& l, cudaStream_t s);
     // V-cycle from planar level m, whose smoother values are VT
     template <typename VT>
-    void vcycle(int m, const double* b, double* z, double* S, double* part, int* counter, const double* zold,
-                cudaStream_t s, bool started);
+    void vcycle(int m, const double* b, double* z, double* part, const double* zold, cudaStream_t s, bool started);
     void first_coarse(cudaStream_t s);  // from the last planar level's residual into its iterate
     int planar_ = 1;
     CornerView corner_;
@@ -326,12 +325,11 @@ class AmgPcg {
     const BsrStructure* S_ = nullptr;
     const double* vals64_ = nullptr;
     const double* dinv64_ = nullptr;
-    DBuf<double> r_, z_, z2_, p_, q_, part_, sc_;
+    DBuf<double> r_, z_, z2_, p_, q_, part_, rd_part_, sc_;
     DBuf<float> vals32_[2];  // per planar level
     DBuf<__half> vals16_[2];
     DBuf<float4> sq4_[2];
     DBuf<float> hs_;  // FP16 smoother directions: the current V-cycle's {2^k, 2^-k}
-    DBuf<int> counter_;
     bool fresh_ = false, stale_ = false;  // the hierarchy was (re)computed for this solve; should be for the next
     long long first_iters_ = 0;
     // the captured iterations, kept while the hierarchy is: what they were captured with
