@@ -410,15 +410,26 @@ __global__ void __launch_bounds__(256) k_apply4(int nelem, const int32_t* __rest
     }
 }
 
+// Warp per element in two phases. First a lane per Gauss point sums J = dN X and H = dN V over the
+// element's nodes (node data broadcast from shared memory) and forms T = w J^-1 sigma (sigma from the
+// strain of J^-1 H); then a lane per node sums f = dN^T T over the Gauss points. No lane needs
+// another's sum: with a lane per node throughout, every Gauss point took 15-17 warp reductions of
+// doubles (~4,600 shuffles per element), which bounded the kernel. 9,240 elements with
+// temperature-dependent constants: 267 -> 43 us (internal and thermal force averaged).
+constexpr int kDnStride = 61;  // doubles per Gauss point of dN in shared memory: odd, so that lanes of different
+constexpr int kNStride = 21;   // Gauss points read different banks
 __global__ void __launch_bounds__(256) k_apply20(int nelem, const int32_t* __restrict__ conn,
                                                  const int32_t* __restrict__ mat, const double* __restrict__ X,
                                                  ApplyArgs A, MatDev md, RuleTables rt, double* __restrict__ fe,
                                                  int* err) {
-    __shared__ double s_dn[kGp20 * 60];
-    __shared__ double s_n[kGp20 * 20];
+    __shared__ double s_dn[kGp20 * kDnStride];
+    __shared__ double s_n[kGp20 * kNStride];
     __shared__ double s_w[kGp20];
-    for (int i = threadIdx.x; i < kGp20 * 60; i += blockDim.x) s_dn[i] = rt.dn20_d[i];
-    for (int i = threadIdx.x; i < kGp20 * 20; i += blockDim.x) s_n[i] = rt.n20_d[i];
+    // per warp and node {x, v}, and {T current, T initial}; then per Gauss point T (9 doubles)
+    __shared__ __align__(16) double s_el[kWarps20][kGp20 * 9 + 1];
+    __shared__ __align__(16) double s_t[kWarps20][40];
+    for (int i = threadIdx.x; i < kGp20 * 60; i += blockDim.x) s_dn[i / 60 * kDnStride + i % 60] = rt.dn20_d[i];
+    for (int i = threadIdx.x; i < kGp20 * 20; i += blockDim.x) s_n[i / 20 * kNStride + i % 20] = rt.n20_d[i];
     for (int i = threadIdx.x; i < kGp20; i += blockDim.x) s_w[i] = rt.w20[i];
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -431,81 +442,102 @@ __global__ void __launch_bounds__(256) k_apply20(int nelem, const int32_t* __res
     }
     const bool thermal = A.cth != 0.0 && md.a_len[k] > 0;
     const bool t_dep = md.e_len[k] > 1 || md.nu_len[k] > 1 || thermal;
-    double x0 = 0, x1 = 0, x2 = 0, v0 = 0, v1 = 0, v2 = 0, tca = 0, tia = 0;
+    const bool strain = A.cv != 0.0 && A.v;
+    double* el = s_el[warp];
+    double* st = s_t[warp];
     if (lane < 20) {
-        int nd = conn[20 * e + lane];
-        x0 = X[3 * nd];
-        x1 = X[3 * nd + 1];
-        x2 = X[3 * nd + 2];
-        if (A.uconf) {
-            x0 += A.uconf[3 * nd];
-            x1 += A.uconf[3 * nd + 1];
-            x2 += A.uconf[3 * nd + 2];
-        }
-        if (A.v) {
-            v0 = A.v[3 * nd];
-            v1 = A.v[3 * nd + 1];
-            v2 = A.v[3 * nd + 2];
-        }
-        tca = A.tcur[nd];
-        tia = A.tinit[nd];
-    }
-    Lame L;
-    if (!t_dep) material_d(md, k, 0.0, &L);
-    double f0 = 0, f1 = 0, f2 = 0;
-    int bad = 0;
-    for (int gp = 0; gp < kGp20; ++gp) {
-        double d0 = 0, d1 = 0, d2 = 0;
-        if (lane < 20) {
-            d0 = s_dn[gp * 60 + lane];
-            d1 = s_dn[gp * 60 + 20 + lane];
-            d2 = s_dn[gp * 60 + 40 + lane];
-        }
-        double J[9] = {d0 * x0, d0 * x1, d0 * x2, d1 * x0, d1 * x1, d1 * x2, d2 * x0, d2 * x1, d2 * x2};
+        const int nd = conn[20 * e + lane];
 #pragma unroll
-        for (int c = 0; c < 9; ++c) J[c] = warp_sum(J[c]);
-        double dth = 0.0;
-        if (t_dep) {
-            double nn = lane < 20 ? s_n[gp * 20 + lane] : 0.0;
-            double tc = warp_sum(nn * tca);
-            material_d(md, k, tc, &L);
-            if (thermal) {
-                double ti = warp_sum(nn * tia);
-                dth = thermal_delta(md, k, tc, ti);
+        for (int c = 0; c < 3; ++c) {
+            el[6 * lane + c] = X[3 * nd + c] + (A.uconf ? A.uconf[3 * nd + c] : 0.0);
+            el[6 * lane + 3 + c] = A.v ? A.v[3 * nd + c] : 0.0;
+        }
+        st[2 * lane] = A.tcur[nd];
+        st[2 * lane + 1] = A.tinit[nd];
+    }
+    __syncwarp();
+    double T[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (lane < kGp20) {
+        const double* dn = s_dn + lane * kDnStride;
+        double J[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, H[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 5
+        for (int a = 0; a < 20; ++a) {
+            const double2 p = *reinterpret_cast<const double2*>(el + 6 * a);      // x0 x1
+            const double2 q = *reinterpret_cast<const double2*>(el + 6 * a + 2);  // x2 v0
+            const double2 r = *reinterpret_cast<const double2*>(el + 6 * a + 4);  // v1 v2
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double g = dn[d * 20 + a];
+                J[3 * d] += g * p.x;
+                J[3 * d + 1] += g * p.y;
+                J[3 * d + 2] += g * q.x;
+                H[3 * d] += g * q.y;
+                H[3 * d + 1] += g * r.x;
+                H[3 * d + 2] += g * r.y;
             }
         }
-        double Ji[9];
-        double det = inv3(J, Ji);
-        if (det == 0.0) bad = 1;
-        double w = fabs(det) * s_w[gp];
-        double g0 = Ji[0] * d0 + Ji[1] * d1 + Ji[2] * d2;
-        double g1 = Ji[3] * d0 + Ji[4] * d1 + Ji[5] * d2;
-        double g2 = Ji[6] * d0 + Ji[7] * d1 + Ji[8] * d2;
-        double eps[6];
-        if (A.cv != 0.0) {
-            eps[0] = warp_sum(g0 * v0);
-            eps[1] = warp_sum(g1 * v1);
-            eps[2] = warp_sum(g2 * v2);
-            eps[3] = warp_sum(g1 * v0 + g0 * v1);
-            eps[4] = warp_sum(g2 * v1 + g1 * v2);
-            eps[5] = warp_sum(g2 * v0 + g0 * v2);
-#pragma unroll
-            for (int i = 0; i < 6; ++i) eps[i] *= A.cv;
+        Lame L;
+        double dth = 0.0;
+        if (t_dep) {
+            double tc = 0.0, ti = 0.0;
+            for (int a = 0; a < 20; ++a) {
+                const double n = s_n[lane * kNStride + a];
+                tc += n * st[2 * a];
+                ti += n * st[2 * a + 1];
+            }
+            material_d(md, k, tc, &L);
+            if (thermal) dth = thermal_delta(md, k, tc, ti);
         } else {
+            material_d(md, k, 0.0, &L);
+        }
+        double Ji[9];
+        const double det = inv3(J, Ji);
+        if (det == 0.0) atomicOr(err, kErrSingularJ);
+        const double w = fabs(det) * s_w[lane];
+        double eps[6] = {0, 0, 0, 0, 0, 0};
+        if (strain) {  // G = J^-1 H: G[i][c] = d v_c / d x_i
+            double G[9];
 #pragma unroll
-            for (int i = 0; i < 6; ++i) eps[i] = 0.0;
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    G[3 * i + c] = Ji[3 * i] * H[c] + Ji[3 * i + 1] * H[3 + c] + Ji[3 * i + 2] * H[6 + c];
+            eps[0] = A.cv * G[0];
+            eps[1] = A.cv * G[4];
+            eps[2] = A.cv * G[8];
+            eps[3] = A.cv * (G[3] + G[1]);
+            eps[4] = A.cv * (G[7] + G[5]);
+            eps[5] = A.cv * (G[6] + G[2]);
         }
         eps[0] -= A.cth * dth;
         eps[1] -= A.cth * dth;
         eps[2] -= A.cth * dth;
         double s[6];
         stress_from(L, eps, s);
-        f0 += (g0 * s[0] + g1 * s[3] + g2 * s[5]) * w;
-        f1 += (g1 * s[1] + g0 * s[3] + g2 * s[4]) * w;
-        f2 += (g2 * s[2] + g1 * s[4] + g0 * s[5]) * w;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {  // T[d][i] = w sum_j Ji[j][d] sigma_ij
+            const double j0 = w * Ji[d], j1 = w * Ji[3 + d], j2 = w * Ji[6 + d];
+            T[3 * d] = j0 * s[0] + j1 * s[3] + j2 * s[5];
+            T[3 * d + 1] = j0 * s[3] + j1 * s[1] + j2 * s[4];
+            T[3 * d + 2] = j0 * s[5] + j1 * s[4] + j2 * s[2];
+        }
     }
-    if (bad && lane == 0) atomicOr(err, kErrSingularJ);
+    __syncwarp();  // every lane has read the node data
+    if (lane < kGp20)
+#pragma unroll
+        for (int c = 0; c < 9; ++c) el[9 * lane + c] = T[c];
+    __syncwarp();
     if (lane < 20) {
+        double f0 = 0.0, f1 = 0.0, f2 = 0.0;
+#pragma unroll 3
+        for (int gp = 0; gp < kGp20; ++gp) {
+            const double* t = el + 9 * gp;
+            const double d0 = s_dn[gp * kDnStride + lane], d1 = s_dn[gp * kDnStride + 20 + lane],
+                         d2 = s_dn[gp * kDnStride + 40 + lane];
+            f0 += d0 * t[0] + d1 * t[3] + d2 * t[6];
+            f1 += d0 * t[1] + d1 * t[4] + d2 * t[7];
+            f2 += d0 * t[2] + d1 * t[5] + d2 * t[8];
+        }
         double* out = fe + ((size_t)e * 20 + lane) * 3;
         out[0] = f0;
         out[1] = f1;
