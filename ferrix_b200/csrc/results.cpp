@@ -16,8 +16,10 @@ using namespace fx;
 
 namespace {
 
-// S, E: 6 Voigt components per node (xx, yy, zz, xy, yz, zx), node-index order.
-void nodal_stress_strain(fx_model* m, std::vector<double>& S, std::vector<double>& E) {
+// S, E (either may be null): 6 Voigt components per node (xx, yy, zz, xy, yz, zx), node-index
+// order, copied straight into the caller's arrays (through vectors of their own, 6.5 MB of results took
+// 1.6 instead of 1.0 ms).
+void nodal_stress_strain(fx_model* m, double* S, double* E) {
     if (!m->state_ready) fail(FX_INVALID_ARGUMENT, "fx_state_initialize was not called");
     ensure_structure(m);
     ModelDev& d = m->dev;
@@ -33,10 +35,8 @@ void nodal_stress_strain(fx_model* m, std::vector<double>& S, std::vector<double
                         m->ctx->tables.view(), (int)n, d.S.node_ptr.ptr, d.S.node_slots.ptr, buf.ptr, dS.ptr, dE.ptr,
                         d.err.ptr, s);
     check_device_errors(m, "stress recovery");
-    S.resize(6 * (size_t)n);
-    E.resize(6 * (size_t)n);
-    dS.download(S.data(), S.size(), s);
-    dE.download(E.data(), E.size(), s);
+    if (S) dS.download(S, 6 * (size_t)n, s);
+    if (E) dE.download(E, 6 * (size_t)n, s);
     stream_wait(s, "stress download");
 }
 
@@ -92,10 +92,7 @@ int fx_nodal_stress_strain(fx_model* m, double* S, double* E) {
             int64_t* v;
             ~R() { g_launch_counter = v; }
         } r{saved};
-        std::vector<double> hs, he;
-        nodal_stress_strain(m, hs, he);
-        if (S) std::memcpy(S, hs.data(), hs.size() * sizeof(double));
-        if (E) std::memcpy(E, he.data(), he.size() * sizeof(double));
+        nodal_stress_strain(m, S, E);
         return FX_OK;
     });
 }
@@ -110,10 +107,11 @@ int fx_write_vtk(fx_model* m, const char* path) {
             int64_t* v;
             ~R() { g_launch_counter = v; }
         } r{saved};
-        std::vector<double> S, E;
-        nodal_stress_strain(m, S, E);
+        if (!m->state_ready) fail(FX_INVALID_ARGUMENT, "fx_state_initialize was not called");
         const DenseModel& D = m->dense;
         const int64_t n = D.n_nodes;
+        std::vector<double> S(6 * (size_t)n), E(6 * (size_t)n);
+        nodal_stress_strain(m, S.data(), E.data());
         std::vector<double> u(3 * (size_t)n), tc((size_t)n);
         m->dev.u.download(u.data(), u.size(), m->ctx->stream);
         m->dev.tcur.download(tc.data(), tc.size(), m->ctx->stream);
