@@ -391,6 +391,22 @@ __global__ void __launch_bounds__(128) k_dense_from_bsr(int n, const int32_t* __
     }
 }
 
+// the same from a planar level's BSR3
+__global__ void __launch_bounds__(128) k_dense_from_planar(int n, const int32_t* __restrict__ row_ptr,
+                                                           const int32_t* __restrict__ goff,
+                                                           const int32_t* __restrict__ cols,
+                                                           const double* __restrict__ vals, double* __restrict__ A) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const int64_t nd = 3 * (int64_t)n, g0 = goff[i], ng = goff[i + 1] - g0;
+    const int nb = row_ptr[i + 1] - row_ptr[i];
+    for (int it = lane; it < 9 * nb; it += 32) {
+        const int e = it / nb, k = it - e * nb;
+        A[(3 * (int64_t)i + e / 3) * nd + 3 * (int64_t)cols[4 * g0 + k] + e % 3] =
+            vals[(g0 * 9 + e * ng + k / 4) * 4 + (k & 3)];
+    }
+}
+
 // Coarsest level: blocked Gauss-Jordan inverse of the dense SPD matrix (no pivoting), kPanel
 // pivots per launch. With P the inverse of the pivot block A[K, K], panel K maps A to
 //   B[K, K] = P, B[K, j] = P A[K, j], B[i, K] = -A[i, K] P, B[i, j] = A[i, j] - A[i, K] P A[K, j].
@@ -601,6 +617,10 @@ __global__ void k_dot_part(int64_t n, const double* __restrict__ a, const double
         part[blockIdx.x] = s;
     }
 }
+
+// partial sums of (b.z, b.zold) as a V-cycle's last smoothing step leaves them (zold null: 0)
+__global__ void __launch_bounds__(256) k_pair_part(int64_t n, const double* __restrict__ b, const double* __restrict__ z,
+                                                   const double* __restrict__ zold, double* __restrict__ part);
 
 // |a|^2 and |b|^2 in two launches (fixed order): partials of a in part[0 .. nb), of b in part[nb .. 2 nb)
 __global__ void __launch_bounds__(256) k_norm2_part(int64_t n, const double* __restrict__ a,
@@ -822,6 +842,16 @@ __device__ __forceinline__ void cta_partials(double v, double v2, bool two, doub
         for (int k = 0; k < nw; ++k) t += sh[threadIdx.x][k];
         part[(two ? 2 : 1) * blockIdx.x + threadIdx.x] = t;
     }
+}
+
+__global__ void __launch_bounds__(256) k_pair_part(int64_t n, const double* __restrict__ b, const double* __restrict__ z,
+                                                   const double* __restrict__ zold, double* __restrict__ part) {
+    double t = 0.0, u = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+        t += b[i] * z[i];
+        if (zold) u += b[i] * zold[i];
+    }
+    cta_partials(t, u, true, part);
 }
 
 #ifndef FX_L0_MIN_BLOCKS
@@ -1665,8 +1695,12 @@ void Amg::coarsest_inverse(AmgLevel& l, cudaStream_t s) {
     const int64_t nd = (int64_t)l.n * l.bs;
     l.dense_inv.alloc((size_t)nd * nd, s);
     l.dense_inv.zero(s);
-    FX_LAUNCH(k_dense_from_bsr<6>, grid_for((int64_t)l.n * 32, 128), 128, 0, s, l.n, l.row_ptr.ptr, l.cols.ptr,
-              l.vals.ptr, l.dense_inv.ptr);
+    if (l.S0)
+        FX_LAUNCH(k_dense_from_planar, grid_for((int64_t)l.n * 32, 128), 128, 0, s, l.n, l.S0->row_ptr.ptr,
+                  l.S0->goff.ptr, l.S0->cols.ptr, l.vals0, l.dense_inv.ptr);
+    else
+        FX_LAUNCH(k_dense_from_bsr<6>, grid_for((int64_t)l.n * 32, 128), 128, 0, s, l.n, l.row_ptr.ptr, l.cols.ptr,
+                  l.vals.ptr, l.dense_inv.ptr);
     DBuf<uint8_t> dead;
     dead.alloc(nd, s);
     DBuf<double> diag0, other, pivot;
@@ -1755,9 +1789,17 @@ static void planar_work(AmgLevel& l, bool result, cudaStream_t s) {
 }
 
 void Amg::setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz, double cell0, double node_volume,
-                cudaStream_t s, AmgStats* st) {
+                bool dense, cudaStream_t s, AmgStats* st) {
     EventTimer timer;
     timer.start(s);
+    auto done = [&] {
+        if (st) {
+            st->levels = (int)L.size();
+            st->sizes.clear();
+            for (auto& l : L) st->sizes.push_back(l.n * l.bs);
+            st->setup_ms = timer.stop_ms(s);
+        }
+    };
     L.clear();
     L.reserve(kMaxLevels + 1);
     planar_ = corner ? 2 : 1;
@@ -1771,6 +1813,14 @@ void Amg::setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz
             L[m].pscale = 1.0 / kAmgOvercorrect;
             estimate_lmax(L[m], red_, s, false);
         }
+    }
+    if (dense && dense_planar(L.back().n)) {
+        AmgLevel& l = L.back();
+        l.lmax = 1.0;  // (no smoothing here)
+        l.coarsest = true;
+        coarsest_inverse(l, s);
+        done();
+        return;
     }
     // the points of the last planar level and their bounding box (cell keys of every level are
     // taken from its lower corner)
@@ -1886,12 +1936,7 @@ void Amg::setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz
         l1.kcs.alloc(8, s);
         l1.kcs.zero(s);
     }
-    if (st) {
-        st->levels = (int)L.size();
-        st->sizes.clear();
-        for (auto& l : L) st->sizes.push_back(l.n * l.bs);
-        st->setup_ms = timer.stop_ms(s);
-    }
+    done();
 }
 
 void Amg::refresh(const PlanarIn* in, cudaStream_t s, AmgStats* st) {
@@ -2091,6 +2136,12 @@ template <typename VT>
 void Amg::vcycle(int m, const double* b, double* z, double* part, const double* zold, cudaStream_t s,
                  bool started) {
     AmgLevel& l = L[m];
+    if (l.coarsest) {  // z = A^-1 b
+        const int64_t nd = 3 * (int64_t)l.n;
+        FX_LAUNCH(k_dense_matvec, grid_for(nd * 32, kLnThreads), kLnThreads, 0, s, (int)nd, l.dense_inv.ptr, b, z);
+        if (part) FX_LAUNCH(k_pair_part, apply_grid(), 256, 0, s, nd, b, z, zold, part);
+        return;
+    }
     const VT* vals;
     if constexpr (std::is_same<VT, __half>::value) vals = l.vals16;
     else if constexpr (std::is_same<VT, float>::value) vals = l.vals32;
@@ -2320,6 +2371,7 @@ void Amg::describe(ClInst& o) const {
         p.lt = l.t.ptr;
         p.b = l.b.ptr;
         p.z = l.xs.ptr;
+        p.dense_inv = l.coarsest ? l.dense_inv.ptr : nullptr;
         p.d4a = l.d4a.ptr;
         p.d4b = l.d4b.ptr;
         p.x4 = l.x4.ptr;
@@ -2414,7 +2466,7 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
     } else {
         drop_graph();
         amg.built_for = 0;  // (a failed setup leaves nothing to reuse)
-        amg.setup(in, corner, corner ? corner->xyz.ptr : xyz, cell0, node_volume, s, st);
+        amg.setup(in, corner, corner ? corner->xyz.ptr : xyz, cell0, node_volume, corner || !persistent, s, st);
         amg.built_for = S.id;
         fresh_ = true;
         stale_ = false;

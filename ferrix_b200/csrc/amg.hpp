@@ -18,6 +18,8 @@
 //   * Chebyshev smoothing of degree 2 on D^-1 A (D = block diagonal) with the
 //     largest eigenvalue from power iteration; dense inverse at the coarsest
 //     level.
+//   * a last planar level that is small enough itself (kDensePlanarDof) takes the dense inverse
+//     and ends the hierarchy: the corner level of small C3D20 meshes, or a small C3D4 system whole.
 // Application: one V-cycle per PCG iteration.
 #pragma once
 
@@ -107,8 +109,9 @@ class Amg {
     // in: the fine matrix and, with a corner level (corner != null), that level's. xyz: FP64
     // coordinates (device, 3 per node) of the last planar level's nodes. cell0: edge of the first
     // aggregates' cells, 0 = chosen from the mesh (pick_cell; node_volume: volume per such node).
+    // dense: the last planar level may be the coarsest (dense_planar()).
     void setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz, double cell0, double node_volume,
-               cudaStream_t s, AmgStats* st);
+               bool dense, cudaStream_t s, AmgStats* st);
     // New matrix values on the structure of the last setup: aggregates, prolongators (values
     // included) and coarse patterns are kept; coarse values, block inverses, eigenvalue
     // estimates and the coarsest inverse are recomputed.
@@ -233,6 +236,7 @@ struct ClPlanar {
     const float4* sq4 = nullptr;  // FP16 smoother: the FP32 iterate copy is scaled by sqrt(a_ii)
     double *lr = nullptr, *lx = nullptr, *ld = nullptr, *lt = nullptr;
     double *b = nullptr, *z = nullptr;  // the corner level's right-hand side and result
+    const double* dense_inv = nullptr;  // the corner level as the coarsest
     float *d4a = nullptr, *d4b = nullptr, *x4 = nullptr;
     double c2_start = 0.0, c1[8] = {}, c2[8] = {};
 };
@@ -273,6 +277,12 @@ void launch_coarse_grid(const ClInst* inst, GridBarState* st, double* flag, bool
 // took 243-324 ms against 183 ms for the multi-launch path on every stream (B200).
 constexpr int64_t kClDefaultMaxDof = 2000;
 
+// A last planar level of at most this many DOF is inverted as it is: 3 DOF per row, so the inverse of
+// 1,200 DOF (~0.6 ms) replaces the transfer's setup (~0.4 ms) and a smaller inverse, and the CG needs 20 %
+// fewer iterations of fewer launches.
+constexpr int kDensePlanarDof = 1200;
+inline bool dense_planar(int64_t rows) { return 3 * rows <= kDensePlanarDof; }
+
 // The default of the option amg_aggregate_nodes: with it the hierarchy chooses its cells (pick_cell).
 constexpr int kAmgAggregateNodes = 40;
 
@@ -308,6 +318,7 @@ class AmgPcg {
     // For the persistent solve: set up (or refresh) the hierarchy for the system and
     // allocate the CG vectors, without iterating; then describe it for the kernel.
     // corner: the corner level with its matrix, or null; cell0, node_volume: Amg::setup
+    // persistent: for the persistent solve (which has no dense fine level)
     void prepare(const BsrStructure& S, const double* vals64, const double* dinv64, const double* xyz,
                  const CornerLevel* corner, double cell0, double node_volume, const PcgOptions& opt, cudaStream_t s,
                  AmgStats* st, bool reuse, bool persistent = false);

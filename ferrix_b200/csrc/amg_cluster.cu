@@ -574,9 +574,14 @@ __device__ double vcycle(const ClInst& I, Vg g, int degree, double alpha, cg::cl
     if (I.planar == 2) {
         corner_restrict_op<G32>(g, I);
         cl.sync();
-        planar_down<VT, G32>(I.pl[1], g, degree, cl, eA, eB, eA4, eB4);
-        coarse_cycle<G32>(I, g, degree, alpha, bar);
-        planar_up<VT, G32>(I.pl[1], g, I.pl[1].b, I.pl[1].z, degree, false, cl, eA, eB, eA4, eB4);
+        if (I.pl[1].dense_inv) {
+            dense_op(g, 3 * I.pl[1].n, I.pl[1].dense_inv, I.pl[1].b, I.pl[1].z);
+            cl.sync();
+        } else {
+            planar_down<VT, G32>(I.pl[1], g, degree, cl, eA, eB, eA4, eB4);
+            coarse_cycle<G32>(I, g, degree, alpha, bar);
+            planar_up<VT, G32>(I.pl[1], g, I.pl[1].b, I.pl[1].z, degree, false, cl, eA, eB, eA4, eB4);
+        }
         corner_prolong_op<G32>(g, I, alpha * I.corner_scale);
         cl.sync();
     } else {

@@ -702,7 +702,11 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
                 if (!d.amg) d.amg = std::make_unique<AmgPcg>();
                 const CornerLevel* corner = d.corner.usable ? &d.corner : nullptr;
                 const int64_t ndof = 3 * r.m->dense.n_nodes;
-                if (!po.amg_kcycle && po.amg_persistent_max_dof > 0 && ndof <= po.amg_persistent_max_dof) {
+                // by default a system that the dense inverse covers (or its corner level) takes the
+                // multi-launch path: 1,194-DOF C3D20 deck 1.0 against 2.1 ms of CG
+                const bool dense = r.o.amg_persistent_max_dof == 0 &&
+                                   dense_planar(corner ? corner->n : r.m->dense.n_nodes);
+                if (!po.amg_kcycle && po.amg_persistent_max_dof > 0 && ndof <= po.amg_persistent_max_dof && !dense) {
                     // small system: hierarchy now, its whole CG in the round's persistent launch below
                     guard(i, [&] {
                         d.amg->prepare(d.S, d.vals64.ptr, d.minv64.ptr, r.amg_xyz.ptr, corner, r.amg_cell,

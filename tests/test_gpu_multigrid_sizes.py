@@ -120,3 +120,20 @@ def test_kept_hierarchy_over_newton_iterations(ctx, npe, persistent):
     u, stats = _solve(ctx, text, amg_persistent_max_dof=persistent)
     assert stats["linear_solves"] > 2 * stats["increments"]
     assert float(np.linalg.norm(u - ref) / np.linalg.norm(ref)) <= 1e-8, stats
+
+
+@pytest.mark.parametrize("prec", [fx.PREC_FP64, fx.PREC_MIXED])
+@pytest.mark.parametrize("npe,cells", [(4, (1, 1, 1)), (4, (2, 1, 3)), (4, (3, 3, 23)), (4, (3, 3, 24)), (4, (3, 3, 25)),
+                                       (20, (3, 3, 24)), (20, (3, 3, 25))])
+def test_dense_planar_level(ctx, npe, cells, prec):
+    """Small systems whose fine level (C3D4) or corner level (C3D20) takes the dense inverse itself, up to
+    its largest size (400 nodes or corners) and just beyond."""
+    lengths = tuple(float(c) for c in cells)
+    spec = decks.c3d20_box_spec(*cells, lengths=lengths)
+    if npe == 4:
+        spec.mesh = decks.tet_box(*cells, *lengths)
+    text = decks.write_deck(spec)
+    ref = static_step.Runner(inp.parse_inp_text(text)).run().displacements
+    u, stats = _solve(ctx, text, precision=prec)
+    # FP64: 1e-10 as elsewhere; these slender columns leave up to 1e-9 at the mixed solver's residual
+    assert float(np.linalg.norm(u - ref) / np.linalg.norm(ref)) <= (1e-10 if prec == fx.PREC_FP64 else 1e-8), stats
