@@ -1923,7 +1923,7 @@ void Amg::setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz
         c.n = na;
         c.bs = 6;
         c.vals.alloc((size_t)c.nblocks * 36, s);
-        galerkin_product(fine_view(lf), lf.tr, c.vals.ptr, s);
+        galerkin_product(fine_view(lf), lf.tr, c.row_ptr.ptr, c.cols.ptr, c.vals.ptr, s);
         // next level points and near-null-space
         coords = std::move(cent);
         Rprev = std::move(Rnext);
@@ -1954,7 +1954,8 @@ void Amg::refresh(const PlanarIn* in, cudaStream_t s, AmgStats* st) {
         }
         if (!l.S0) planar_values(l, s);
         estimate_lmax(l, red_, s, true);
-        if (!l.corner_next) galerkin_product(fine_view(l), l.tr, L[lev + 1].vals.ptr, s);
+        if (!l.corner_next)
+            galerkin_product(fine_view(l), l.tr, L[lev + 1].row_ptr.ptr, L[lev + 1].cols.ptr, L[lev + 1].vals.ptr, s);
     }
     if (st) {
         st->levels = (int)L.size();

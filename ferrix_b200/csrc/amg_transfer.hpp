@@ -2,11 +2,11 @@
 // A_c = P^T A P with it (Vanek, Mandel & Brezina 1996).
 //
 // P = (I - omega D^-1 A) Q: every fine row reaches the aggregates of its matrix
-// neighbours. Both sparse products, W = A P and A_c = P^T W, are built once as lists of
-// operand pairs sorted by the (row, column) of the entry they contribute to (expand,
-// sort, compress); the numeric kernels sum each entry's pairs in that fixed order (no
-// atomics: results do not depend on timing) and are repeated when only the matrix
-// values change.
+// neighbours. The sparse products W = A P and A_c = P^T W are formed row by row, their patterns once
+// and their values again when only the matrix values change; rows too long for shared memory
+// take lists of operand pairs sorted by the (row, column) of the entry they contribute to
+// (expand, sort, compress). Every sum has a fixed order (no atomics: results do not
+// depend on timing).
 #pragma once
 
 #include <cstdint>
@@ -59,13 +59,17 @@ struct PairList {
 
 // Transfer of a level to the next: P's entries by fine row (ptr, col; val: row-major blocks, what
 // the products read; val32: the cycle's interleaved copy) and by aggregate (t_ptr, t_row, t_val32),
-// see transfer.cuh, and the pair lists of W = A P and A_c = P^T W.
+// t_ent: the entry), see transfer.cuh, and W's pattern with the largest rows of W and A_c (by_rows), or
+// the pair lists of W = A P and A_c = P^T W.
 struct Transfer {
     int n = 0, na = 0, bs = 3;
     int64_t nnz = 0;
-    DBuf<int32_t> ptr, col, t_ptr, t_row;
+    DBuf<int32_t> ptr, col, t_ptr, t_row, t_ent;
     DBuf<double> val;
     DBuf<double2> val32, t_val32;
+    bool by_rows = false;
+    DBuf<int32_t> w_ptr, w_col;
+    int most_w = 0, most_c = 0;
     PairList w, c;
 };
 
@@ -76,7 +80,8 @@ struct Transfer {
 bool build_transfer(const FineView& F, int na, const int32_t* agg, const double* Q, const double* dinv, double omega,
                     Transfer& t, DBuf<int32_t>& c_ptr, DBuf<int32_t>& c_cols, int64_t* ncb, DBuf<uint8_t>& tmp,
                     cudaStream_t s);
-// c_vals (36 per block) = P^T A P
-void galerkin_product(const FineView& F, const Transfer& t, double* c_vals, cudaStream_t s);
+// c_vals (36 per block of the pattern c_ptr, c_cols) = P^T A P
+void galerkin_product(const FineView& F, const Transfer& t, const int32_t* c_ptr, const int32_t* c_cols,
+                      double* c_vals, cudaStream_t s);
 
 }  // namespace fx

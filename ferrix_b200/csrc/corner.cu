@@ -338,13 +338,16 @@ void corner_weights(CornerLevel& c, const double* xyz, cudaStream_t s) {
     FX_LAUNCH(k_corner_xyz, grid_for(c.n), 256, 0, s, c.n, c.fine_of.ptr, xyz, c.xyz.ptr);
 }
 
+void allow_shared_corner() {
+    FX_CUDA_CHECK(cudaFuncSetAttribute(k_corner_elements, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kWarpsG * kSharedG));
+}
+
 void corner_matrix(CornerLevel& c, const ElemView& g4, const ElemView& g20, const double* ebuf, const BcView& bc,
                    const unsigned long long* maxdiag, cudaStream_t s) {
     const size_t v4 = (size_t)g4.n * kPairs4 * 9;
     c.ebuf.alloc(v4 + (size_t)g20.n * kPairs8 * 9 + 9, s);
     if (v4) FX_CUDA_CHECK(cudaMemcpyAsync(c.ebuf.ptr, ebuf, v4 * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    FX_CUDA_CHECK(cudaFuncSetAttribute(k_corner_elements, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kWarpsG * kSharedG));
     FX_LAUNCH(k_corner_elements, grid_for(g20.n, kWarpsG), 32 * kWarpsG, kWarpsG * kSharedG, s, g20.n, g20.conn,
               c.corner_of.ptr, c.par.ptr, c.wgt.ptr, ebuf + v4, c.ebuf.ptr + v4);
     c.vals.alloc((size_t)c.S.n_groups * 36, s);

@@ -121,6 +121,10 @@ inline int guarded(fx_ctx* ctx, F&& f) {
 
 namespace fx {
 
+// The kernels that take more than 48 KB of dynamic shared memory are allowed it; for each new context.
+void allow_shared_transfer();
+void allow_shared_corner();
+
 void ensure_dense(fx_model* m);
 // One kernel of each source file's module, and the loading of every kernel of
 // those modules on the current device (once per device and process): with lazy

@@ -137,3 +137,28 @@ def test_dense_planar_level(ctx, npe, cells, prec):
     u, stats = _solve(ctx, text, precision=prec)
     # FP64: 1e-10 as elsewhere; these slender columns leave up to 1e-9 at the mixed solver's residual
     assert float(np.linalg.norm(u - ref) / np.linalg.norm(ref)) <= (1e-10 if prec == fx.PREC_FP64 else 1e-8), stats
+
+
+@pytest.mark.parametrize("nodes", [0, 2])
+def test_hub_node(ctx, nodes):
+    """A ball of C3D4 elements around one node: with two nodes per aggregate, that node's row reaches more
+    aggregates than the row-wise products hold, which then go by sorted operand pairs."""
+    k = np.arange(1500)
+    z = 1.0 - (2.0 * k + 1.0) / len(k)
+    phi = k * np.pi * (3.0 - np.sqrt(5.0))
+    r = np.sqrt(1.0 - z * z)
+    sphere = np.stack([r * np.cos(phi), r * np.sin(phi), z], axis=1)
+    from scipy.spatial import ConvexHull
+    tri = ConvexHull(sphere).simplices
+    xyz = np.concatenate([[[0.0, 0.0, 0.0]], sphere])
+    conn = np.concatenate([np.zeros((len(tri), 1), dtype=np.int64), tri + 1], axis=1)
+    v = np.einsum("ij,ij->i", np.cross(xyz[conn[:, 1]], xyz[conn[:, 2]]), xyz[conn[:, 3]])
+    conn[v < 0, 1], conn[v < 0, 2] = conn[v < 0, 2].copy(), conn[v < 0, 1].copy()
+    lattice = np.ones((len(xyz), 3), dtype=np.int64)
+    lattice[xyz[:, 2] < -0.7] = 0  # clamped cap
+    lattice[xyz[:, 2] > 0.7] = 2   # loaded cap
+    mesh = decks.BoxMesh(xyz, conn, 4, lattice, (2, 2, 2), (2.0, 2.0, 2.0))
+    text = decks.write_deck(decks.DeckSpec(mesh, [(2.0e5, 0.3, None)], load_total=(100.0, 50.0, -200.0)))
+    ref = static_step.Runner(inp.parse_inp_text(text)).run().displacements
+    u, stats = _solve(ctx, text, precision=fx.PREC_FP64, amg_aggregate_nodes=nodes, amg_persistent_max_dof=-1)
+    assert float(np.linalg.norm(u - ref) / np.linalg.norm(ref)) <= 1e-10, stats
