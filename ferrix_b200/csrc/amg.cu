@@ -290,11 +290,11 @@ __global__ void __launch_bounds__(128) k_planar6(int n, const int32_t* __restric
 template <int BS>
 __global__ void __launch_bounds__(32 * kRestrictWarps)
     k_restrict(const int32_t* __restrict__ t_ptr, const int32_t* __restrict__ t_row, const double2* __restrict__ t_val,
-               const double* __restrict__ rf, double* __restrict__ bc, CoarseStart cs) {
+               const double* rf, double* __restrict__ bc, CoarseStart cs) {
     __shared__ double sh[kRestrictWarps][6];
     const int a = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double t[6];
-    restrict_agg<BS, false>(t_row, t_val, rf, t_ptr[a], t_ptr[a + 1], w, lane, t);
+    restrict_agg<BS, false>(t_row, t_val, rf, t_ptr[a], t_ptr[a + 1], w, lane, t, ChainWait());
     if (lane == 0)
 #pragma unroll
         for (int c = 0; c < 6; ++c) sh[w][c] = t[c];
@@ -333,7 +333,7 @@ constexpr int kProlongRows = BS == 3 ? 64 : 16;
 template <int BS>
 __global__ void __launch_bounds__(256) k_prolong(int n, const int32_t* __restrict__ p_ptr,
                                                  const int32_t* __restrict__ p_col, const double2* __restrict__ p_val,
-                                                 const double* __restrict__ xc, double* __restrict__ xf, double alpha,
+                                                 const double* xc, double* xf, double alpha,
                                                  float* __restrict__ x4, const float4* __restrict__ sq4) {
     constexpr int ST = BS | 1;  // odd stride: no bank conflicts
     __shared__ double sh[256 * ST];
@@ -347,16 +347,25 @@ __global__ void __launch_bounds__(256) k_prolong(int n, const int32_t* __restric
     if (own) {
         p0 = p_ptr[j];
         p1 = p_ptr[j + 1];
-        x0 = xf[k];
         if (BS == 3 && x4 && sq4) q = (double)reinterpret_cast<const float*>(sq4)[4 * (int64_t)j + c];
     }
+    double2 v[3 * BS];
+    int col = 0;
+    auto load = [&](int e) {
+        if (e >= e1) return;
+        col = __ldg(p_col + e);
+#pragma unroll
+        for (int u = 0; u < 3 * BS; ++u) v[u] = __ldg(p_val + p32<BS>(e, u));
+    };
+    load(e0 + (int)threadIdx.x);
+    chain_wait();
+    if (own) x0 = xf[k];
     for (int tile = e0; tile < e1; tile += 256) {  // CTA-uniform
         const int e = tile + (int)threadIdx.x;
+        if (tile > e0) load(e);
         if (e < e1) {
-            double2 v[3 * BS], w[3];
-#pragma unroll
-            for (int u = 0; u < 3 * BS; ++u) v[u] = __ldg(p_val + p32<BS>(e, u));
-            const double2* x = reinterpret_cast<const double2*>(xc + (int64_t)p_col[e] * 6);
+            double2 w[3];
+            const double2* x = reinterpret_cast<const double2*>(xc + (int64_t)col * 6);
 #pragma unroll
             for (int h = 0; h < 3; ++h) w[h] = x[h];
 #pragma unroll
@@ -367,9 +376,9 @@ __global__ void __launch_bounds__(256) k_prolong(int n, const int32_t* __restric
         __syncthreads();
     }
     if (!own) return;
-    const double v = x0 + alpha * t;
-    xf[k] = v;
-    if (BS == 3 && x4) x4[4 * (int64_t)j + c] = (float)(v * q);
+    const double xn = x0 + alpha * t;
+    xf[k] = xn;
+    if (BS == 3 && x4) x4[4 * (int64_t)j + c] = (float)(xn * q);
 }
 
 // ------------------------------------------------------------------ coarsest level
@@ -508,10 +517,9 @@ __global__ void __launch_bounds__(256) k_gj_first(int nd, const double* __restri
 // separate launches for the pivot inverse (16-18 us), panel rows (9), update (8) and panel
 // columns (4) instead: the NLGEOM beam of 16k DOF, with 85 inverses of 168 DOF, took 370 ms
 // against 355, the 14,883-DOF cantilever 9.44 against 9.15 ms from deck text.
-__global__ void __launch_bounds__(256) k_gj_panel(int nd, int k0, const double* __restrict__ A,
-                                                  double* __restrict__ B, const double* __restrict__ P,
-                                                  double* __restrict__ P_next, const double* __restrict__ diag,
-                                                  int* __restrict__ singular) {
+__global__ void __launch_bounds__(256) k_gj_panel(int nd, int k0, const double* A, double* __restrict__ B,
+                                                  const double* P, double* __restrict__ P_next,
+                                                  const double* __restrict__ diag, int* __restrict__ singular) {
     __shared__ __align__(16) double Ps[kPanel][kPanel + 2];     // P, zero outside the panel
     __shared__ double Rs[kPanel][kPanel];                       // A[K, j0 + c], then P A[K, j0 + c]
     __shared__ __align__(16) double Ls[kTileRows][kPanel + 2];  // A[i0 + r, K]
@@ -520,6 +528,7 @@ __global__ void __launch_bounds__(256) k_gj_panel(int nd, int k0, const double* 
     const int b = min(kPanel, nd - k0);
     const bool panel_col = j0 == k0;
     const int j = j0 + tx;
+    chain_wait();
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
         const int r = ty + 8 * u;
@@ -593,11 +602,10 @@ __global__ void __launch_bounds__(256) k_dense_zero_dead(int nd, double* __restr
         if (dead[r] || dead[c]) A[(int64_t)r * nd + c] = 0.0;
 }
 
-__global__ void k_dense_matvec(int nd, const double* __restrict__ A, const double* __restrict__ x,
-                               double* __restrict__ y) {
+__global__ void k_dense_matvec(int nd, const double* __restrict__ A, const double* x, double* __restrict__ y) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= nd) return;
-    const double t = dense_row_dot<false>(A + (int64_t)warp * nd, x, nd, lane);
+    const double t = dense_row_dot<false>(A + (int64_t)warp * nd, x, nd, lane, ChainWait());
     if (lane == 0) y[warp] = t;
 }
 
@@ -619,8 +627,8 @@ __global__ void k_dot_part(int64_t n, const double* __restrict__ a, const double
 }
 
 // partial sums of (b.z, b.zold) as a V-cycle's last smoothing step leaves them (zold null: 0)
-__global__ void __launch_bounds__(256) k_pair_part(int64_t n, const double* __restrict__ b, const double* __restrict__ z,
-                                                   const double* __restrict__ zold, double* __restrict__ part);
+__global__ void __launch_bounds__(256) k_pair_part(int64_t n, const double* b, const double* z,
+                                                   const double* zold, double* __restrict__ part);
 
 // |a|^2 and |b|^2 in two launches (fixed order): partials of a in part[0 .. nb), of b in part[nb .. 2 nb)
 __global__ void __launch_bounds__(256) k_norm2_part(int64_t n, const double* __restrict__ a,
@@ -692,7 +700,7 @@ __global__ void k_fin(int nb, const double* __restrict__ part, double* __restric
 
 // Sum of n partial sums (entries of `stride` doubles; minus the second double of each with diff), in
 // every thread of a CTA of 256.
-__device__ __forceinline__ double cta_total(const double* __restrict__ part, int n, int stride, bool diff) {
+__device__ __forceinline__ double cta_total(const double* part, int n, int stride, bool diff) {
     __shared__ double s_tot[8];
     double t = 0.0;
     for (int k = threadIdx.x; k < n; k += 256)
@@ -729,9 +737,9 @@ __global__ void k_rdr_part(int n, const double* __restrict__ r, const double* __
 
 // p = z + beta p with beta = (r.z - r.z_old) / r.z_prev from the V-cycle's partial sums (pairs; z_old only
 // in the flexible CG), r.z into S[8] and r.D^-1 r from the update's partial sums into S[2]
-__global__ void __launch_bounds__(256) k_xpby(int64_t n, const double* __restrict__ z, double* __restrict__ S,
-                                              const double* __restrict__ rz_part, int n_rz, bool flexible,
-                                              const double* __restrict__ rd_part, int n_rd, double* __restrict__ p) {
+__global__ void __launch_bounds__(256) k_xpby(int64_t n, const double* z, double* S, const double* rz_part, int n_rz,
+                                              bool flexible, const double* rd_part, int n_rd, double* p) {
+    chain_wait();
     const double prev = S[0];  // (S[0] is moved on by the next update only)
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const double zv = i < n ? z[i] : 0.0, pv = i < n ? p[i] : 0.0;
@@ -844,8 +852,9 @@ __device__ __forceinline__ void cta_partials(double v, double v2, bool two, doub
     }
 }
 
-__global__ void __launch_bounds__(256) k_pair_part(int64_t n, const double* __restrict__ b, const double* __restrict__ z,
-                                                   const double* __restrict__ zold, double* __restrict__ part) {
+__global__ void __launch_bounds__(256) k_pair_part(int64_t n, const double* b, const double* z,
+                                                   const double* zold, double* __restrict__ part) {
+    chain_wait();
     double t = 0.0, u = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
         t += b[i] * z[i];
@@ -955,8 +964,9 @@ __global__ void __launch_bounds__(256, std::is_same<VT, __half>::value ? kL0MinB
     const int rows_per_grid = (gridDim.x * blockDim.x) >> kL0LaneShift;
     // uniform trip count per warp: the warp's rows share one base
     const int nb = ((o.n + kL0RowsPerWarp - 1) / kL0RowsPerWarp) * kL0RowsPerWarp;
-    const double* __restrict__ v = o.v;
+    const double* v = o.v;
     double dsum = 0.0, dsum2 = 0.0;
+    chain_wait();
     for (int base = row0 - (row0 & (kL0RowsPerWarp - 1)); base < nb; base += rows_per_grid) {
         const int row = base + (row0 & (kL0RowsPerWarp - 1));
         const bool valid = row < o.n;
@@ -971,7 +981,7 @@ __global__ void __launch_bounds__(256, std::is_same<VT, __half>::value ? kL0MinB
         float2 hsc = make_float2(1.f, 1.f);  // {2^k, 2^-k}: .x is read where the direction is stored
         auto load_epi = [&]() {
         if (H && epi) sqi = __ldg(o.sq4 + row);
-        if (kH16g && epi && o.hs) hsc.y = __ldg(o.hs + 1);
+        if (kH16g && epi && o.hs) hsc.y = o.hs[1];
         if (epi) {
             if (MODE == kL0Cheb0 || MODE == kL0ChebK) {
                 const double* src = MODE == kL0Cheb0 ? o.b : o.r;
@@ -1028,13 +1038,13 @@ __global__ void __launch_bounds__(256, std::is_same<VT, __half>::value ? kL0MinB
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     if constexpr (kH16g) {
-                        const uint2 u = __ldg(reinterpret_cast<const uint2*>(o.v4) + cj[q]);
+                        const uint2 u = reinterpret_cast<const uint2*>(o.v4)[cj[q]];
                         const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
                         xv[q][0] = a.x;
                         xv[q][1] = a.y;
                         xv[q][2] = __half2float(__ushort_as_half((unsigned short)(u.y & 0xffffu)));
                     } else {
-                        const float4 t = __ldg(o.v4 + cj[q]);
+                        const float4 t = o.v4[cj[q]];
                         xv[q][0] = t.x;
                         xv[q][1] = t.y;
                         xv[q][2] = t.z;
@@ -1044,7 +1054,7 @@ __global__ void __launch_bounds__(256, std::is_same<VT, __half>::value ? kL0MinB
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
 #pragma unroll
-                    for (int k = 0; k < 3; ++k) xv[q][k] = (GT)__ldg(v + 3 * (int64_t)cj[q] + k);
+                    for (int k = 0; k < 3; ++k) xv[q][k] = (GT)v[3 * (int64_t)cj[q] + k];
             }
             const VT* vb = o.vals + ((int64_t)g0 * 9 + g) * 4;
             const int64_t pl = (int64_t)ng * 4;
@@ -1101,7 +1111,7 @@ __global__ void __launch_bounds__(256, std::is_same<VT, __half>::value ? kL0MinB
             o.r[o3 + c] = c == 0 ? rr[0] : (c == 1 ? rr[1] : rr[2]);
             const double dn = (MODE == kL0Cheb0 ? 0.0 : o.c1 * vc) + o.c2 * z;
             if (kH16) {
-                if (o.hs) hsc.x = __ldg(o.hs);
+                if (o.hs) hsc.x = o.hs[0];
                 reinterpret_cast<unsigned short*>(o.d4_out)[4 * (int64_t)row + c] = (unsigned short)h16_bits(
                     (float)(dn * (double)(c == 0 ? sqi.x : (c == 1 ? sqi.y : sqi.z))) * hsc.x);
             } else if (G32) o.d4_out[4 * (int64_t)row + c] = (float)(H ? dn * (double)(c == 0 ? sqi.x : (c == 1 ? sqi.y : sqi.z)) : dn);
@@ -1193,16 +1203,12 @@ constexpr int kLnThreads = FX_LN_THREADS;
 // registers, enough for a lane's whole 6x6 block and its gathered 6-vector in flight
 // without spills. On the 417k-DOF box a default solve took 51.9-52.4 ms with 4, against
 // 52.9-53.2 with 6 (80 registers), 52.5-53.2 with 7 (72, spilling) and 52.3-52.5 with 8
-// (64, the epilogue operands loaded after the row sums, FX_LN_LATE_EPI).
+// (64). The epilogue's operands are loaded after the row sums: before them, behind the wait for
+// the kernel ahead, two of the modes spilled, at the same time per solve.
 #ifndef FX_LN_MIN_BLOCKS
 #define FX_LN_MIN_BLOCKS 4
 #endif
 constexpr int kLnMinBlocks = FX_LN_MIN_BLOCKS;
-#ifndef FX_LN_LATE_EPI
-#define FX_LN_LATE_EPI 0
-#endif
-constexpr bool kLnLateEpi = FX_LN_LATE_EPI != 0;  // epilogue operands loaded after the row sums
-
 struct LnOp {
     int n;
     const int32_t* row_ptr;
@@ -1226,7 +1232,11 @@ __global__ void __launch_bounds__(kLnThreads, kLnMinBlocks) k_ln_op(LnOp o) {
     const int c = lane < 6 ? lane : 0;
     const bool epi = lane < 6;
     double src6[6] = {0, 0, 0, 0, 0, 0}, Dr[6] = {0, 0, 0, 0, 0, 0}, vc = 0.0, xoc = 0.0, bc = 0.0;
-    auto load_epi = [&]() {  // row-local operands of the epilogue
+    // lanes over the row's blocks; every lane ends with the six row sums
+    const int b0 = o.row_ptr[row];
+    double acc[6];
+    coarse_row6<false>(o.cols, o.vals, o.v, b0, o.row_ptr[row + 1] - b0, lane, acc, ChainWait());
+    // row-local operands of the epilogue
     if (epi) {
         if (MODE == kL0Cheb0 || MODE == kL0ChebK) {
             const double* src = MODE == kL0Cheb0 ? o.b : o.r;
@@ -1246,13 +1256,6 @@ __global__ void __launch_bounds__(kLnThreads, kLnMinBlocks) k_ln_op(LnOp o) {
             src6[0] = o.r[o6 + c];
         }
     }
-    };
-    if (!kLnLateEpi) load_epi();
-    // lanes over the row's blocks; every lane ends with the six row sums
-    const int b0 = o.row_ptr[row];
-    double acc[6];
-    coarse_row6<false>(o.cols, o.vals, o.v, b0, o.row_ptr[row + 1] - b0, lane, acc);
-    if (kLnLateEpi) load_epi();
     double axc = acc[0];
 #pragma unroll
     for (int r = 1; r < 6; ++r)
@@ -1364,15 +1367,15 @@ __global__ void k_l0_cheb_start(int n, const double* __restrict__ dinv, const do
 // b = P^T r of the corner level (a group of lanes per corner) fused with the level's first
 // pre-smoothing step from x = 0, as k_l0_cheb_start (hs: the V-cycle's scale of FP16 directions,
 // already published)
-__global__ void __launch_bounds__(256) k_corner_restrict(CornerView V, const double* __restrict__ rf,
+__global__ void __launch_bounds__(256) k_corner_restrict(CornerView V, const double* rf,
                                                          double* __restrict__ b, const double* __restrict__ dinv,
                                                          double* __restrict__ r, double* __restrict__ x,
                                                          double* __restrict__ d, float4* __restrict__ d4, double c2,
                                                          const float4* __restrict__ sq4,
-                                                         const float* __restrict__ hs) {
+                                                         const float* hs) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / kCornerLanes, sub = t % kCornerLanes;
     double v[3];
-    corner_restrict_row<false>(V, rf, i < V.n ? i : -1, sub, v);
+    corner_restrict_row<false>(V, rf, i < V.n ? i : -1, sub, v, ChainWait());
     if (i >= V.n || sub != 0) return;
     const int64_t o3 = 3 * (int64_t)i;
     const double* D = dinv + 9 * (int64_t)i;
@@ -1390,13 +1393,13 @@ __global__ void __launch_bounds__(256) k_corner_restrict(CornerView V, const dou
 }
 
 // x += alpha P x_c from the corner level, and the FP32 copy of x for the smoother's gathers
-__global__ void __launch_bounds__(256) k_corner_prolong(CornerView V, const double* __restrict__ xc,
-                                                        double* __restrict__ xf, double alpha,
+__global__ void __launch_bounds__(256) k_corner_prolong(CornerView V, const double* xc,
+                                                        double* xf, double alpha,
                                                         float4* __restrict__ x4, const float4* __restrict__ sq4) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= V.n_fine) return;
     double u[3];
-    corner_prolong_node<false>(V, xc, j, u);
+    corner_prolong_node<false>(V, xc, j, u, ChainWait());
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         u[k] = xf[3 * (int64_t)j + k] + alpha * u[k];
@@ -1411,10 +1414,10 @@ __global__ void __launch_bounds__(256) k_corner_prolong(CornerView V, const doub
 // hs != null (FP16 directions): the V-cycle's scale comes from S[2], the previous residual's
 // r.D^-1 r (the new one is summed later), and is published in hs for the V-cycle's later launches.
 // A thread per node, the node's operands loaded before the sum of the partials.
-__global__ void __launch_bounds__(256) k_amg_update_start(int n, double* __restrict__ S,
-                                                          const double* __restrict__ pq_part, int n_pq,
-                                                          const double* __restrict__ p, const double* __restrict__ q,
-                                                          double* __restrict__ x, double* __restrict__ r,
+__global__ void __launch_bounds__(256) k_amg_update_start(int n, double* S,
+                                                          const double* pq_part, int n_pq,
+                                                          const double* p, const double* q,
+                                                          double* x, double* r,
                                                           const double* __restrict__ dinv, double* __restrict__ part,
                                                           double* __restrict__ r0, double* __restrict__ x0,
                                                           double* __restrict__ d0, float4* __restrict__ d4,
@@ -1424,6 +1427,10 @@ __global__ void __launch_bounds__(256) k_amg_update_start(int n, double* __restr
     const bool own = i < n;
     const int64_t o3 = 3 * (int64_t)i;
     double pv[3], qv[3], xv[3], rv[3], D[9];
+    if (own)
+#pragma unroll
+        for (int c = 0; c < 9; ++c) D[c] = dinv[9 * (int64_t)i + c];
+    chain_wait();
     if (own) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -1432,8 +1439,6 @@ __global__ void __launch_bounds__(256) k_amg_update_start(int n, double* __restr
             xv[c] = x[o3 + c];
             rv[c] = r[o3 + c];
         }
-#pragma unroll
-        for (int c = 0; c < 9; ++c) D[c] = dinv[9 * (int64_t)i + c];
     }
     const double rz = S[8];
     const float2 hsc = hs ? h16_scale(S[2]) : make_float2(1.0f, 1.0f);
@@ -1715,7 +1720,7 @@ void Amg::coarsest_inverse(AmgLevel& l, cudaStream_t s) {
     FX_LAUNCH(k_gj_first, 1, 256, 0, s, (int)nd, l.dense_inv.ptr, diag0.ptr, singular.ptr, P[0]);
     const dim3 tiles(grid_for(nd, kPanel), grid_for(nd, kTileRows));
     for (int k0 = 0; k0 < (int)nd; k0 += kPanel) {
-        FX_LAUNCH(k_gj_panel, tiles, 256, 0, s, (int)nd, k0, l.dense_inv.ptr, other.ptr, P[0], P[1], diag0.ptr,
+        FX_LAUNCH_CHAIN(k_gj_panel, tiles, 256, 0, s, (int)nd, k0, l.dense_inv.ptr, other.ptr, P[0], P[1], diag0.ptr,
                   singular.ptr);
         l.dense_inv.swap(other);
         std::swap(P[0], P[1]);
@@ -2033,7 +2038,7 @@ void Amg::cycle(int lev, const double* b, double* x, cudaStream_t s, bool starte
     AmgLevel& l = L[lev];
     const int64_t nd = (int64_t)l.n * l.bs;
     if (l.coarsest) {
-        FX_LAUNCH(k_dense_matvec, grid_for(nd * 32, kLnThreads), kLnThreads, 0, s, (int)nd, l.dense_inv.ptr, b, x);
+        FX_LAUNCH_CHAIN(k_dense_matvec, grid_for(nd * 32, kLnThreads), kLnThreads, 0, s, (int)nd, l.dense_inv.ptr, b, x);
         return;
     }
     AmgLevel& c = L[lev + 1];
@@ -2056,19 +2061,19 @@ void Amg::cycle(int lev, const double* b, double* x, cudaStream_t s, bool starte
         o.xo = xs;
         o.c1 = k.c1[st];
         o.c2 = k.c2[st];
-        FX_LAUNCH(k_ln_op<kL0ChebK>, grid, kLnThreads, 0, s, o);
+        FX_LAUNCH_CHAIN(k_ln_op<kL0ChebK>, grid, kLnThreads, 0, s, o);
         std::swap(dA, dB);
     }
     {
         LnOp o = ln_op(l);
         o.v = dA;
         o.r = l.r.ptr;
-        FX_LAUNCH(k_ln_op<kL0RUpd>, grid, kLnThreads, 0, s, o);  // r = b - A xs
+        FX_LAUNCH_CHAIN(k_ln_op<kL0RUpd>, grid, kLnThreads, 0, s, o);  // r = b - A xs
     }
-    FX_LAUNCH(k_restrict<6>, (unsigned)l.tr.na, 32 * kRestrictWarps, 0, s, l.tr.t_ptr.ptr, l.tr.t_row.ptr,
+    FX_LAUNCH_CHAIN(k_restrict<6>, (unsigned)l.tr.na, 32 * kRestrictWarps, 0, s, l.tr.t_ptr.ptr, l.tr.t_row.ptr,
               l.tr.t_val32.ptr, l.r.ptr, c.b.ptr, coarse_start(lev + 1));
     coarse(lev + 1, s);
-    FX_LAUNCH(k_prolong<6>, grid_for(l.n, kProlongRows<6>), 256, 0, s, l.n, l.tr.ptr.ptr, l.tr.col.ptr,
+    FX_LAUNCH_CHAIN(k_prolong<6>, grid_for(l.n, kProlongRows<6>), 256, 0, s, l.n, l.tr.ptr.ptr, l.tr.col.ptr,
               l.tr.val32.ptr, c.x.ptr, xs,
               alpha_ * l.pscale, nullptr, nullptr);
     {
@@ -2079,7 +2084,7 @@ void Amg::cycle(int lev, const double* b, double* x, cudaStream_t s, bool starte
         o.d_out = dA;
         o.xo = x;
         o.c2 = k.c2_start;
-        FX_LAUNCH(k_ln_op<kL0Cheb0>, grid, kLnThreads, 0, s, o);
+        FX_LAUNCH_CHAIN(k_ln_op<kL0Cheb0>, grid, kLnThreads, 0, s, o);
     }
     for (int st = 1; st < degree_; ++st) {
         LnOp o = ln_op(l);
@@ -2089,7 +2094,7 @@ void Amg::cycle(int lev, const double* b, double* x, cudaStream_t s, bool starte
         o.xo = x;
         o.c1 = k.c1[st];
         o.c2 = k.c2[st];
-        FX_LAUNCH(k_ln_op<kL0ChebK>, grid, kLnThreads, 0, s, o);
+        FX_LAUNCH_CHAIN(k_ln_op<kL0ChebK>, grid, kLnThreads, 0, s, o);
         std::swap(dA, dB);
     }
 }
@@ -2122,10 +2127,10 @@ void Amg::first_coarse(cudaStream_t s) {
         launch_coarse_grid(desc_.ptr, gbar_.ptr, gflag_, g32, degree_, alpha_, s);
         return;
     }
-    FX_LAUNCH(k_restrict<3>, (unsigned)l.tr.na, 32 * kRestrictWarps, 0, s, l.tr.t_ptr.ptr, l.tr.t_row.ptr,
+    FX_LAUNCH_CHAIN(k_restrict<3>, (unsigned)l.tr.na, 32 * kRestrictWarps, 0, s, l.tr.t_ptr.ptr, l.tr.t_row.ptr,
               l.tr.t_val32.ptr, l.r.ptr, c.b.ptr, coarse_start(planar_));
     coarse(planar_, s);
-    FX_LAUNCH(k_prolong<3>, grid_for(l.n, kProlongRows<3>), 256, 0, s, l.n, l.tr.ptr.ptr, l.tr.col.ptr,
+    FX_LAUNCH_CHAIN(k_prolong<3>, grid_for(l.n, kProlongRows<3>), 256, 0, s, l.n, l.tr.ptr.ptr, l.tr.col.ptr,
               l.tr.val32.ptr, c.x.ptr, l.x.ptr, alpha_ * l.pscale, g32 ? l.x4.ptr : nullptr, l.sq4);
 }
 
@@ -2139,8 +2144,8 @@ void Amg::vcycle(int m, const double* b, double* z, double* part, const double* 
     AmgLevel& l = L[m];
     if (l.coarsest) {  // z = A^-1 b
         const int64_t nd = 3 * (int64_t)l.n;
-        FX_LAUNCH(k_dense_matvec, grid_for(nd * 32, kLnThreads), kLnThreads, 0, s, (int)nd, l.dense_inv.ptr, b, z);
-        if (part) FX_LAUNCH(k_pair_part, apply_grid(), 256, 0, s, nd, b, z, zold, part);
+        FX_LAUNCH_CHAIN(k_dense_matvec, grid_for(nd * 32, kLnThreads), kLnThreads, 0, s, (int)nd, l.dense_inv.ptr, b, z);
+        if (part) FX_LAUNCH_CHAIN(k_pair_part, apply_grid(), 256, 0, s, nd, b, z, zold, part);
         return;
     }
     const VT* vals;
@@ -2177,7 +2182,7 @@ void Amg::vcycle(int m, const double* b, double* z, double* part, const double* 
         o.xo = l.x.ptr;
         o.c1 = k.c1[st];
         o.c2 = k.c2[st];
-        FX_LAUNCH((k_l0_op<VT, kL0ChebK, g32>), grid, 256, 0, s, o);
+        FX_LAUNCH_CHAIN((k_l0_op<VT, kL0ChebK, g32>), grid, 256, 0, s, o);
         std::swap(dA, dB);
         std::swap(dA4, dB4);
     }
@@ -2186,15 +2191,15 @@ void Amg::vcycle(int m, const double* b, double* z, double* part, const double* 
         o.v = dA;
         o.v4 = dA4;
         o.r = l.r.ptr;
-        FX_LAUNCH((k_l0_op<VT, kL0RUpd, g32>), grid, 256, 0, s, o);  // r = b - A x
+        FX_LAUNCH_CHAIN((k_l0_op<VT, kL0RUpd, g32>), grid, 256, 0, s, o);  // r = b - A x
     }
     if (l.corner_next) {
         AmgLevel& c = L[m + 1];
         const Start0 c0 = start_of(c);
-        FX_LAUNCH(k_corner_restrict, grid_for((int64_t)c.n * kCornerLanes), 256, 0, s, corner_, l.r.ptr, c.b.ptr,
+        FX_LAUNCH_CHAIN(k_corner_restrict, grid_for((int64_t)c.n * kCornerLanes), 256, 0, s, corner_, l.r.ptr, c.b.ptr,
                   c.dinv0, c0.r, c0.x, c0.d, c0.d4, c0.c2, c0.sq4, c0.hs);
         vcycle<VT>(m + 1, c.b.ptr, c.xs.ptr, nullptr, nullptr, s, true);
-        FX_LAUNCH(k_corner_prolong, grid_for(l.n), 256, 0, s, corner_, c.result(), l.x.ptr, alpha_ * l.pscale,
+        FX_LAUNCH_CHAIN(k_corner_prolong, grid_for(l.n), 256, 0, s, corner_, c.result(), l.x.ptr, alpha_ * l.pscale,
                   g32 ? x4 : nullptr, l.sq4);
     } else {
         first_coarse(s);
@@ -2225,9 +2230,9 @@ void Amg::vcycle(int m, const double* b, double* z, double* part, const double* 
             o.zold = zold;
             o.part = part;
         }
-        if (st == 0) FX_LAUNCH((k_l0_op<VT, kL0Cheb0, g32>), grid, 256, 0, s, o);
+        if (st == 0) FX_LAUNCH_CHAIN((k_l0_op<VT, kL0Cheb0, g32>), grid, 256, 0, s, o);
         else {
-            FX_LAUNCH((k_l0_op<VT, kL0ChebK, g32>), grid, 256, 0, s, o);
+            FX_LAUNCH_CHAIN((k_l0_op<VT, kL0ChebK, g32>), grid, 256, 0, s, o);
             std::swap(dA, dB);
             std::swap(dA4, dB4);
         }
@@ -2571,12 +2576,12 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
         o.y = q_.ptr;
         o.dot = 1;
         o.part = part_.ptr;
-        FX_LAUNCH((k_l0_op<double, kL0Apply>), g0, 256, 0, s, o);  // q = A p, p.q
+        FX_LAUNCH_CHAIN((k_l0_op<double, kL0Apply>), g0, 256, 0, s, o);  // q = A p, p.q
         const Amg::Start0 s0 = amg.start0();
-        FX_LAUNCH(k_amg_update_start, gu, 256, 0, s, n, sc_.ptr, part_.ptr, (int)g0, p_.ptr, q_.ptr, x, r_.ptr, dinv64,
+        FX_LAUNCH_CHAIN(k_amg_update_start, gu, 256, 0, s, n, sc_.ptr, part_.ptr, (int)g0, p_.ptr, q_.ptr, x, r_.ptr, dinv64,
                   rd_part_.ptr, s0.r, s0.x, s0.d, s0.d4, s0.c2, s0.sq4, s0.hs);  // x, r; the V-cycle's first step
         amg.apply(r_.ptr, zn, part_.ptr, amg.kcycle() ? zo : nullptr, s, true);  // z, r.z
-        FX_LAUNCH(k_xpby, gx, 256, 0, s, nd, zn, sc_.ptr, part_.ptr, (int)gz, amg.kcycle(), rd_part_.ptr, (int)gu,
+        FX_LAUNCH_CHAIN(k_xpby, gx, 256, 0, s, nd, zn, sc_.ptr, part_.ptr, (int)gz, amg.kcycle(), rd_part_.ptr, (int)gu,
                   p_.ptr);
     };
     // Two iterations per graph (z alternates). Between host checks as many replays are queued as the

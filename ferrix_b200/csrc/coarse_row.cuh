@@ -13,6 +13,8 @@
 
 #include <cstdint>
 
+#include "device.cuh"
+
 namespace fx {
 
 // Loads of the source vector: through L2 only (CG = true) when other CTAs of the
@@ -27,9 +29,12 @@ __device__ __forceinline__ double2 coarse_ld2(const double* p) {
 // every lane of the warp. The lane's blocks are summed in block order; the lanes' sums
 // are added by xor shuffles over 16, 8, 4, 2, 1 (both partners add the same two values,
 // so all lanes hold identical bits).
-template <bool CG>
+// wait: called in every lane before v is read, with the first block's values in flight.
+template <bool CG, typename Wait = NoWait>
 __device__ __forceinline__ void coarse_row6(const int32_t* __restrict__ cols, const double2* __restrict__ vals,
-                                            const double* v, int b0, int nblk, int lane, double (&acc)[6]) {
+                                            const double* v, int b0, int nblk, int lane, double (&acc)[6],
+                                            Wait wait = Wait()) {
+    if (lane >= nblk) wait();
 #pragma unroll
     for (int r = 0; r < 6; ++r) acc[r] = 0.0;
     for (int j = lane; j < nblk; j += 32) {
@@ -39,6 +44,7 @@ __device__ __forceinline__ void coarse_row6(const int32_t* __restrict__ cols, co
         double2 m[18];
 #pragma unroll
         for (int k = 0; k < 18; ++k) m[k] = __ldg(a + (int64_t)k * nblk);
+        if (j == lane) wait();
         const double* xs = v + 6 * (int64_t)col;
         const double2 x0 = coarse_ld2<CG>(xs), x1 = coarse_ld2<CG>(xs + 2), x2 = coarse_ld2<CG>(xs + 4);
 #pragma unroll
@@ -56,16 +62,24 @@ __device__ __forceinline__ void coarse_row6(const int32_t* __restrict__ cols, co
 // A[c] x[c] for c = l, l + 32, ... in that order (8 columns' loads in flight before their
 // products), then the lanes' sums by an xor tree. Shared by the per-step and the
 // persistent / cooperative coarse kernels.
-template <bool CG>
-__device__ __forceinline__ double dense_row_dot(const double* __restrict__ a, const double* x, int nd, int lane) {
+// wait: called in every lane before x is read, with the first columns' loads in flight.
+template <bool CG, typename Wait = NoWait>
+__device__ __forceinline__ double dense_row_dot(const double* __restrict__ a, const double* x, int nd, int lane,
+                                                Wait wait = Wait()) {
     constexpr int U = 8;
     double t = 0.0;
+    if (lane >= nd) wait();
     for (int c0 = lane; c0 < nd; c0 += 32 * U) {
         double av[U], xv[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int c = c0 + 32 * u;
             av[u] = c < nd ? __ldg(a + c) : 0.0;
+        }
+        if (c0 == lane) wait();
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + 32 * u;
             xv[u] = c < nd ? (CG ? __ldcg(x + c) : x[c]) : 0.0;
         }
 #pragma unroll

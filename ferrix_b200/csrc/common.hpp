@@ -67,6 +67,33 @@ extern thread_local int64_t* g_launch_counter;
         if (::fx::debug_sync()) ::fx::stream_wait((stream), #kernel, 20.0);                          \
     } while (0)
 
+// A launch that may begin before the kernel ahead of it in the stream has ended (programmatic dependent
+// launch): its CTAs become resident when that kernel's have left, without waiting for its writes to be
+// flushed, and wait for those in chain_wait() (device.cuh).
+#define FX_LAUNCH_CHAIN(kernel, grid, block, smem, stream, ...)                                      \
+    do {                                                                                             \
+        ::fx::launch_chain((kernel), (grid), (block), (smem), (stream), __VA_ARGS__);                \
+        if (::fx::g_launch_counter) ++*::fx::g_launch_counter;                                       \
+        if (::fx::debug_sync()) ::fx::stream_wait((stream), #kernel, 20.0);                          \
+    } while (0)
+
+#ifdef __CUDACC__
+template <typename... P, typename... A>
+inline void launch_chain(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    FX_CUDA_CHECK(cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...));
+}
+#endif
+
 // Stream-ordered device buffer (cudaMallocAsync / cudaFreeAsync).
 template <typename T>
 struct DBuf {

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "corner.hpp"
+#include "device.cuh"
 
 namespace fx {
 
@@ -20,18 +21,19 @@ constexpr int kCornerLanes = 8;  // lanes per corner of the restriction: one rou
 
 // (P^T r) of corner i by a group of kCornerLanes lanes (sub: lane within it), the lanes' sums
 // added by an xor tree; every lane of the warp takes part, with i < 0 for a group without a corner.
-template <bool CG>
+// wait: called in every lane before r is read, with the list's ends and the corner's node at hand.
+template <bool CG, typename Wait = NoWait>
 __device__ __forceinline__ void corner_restrict_row(const CornerView& V, const double* r, int i, int sub,
-                                                    double (&t)[3]) {
+                                                    double (&t)[3], Wait wait = Wait()) {
     auto ld = [&](int64_t k) { return CG ? __ldcg(r + k) : r[k]; };
     t[0] = t[1] = t[2] = 0.0;
+    const int e0 = i >= 0 ? __ldg(V.ch_ptr + i) : 0, e1 = i >= 0 ? __ldg(V.ch_ptr + i + 1) : 0;
+    const int64_t o = i >= 0 && sub == 0 ? 3 * (int64_t)__ldg(V.fine_of + i) : 0;
+    wait();
     if (i >= 0) {
-        if (sub == 0) {
-            const int64_t o = 3 * (int64_t)__ldg(V.fine_of + i);
+        if (sub == 0)
             for (int k = 0; k < 3; ++k) t[k] = ld(o + k);
-        }
-        const int e1 = __ldg(V.ch_ptr + i + 1);
-        for (int e = __ldg(V.ch_ptr + i) + sub; e < e1; e += kCornerLanes) {
+        for (int e = e0 + sub; e < e1; e += kCornerLanes) {
             const int item = __ldg(V.ch + e), node = item >> 1;
             const MidWeight w = mid_weight(V.wgt, node);
             const double r0 = ld(3 * (int64_t)node), r1 = ld(3 * (int64_t)node + 1), r2 = ld(3 * (int64_t)node + 2);
@@ -49,11 +51,14 @@ __device__ __forceinline__ void corner_restrict_row(const CornerView& V, const d
 }
 
 // (P x_c) of fine node j
-template <bool CG>
-__device__ __forceinline__ void corner_prolong_node(const CornerView& V, const double* xc, int j, double (&u)[3]) {
+// wait: called before xc is read, with the node's parents at hand.
+template <bool CG, typename Wait = NoWait>
+__device__ __forceinline__ void corner_prolong_node(const CornerView& V, const double* xc, int j, double (&u)[3],
+                                                    Wait wait = Wait()) {
     auto ld = [&](int64_t k) { return CG ? __ldcg(xc + k) : xc[k]; };
     const int i = __ldg(V.corner_of + j);
     const int2 p = __ldg(V.par + j);
+    wait();
     u[0] = u[1] = u[2] = 0.0;
     if (i >= 0) {
         for (int k = 0; k < 3; ++k) u[k] = ld(3 * (int64_t)i + k);

@@ -83,6 +83,20 @@ __device__ __forceinline__ T inv3(const T J[9], T Ji[9]) {
     return det;
 }
 
+// In a kernel launched by FX_LAUNCH_CHAIN: waits for the end of all kernels ahead of it in the stream and
+// for their writes. What those write is read after this call, by ordinary loads (no __ldg, no
+// const __restrict__); before it only what was there before the last launch that was not chained
+// (a chain's matrices, transfers and index lists). The kernels do not let the next one start early
+// (cudaTriggerProgrammaticLaunchCompletion): CTAs that wait while the kernel ahead still works made a
+// 16k-DOF Newton solve's 2,774 iterations 131 ms, 117 without, 123 with ordinary launches.
+__device__ __forceinline__ void chain_wait() { cudaGridDependencySynchronize(); }
+struct ChainWait {
+    __device__ __forceinline__ void operator()() const { chain_wait(); }
+};
+struct NoWait {
+    __device__ __forceinline__ void operator()() const {}
+};
+
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

@@ -34,16 +34,21 @@ __host__ __device__ constexpr int64_t p32_size(int64_t n) {  // pairs
 // cooperative kernels run them one after another in one warp.
 // CG: r is written by other CTAs of the same launch (read through L2).
 constexpr int kRestrictWarps = 4;
-template <int BS, bool CG>
+// wait: called in every lane before r is read, with the first entry's loads in flight.
+template <int BS, bool CG, typename Wait = NoWait>
 __device__ __forceinline__ void restrict_agg(const int32_t* __restrict__ t_row, const double2* __restrict__ t_val,
-                                             const double* r, int p0, int p1, int v, int lane, double (&t)[6]) {
+                                             const double* r, int p0, int p1, int v, int lane, double (&t)[6],
+                                             Wait wait = Wait()) {
+    const int first = p0 + 32 * v + lane;
+    if (first >= p1) wait();
 #pragma unroll
     for (int c = 0; c < 6; ++c) t[c] = 0.0;
-    for (int p = p0 + 32 * v + lane; p < p1; p += 32 * kRestrictWarps) {
+    for (int p = first; p < p1; p += 32 * kRestrictWarps) {
         const double* rr = r + (int64_t)BS * __ldg(t_row + p);
         double2 w[3 * BS];
 #pragma unroll
         for (int q = 0; q < 3 * BS; ++q) w[q] = __ldg(t_val + p32<BS>(p, q));
+        if (p == first) wait();
         double rv[BS];
 #pragma unroll
         for (int k = 0; k < BS; ++k) rv[k] = CG ? __ldcg(rr + k) : rr[k];

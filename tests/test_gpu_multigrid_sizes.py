@@ -162,3 +162,22 @@ def test_hub_node(ctx, nodes):
     ref = static_step.Runner(inp.parse_inp_text(text)).run().displacements
     u, stats = _solve(ctx, text, precision=fx.PREC_FP64, amg_aggregate_nodes=nodes, amg_persistent_max_dof=-1)
     assert float(np.linalg.norm(u - ref) / np.linalg.norm(ref)) <= 1e-10, stats
+
+
+@pytest.mark.parametrize("prec", [fx.PREC_FP64, fx.PREC_MIXED])
+@pytest.mark.parametrize("cycle", [0, 1])
+@pytest.mark.parametrize("npe,cells,nodes", [(4, (4, 5, 9), 0), (4, (6, 6, 14), 4), (4, (6, 6, 14), 40),
+                                             (20, (2, 2, 6), 0), (20, (5, 5, 12), 4)])
+def test_chained_launches(ctx, npe, cells, nodes, cycle, prec):
+    """Each kernel of the iteration may begin before the one ahead has ended: replayed from graphs and
+    launched one by one, with one, two and more levels under the cycle, the solve gives the same bits."""
+    spec = decks.c3d20_box_spec(*cells, lengths=tuple(float(c) for c in cells))
+    if npe == 4:
+        spec.mesh = decks.tet_box(*cells, *(float(c) for c in cells))
+    text = decks.write_deck(spec)
+    ref = static_step.Runner(inp.parse_inp_text(text)).run().displacements
+    runs = [_solve(ctx, text, precision=prec, amg_cycle=cycle, amg_aggregate_nodes=nodes, use_graphs=g,
+                   amg_persistent_max_dof=-1) for g in (1, 0, 1, 1)]
+    for u, stats in runs:
+        assert np.array_equal(u, runs[0][0]) and stats["pcg_iterations"] == runs[0][1]["pcg_iterations"]
+        assert float(np.linalg.norm(u - ref) / np.linalg.norm(ref)) <= (1e-10 if prec == fx.PREC_FP64 else 1e-8), stats
