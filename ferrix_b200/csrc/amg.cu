@@ -2570,7 +2570,7 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
     auto iteration = [&]() {
         double* zn = parity ? z_.ptr : z2_.ptr;
         const double* zo = parity ? z2_.ptr : z_.ptr;
-        parity ^= 1;
+        if (amg.kcycle()) parity ^= 1;
         L0Op<double> o = l0_op<double>(l0, vals64);
         o.v = p_.ptr;
         o.y = q_.ptr;
@@ -2584,13 +2584,15 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
         FX_LAUNCH_CHAIN(k_xpby, gx, 256, 0, s, nd, zn, sc_.ptr, part_.ptr, (int)gz, amg.kcycle(), rd_part_.ptr, (int)gu,
                   p_.ptr);
     };
-    // Two iterations per graph (z alternates). Between host checks as many replays are queued as the
+    // Two iterations per graph (z alternates in the flexible CG), one for large systems, where half an
+    // iteration too many on average costs more than the gap between two graphs (2-3 us; 93k DOF: 29
+    // iterations instead of 30, 7.55 and 7.38 ms a solve). Between host checks as many replays are queued as the
     // residual's fall so far says are surely needed (60 % of the estimate, at most 12 iterations, 4 where
     // an iteration takes several times the ~14 us that a check idles the GPU for): iterations queued
     // past the end cost more than checks.
     // (A device-side loop as a WHILE graph node, one or four iterations per body, measured 1-7 %
     // slower per iteration on B200 than host-polled replays.)
-    const int per_graph = 2;
+    const int per_graph = n > 30000 && !amg.kcycle() ? 1 : 2;
     const bool graphs = opt.graphs && !debug_sync();
     const void* key[4] = {x, vals64, dinv64, r_.ptr};
     if (gexec_ && (!graphs || !std::equal(key, key + 4, graph_key_))) drop_graph();
