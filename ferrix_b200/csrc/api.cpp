@@ -165,7 +165,6 @@ int fx_ctx_create(int device, fx_ctx** out) {
         // here and not before each launch: set from several threads per solve, a batch of 24 small decks
         // took 57 ms, and 52 ms this way
         allow_shared_transfer();
-        allow_shared_corner();
         // keep freed stream-ordered allocations in this process's pool between solves
         // instead of returning them to the driver at every synchronisation
         cudaMemPool_t pool;

@@ -1,4 +1,6 @@
 // Corner level of C3D20 meshes (see corner.hpp): structure, weights and Galerkin matrix.
+#include <cuda_pipeline_primitives.h>
+
 #include <cub/cub.cuh>
 
 #include "common.hpp"
@@ -132,6 +134,101 @@ __global__ void k_corner_xyz(int n, const int32_t* __restrict__ fine_of, const d
     for (int k = 0; k < 3; ++k) out[3 * (int64_t)i + k] = x[3 * (int64_t)fine_of[i] + k];
 }
 
+// Element Galerkin matrices P_e^T K_e P_e (36 node-pair blocks of the 8 corners) from the 210 blocks
+// of K_e. CTA per element: K_e is staged in shared memory by asynchronous 16-byte copies (15 kB, read once:
+// the floor is that traffic), T = K_e P_e (160 blocks: C = I/2 +- (t I - f d^T) of a mid node applied from
+// the right acts on rows alone, so 16 threads per corner take a block row at a time) is formed beside it,
+// then P_e^T T by a thread per block column. 32k elements: 255 us, bound by shared memory; 404 with
+// copies through registers, 445 with a warp per element and a lane per block.
+constexpr int kThreadsG = 128;
+__global__ void __launch_bounds__(kThreadsG) k_corner_elements(const int32_t* __restrict__ conn,
+                                                               const int32_t* __restrict__ corner_of,
+                                                               const int2* __restrict__ par,
+                                                               const double* __restrict__ wgt,
+                                                               const double* __restrict__ ebuf,
+                                                               double* __restrict__ out) {
+    __shared__ __align__(16) double K[kPairs20 * 9];
+    __shared__ double T[160 * 9];
+    __shared__ double W[12 * 8];  // per mid node {t, f, d, sign of its first local corner}
+    const int tid = threadIdx.x;
+    const int64_t e = blockIdx.x;
+    const double* src = ebuf + e * (kPairs20 * 9);
+    // (K_e starts on a multiple of 16 bytes: 15,120 per C3D20 element after 720 per C3D4)
+    for (int i = tid; i < kPairs20 * 9 / 2; i += kThreadsG) __pipeline_memcpy_async(K + 2 * i, src + 2 * i, 16);
+    __pipeline_commit();
+    if (tid < 96) {
+        const int k = tid >> 3, node = conn[20 * e + 8 + k];
+        if ((tid & 7) < 7) W[tid] = wgt[8 * (int64_t)node + (tid & 7)];
+        else W[tid] = corner_of[conn[20 * e + kEdge[k][0]]] == par[node].x ? -1.0 : 1.0;
+    }
+    __pipeline_wait_prior(0);
+    __syncthreads();
+    auto sign = [&](int k, int a) { return kEdge[k][0] == a ? W[8 * k + 7] : -W[8 * k + 7]; };
+    {  // rows of T_ib = K_ib + sum over b's mid nodes m of K_im C_mb: 16 threads per corner b, with its weights
+        const int b = tid >> 4;
+        int m[3];
+        double w0[3], f[3][3], d[3][3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+            const int k = kCornerEdge[b][u];
+            const double* w = W + 8 * k;
+            const double sg = sign(k, b);
+            m[u] = 8 + k;
+            w0[u] = 0.5 + sg * w[0];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                f[u][c] = w[1 + c];
+                d[u][c] = sg * w[4 + c];
+            }
+        }
+        for (int t = tid & 15; t < 60; t += 16) {
+            const int i = t / 3, r = t - 3 * i;
+            auto row = [&](int j, double y[3]) {  // of K_ij
+                const double* blk = K + 9 * pair_index(20, min(i, j), max(i, j)) + (i <= j ? 3 * r : r);
+                const int st = i <= j ? 1 : 3;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) y[c] = blk[c * st];
+            };
+            double o[3], y[3];
+            row(b, o);
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                row(m[u], y);
+                const double yf = y[0] * f[u][0] + y[1] * f[u][1] + y[2] * f[u][2];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) o[c] += w0[u] * y[c] - yf * d[u][c];
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) T[180 * b + 3 * t + c] = o[c];  // block (b, i): at 20 b + i
+        }
+    }
+    __syncthreads();
+    if (tid < kPairs8 * 3) {  // column c of block q = (a, b): T_ab + sum over a's mid nodes m of C_ma^T T_mb
+        const int q = tid / 3, c = tid - 3 * q;
+        int a = 0, at = q;
+        while (at >= 8 - a) at -= 8 - a++;
+        const int b = a + at;
+        double o[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) o[r] = T[9 * (20 * b + a) + 3 * r + c];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+            const int k = kCornerEdge[a][u];
+            const double* w = W + 8 * k;
+            const double* y = T + 9 * (20 * b + 8 + k) + c;
+            const double sg = sign(k, a);
+            const double fy = w[1] * y[0] + w[2] * y[3] + w[3] * y[6];
+#pragma unroll
+            for (int r = 0; r < 3; ++r) o[r] += (0.5 + sg * w[0]) * y[3 * r] - sg * w[4 + r] * fy;
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) K[9 * q + 3 * r + c] = o[r];  // (K_e is not read any more)
+    }
+    __syncthreads();
+    for (int i = tid; i < kPairs8 * 9; i += kThreadsG) out[e * (kPairs8 * 9) + i] = K[i];
+}
+static_assert(kThreadsG == 128 && kPairs8 * 3 <= kThreadsG, "16 threads per corner; a thread per block column");
+
 // C = I / 2 +- M of a mid node towards one corner: y (3x3, row-major) -> y C (right) or C^T y (left)
 __device__ __forceinline__ void mul_right(const double y[9], const MidWeight& w, double sg, double o[9]) {
 #pragma unroll
@@ -147,74 +244,6 @@ __device__ __forceinline__ void mul_left(const double y[9], const MidWeight& w, 
         const double fy = w.f[0] * y[c] + w.f[1] * y[3 + c] + w.f[2] * y[6 + c];
 #pragma unroll
         for (int r = 0; r < 3; ++r) o[3 * r + c] += (0.5 + sg * w.t) * y[3 * r + c] - sg * w.d[r] * fy;
-    }
-}
-
-// Element Galerkin matrices P_e^T K_e P_e (36 node-pair blocks of the 8 corners) from the 210 blocks
-// of K_e. Warp per element: K_e is staged in shared memory by consecutive loads (15 kB, read once:
-// the bound is that traffic), T = K_e P_e (160 blocks) is formed beside it and then P_e^T T.
-constexpr int kWarpsG = 4;
-constexpr int kSharedG = (kPairs20 * 9 + 160 * 9 + 12 * 8) * (int)sizeof(double);
-__global__ void __launch_bounds__(32 * kWarpsG) k_corner_elements(int nelem, const int32_t* __restrict__ conn,
-                                                                  const int32_t* __restrict__ corner_of,
-                                                                  const int2* __restrict__ par,
-                                                                  const double* __restrict__ wgt,
-                                                                  const double* __restrict__ ebuf,
-                                                                  double* __restrict__ out) {
-    extern __shared__ __align__(16) double sh[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* K = sh + (size_t)warp * (kSharedG / sizeof(double));
-    double* T = K + kPairs20 * 9;
-    double* W = T + 160 * 9;  // per mid node {t, f, d, sign of its first local corner}
-    const int64_t e = (int64_t)blockIdx.x * kWarpsG + warp;
-    if (e >= nelem) return;  // warp-uniform
-    const double* src = ebuf + e * (kPairs20 * 9);
-    for (int i = lane; i < kPairs20 * 9; i += 32) K[i] = __ldcs(src + i);
-    if (lane < 12) {
-        const int node = conn[20 * e + 8 + lane];
-        for (int k = 0; k < 7; ++k) W[8 * lane + k] = wgt[8 * (int64_t)node + k];
-        W[8 * lane + 7] = corner_of[conn[20 * e + kEdge[lane][0]]] == par[node].x ? -1.0 : 1.0;
-    }
-    __syncwarp();
-    auto weight = [&](int k) {
-        const double* w = W + 8 * k;
-        return MidWeight{w[0], {w[1], w[2], w[3]}, {w[4], w[5], w[6]}};
-    };
-    auto sign = [&](int k, int a) { return kEdge[k][0] == a ? W[8 * k + 7] : -W[8 * k + 7]; };
-    auto block = [&](int i, int j, double y[9]) {  // K_ij
-        const double* b = K + 9 * pair_index(20, min(i, j), max(i, j));
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) y[3 * r + c] = i <= j ? b[3 * r + c] : b[3 * c + r];
-    };
-    for (int q = lane; q < 160; q += 32) {  // T_ib = K_ib + sum over b's mid nodes m of K_im C_mb
-        const int i = q >> 3, b = q & 7;
-        double t[9], y[9];
-        block(i, b, t);
-        for (int u = 0; u < 3; ++u) {
-            const int k = kCornerEdge[b][u];
-            block(i, 8 + k, y);
-            mul_right(y, weight(k), sign(k, b), t);
-        }
-#pragma unroll
-        for (int c = 0; c < 9; ++c) T[9 * q + c] = t[c];
-    }
-    __syncwarp();
-    double* o = out + e * (kPairs8 * 9);
-    for (int q = lane; q < kPairs8; q += 32) {
-        int a = 0, r = q;
-        while (r >= 8 - a) r -= 8 - a++;
-        const int b = a + r;
-        double t[9];
-#pragma unroll
-        for (int c = 0; c < 9; ++c) t[c] = T[9 * (8 * a + b) + c];
-        for (int u = 0; u < 3; ++u) {
-            const int k = kCornerEdge[a][u];
-            mul_left(T + 9 * (8 * (8 + k) + b), weight(k), sign(k, a), t);
-        }
-#pragma unroll
-        for (int c = 0; c < 9; ++c) o[9 * q + c] = t[c];
     }
 }
 
@@ -338,18 +367,14 @@ void corner_weights(CornerLevel& c, const double* xyz, cudaStream_t s) {
     FX_LAUNCH(k_corner_xyz, grid_for(c.n), 256, 0, s, c.n, c.fine_of.ptr, xyz, c.xyz.ptr);
 }
 
-void allow_shared_corner() {
-    FX_CUDA_CHECK(cudaFuncSetAttribute(k_corner_elements, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kWarpsG * kSharedG));
-}
-
 void corner_matrix(CornerLevel& c, const ElemView& g4, const ElemView& g20, const double* ebuf, const BcView& bc,
                    const unsigned long long* maxdiag, cudaStream_t s) {
     const size_t v4 = (size_t)g4.n * kPairs4 * 9;
     c.ebuf.alloc(v4 + (size_t)g20.n * kPairs8 * 9 + 9, s);
     if (v4) FX_CUDA_CHECK(cudaMemcpyAsync(c.ebuf.ptr, ebuf, v4 * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    FX_LAUNCH(k_corner_elements, grid_for(g20.n, kWarpsG), 32 * kWarpsG, kWarpsG * kSharedG, s, g20.n, g20.conn,
-              c.corner_of.ptr, c.par.ptr, c.wgt.ptr, ebuf + v4, c.ebuf.ptr + v4);
+    if (g20.n)
+        FX_LAUNCH(k_corner_elements, (unsigned)g20.n, kThreadsG, 0, s, g20.conn, c.corner_of.ptr, c.par.ptr, c.wgt.ptr,
+                  ebuf + v4, c.ebuf.ptr + v4);
     c.vals.alloc((size_t)c.S.n_groups * 36, s);
     launch_bsr_gather<double>(c.S, c.ebuf.ptr, c.vals.ptr, s);
     if (bc.n) {

@@ -123,7 +123,6 @@ namespace fx {
 
 // The kernels that take more than 48 KB of dynamic shared memory are allowed it; for each new context.
 void allow_shared_transfer();
-void allow_shared_corner();
 
 void ensure_dense(fx_model* m);
 // One kernel of each source file's module, and the loading of every kernel of
