@@ -14,8 +14,8 @@ One step = one StaticStep::solve of that deck to a displacement accurate to
 1e-8 against the FP64 direct solution: residual, symbolic pattern (rebuilt every
 step), element stiffness + BSR3 assembly, penalty BCs, PCG to the stated
 tolerance, update, convergence re-check. The default solver is the FP64 CG with
-the aggregation-multigrid preconditioner whose fine-level smoother reads FP32
-matrix values (`--precision mixed --preconditioner amg`); the comparison arms
+the smoothed-aggregation multigrid preconditioner whose smoother reads FP16 values of
+the scaled matrix (`--precision mixed --preconditioner amg`); the comparison arms
 time the other solvers on the same deck, among them the plain FP64 GPU PCG
 (scalar CSR + Jacobi, the reference IterativeSolver's algorithm). `value` is solves/s over all ranks with
 the model already resident on the device; `e2e` is the same through the public

@@ -99,7 +99,8 @@ typedef struct {
     double amg_cheb_ratio;   /* FX_PRECOND_AMG: lmax / lmin of the first-kind Chebyshev interval; 0 = 12 */
     int amg_persistent_max_dof; /* FX_PRECOND_AMG, V-cycle: systems of at most this many DOF run their
                                    whole CG in one persistent launch, one thread-block cluster per system
-                                   (all such systems of a round in the same launch); 0 = default (2,000);
+                                   (all such systems of a round in the same launch); 0 = default (2,000,
+                                   and not where the dense inverse covers the level it starts from);
                                    < 0 = never (one launch per CG step and phase) */
     int amg_fused_coarse;       /* FX_PRECOND_AMG, V-cycle, systems on the multi-launch path: 1 = the coarse
                                    part of each V-cycle (restriction, coarse levels, dense coarsest solve,
