@@ -2603,12 +2603,19 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
     const void* key[4] = {x, vals64, dinv64, r_.ptr};
     if (gexec_ && (!graphs || !std::equal(key, key + 4, graph_key_))) drop_graph();
     if (graphs && !gexec_) {
-        cudaGraph_t g;
+        cudaGraph_t g = nullptr;
         int64_t count = 0;
         int64_t* saved = g_launch_counter;
-        g_launch_counter = &count;
         FX_CUDA_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        for (int k = 0; k < per_graph; ++k) iteration();
+        g_launch_counter = &count;
+        try {
+            for (int k = 0; k < per_graph; ++k) iteration();
+        } catch (...) {  // (a batch goes on with its other systems on this stream)
+            g_launch_counter = saved;
+            if (cudaStreamEndCapture(s, &g) == cudaSuccess && g) cudaGraphDestroy(g);
+            cudaGetLastError();
+            throw;
+        }
         const cudaError_t ce = cudaStreamEndCapture(s, &g);
         g_launch_counter = saved;
         FX_CUDA_CHECK(ce);

@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <new>
 
 #include "engine.hpp"
 #include "pcg_csr.hpp"
@@ -626,15 +627,13 @@ struct StepRunner {
     }
 };
 
-// Advances all runners in lockstep rounds; runners share the context stream.
-// Returns per-runner status (FX_OK or the error that stopped that model).
+// Advances all runners in lockstep rounds; runners share the context stream. What is one model's own
+// runs under guard(), so that its failure ends that model only; the failure of a launch or a wait that
+// several share leaves as an exception.
 static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<int>& status,
-                       std::vector<std::string>& msgs) {
+                       std::vector<std::string>& msgs, std::vector<char>& alive) {
     cudaStream_t s = ctx->stream;
     const size_t n = rs.size();
-    status.assign(n, FX_OK);
-    msgs.assign(n, std::string());
-    std::vector<char> alive(n, 1);
     auto guard = [&](size_t i, auto&& f) {
         if (!alive[i]) return;
         try {
@@ -693,9 +692,19 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
         ph.start(s);
         std::vector<size_t> csr_ids, bsr_ids, cluster_ids;
         for (size_t i : solve) (rs[i]->csr || rs[i]->amg ? csr_ids : bsr_ids).push_back(i);
-        for (size_t i : csr_ids) {
-            StepRunner& r = *rs[i];
-            if (r.amg) {
+        for (size_t i : csr_ids)
+            guard(i, [&] {
+                StepRunner& r = *rs[i];
+                if (!r.amg) {
+                    PcgOptions pc = po;
+                    if (r.csr_reference) {  // iterative.rs:26-122 called with tol 1e-8, max_iter 1000 (static_step.rs:204)
+                        pc.rtol = 1e-8;
+                        pc.max_iter = 1000;
+                    }
+                    r.csr_status = ctx->pcgcsr.solve(r.csr_sys, r.m->dev.R.ptr, r.m->dev.du.ptr, pc, r.csr_reference, s,
+                                                     &ctx->launches, &r.csr_iters, &r.csr_relres);
+                    return;
+                }
                 AmgStats ast;
                 const bool reuse = r.reuse_hierarchy();
                 ModelDev& d = r.m->dev;
@@ -706,32 +715,21 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
                 // multi-launch path: 1,194-DOF C3D20 deck 1.0 against 2.1 ms of CG
                 const bool dense = r.o.amg_persistent_max_dof == 0 &&
                                    dense_planar(corner ? corner->n : r.m->dense.n_nodes);
-                if (!po.amg_kcycle && po.amg_persistent_max_dof > 0 && ndof <= po.amg_persistent_max_dof && !dense) {
+                const bool persistent =
+                    !po.amg_kcycle && po.amg_persistent_max_dof > 0 && ndof <= po.amg_persistent_max_dof && !dense;
+                if (persistent) {
                     // small system: hierarchy now, its whole CG in the round's persistent launch below
-                    guard(i, [&] {
-                        d.amg->prepare(d.S, d.vals64.ptr, d.minv64.ptr, r.amg_xyz.ptr, corner, r.amg_cell,
-                                       r.amg_node_volume, po, s, &ast, reuse, true);
-                        r.S.amg_levels = ast.levels;
-                        r.S.amg_setup_ms += ast.setup_ms;
-                        cluster_ids.push_back(i);
-                    });
-                    continue;
+                    d.amg->prepare(d.S, d.vals64.ptr, d.minv64.ptr, r.amg_xyz.ptr, corner, r.amg_cell,
+                                   r.amg_node_volume, po, s, &ast, reuse, true);
+                    cluster_ids.push_back(i);
+                } else {
+                    r.csr_status = d.amg->solve(d.S, d.vals64.ptr, d.minv64.ptr, r.amg_xyz.ptr, corner, r.amg_cell,
+                                                r.amg_node_volume, d.R.ptr, d.du.ptr, po, s, &ctx->launches,
+                                                &r.csr_iters, &r.csr_relres, &ast, reuse);
                 }
-                r.csr_status = d.amg->solve(d.S, d.vals64.ptr, d.minv64.ptr, r.amg_xyz.ptr, corner, r.amg_cell,
-                                            r.amg_node_volume, d.R.ptr, d.du.ptr, po, s, &ctx->launches, &r.csr_iters,
-                                            &r.csr_relres, &ast, reuse);
                 r.S.amg_levels = ast.levels;
                 r.S.amg_setup_ms += ast.setup_ms;
-                continue;
-            }
-            PcgOptions pc = po;
-            if (r.csr_reference) {  // iterative.rs:26-122 called with tol 1e-8, max_iter 1000 (static_step.rs:204)
-                pc.rtol = 1e-8;
-                pc.max_iter = 1000;
-            }
-            r.csr_status = ctx->pcgcsr.solve(r.csr_sys, r.m->dev.R.ptr, r.m->dev.du.ptr, pc, r.csr_reference, s,
-                                             &ctx->launches, &r.csr_iters, &r.csr_relres);
-        }
+            });
         if (!cluster_ids.empty()) {
             // every small multigrid system of the round in one persistent launch (a cluster each)
             std::vector<ClInst> desc;
@@ -794,6 +792,29 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
     stream_wait(s, "stream");
 }
 
+// run_rounds() with a status for every model: FX_OK or what stopped it. What stops the rounds as a whole
+// stops all models that were still on the way.
+static void solve_runners(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<int>& status,
+                          std::vector<std::string>& msgs) {
+    status.assign(rs.size(), FX_OK);
+    msgs.assign(rs.size(), std::string());
+    std::vector<char> alive(rs.size(), 1);
+    auto stop = [&](int st, const char* what) {
+        for (size_t i = 0; i < rs.size(); ++i)
+            if (alive[i]) {
+                status[i] = st;
+                msgs[i] = what;
+            }
+    };
+    try {
+        run_rounds(ctx, rs, status, msgs, alive);
+    } catch (const Error& e) {
+        stop(e.status, e.what());
+    } catch (const std::bad_alloc&) {
+        stop(FX_GENERIC, "Generic error: host allocation failed");
+    }
+}
+
 int step_solve(fx_model* m, int k, const fx_solve_opts& o, fx_step_stats* st, fx_increment_cb cb, void* user) {
     fx_ctx* ctx = m->ctx;
     int64_t* saved = g_launch_counter;
@@ -813,8 +834,8 @@ int step_solve(fx_model* m, int k, const fx_solve_opts& o, fx_step_stats* st, fx
     std::vector<StepRunner*> rs{&r};
     std::vector<int> status;
     std::vector<std::string> msgs;
-    run_rounds(ctx, rs, status, msgs);
-    r.S.t_total_ms = tot.stop_ms(ctx->stream);
+    solve_runners(ctx, rs, status, msgs);
+    if (status[0] != FX_CUDA) r.S.t_total_ms = tot.stop_ms(ctx->stream);
     if (st) *st = r.S;
     if (status[0] != FX_OK) fail(status[0], msgs[0]);
     return FX_OK;
@@ -847,8 +868,9 @@ static int batch_solve_on(fx_ctx* ctx, fx_model* const* models, int n, const fx_
     }
     std::vector<int> status;
     std::vector<std::string> msgs;
-    run_rounds(ctx, rs, status, msgs);
-    double ms = tot.stop_ms(ctx->stream);
+    solve_runners(ctx, rs, status, msgs);
+    const bool broken = std::find(status.begin(), status.end(), (int)FX_CUDA) != status.end();
+    const double ms = broken ? 0.0 : tot.stop_ms(ctx->stream);
     int rc = FX_OK;
     size_t j = 0;
     for (int i = 0; i < n; ++i) {
@@ -869,6 +891,17 @@ static int batch_solve_on(fx_ctx* ctx, fx_model* const* models, int n, const fx_
     return rc;
 }
 
+// batch_solve_on() under guarded(): a call that ends with an error and without a model's own status
+// leaves that error as the status of each of its models.
+static int batch_solve_guarded(fx_ctx* ctx, fx_model* const* models, int n, const fx_solve_opts& o, int* status,
+                               fx_step_stats* stats) {
+    std::vector<int> st(n, FX_OK);
+    const int rc = guarded(ctx, [&] { return batch_solve_on(ctx, models, n, o, st.data(), stats); });
+    if (rc != FX_OK && std::all_of(st.begin(), st.end(), [](int v) { return v == FX_OK; })) st.assign(n, rc);
+    if (status) std::copy(st.begin(), st.end(), status);
+    return rc;
+}
+
 // A batch of several models is spread over kBatchWorkers worker contexts of the
 // caller's context (own streams and host threads; balanced by DOF, largest first):
 // each worker runs its models' rounds (assembly, multigrid setup with its host round
@@ -884,7 +917,7 @@ int batch_solve(fx_ctx* ctx, fx_model* const* models, int n, const fx_solve_opts
                 fx_step_stats* stats) {
     const fx_solve_opts& o = o_in;
     const int K = std::min(kBatchWorkers, n);
-    if (K <= 1) return batch_solve_on(ctx, models, n, o, status_out, stats);
+    if (K <= 1) return batch_solve_guarded(ctx, models, n, o, status_out, stats);
     for (int i = 0; i < n; ++i)
         if (!models[i] || models[i]->ctx != ctx) {
             ctx->last_error = "model not bound to this context";
@@ -927,9 +960,7 @@ int batch_solve(fx_ctx* ctx, fx_model* const* models, int n, const fx_solve_opts
             }
             std::vector<int> st(ms.size(), FX_OK);
             std::vector<fx_step_stats> ss(ms.size());
-            rcs[k] = guarded(w, [&] {
-                return batch_solve_on(w, ms.data(), (int)ms.size(), o, st.data(), ss.data());
-            });
+            rcs[k] = batch_solve_guarded(w, ms.data(), (int)ms.size(), o, st.data(), ss.data());
             if (rcs[k] != FX_OK) errs[k] = w->last_error;
             cudaStreamSynchronize(w->stream);
             for (size_t j = 0; j < ms.size(); ++j) {
