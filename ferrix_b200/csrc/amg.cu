@@ -421,13 +421,18 @@ __global__ void __launch_bounds__(128) k_dense_from_planar(int n, const int32_t*
 //   B[K, K] = P, B[K, j] = P A[K, j], B[i, K] = -A[i, K] P, B[i, j] = A[i, j] - A[i, K] P A[K, j].
 // A and B alternate between two buffers, so that every tile is computed from A alone by its own
 // CTA and a panel is one launch; the CTA that holds the next pivot block inverts it as
-// soon as it is updated. DOFs with a vanishing diagonal are decoupled first and get
+// soon as it is updated. DOFs without stiffness (k_dense_decouple) are decoupled first and get
 // zero rows/columns in the inverse.
 constexpr int kPanel = 32;
 constexpr int kTileRows = 64;  // rows of a tile (kPanel columns): P A[K, j] is formed once per tile
 
-__global__ void __launch_bounds__(1024) k_dense_decouple(int nd, double* __restrict__ A, uint8_t* __restrict__ dead,
-                                                         double* __restrict__ diag) {
+// dead[k] = 1 for the DOFs to decouple. 6x6 levels: a diagonal below 1e-12 of the largest, the columns that
+// a rank-deficient aggregate's factorisation left empty. Planar levels: none but a zero diagonal (a
+// node of no element). There the largest is the constraints' penalty, 1e6 times the stiffest
+// material's, and the inverse is the only thing that acts on a soft material's nodes: with the 6x6 levels'
+// rule, steel beside a material 4e6 times softer did not converge.
+__global__ void __launch_bounds__(1024) k_dense_decouple(int nd, double rel, double* __restrict__ A,
+                                                         uint8_t* __restrict__ dead, double* __restrict__ diag) {
     __shared__ double s_red[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     double m = 0.0;
@@ -439,7 +444,7 @@ __global__ void __launch_bounds__(1024) k_dense_decouple(int nd, double* __restr
     for (int w = 0; w < nw; ++w) dmax = fmax(dmax, s_red[w]);
     int any = 0;
     for (int k = threadIdx.x; k < nd; k += blockDim.x) {
-        dead[k] = !(fabs(A[(int64_t)k * nd + k]) > 1e-12 * dmax);
+        dead[k] = !(fabs(A[(int64_t)k * nd + k]) > rel * dmax);
         any |= dead[k];
     }
     if (__syncthreads_or(any)) {  // (rank-deficient aggregates only: the pass over A takes ~50 us at 700 DOF)
@@ -1721,7 +1726,7 @@ void Amg::coarsest_inverse(AmgLevel& l, cudaStream_t s) {
     singular.zero(s);
     other.alloc((size_t)nd * nd, s);
     pivot.alloc(2 * kPanel * kPanel, s);
-    FX_LAUNCH(k_dense_decouple, 1, 1024, 0, s, (int)nd, l.dense_inv.ptr, dead.ptr, diag0.ptr);
+    FX_LAUNCH(k_dense_decouple, 1, 1024, 0, s, (int)nd, l.S0 ? 0.0 : 1e-12, l.dense_inv.ptr, dead.ptr, diag0.ptr);
     double* P[2] = {pivot.ptr, pivot.ptr + kPanel * kPanel};
     FX_LAUNCH(k_gj_first, 1, 256, 0, s, (int)nd, l.dense_inv.ptr, diag0.ptr, singular.ptr, P[0]);
     const dim3 tiles(grid_for(nd, kPanel), grid_for(nd, kTileRows));
