@@ -1830,7 +1830,7 @@ void Amg::setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz
             estimate_lmax(L[m], red_, s, false);
         }
     }
-    if (dense && dense_planar(L.back().n)) {
+    if (dense && cell0 <= 0.0 && dense_planar(L.back().n)) {
         AmgLevel& l = L.back();
         l.lmax = 1.0;  // (no smoothing here)
         l.coarsest = true;

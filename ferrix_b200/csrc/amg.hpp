@@ -109,7 +109,7 @@ class Amg {
     // in: the fine matrix and, with a corner level (corner != null), that level's. xyz: FP64
     // coordinates (device, 3 per node) of the last planar level's nodes. cell0: edge of the first
     // aggregates' cells, 0 = chosen from the mesh (pick_cell; node_volume: volume per such node).
-    // dense: the last planar level may be the coarsest (dense_planar()).
+    // dense: the last planar level may be the coarsest (dense_planar()); not with a cell0 of the caller's.
     void setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz, double cell0, double node_volume,
                bool dense, cudaStream_t s, AmgStats* st);
     // New matrix values on the structure of the last setup: aggregates, prolongators (values

@@ -713,7 +713,7 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
                 const int64_t ndof = 3 * r.m->dense.n_nodes;
                 // by default a system that the dense inverse covers (or its corner level) takes the
                 // multi-launch path: 1,194-DOF C3D20 deck 1.0 against 2.1 ms of CG
-                const bool dense = r.o.amg_persistent_max_dof == 0 &&
+                const bool dense = r.o.amg_persistent_max_dof == 0 && r.amg_cell <= 0.0 &&
                                    dense_planar(corner ? corner->n : r.m->dense.n_nodes);
                 const bool persistent =
                     !po.amg_kcycle && po.amg_persistent_max_dof > 0 && ndof <= po.amg_persistent_max_dof && !dense;

@@ -1,0 +1,55 @@
+"""An aggregate size that the caller asks for is used, also where the dense inverse would cover the system:
+the level count shows the aggregated level, and the coarsest level's inverse is tested at the sizes
+around its 32-pivot panels and 64-row tiles on a system above the dense size.
+
+Tolerance: 1e-10 against the oracle's FP64 direct solution at a residual target of 1e-11, as the other
+tests of the multigrid's sizes."""
+import numpy as np
+import pytest
+
+import ferrix_b200 as fx
+from ferrix_b200 import decks
+from oracle import inp, static_step
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = fx.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.fixture(scope="module")
+def solved():
+    out = {}
+    for name, text in (("small", decks.c3d4_cantilever(4, 5, 9)),   # 300 nodes
+                       ("large", decks.c3d4_cantilever(5, 6, 11)),  # 504 nodes
+                       ("corners", decks.c3d20_box(2, 2, 6, lengths=(2.0, 2.0, 6.0)))):  # 63 corners
+        out[name] = text, static_step.Runner(inp.parse_inp_text(text)).run().displacements
+    return out
+
+
+def _solve(ctx, solved, name, **kw):
+    text, ref = solved[name]
+    p = fx.Project.from_inp_text(text, ctx)
+    st = fx.SolutionState(p.num_dofs, p.num_nodes)
+    st.initialize(p)
+    stats = p.steps[0].solve(1, p, st, opts=fx.solve_opts(precision=fx.PREC_FP64, rtol=1e-11, **kw))
+    err = float(np.linalg.norm(st.displacements - ref) / np.linalg.norm(ref))
+    p.close()
+    assert err <= 1e-10, (err, stats)
+    return stats["amg_levels"]
+
+
+@pytest.mark.parametrize("persistent", [0, -1])
+def test_small_systems(ctx, solved, persistent):
+    for name, dense in (("small", 1), ("corners", 2)):
+        assert _solve(ctx, solved, name, amg_persistent_max_dof=persistent) == dense
+        assert _solve(ctx, solved, name, amg_aggregate_nodes=12, amg_persistent_max_dof=persistent) == dense + 1
+
+
+@pytest.mark.parametrize("nodes", [3, 4, 5, 8, 12, 20, 33, 45, 47, 50, 75, 120, 300, 5000])
+def test_coarsest_inverse_sizes(ctx, solved, nodes):
+    assert _solve(ctx, solved, "large", amg_aggregate_nodes=nodes, amg_persistent_max_dof=-1) == 2
