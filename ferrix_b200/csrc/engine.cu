@@ -337,12 +337,12 @@ struct StepRunner {
             if (d.corner.built_for != d.S.id)
                 build_corner_level(d.g4(), d.g20(), (int)m->dense.n_nodes, d.S.id, d.corner, m->ctx->stream);
             // volume per node of the level that is aggregated; aggregate cells holding the asked
-            // number of its nodes on average, or (the default) chosen by the hierarchy
+            // number of the mesh's nodes on average, or (the default) chosen by the hierarchy
             const double vol = m->dense.volume > 0.0 ? m->dense.volume : 1.0;
-            const int64_t nodes = d.corner.usable ? d.corner.n : m->dense.n_nodes;
-            amg_node_volume = vol / (double)std::max<int64_t>(1, nodes);
+            const int64_t n = m->dense.n_nodes;
+            amg_node_volume = vol / (double)std::max<int64_t>(1, d.corner.usable ? d.corner.n : n);
             const bool chosen = o.amg_aggregate_nodes > 0 && o.amg_aggregate_nodes != kAmgAggregateNodes;
-            amg_cell = chosen ? std::cbrt((double)o.amg_aggregate_nodes * amg_node_volume) : 0.0;
+            amg_cell = chosen ? std::cbrt((double)o.amg_aggregate_nodes * vol / (double)std::max<int64_t>(1, n)) : 0.0;
         }
         cudaStream_t s = m->ctx->stream;
         ModelDev& d = m->dev;

@@ -85,10 +85,10 @@ typedef struct {
     int reference_iterative; /* SOLVER=ITERATIVE steps: reference semantics (Jacobi PCG, absolute
                                 sqrt(r.z) < 1e-8, at most 1000 iterations; iterative.rs:26-136) */
     int preconditioner;     /* fx_preconditioner */
-    int amg_aggregate_nodes; /* FX_PRECOND_AMG: mean nodes per aggregate of the first aggregated level (cell
-                                size; C3D20 meshes: of element corners); 0 or 40 (the default) = chosen from
-                                the mesh, 20 to 80, and none where the dense inverse covers the level (400
-                                nodes or corners) */
+    int amg_aggregate_nodes; /* FX_PRECOND_AMG: mean nodes of the mesh per aggregate of the first aggregated
+                                level (cell size); 0 or 40 (the default) = chosen from the mesh, 20 to 80 nodes
+                                of that level (C3D20 meshes: element corners), and none where the dense inverse
+                                covers the level (400 nodes or corners) */
     int amg_smoother_degree; /* FX_PRECOND_AMG: Chebyshev steps per pre/post smoothing, 1..8; 0 = 2 */
     int amg_cycle;           /* FX_PRECOND_AMG: 0 = V-cycle, 1 = K-cycle at the first coarse level (two
                                 flexible-CG steps per coarse correction; the outer CG is then flexible) */

@@ -1,5 +1,5 @@
-"""An aggregate size that the caller asks for is used, also where the dense inverse would cover the system:
-the level count shows the aggregated level, and the coarsest level's inverse is tested at the sizes
+"""An aggregate size that the caller asks for is used, also where the dense inverse would cover the system,
+and counts the mesh's nodes: the level count shows the aggregated level, and the coarsest level's inverse is tested at the sizes
 around its 32-pivot panels and 64-row tiles on a system above the dense size.
 
 Tolerance: 1e-10 against the oracle's FP64 direct solution at a residual target of 1e-11, as the other
@@ -53,3 +53,18 @@ def test_small_systems(ctx, solved, persistent):
 @pytest.mark.parametrize("nodes", [3, 4, 5, 8, 12, 20, 33, 45, 47, 50, 75, 120, 300, 5000])
 def test_coarsest_inverse_sizes(ctx, solved, nodes):
     assert _solve(ctx, solved, "large", amg_aggregate_nodes=nodes, amg_persistent_max_dof=-1) == 2
+
+
+def test_counts_mesh_nodes(ctx):
+    """1,820 corners among 6,768 nodes: 16 nodes of the mesh per aggregate leave 408 aggregates, more than the dense
+    inverse's 200 (one more level); 16 corners, or 64 nodes, leave 132."""
+    text = decks.c3d20_box(6, 9, 25, lengths=(6.0, 9.0, 25.0))
+    levels = []
+    for nodes in (16, 64):
+        p = fx.Project.from_inp_text(text, ctx)
+        assert p.num_nodes == 6768
+        st = fx.SolutionState(p.num_dofs, p.num_nodes)
+        st.initialize(p)
+        levels.append(p.steps[0].solve(1, p, st, opts=fx.solve_opts(amg_aggregate_nodes=nodes))["amg_levels"])
+        p.close()
+    assert levels == [4, 3]
