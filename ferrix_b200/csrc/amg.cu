@@ -2086,7 +2086,7 @@ void Amg::cycle(int lev, const double* b, double* x, cudaStream_t s, bool starte
     coarse(lev + 1, s);
     FX_LAUNCH_CHAIN(k_prolong<6>, grid_for(l.n, kProlongRows<6>), 256, 0, s, l.n, l.tr.ptr.ptr, l.tr.col.ptr,
               l.tr.val32.ptr, c.x.ptr, xs,
-              alpha_ * l.pscale, nullptr, nullptr);
+              alpha_ * pscale(l), nullptr, nullptr);
     {
         LnOp o = ln_op(l);
         o.v = xs;
@@ -2142,7 +2142,7 @@ void Amg::first_coarse(cudaStream_t s) {
               l.tr.t_val32.ptr, l.r.ptr, c.b.ptr, coarse_start(planar_));
     coarse(planar_, s);
     FX_LAUNCH_CHAIN(k_prolong<3>, grid_for(l.n, kProlongRows<3>), 256, 0, s, l.n, l.tr.ptr.ptr, l.tr.col.ptr,
-              l.tr.val32.ptr, c.x.ptr, l.x.ptr, alpha_ * l.pscale, g32 ? l.x4.ptr : nullptr, l.sq4);
+              l.tr.val32.ptr, c.x.ptr, l.x.ptr, alpha_ * pscale(l), g32 ? l.x4.ptr : nullptr, l.sq4);
 }
 
 // A planar level with the fused operators: pre-smoothing from x = 0 (one elementwise
@@ -2210,7 +2210,7 @@ void Amg::vcycle(int m, const double* b, double* z, double* part, const double* 
         FX_LAUNCH_CHAIN(k_corner_restrict, grid_for((int64_t)c.n * kCornerLanes), 256, 0, s, corner_, l.r.ptr, c.b.ptr,
                   c.dinv0, c0.r, c0.x, c0.d, c0.d4, c0.c2, c0.sq4, c0.hs);
         vcycle<VT>(m + 1, c.b.ptr, c.xs.ptr, nullptr, nullptr, s, true);
-        FX_LAUNCH_CHAIN(k_corner_prolong, grid_for(l.n), 256, 0, s, corner_, c.result(), l.x.ptr, alpha_ * l.pscale,
+        FX_LAUNCH_CHAIN(k_corner_prolong, grid_for(l.n), 256, 0, s, corner_, c.result(), l.x.ptr, alpha_ * pscale(l),
                   g32 ? x4 : nullptr, l.sq4);
     } else {
         first_coarse(s);
@@ -2363,9 +2363,9 @@ double profile_smoother_op(const BsrStructure& S, const double* vals64, const do
     return ms;
 }
 
-static ClTransfer cl_transfer(const AmgLevel& l) {
+static ClTransfer cl_transfer(const AmgLevel& l, double pscale) {
     const Transfer& t = l.tr;
-    return ClTransfer{t.na, t.ptr.ptr, t.col.ptr, t.t_ptr.ptr, t.t_row.ptr, t.val32.ptr, t.t_val32.ptr, l.pscale};
+    return ClTransfer{t.na, t.ptr.ptr, t.col.ptr, t.t_ptr.ptr, t.t_row.ptr, t.val32.ptr, t.t_val32.ptr, pscale};
 }
 
 void Amg::describe(ClInst& o) const {
@@ -2400,8 +2400,8 @@ void Amg::describe(ClInst& o) const {
         }
     }
     o.corner = corner_;
-    o.corner_scale = L[0].pscale;
-    o.tr = cl_transfer(L[planar_ - 1]);
+    o.corner_scale = pscale(L[0]);
+    o.tr = cl_transfer(L[planar_ - 1], pscale(L[planar_ - 1]));
     for (size_t m = planar_; m < L.size() && m < (size_t)kClMaxLevels; ++m) {
         const AmgLevel& l = L[m];
         ClLevel& c = o.lev[m];
@@ -2412,7 +2412,7 @@ void Amg::describe(ClInst& o) const {
         c.vals = l.pvals.ptr;
         c.dinv = l.dinv.ptr;
         c.dense_inv = l.dense_inv.ptr;
-        c.tr = cl_transfer(l);
+        c.tr = cl_transfer(l, pscale(l));
         c.x = l.x.ptr;
         c.b = l.b.ptr;
         c.r = l.r.ptr;
@@ -2490,7 +2490,7 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
     }
     amg.set_cycle(opt.amg_kcycle);
     amg.set_smoother_kind(opt.amg_cheb_kind);
-    amg.set_overcorrect(opt.amg_overcorrect);
+    amg.set_overcorrect(opt.amg_overcorrect, opt.amg_overcorrect_all);
     amg.set_cheb_ratio(opt.amg_cheb_ratio);
     S_ = &S;
     vals64_ = vals64;

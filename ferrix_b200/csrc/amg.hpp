@@ -135,7 +135,12 @@ class Amg {
     // Chebyshev smoother: 0 = first kind on [lmax/30, lmax], 1 = fourth kind
     void set_smoother_kind(int kind) { cheb_kind_ = kind; }
     // coarse corrections x += alpha P e; first-kind Chebyshev interval [lmax / ratio, lmax]
-    void set_overcorrect(double alpha) { alpha_ = alpha; }
+    // scale of coarse corrections; all: of every one (PcgOptions), else of a level's times its pscale
+    void set_overcorrect(double alpha, bool all) {
+        alpha_ = alpha;
+        alpha_all_ = all;
+    }
+    double pscale(const AmgLevel& l) const { return alpha_all_ ? 1.0 : l.pscale; }
     void set_cheb_ratio(double ratio) { cheb_ratio_ = ratio; }
     bool kcycle() const { return kcycle_; }
     // z = cycle(r), FP64 vectors of 3 * n_nodes. With part != null the last smoothing step also
@@ -188,6 +193,7 @@ class Amg {
     int64_t part_slots_ = 0;
     int cheb_kind_ = 0;
     double alpha_ = 1.0, cheb_ratio_ = 30.0;
+    bool alpha_all_ = false;
     int degree_ = 2;
     const double* rdr_ = nullptr;
     float* hs_ = nullptr;

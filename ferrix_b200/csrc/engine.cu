@@ -656,7 +656,8 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
         po.amg_kcycle = rs[0]->o.amg_cycle == 1;
         po.amg_cheb_kind = rs[0]->o.amg_smoother == 1 ? 1 : 0;
         const double oc = rs[0]->o.amg_overcorrect;
-        po.amg_overcorrect = oc > 0.0 && oc < 2.0 ? oc : kAmgOvercorrect;
+        po.amg_overcorrect_all = oc > 0.0 && oc < 2.0 && oc != kAmgOvercorrect;
+        po.amg_overcorrect = po.amg_overcorrect_all ? oc : kAmgOvercorrect;
         po.amg_cheb_ratio = rs[0]->o.amg_cheb_ratio > 1.0 ? rs[0]->o.amg_cheb_ratio : kAmgChebRatio;
         po.amg_fused_coarse = rs[0]->o.amg_fused_coarse == 1;
         po.amg_fp16 = rs[0]->o.amg_fp16_smoother >= 0;

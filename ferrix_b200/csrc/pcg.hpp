@@ -84,9 +84,9 @@ struct PcgSystem {
 
 // Multigrid defaults, from a sweep on the 417k-DOF C3D20 box (136 -> 100 CG
 // iterations) and a population of C3D4 / C3D20 boxes (13 % less time):
-// coarse corrections scaled by 1.7 (aggregation without prolongator smoothing
-// under-corrects; a smoothed transfer, which does not, scales its corrections by the
-// option's value over 1.7, so by 1 by default), first-kind Chebyshev on [lmax / 12, lmax].
+// coarse corrections scaled by 1.7 through an unsmoothed transfer (aggregation without prolongator
+// smoothing under-corrects) and by 1 through a smoothed one or the corner level's, first-kind
+// Chebyshev on [lmax / 12, lmax].
 constexpr double kAmgOvercorrect = 1.7;
 constexpr double kAmgChebRatio = 12.0;
 
@@ -117,7 +117,8 @@ struct PcgOptions {
     bool amg_fp32 = false;    // FP32 fine-matrix values in the level-0 smoother
     bool amg_kcycle = false;  // K-cycle at the first coarse level (flexible outer CG)
     int amg_cheb_kind = 0;    // 0: Chebyshev of the first kind on [lmax/ratio, lmax], 1: fourth kind
-    double amg_overcorrect = kAmgOvercorrect;  // scale of every coarse correction
+    double amg_overcorrect = kAmgOvercorrect;  // scale of coarse corrections: through unsmoothed transfers, or
+    bool amg_overcorrect_all = false;          // (a value of the caller's) through every one
     double amg_cheb_ratio = kAmgChebRatio;  // lmax / lmin of the first-kind Chebyshev interval
     int64_t amg_persistent_max_dof = 0;     // systems up to this size: one persistent cluster launch (< 0: never)
     bool amg_fused_coarse = true;           // coarse part of each V-cycle as one cooperative launch

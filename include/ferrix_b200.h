@@ -94,9 +94,9 @@ typedef struct {
                                 flexible-CG steps per coarse correction; the outer CG is then flexible) */
     int amg_smoother;        /* FX_PRECOND_AMG: 0 = Chebyshev of the first kind on [lmax/ratio, lmax],
                                 1 = Chebyshev of the fourth kind (Lottes 2023) */
-    double amg_overcorrect;  /* FX_PRECOND_AMG: coarse corrections are scaled by this factor, in (0, 2), through
-                                an unsmoothed transfer, and by the factor over 1.7 through a smoothed one or the
-                                corner level's (which do not under-correct); 0 = 1.7 */
+    double amg_overcorrect;  /* FX_PRECOND_AMG: coarse corrections are scaled by this factor, in (0, 2); 0 or 1.7
+                                (the default) = 1.7 through an unsmoothed transfer and 1 through a smoothed one or
+                                the corner level's, which do not under-correct */
     double amg_cheb_ratio;   /* FX_PRECOND_AMG: lmax / lmin of the first-kind Chebyshev interval; 0 = 12 */
     int amg_persistent_max_dof; /* FX_PRECOND_AMG, V-cycle: systems of at most this many DOF run their
                                    whole CG in one persistent launch, one thread-block cluster per system

@@ -68,3 +68,16 @@ def test_counts_mesh_nodes(ctx):
         levels.append(p.steps[0].solve(1, p, st, opts=fx.solve_opts(amg_aggregate_nodes=nodes))["amg_levels"])
         p.close()
     assert levels == [4, 3]
+
+
+def test_correction_scale(ctx):
+    """Smoothed transfers take their corrections unscaled by default: asked for as 1.0 it is the same cycle."""
+    text = decks.c3d4_cantilever(8, 8, 30)
+    its = []
+    for kw in ({}, dict(amg_overcorrect=1.0)):
+        p = fx.Project.from_inp_text(text, ctx)
+        st = fx.SolutionState(p.num_dofs, p.num_nodes)
+        st.initialize(p)
+        its.append(p.steps[0].solve(1, p, st, opts=fx.solve_opts(rtol=1e-10, **kw))["pcg_iterations"])
+        p.close()
+    assert its[0] == its[1]
