@@ -2604,7 +2604,11 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
     // (A device-side loop as a WHILE graph node, one or four iterations per body, measured 1-7 %
     // slower per iteration on B200 than host-polled replays.)
     const int per_graph = n > 30000 && !amg.kcycle() ? 1 : 2;
-    const bool graphs = opt.graphs && !debug_sync();
+    // A hierarchy that ends with a planar level's dense inverse converges in 4 to 20 iterations of short
+    // kernels: capturing and instantiating them costs more than it saves, and most beside other
+    // threads that do the same (64 decks of 132 / 1,194 DOF as a batch 50 / 63 ms with graphs, 32 / 38 without;
+    // alone 1.28 / 1.69 and 1.09 / 1.53; without the dense level, 64 x 1,512 DOF, 33 and 34).
+    const bool graphs = opt.graphs && !debug_sync() && !amg.L[amg.planar() - 1].coarsest;
     const void* key[4] = {x, vals64, dinv64, r_.ptr};
     if (gexec_ && (!graphs || !std::equal(key, key + 4, graph_key_))) drop_graph();
     if (graphs && !gexec_) {
