@@ -2449,7 +2449,7 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
         in[1].vals = corner->vals.ptr;
         in[1].dinv = corner->minv.ptr;
     }
-    const bool f16 = opt.amg_fp32 && opt.amg_fp16 && !persistent;
+    const bool f16 = opt.amg_fp32 && opt.amg_fp16 > 0 && !persistent;
     const bool keep = keeps(S, reuse) && amg.planar() == (corner ? 2 : 1);
     for (int m = 0; m < (corner && !keep ? 2 : 1); ++m) {
         const BsrStructure& Sm = *in[m].S;

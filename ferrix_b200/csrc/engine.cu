@@ -627,6 +627,18 @@ struct StepRunner {
     }
 };
 
+// Values of the mixed fine-level smoother where the caller leaves them open. FP16 rounds the matrix by 5e-4
+// of its entries; where a stiff part hangs on a soft one, its rigid motion, which those entries should cancel, leaves
+// a residual of that size against the soft part's stiffness, and the smoother spoils what the coarse levels
+// gain: a 13k-DOF C3D20 bar with its clamped half softer by 1e2 / 1e3 / 1e4 / 1e5 took 28-52 / 26-52 / 62-90 / over
+// 200 iterations or did not converge, with FP32 at 1e5 at most 68, in FP64 20-58. The sizes of the persistent
+// launch (FP32) keep its precision on the multi-launch path.
+constexpr double kMaxContrast16 = 100.0;
+static void smoother_precision(const DenseModel& D, PcgOptions& po) {
+    if (po.amg_fp16 != 0) return;
+    po.amg_fp16 = D.e_contrast <= kMaxContrast16 && 3 * D.n_nodes > kClDefaultMaxDof ? 1 : -1;
+}
+
 // Advances all runners in lockstep rounds; runners share the context stream. What is one model's own
 // runs under guard(), so that its failure ends that model only; the failure of a launch or a wait that
 // several share leaves as an exception.
@@ -644,8 +656,9 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
             alive[i] = 0;
         }
     };
-    PcgOptions po;
+    PcgOptions shared;
     if (!rs.empty()) {
+        PcgOptions& po = shared;
         po.rtol = rs[0]->o.rtol;
         po.max_iter = rs[0]->o.max_iter;
         po.poll = rs[0]->o.poll_interval;
@@ -660,7 +673,8 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
         po.amg_overcorrect = po.amg_overcorrect_all ? oc : kAmgOvercorrect;
         po.amg_cheb_ratio = rs[0]->o.amg_cheb_ratio > 1.0 ? rs[0]->o.amg_cheb_ratio : kAmgChebRatio;
         po.amg_fused_coarse = rs[0]->o.amg_fused_coarse == 1;
-        po.amg_fp16 = rs[0]->o.amg_fp16_smoother >= 0;
+        const int h = rs[0]->o.amg_fp16_smoother;
+        po.amg_fp16 = h < 0 ? -1 : h > 0 ? 1 : 0;
         // persistent cluster solve for tiny systems (a cluster's few SMs are latency-bound
         // where the multi-launch path uses the whole GPU); all of a round's in one launch
         const int pm = rs[0]->o.amg_persistent_max_dof;
@@ -697,7 +711,7 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
             guard(i, [&] {
                 StepRunner& r = *rs[i];
                 if (!r.amg) {
-                    PcgOptions pc = po;
+                    PcgOptions pc = shared;
                     if (r.csr_reference) {  // iterative.rs:26-122 called with tol 1e-8, max_iter 1000 (static_step.rs:204)
                         pc.rtol = 1e-8;
                         pc.max_iter = 1000;
@@ -707,6 +721,8 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
                     return;
                 }
                 AmgStats ast;
+                PcgOptions po = shared;
+                smoother_precision(r.m->dense, po);
                 const bool reuse = r.reuse_hierarchy();
                 ModelDev& d = r.m->dev;
                 if (!d.amg) d.amg = std::make_unique<AmgPcg>();
@@ -741,7 +757,8 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
             d_desc.upload(desc, s);
             d_res.alloc(desc.size(), s);
             const AmgPcg& a0 = *rs[cluster_ids[0]]->m->dev.amg;
-            launch_amg_cluster(d_desc.ptr, d_res.ptr, (int)desc.size(), po.amg_fp32, po.rtol, po.max_iter,
+            launch_amg_cluster(d_desc.ptr, d_res.ptr, (int)desc.size(), shared.amg_fp32, shared.rtol,
+                               shared.max_iter,
                                a0.amg.degree(), a0.amg.overcorrect(), s);
             std::vector<ClResult> res(desc.size());
             d_res.download(res.data(), res.size(), s);
@@ -763,11 +780,11 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
                 if (rs[i]->fp64) v64.push_back(&rs[i]->sys64);
                 else v32.push_back(&rs[i]->sys32);
             }
-            if (!v64.empty()) ctx->pcg64.solve(v64, po, s, &ctx->launches);
+            if (!v64.empty()) ctx->pcg64.solve(v64, shared, s, &ctx->launches);
             if (!v32.empty()) {
-                PcgOptions p32 = po;  // mixed: the tightened residual target, also for its FP64 finish
-                p32.rtol = po.rtol * kMixedBjResidualFactor;
-                p32.accept_rtol = po.rtol;
+                PcgOptions p32 = shared;  // mixed: the tightened residual target, also for its FP64 finish
+                p32.rtol = shared.rtol * kMixedBjResidualFactor;
+                p32.accept_rtol = shared.rtol;
                 ctx->pcg32.solve(v32, p32, s, &ctx->launches);
                 std::vector<PcgSystem<double>*> fb;
                 for (size_t i : bsr_ids)

@@ -1192,6 +1192,20 @@ DenseModel build_dense(const Project& p) {
         m.t.push_back(0.0);
         m.v.push_back(0.0);
     }
+    std::vector<char> used(p.materials.size(), p.materials.size() == 1);
+    if (used.size() > 1)
+        for (int32_t k : mat)
+            if (k >= 0) used[(size_t)k] = 1;
+    double lo = 0.0, hi = 0.0;
+    for (size_t k = 0; k < used.size(); ++k)
+        if (used[k] && p.materials[k].has_e)
+            for (const auto& tv : p.materials[k].e.data) {
+                const double e = std::fabs(tv.second);
+                if (!(e > 0.0)) continue;
+                lo = lo > 0.0 ? std::min(lo, e) : e;
+                hi = std::max(hi, e);
+            }
+    if (lo > 0.0) d.e_contrast = hi / lo;
     return d;
 }
 

@@ -114,7 +114,7 @@ struct PcgOptions {
     double accept_rtol = 0.0;
     // multigrid preconditioner
     int amg_degree = 2;       // Chebyshev smoothing steps per pre/post smoothing
-    bool amg_fp32 = false;    // FP32 fine-matrix values in the level-0 smoother
+    bool amg_fp32 = false;    // mixed precision: FP32 (or FP16, below) fine-matrix values in the level-0 smoother
     bool amg_kcycle = false;  // K-cycle at the first coarse level (flexible outer CG)
     int amg_cheb_kind = 0;    // 0: Chebyshev of the first kind on [lmax/ratio, lmax], 1: fourth kind
     double amg_overcorrect = kAmgOvercorrect;  // scale of coarse corrections: through unsmoothed transfers, or
@@ -122,7 +122,7 @@ struct PcgOptions {
     double amg_cheb_ratio = kAmgChebRatio;  // lmax / lmin of the first-kind Chebyshev interval
     int64_t amg_persistent_max_dof = 0;     // systems up to this size: one persistent cluster launch (< 0: never)
     bool amg_fused_coarse = true;           // coarse part of each V-cycle as one cooperative launch
-    bool amg_fp16 = false;                  // level-0 smoothing with FP16 values of the scaled matrix
+    int amg_fp16 = -1;  // mixed, multi-launch path: FP16 values of the scaled matrix; 1 on, -1 off, 0 by the system
 };
 
 template <typename T>

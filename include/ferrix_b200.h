@@ -109,8 +109,9 @@ typedef struct {
                                    per step (default; measured faster on B200) */
     int amg_fp16_smoother;      /* FX_PRECOND_AMG with FX_PREC_MIXED, systems on the multi-launch path: the
                                    fine-level smoother reads FP16 values of the diagonally scaled matrix
-                                   D^-1/2 K D^-1/2 (entries within [-1, 1]); 0 = default (FP16), 1 = FP16,
-                                   -1 = FP32 values of K */
+                                   D^-1/2 K D^-1/2 (entries within [-1, 1]); 1 = FP16, -1 = FP32 values of K,
+                                   0 = default: FP16 above 2,000 DOF where the materials' Young's moduli lie
+                                   within a factor of 100, else FP32 */
 } fx_solve_opts;
 
 /* Preconditioner of the BSR3 PCG. */
@@ -118,7 +119,8 @@ typedef enum {
     FX_PRECOND_BLOCK_JACOBI = 0, /* 3x3 block-Jacobi */
     FX_PRECOND_AMG = 1           /* smoothed-aggregation multigrid V-cycle (rigid-body near-null-space; C3D20
                                     meshes: below a level of the element corners), FP64 CG;
-                                    with FX_PREC_MIXED the fine-level smoother reads FP32 matrix values */
+                                    with FX_PREC_MIXED the fine-level smoother reads FP16 or FP32 matrix values
+                                    (amg_fp16_smoother) */
 } fx_preconditioner;
 
 typedef struct {
