@@ -160,8 +160,7 @@ class Amg {
         const float4* sq4;  // FP16 smoother: the float4 direction is written scaled by sqrt(a_ii)
         float* hs;          // FP16 directions: where the start publishes the V-cycle's scale (else null)
     };
-    Start0 start0() const { return start_of(L[0]); }
-    Start0 start_of(const AmgLevel& l) const;
+    Start0 start0() const;
     // the hierarchy, smoother coefficients and work vectors, for the persistent solve
     void describe(ClInst& out) const;
     // The coarse part of each V-cycle as one cooperative launch (on: after every setup /
@@ -183,8 +182,9 @@ class Amg {
     CoarseStart coarse_start(int m) const;
     void coarse(int m, cudaStream_t s);
     void coarsest_inverse(AmgLevel& l, cudaStream_t s);
-    // V-cycle from planar level m, whose smoother values are VT
+    // V-cycle from planar level m (whose smoother values are VT)
     template <typename VT>
+    void vcycle_of(int m, const double* b, double* z, double* part, const double* zold, cudaStream_t s, bool started);
     void vcycle(int m, const double* b, double* z, double* part, const double* zold, cudaStream_t s, bool started);
     void first_coarse(cudaStream_t s);  // from the last planar level's residual into its iterate
     int planar_ = 1;
@@ -343,9 +343,9 @@ class AmgPcg {
     const double* vals64_ = nullptr;
     const double* dinv64_ = nullptr;
     DBuf<double> r_, z_, z2_, p_, q_, part_, rd_part_, sc_;
-    DBuf<float> vals32_[2];  // per planar level
-    DBuf<__half> vals16_[2];
-    DBuf<float4> sq4_[2];
+    DBuf<float> vals32_;
+    DBuf<__half> vals16_;
+    DBuf<float4> sq4_;
     DBuf<float> hs_;  // FP16 smoother directions: the current V-cycle's {2^k, 2^-k}
     bool fresh_ = false, stale_ = false;  // the hierarchy was (re)computed for this solve; should be for the next
     long long first_iters_ = 0;

@@ -359,7 +359,6 @@ __device__ __noinline__ double start0_op(Vg g, const ClInst& I, double alpha, bo
 }
 
 // Restriction to the corner level with its first smoothing step from x = 0
-template <bool G32>
 __device__ __noinline__ void corner_restrict_op(Vg g, const ClInst& I) {
     const ClPlanar& P = I.pl[1];
     const int sub = g.t % kCornerLanes;
@@ -371,16 +370,14 @@ __device__ __noinline__ void corner_restrict_op(Vg g, const ClInst& I) {
         if (i >= P.n || sub != 0) continue;
         const int64_t o3 = 3 * (int64_t)i;
         const double* D = P.dinv0 + 9 * (int64_t)i;
-        double t[3];
         for (int c = 0; c < 3; ++c) {
-            t[c] = P.c2_start * (__ldg(D + 3 * c) * v[0] + __ldg(D + 3 * c + 1) * v[1] + __ldg(D + 3 * c + 2) * v[2]);
+            const double t =
+                P.c2_start * (__ldg(D + 3 * c) * v[0] + __ldg(D + 3 * c + 1) * v[1] + __ldg(D + 3 * c + 2) * v[2]);
             P.b[o3 + c] = v[c];
             P.lr[o3 + c] = v[c];
-            P.lx[o3 + c] = t[c];
+            P.lx[o3 + c] = t;
+            P.ld[o3 + c] = t;
         }
-        if (G32) reinterpret_cast<float4*>(P.d4a)[i] = make_float4((float)t[0], (float)t[1], (float)t[2], 0.0f);
-        else
-            for (int c = 0; c < 3; ++c) P.ld[o3 + c] = t[c];
     }
 }
 
@@ -572,15 +569,15 @@ __device__ double vcycle(const ClInst& I, Vg g, int degree, double alpha, cg::cl
     ClusterBar bar{cl};
     planar_down<VT, G32>(I.pl[0], g, degree, cl, dA, dB, dA4, dB4);
     if (I.planar == 2) {
-        corner_restrict_op<G32>(g, I);
+        corner_restrict_op(g, I);
         cl.sync();
         if (I.pl[1].dense_inv) {
             dense_op(g, 3 * I.pl[1].n, I.pl[1].dense_inv, I.pl[1].b, I.pl[1].z);
             cl.sync();
         } else {
-            planar_down<VT, G32>(I.pl[1], g, degree, cl, eA, eB, eA4, eB4);
-            coarse_cycle<G32>(I, g, degree, alpha, bar);
-            planar_up<VT, G32>(I.pl[1], g, I.pl[1].b, I.pl[1].z, degree, false, cl, eA, eB, eA4, eB4);
+            planar_down<double, false>(I.pl[1], g, degree, cl, eA, eB, eA4, eB4);
+            coarse_cycle<false>(I, g, degree, alpha, bar);
+            planar_up<double, false>(I.pl[1], g, I.pl[1].b, I.pl[1].z, degree, false, cl, eA, eB, eA4, eB4);
         }
         corner_prolong_op<G32>(g, I, alpha * I.corner_scale);
         cl.sync();
