@@ -2470,6 +2470,7 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
         in[0].vals32 = vals32_.ptr;
     }
     amg.set_degree(opt.amg_degree);
+    kept_ = keep;
     if (keep) {
         amg.keep(in[0], st);
     } else if (reuse && amg.built_for == S.id && !amg.L.empty() && amg.L[0].n == n && amg.planar() == (corner ? 2 : 1)) {
@@ -2636,6 +2637,7 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
     long long it = 0;
     int rc = FX_OK;
     const double rtol2 = opt.rtol * opt.rtol;
+    const long long max_iter = kept_ ? std::min<long long>(opt.max_iter, 2 * first_iters_ + 50) : opt.max_iter;
     double seen = -1.0;  // r.D^-1 r at the check before, and the iterations queued since
     int queued = 0;
     while (true) {
@@ -2647,7 +2649,11 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
             break;
         }
         if (h[3] <= 0.0 || h[2] <= rtol2 * h[3]) break;
-        if (it >= opt.max_iter) {
+        if (kept_ && h[8] < 0.0) {  // (AmgPcg::keeps)
+            rc = FX_NUMERICAL;
+            break;
+        }
+        if (it >= max_iter) {
             rc = FX_CONVERGENCE;
             break;
         }
@@ -2658,7 +2664,7 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
             next = (int)(left < 20.0 ? 0.6 * left : 12.0);
             if (n > 30000) next = std::min(next, 4);
         }
-        next = (int)std::min<long long>(std::max(next, 1), std::max<long long>(1, opt.max_iter - it));
+        next = (int)std::min<long long>(std::max(next, 1), std::max<long long>(1, max_iter - it));
         const int replays = (next + per_graph - 1) / per_graph;
         for (int k = 0; k < replays; ++k) {
             if (gexec_) {

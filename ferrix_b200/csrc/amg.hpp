@@ -308,13 +308,18 @@ class AmgPcg {
     ~AmgPcg() { drop_graph(); }
     // Whether the next solve on this structure keeps the hierarchy below the fine level as it is
     // (reuse: the caller allows it, the matrix being a later Newton tangent of the same increment).
-    // A V-cycle with a lagged coarse operator is still symmetric positive definite and the CG tests
-    // the true system, so only its iteration count can suffer: once a solve on the kept hierarchy takes
-    // a quarter (and more than 4 iterations) longer than the first one did, the next one
-    // recomputes it. (NLGEOM beam, 16k DOF: setups 80 of 215 ms with every tangent's recomputed.)
+    // A V-cycle with a lagged coarse operator is symmetric, and positive definite as long as the fine level's kept
+    // eigenvalue estimate bounds the new tangent's (the smoother's Chebyshev polynomial of the default interval and
+    // degree exceeds 1 from 13/12 of it on); the CG tests the true system. So a solve on the kept
+    // hierarchy may take longer, and can fail: once one takes a quarter (and more than 4 iterations) longer than
+    // the first did, the next recomputes the hierarchy; one that fails, finds a negative r.z or takes twice the
+    // first's iterations and 50 ends, to be done over on a recomputed one (kept(), outdate()). (NLGEOM beam, 16k DOF:
+    // setups 80 of 215 ms with every tangent's recomputed.)
     bool keeps(const BsrStructure& S, bool reuse) const {
         return reuse && amg.built_for == S.id && !amg.L.empty() && amg.L[0].n == S.n_rows && !stale_;
     }
+    bool kept() const { return kept_; }  // the last solve was on the kept hierarchy
+    void outdate() { stale_ = true; }    // the next one recomputes it
     // iterations of the solve that prepare() was called for (solve() calls it itself)
     void solved(long long iterations) {
         if (fresh_) first_iters_ = iterations;
@@ -347,6 +352,7 @@ class AmgPcg {
     DBuf<__half> vals16_;
     DBuf<float4> sq4_;
     DBuf<float> hs_;  // FP16 smoother directions: the current V-cycle's {2^k, 2^-k}
+    bool kept_ = false;
     bool fresh_ = false, stale_ = false;  // the hierarchy was (re)computed for this solve; should be for the next
     long long first_iters_ = 0;
     // the captured iterations, kept while the hierarchy is: what they were captured with

@@ -486,6 +486,40 @@ struct StepRunner {
     // hierarchy built at the increment's first tangent (AmgPcg::keeps)
     bool reuse_hierarchy() const { return step->nlgeom && it > 0; }
 
+    // the corner level's matrix of the last assembled tangent
+    void corner_values() {
+        ModelDev& d = m->dev;
+        corner_matrix(d.corner, d.g4(), d.g20(), d.ebuf64.ptr, bcv, d.maxdiag.ptr, m->ctx->stream);
+    }
+
+    // The prepared system by the multigrid CG; persistent: its set-up only.
+    void solve_amg(const PcgOptions& po, bool reuse, bool persistent) {
+        ModelDev& d = m->dev;
+        cudaStream_t s = m->ctx->stream;
+        AmgStats ast;
+        const CornerLevel* corner = d.corner.usable ? &d.corner : nullptr;
+        if (persistent)
+            d.amg->prepare(d.S, d.vals64.ptr, d.minv64.ptr, amg_xyz.ptr, corner, amg_cell, amg_node_volume, po, s,
+                           &ast, reuse, true);
+        else
+            csr_status = d.amg->solve(d.S, d.vals64.ptr, d.minv64.ptr, amg_xyz.ptr, corner, amg_cell, amg_node_volume,
+                                      d.R.ptr, d.du.ptr, po, s, &m->ctx->launches, &csr_iters, &csr_relres, &ast,
+                                      reuse);
+        S.amg_levels = ast.levels;
+        S.amg_setup_ms += ast.setup_ms;
+    }
+
+    // A solve on a kept hierarchy that failed, over again on one computed for its matrix.
+    void solve_amg_over(const PcgOptions& po) {
+        ModelDev& d = m->dev;
+        if (csr_status == FX_OK || !d.amg->kept()) return;
+        const long long spent = csr_iters;
+        d.amg->outdate();
+        if (d.corner.usable) corner_values();
+        solve_amg(po, true, false);
+        csr_iters += spent;
+    }
+
     // tangent, penalty, block-Jacobi (static_step.rs:173-199)
     void prepare_solve() {
         ModelDev& d = m->dev;
@@ -514,7 +548,7 @@ struct StepRunner {
             const bool reuse = reuse_hierarchy();
             if (d.corner.usable && !(d.amg && d.amg->keeps(d.S, reuse))) {
                 if (!reuse || !d.corner.wgt.ptr) corner_weights(d.corner, amg_xyz.ptr, s);  // (a refresh keeps them)
-                corner_matrix(d.corner, d.g4(), d.g20(), d.ebuf64.ptr, bcv, d.maxdiag.ptr, s);
+                corner_values();
             }
         } else if (fp64) {
             launch_penalty<double>(d.S, d.vals64.ptr, bcv, d.maxdiag.ptr, d.R.ptr, ucur.ptr, s);
@@ -720,32 +754,21 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
                                                      &ctx->launches, &r.csr_iters, &r.csr_relres);
                     return;
                 }
-                AmgStats ast;
                 PcgOptions po = shared;
                 smoother_precision(r.m->dense, po);
-                const bool reuse = r.reuse_hierarchy();
                 ModelDev& d = r.m->dev;
                 if (!d.amg) d.amg = std::make_unique<AmgPcg>();
-                const CornerLevel* corner = d.corner.usable ? &d.corner : nullptr;
                 const int64_t ndof = 3 * r.m->dense.n_nodes;
                 // by default a system that the dense inverse covers (or its corner level) takes the
                 // multi-launch path: 1,194-DOF C3D20 deck 1.0 against 2.1 ms of CG
                 const bool dense = r.o.amg_persistent_max_dof == 0 && r.amg_cell <= 0.0 &&
-                                   dense_planar(corner ? corner->n : r.m->dense.n_nodes);
+                                   dense_planar(d.corner.usable ? d.corner.n : r.m->dense.n_nodes);
                 const bool persistent =
                     !po.amg_kcycle && po.amg_persistent_max_dof > 0 && ndof <= po.amg_persistent_max_dof && !dense;
-                if (persistent) {
-                    // small system: hierarchy now, its whole CG in the round's persistent launch below
-                    d.amg->prepare(d.S, d.vals64.ptr, d.minv64.ptr, r.amg_xyz.ptr, corner, r.amg_cell,
-                                   r.amg_node_volume, po, s, &ast, reuse, true);
-                    cluster_ids.push_back(i);
-                } else {
-                    r.csr_status = d.amg->solve(d.S, d.vals64.ptr, d.minv64.ptr, r.amg_xyz.ptr, corner, r.amg_cell,
-                                                r.amg_node_volume, d.R.ptr, d.du.ptr, po, s, &ctx->launches,
-                                                &r.csr_iters, &r.csr_relres, &ast, reuse);
-                }
-                r.S.amg_levels = ast.levels;
-                r.S.amg_setup_ms += ast.setup_ms;
+                r.solve_amg(po, r.reuse_hierarchy(), persistent);
+                // a small system: its whole CG in the round's persistent launch below
+                if (persistent) cluster_ids.push_back(i);
+                else r.solve_amg_over(po);
             });
         if (!cluster_ids.empty()) {
             // every small multigrid system of the round in one persistent launch (a cluster each)
@@ -770,6 +793,7 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
                 r.m->dev.amg->solved(r.csr_iters);
                 guard(cluster_ids[k], [&] {
                     r.csr_relres = r.m->dev.amg->true_relres(r.m->dev.R.ptr, r.m->dev.du.ptr, s);
+                    r.solve_amg_over(shared);
                 });
             }
         }
