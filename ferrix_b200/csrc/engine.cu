@@ -314,7 +314,8 @@ struct StepRunner {
     double csr_relres = 0.0;
     // aggregation-multigrid preconditioned FP64 CG (FX_PRECOND_AMG)
     bool amg = false;
-    double amg_cell = 0.0, amg_node_volume = 0.0;
+    double amg_cell = 0.0, amg_volume = 1.0;
+    bool no_corner = false;  // this step's hierarchy does without a corner level
     DBuf<double> amg_xyz;
 
     void begin(fx_model* mm, int kk, const fx_solve_opts& oo) {
@@ -336,13 +337,12 @@ struct StepRunner {
             ModelDev& d = m->dev;
             if (d.corner.built_for != d.S.id)
                 build_corner_level(d.g4(), d.g20(), (int)m->dense.n_nodes, d.S.id, d.corner, m->ctx->stream);
-            // volume per node of the level that is aggregated; aggregate cells holding the asked
-            // number of the mesh's nodes on average, or (the default) chosen by the hierarchy
-            const double vol = m->dense.volume > 0.0 ? m->dense.volume : 1.0;
-            const int64_t n = m->dense.n_nodes;
-            amg_node_volume = vol / (double)std::max<int64_t>(1, d.corner.usable ? d.corner.n : n);
+            // aggregate cells holding the asked number of the mesh's nodes on average, or (the default)
+            // chosen by the hierarchy
+            amg_volume = m->dense.volume > 0.0 ? m->dense.volume : 1.0;
+            const double per_node = amg_volume / (double)std::max<int64_t>(1, m->dense.n_nodes);
             const bool chosen = o.amg_aggregate_nodes > 0 && o.amg_aggregate_nodes != kAmgAggregateNodes;
-            amg_cell = chosen ? std::cbrt((double)o.amg_aggregate_nodes * vol / (double)std::max<int64_t>(1, n)) : 0.0;
+            amg_cell = chosen ? std::cbrt((double)o.amg_aggregate_nodes * per_node) : 0.0;
         }
         cudaStream_t s = m->ctx->stream;
         ModelDev& d = m->dev;
@@ -486,6 +486,9 @@ struct StepRunner {
     // hierarchy built at the increment's first tangent (AmgPcg::keeps)
     bool reuse_hierarchy() const { return step->nlgeom && it > 0; }
 
+    CornerLevel* corner() const { return m->dev.corner.usable && !no_corner ? &m->dev.corner : nullptr; }
+    int64_t planar_nodes() const { return corner() ? corner()->n : m->dense.n_nodes; }
+
     // the corner level's matrix of the last assembled tangent
     void corner_values() {
         ModelDev& d = m->dev;
@@ -497,14 +500,23 @@ struct StepRunner {
         ModelDev& d = m->dev;
         cudaStream_t s = m->ctx->stream;
         AmgStats ast;
-        const CornerLevel* corner = d.corner.usable ? &d.corner : nullptr;
-        if (persistent)
-            d.amg->prepare(d.S, d.vals64.ptr, d.minv64.ptr, amg_xyz.ptr, corner, amg_cell, amg_node_volume, po, s,
-                           &ast, reuse, true);
-        else
-            csr_status = d.amg->solve(d.S, d.vals64.ptr, d.minv64.ptr, amg_xyz.ptr, corner, amg_cell, amg_node_volume,
-                                      d.R.ptr, d.du.ptr, po, s, &m->ctx->launches, &csr_iters, &csr_relres, &ast,
-                                      reuse);
+        const double node_volume = amg_volume / (double)std::max<int64_t>(1, planar_nodes());
+        try {
+            if (persistent)
+                d.amg->prepare(d.S, d.vals64.ptr, d.minv64.ptr, amg_xyz.ptr, corner(), amg_cell, node_volume, po, s,
+                               &ast, reuse, true);
+            else
+                csr_status = d.amg->solve(d.S, d.vals64.ptr, d.minv64.ptr, amg_xyz.ptr, corner(), amg_cell,
+                                          node_volume, d.R.ptr, d.du.ptr, po, s, &m->ctx->launches, &csr_iters,
+                                          &csr_relres, &ast, reuse);
+        } catch (const Error& e) {
+            // A coarse operator below the corner level may look singular where one below the nodes does not (a stiff
+            // part on flat cells 1e4 times softer): whether the system is, the latter decides.
+            if (e.status != FX_NUMERICAL || !corner()) throw;
+            no_corner = true;
+            solve_amg(po, false, persistent);
+            return;
+        }
         S.amg_levels = ast.levels;
         S.amg_setup_ms += ast.setup_ms;
     }
@@ -515,7 +527,7 @@ struct StepRunner {
         if (csr_status == FX_OK || !d.amg->kept()) return;
         const long long spent = csr_iters;
         d.amg->outdate();
-        if (d.corner.usable) corner_values();
+        if (corner()) corner_values();
         solve_amg(po, true, false);
         csr_iters += spent;
     }
@@ -546,7 +558,7 @@ struct StepRunner {
             launch_axpby(3 * nn, 1.0, d.xyz.ptr, step->nlgeom ? 1.0 : 0.0, step->nlgeom ? ucur.ptr : nullptr,
                          amg_xyz.ptr, s);
             const bool reuse = reuse_hierarchy();
-            if (d.corner.usable && !(d.amg && d.amg->keeps(d.S, reuse))) {
+            if (corner() && !(d.amg && d.amg->keeps(d.S, reuse))) {
                 if (!reuse || !d.corner.wgt.ptr) corner_weights(d.corner, amg_xyz.ptr, s);  // (a refresh keeps them)
                 corner_values();
             }
@@ -762,7 +774,7 @@ static void run_rounds(fx_ctx* ctx, std::vector<StepRunner*>& rs, std::vector<in
                 // by default a system that the dense inverse covers (or its corner level) takes the
                 // multi-launch path: 1,194-DOF C3D20 deck 1.0 against 2.1 ms of CG
                 const bool dense = r.o.amg_persistent_max_dof == 0 && r.amg_cell <= 0.0 &&
-                                   dense_planar(d.corner.usable ? d.corner.n : r.m->dense.n_nodes);
+                                   dense_planar(r.planar_nodes());
                 const bool persistent =
                     !po.amg_kcycle && po.amg_persistent_max_dof > 0 && ndof <= po.amg_persistent_max_dof && !dense;
                 r.solve_amg(po, r.reuse_hierarchy(), persistent);

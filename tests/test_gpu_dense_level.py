@@ -27,9 +27,9 @@ def _ids(a):
     return "\n".join(", ".join(str(int(v) + 1) for v in a[i:i + 12]) for i in range(0, len(a), 12))
 
 
-def two_materials(npe, cells, lengths, stiff, soft):
+def two_materials(npe, cells, lengths, stiff, soft, jitter=0.05):
     """A column clamped at z = 0 whose lower and upper half have Young's moduli stiff and soft."""
-    mesh = decks.tet_box(*cells, *lengths) if npe == 4 else decks.hex20_box(*cells, *lengths, jitter=0.05, seed=1)
+    mesh = decks.tet_box(*cells, *lengths) if npe == 4 else decks.hex20_box(*cells, *lengths, jitter=jitter, seed=1)
     text = decks.write_deck(decks.DeckSpec(mesh, [(stiff, 0.3, None)], load_total=(1.0, 2.0, -1.0)))
     is_soft = mesh.xyz[mesh.conn].mean(axis=1)[:, 2] > lengths[2] / 2
     text = text.replace("*Elset, Elset=Vol\nSolid\n", "*Elset, Elset=Vol\n" + _ids(np.nonzero(~is_soft)[0]) +
@@ -66,3 +66,20 @@ def test_soft_on_stiff(ctx, npe, cells, lengths, contrast, prec):
     text = two_materials(npe, cells, lengths, 2.0e5, 2.0e5 / contrast)
     u, stats = solve(ctx, text, precision=prec)
     assert error(text, u) <= 1e-8, stats
+
+
+@pytest.mark.parametrize("prec", [fx.PREC_FP64, fx.PREC_MIXED])
+@pytest.mark.parametrize("contrast", [1e4, 1e5])
+def test_coarse_operator_below_the_corners(ctx, contrast, prec):
+    """A stiff plate on cells eight times wider than high and much softer: the coarse operator below the corner
+    level has pivots as of a singular one, that below the nodes has not, and the system is solved.
+
+    Tolerance: mean displacement of the loaded face, 1e-6: contrast x unit round-off = 1e-11, and at most 1e2 by the
+    plate's lever on the pad."""
+    text = two_materials(20, (6, 6, 24), (6.0, 6.0, 3.0), 2.0e5 / contrast, 2.0e5, jitter=0.0)
+    u, _ = solve(ctx, text, precision=prec)
+    ref = static_step.Runner(inp.parse_inp_text(text)).run().displacements
+    mesh = decks.hex20_box(6, 6, 24, 6.0, 6.0, 3.0)
+    top = decks.face_nodes(mesh, 2, 1)
+    a, b = (v.reshape(-1, 3)[top].mean(axis=0) for v in (u, ref))
+    assert np.linalg.norm(a - b) <= 1e-6 * np.linalg.norm(b)
