@@ -170,7 +170,8 @@ __global__ void __launch_bounds__(kThreads4) k_stiff4(int nelem, const int32_t* 
         tc += 0.25 * Tcur[nd[a]];
     }
     Lame L{};
-    if (!material_d(md, mat[own ? e : e0], tc, &L)) atomicOr(err, kErrNoMaterial);  // (the host then stops)
+    const bool known = material_d(md, mat[own ? e : e0], tc, &L);
+    if (!known) atomicOr(err, kErrNoMaterial);  // (the host then stops)
     T J[9], Ji[9];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(kThreads4) k_stiff4(int nelem, const int32_t* 
         J[6 + c] = (T)(x[3][c] - x[0][c]);
     }
     T det = inv3(J, Ji);
-    if (det == T(0)) atomicOr(err, kErrSingularJ);
+    if (det == T(0) && known) atomicOr(err, kErrSingularJ);
     T w = fabs(det) * (T)(1.0 / 6.0);
     T g[4][3];
 #pragma unroll
