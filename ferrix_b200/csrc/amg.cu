@@ -23,6 +23,12 @@ constexpr int kMaxLevels = 8;
 // is 1.1 times the power iteration's value: 4/3 over the latter, the optimum of the analysis
 constexpr double kLmaxMargin = 1.1;
 constexpr double kSmoothOmega = 4.0 / 3.0 * kLmaxMargin;
+// Transfers are smoothed but where the caller asks for aggregates of fewer than kSmoothMembers members on a level of
+// more than kSmoothRows rows: smoothed ones reach so many small aggregates there that the Galerkin product costs
+// more than it saves (205k-DOF C3D4 box with 4 / 8 / 16 nodes per aggregate 90 / 27 / 16.4 ms a solve, unsmoothed 17.8 /
+// 12.5 / 11.0; with 24 11.6 and 11.7). The levels below follow the first, but below a corner level (96k-DOF
+// C3D20 box, 8 nodes: 13.6 ms, 12.2 smoothed).
+constexpr int64_t kSmoothMembers = 20, kSmoothRows = 5000;
 
 template <typename Op>
 void cub_call(Op op, DBuf<uint8_t>& tmp, cudaStream_t s) {
@@ -1847,6 +1853,7 @@ void Amg::setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz
     unsigned long long hbox[6];
     FX_CUDA_CHECK(cudaMemcpyAsync(hbox, box.ptr, sizeof(hbox), cudaMemcpyDeviceToHost, s));
     double cell = cell0, extent[3] = {0.0, 0.0, 0.0};
+    bool smooth = true;
     for (int lev = planar_ - 1;; ++lev) {
         AmgLevel& l = L[lev];
         const int64_t nd = (int64_t)l.n * l.bs;
@@ -1925,11 +1932,13 @@ void Amg::setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz
             l.blk_row.alloc(l.nblocks, s);
             FX_LAUNCH(k_expand_rows, grid_for(l.n), 256, 0, s, l.n, l.row_ptr.ptr, l.blk_row.ptr);
         }
+        if (l.S0) smooth = cell0 <= 0.0 || l.n <= kSmoothRows || l.n >= kSmoothMembers * na;
+        else if (planar_ == 2) smooth = true;
         L.emplace_back();
         AmgLevel& c = L.back();
         AmgLevel& lf = L[L.size() - 2];
         const bool smoothed = build_transfer(fine_view(lf), na, agg.ptr, Q.ptr, lf.dinv_ptr(), kSmoothOmega / lf.lmax,
-                                             lf.tr, c.row_ptr, c.cols, &c.nblocks, tmp_, s);
+                                             smooth, lf.tr, c.row_ptr, c.cols, &c.nblocks, tmp_, s);
         lf.pscale = smoothed ? 1.0 / kAmgOvercorrect : 1.0;
         c.n = na;
         c.bs = 6;

@@ -741,20 +741,20 @@ bool build_by_rows(const FineView& F, int na, const int32_t* agg, const double* 
 }  // namespace
 
 bool build_transfer(const FineView& F, int na, const int32_t* agg, const double* Q, const double* dinv, double omega,
-                    Transfer& t, DBuf<int32_t>& c_ptr, DBuf<int32_t>& c_cols, int64_t* ncb, DBuf<uint8_t>& tmp,
-                    cudaStream_t s) {
+                    bool smooth, Transfer& t, DBuf<int32_t>& c_ptr, DBuf<int32_t>& c_cols, int64_t* ncb,
+                    DBuf<uint8_t>& tmp, cudaStream_t s) {
     const int n = F.n, bs = F.bs;
     const int abits = bits_for(na > 1 ? na : 2), nbits = bits_for(n > 1 ? n : 2);
     t.n = n;
     t.na = na;
     t.bs = bs;
-    t.by_rows = build_by_rows(F, na, agg, Q, dinv, omega, t, c_ptr, c_cols, ncb, tmp, s);
+    t.by_rows = smooth && build_by_rows(F, na, agg, Q, dinv, omega, t, c_ptr, c_cols, ncb, tmp, s);
     if (t.by_rows) return true;
     t.w_ptr.release();
     t.w_col.release();
     DBuf<int64_t> cnt, end;
     DBuf<int32_t> w_ptr;
-    bool smooth = F.nblocks > 0;
+    smooth = smooth && F.nblocks > 0;
     int64_t total = 0;
     PairList p;
     while (true) {

@@ -74,12 +74,12 @@ struct Transfer {
 };
 
 // P of the level `F` with aggregates agg (per fine row) and tentative prolongator Q
-// (BS x 6 per fine row): smoothed with omega and the block inverses dinv, or Q itself where the smoothed product would not fit 32-bit item indices. Fills t.ptr .. t.val
-// and both pair lists, and c_ptr (na + 1), c_cols: the block pattern of A_c. Returns whether P
-// is smoothed; *ncb = blocks of A_c.
+// (BS x 6 per fine row): smoothed with omega and the block inverses dinv, or (not `smooth`, or where the
+// smoothed product would not fit 32-bit item indices) Q itself. Fills t and c_ptr (na + 1), c_cols: the
+// block pattern of A_c. Returns whether P is smoothed; *ncb = blocks of A_c.
 bool build_transfer(const FineView& F, int na, const int32_t* agg, const double* Q, const double* dinv, double omega,
-                    Transfer& t, DBuf<int32_t>& c_ptr, DBuf<int32_t>& c_cols, int64_t* ncb, DBuf<uint8_t>& tmp,
-                    cudaStream_t s);
+                    bool smooth, Transfer& t, DBuf<int32_t>& c_ptr, DBuf<int32_t>& c_cols, int64_t* ncb,
+                    DBuf<uint8_t>& tmp, cudaStream_t s);
 // c_vals (36 per block of the pattern c_ptr, c_cols) = P^T A P
 void galerkin_product(const FineView& F, const Transfer& t, const int32_t* c_ptr, const int32_t* c_cols,
                       double* c_vals, cudaStream_t s);

@@ -55,6 +55,35 @@ def test_coarsest_inverse_sizes(ctx, solved, nodes):
     assert _solve(ctx, solved, "large", amg_aggregate_nodes=nodes, amg_persistent_max_dof=-1) == 2
 
 
+@pytest.mark.parametrize("nodes", [4, 8, 16, 24])
+def test_unsmoothed_transfers(ctx, nodes):
+    """Above 5,000 rows small aggregates take the tentative transfer itself (24: the smoothed one)."""
+    text = decks.c3d4_cantilever(13, 13, 28)  # 5,684 nodes
+    ref = static_step.Runner(inp.parse_inp_text(text)).run().displacements
+    p = fx.Project.from_inp_text(text, ctx)
+    st = fx.SolutionState(p.num_dofs, p.num_nodes)
+    for prec, tol in ((fx.PREC_FP64, 1e-10), (fx.PREC_MIXED, 1e-8)):
+        st.initialize(p)
+        p.steps[0].solve(1, p, st, opts=fx.solve_opts(precision=prec, rtol=1e-11, amg_aggregate_nodes=nodes))
+        assert float(np.linalg.norm(st.displacements - ref) / np.linalg.norm(ref)) <= tol
+    p.close()
+
+
+def test_unsmoothed_transfers_below_the_corners(ctx):
+    """The same on a corner level of 5,400 corners, whose lower levels are smoothed: against the default hierarchy, 1e-8."""
+    text = decks.c3d20_box(14, 14, 23, lengths=(14.0, 14.0, 23.0))
+    p = fx.Project.from_inp_text(text, ctx)
+    st = fx.SolutionState(p.num_dofs, p.num_nodes)
+    u = []
+    for nodes in (0, 16, 40):
+        st.initialize(p)
+        p.steps[0].solve(1, p, st, opts=fx.solve_opts(rtol=1e-11, amg_aggregate_nodes=nodes))
+        u.append(st.displacements)
+    p.close()
+    for v in u[1:]:
+        assert float(np.linalg.norm(v - u[0]) / np.linalg.norm(u[0])) <= 1e-8
+
+
 def test_counts_mesh_nodes(ctx):
     """1,820 corners among 6,768 nodes: 16 nodes of the mesh per aggregate leave 408 aggregates, more than the dense
     inverse's 200 (one more level); 16 corners, or 64 nodes, leave 132."""
