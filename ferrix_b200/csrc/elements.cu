@@ -276,15 +276,29 @@ __global__ void __launch_bounds__(32 * kWarpsS20, 4) k_stiff20(int nelem, const 
             if (lane < kGp20) tg += s_n[lane * 21 + a] * t;
         }
     if (lane < kGp20) {
-        T J[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, Ji[9];
+        // The node coordinates cancel in J, so in FP32 its terms go into four sums that are added last: one after
+        // another they left 1.7 times the error of a tree of warp reductions in the matrix.
+        constexpr int P = sizeof(T) == 4 ? 4 : 1;
+        T Jp[P][9], Ji[9];
+#pragma unroll
+        for (int q = 0; q < P; ++q)
+#pragma unroll
+            for (int c = 0; c < 9; ++c) Jp[q][c] = 0;
 #pragma unroll 4
         for (int a = 0; a < 20; ++a)
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 const T g = s_dn[lane * 61 + d * 20 + a];
 #pragma unroll
-                for (int c = 0; c < 3; ++c) J[3 * d + c] = fmat(g, s_x[warp][3 * a + c], J[3 * d + c]);
+                for (int c = 0; c < 3; ++c)
+                    Jp[a % P][3 * d + c] = fmat(g, s_x[warp][3 * a + c], Jp[a % P][3 * d + c]);
             }
+        T J[9];
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+            if constexpr (P == 4) J[c] = (Jp[0][c] + Jp[1][c]) + (Jp[2][c] + Jp[3][c]);
+            else J[c] = Jp[0][c];
+        }
         Lame L;
         material_d(md, k, tg, &L);
         const T det = inv3(J, Ji);
