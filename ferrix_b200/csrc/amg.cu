@@ -1611,9 +1611,11 @@ static void level_spmv(const AmgLevel& l, const double* x, const double* b, doub
 }
 
 // Largest eigenvalue of D^-1 A by 12 power iterations from a fixed hashed start vector, one launch
-// each: a step is x <- c2 D^-1 A x without a normalisation (c2 = 1/4 keeps 12 steps of a spectrum
-// up to ~5,000 within FP32's range), and the eigenvalue is the ratio of the last two vectors' norms.
-// (Normalised after every step, an iteration was six launches, ~18 us on a small level.)
+// each: a step is x <- c2 D^-1 A x without a normalisation, and the eigenvalue is the ratio of the last two vectors' norms.
+// (Normalised after every step, an iteration was six launches, ~18 us on a small level.) Planar levels have
+// eigenvalues of at most the nodes of an element, 20, so that with c2 = 1/4 twelve steps grow a vector by at most 2.4e8;
+// in FP32 it also holds the factors sqrt(a_ii) of the scaled matrix, up to 1e11 with the constraints' penalty on a
+// stiffness of 1e16. The 6x6 levels, whose bound is the blocks of a row, are in FP64.
 // Planar levels: the products come from the FP16 scaled matrix that the smoother reads, through
 // float4 vectors, or from the FP32 copy or the FP64 values with FP64 vectors.
 // warm: start from the vector the previous estimate on this level ended with (a

@@ -33,8 +33,8 @@ void cub_call(Op op, DBuf<uint8_t>& tmp, cudaStream_t s) {
 // accumulated in shared memory over the row's operands one after another (each operand's columns are
 // distinct), so the sums' order is fixed. Nothing of the size of the products is sorted or stored. On a
 // 205k-DOF C3D4 box the setup took 3.5 ms with the pair lists below (0.9 ms of it sorts, 0.8 ms sums that
-// gather both operands of every pair) and 3.25 ms this way. Rows with more than kSetMax columns, or
-// whose values exceed the shared memory, take the pair lists.
+// gather both operands of every pair) and 3.25 ms this way. Rows with more than kSetMax columns take the
+// pair lists.
 
 constexpr int kSet = 512, kSetMax = 384;  // slots of a warp's hash set, distinct columns it may hold
 constexpr int kRowWarps = 8;
@@ -351,10 +351,10 @@ __global__ void __launch_bounds__(32 * kCoarseWarps)
 
 constexpr size_t kRowShared = 200 << 10;
 
-// warps (1, 2, 4, 8) whose `per_warp` bytes fit the shared memory, at most `want`; 0: not even one
+// warps (1, 2, 4, 8) whose `per_warp` bytes fit the shared memory, at most `want`
 int warps_that_fit(size_t per_warp, int want) {
     int w = want;
-    while (w > 0 && per_warp * w > kRowShared) w >>= 1;
+    while (w > 1 && per_warp * w > kRowShared) w >>= 1;
     return w;
 }
 
@@ -392,12 +392,7 @@ void launch_rows(K kernel, int bs, const FineView& F, int most, cudaStream_t s, 
     FX_LAUNCH(kernel, grid_for(F.n, warps), 32 * warps, warps * row, s, F.n, warps, most, F, args...);
 }
 
-// the smallest shared memory per CTA at which `most` columns' rows still have their values in it
-bool rows_fit(int bs, int most_p, int most_w, int most_c) {
-    auto row = [&](int most) { return (size_t)most * (bs * 6 * sizeof(double) + sizeof(int)); };
-    return warps_that_fit(row(most_p), 1) && warps_that_fit(row(most_w), 1) &&
-           warps_that_fit((size_t)most_c * (36 * sizeof(double) + sizeof(int)), 1);
-}
+static_assert(kSetMax * (36 * sizeof(double) + sizeof(int)) <= kRowShared, "a warp's longest row fits the shared memory");
 
 // ------------------------------------------------------------------ products by pair lists
 
@@ -715,7 +710,6 @@ bool build_by_rows(const FineView& F, int na, const int32_t* agg, const double* 
     int most_p = 0;
     t.most_w = t.most_c = 0;
     if (!row_pattern(F.n, SrcP{F, agg}, t.ptr, t.col, &t.nnz, &most_p, tmp, s)) return false;
-    if (!rows_fit(bs, most_p, 1, 1)) return false;
     t.val.alloc((size_t)t.nnz * bs * 6, s);
     if (bs == 3)
         launch_rows(k_p_values<3>, 3, F, most_p, s, agg, Q, (const int32_t*)t.ptr.ptr, (const int32_t*)t.col.ptr, dinv,
@@ -730,10 +724,8 @@ bool build_by_rows(const FineView& F, int na, const int32_t* agg, const double* 
         transpose_and_interleave(t, p_row.ptr, tmp, s);
     }
     if (!row_pattern(F.n, SrcW{F, t.ptr.ptr, t.col.ptr}, t.w_ptr, t.w_col, &t.w.n, &t.most_w, tmp, s)) return false;
-    if (!rows_fit(bs, 1, t.most_w, 1)) return false;
     if (!row_pattern(na, SrcC{t.t_ptr.ptr, t.t_row.ptr, t.w_ptr.ptr, t.w_col.ptr}, c_ptr, c_cols, ncb, &t.most_c, tmp, s))
         return false;
-    if (!rows_fit(bs, 1, 1, t.most_c)) return false;
     t.c.n = *ncb;
     return true;
 }

@@ -3,7 +3,7 @@
 //
 // P = (I - omega D^-1 A) Q: every fine row reaches the aggregates of its matrix
 // neighbours. The sparse products W = A P and A_c = P^T W are formed row by row, their patterns once
-// and their values again when only the matrix values change; rows too long for shared memory
+// and their values again when only the matrix values change; rows of more columns than a warp's hash set holds
 // take lists of operand pairs sorted by the (row, column) of the entry they contribute to
 // (expand, sort, compress). Every sum has a fixed order (no atomics: results do not
 // depend on timing).

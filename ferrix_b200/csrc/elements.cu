@@ -82,12 +82,6 @@ void DeviceTables::init(cudaStream_t s) {
             }
     for (size_t i = 0; i < n.size(); ++i) nf[i] = (float)n[i];
     for (size_t i = 0; i < dn.size(); ++i) dnf[i] = (float)dn[i];
-    std::vector<uint8_t> pairs;
-    for (int a = 0; a < 20; ++a)
-        for (int b = a; b < 20; ++b) {
-            pairs.push_back((uint8_t)a);
-            pairs.push_back((uint8_t)b);
-        }
     // derivatives at the 20 node positions (local coordinates of c3d20.rs:61-84) for stress recovery
     static const double nodes20[20][3] = {{-1, -1, -1}, {1, -1, -1}, {1, 1, -1}, {-1, 1, -1}, {-1, -1, 1},
                                           {1, -1, 1},   {1, 1, 1},   {-1, 1, 1}, {0, -1, -1}, {1, 0, -1},
@@ -101,12 +95,11 @@ void DeviceTables::init(cudaStream_t s) {
     n20_f.upload(nf, s);
     dn20_f.upload(dnf, s);
     w20.upload(wt, s);
-    pair20.upload(pairs, s);
     FX_CUDA_CHECK(cudaStreamSynchronize(s));
 }
 
 RuleTables DeviceTables::view() const {
-    return RuleTables{n20_d.ptr, dn20_d.ptr, n20_f.ptr, dn20_f.ptr, w20.ptr, pair20.ptr, dn20_nodes.ptr};
+    return RuleTables{n20_d.ptr, dn20_d.ptr, n20_f.ptr, dn20_f.ptr, w20.ptr, dn20_nodes.ptr};
 }
 
 // ------------------------------------------------------------------ helpers

@@ -20,7 +20,6 @@ struct ElemView {
 struct DeviceTables {
     DBuf<double> n20_d, dn20_d, w20, dn20_nodes;
     DBuf<float> n20_f, dn20_f;
-    DBuf<uint8_t> pair20;
     void init(cudaStream_t s);
     RuleTables view() const;
 };
