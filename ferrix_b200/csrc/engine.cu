@@ -962,33 +962,10 @@ static int batch_solve_guarded(fx_ctx* ctx, fx_model* const* models, int n, cons
 // trips, the multi-launch CG of each system, one persistent launch for its tiny ones)
 // while the others do theirs, so the kernels of up to kBatchWorkers systems share the
 // GPU. A model takes the same path whichever worker it lands on.
-//
-// The pool grows before the workers start (batch_need). Growing under them, in 32 MB steps, by 0.6-1 GB for
-// 24 new C3D4 decks of 2k-60k DOF, each step may stall every worker: their first solve took 48-54 ms, but 511
-// once. In one step before: 51-57 ms, 42-45 of them the solve.
 #ifndef FX_BATCH_WORKERS
 #define FX_BATCH_WORKERS 4
 #endif
 constexpr int kBatchWorkers = FX_BATCH_WORKERS;
-
-// Spare pool memory for a batch of models in `order` (largest first): what each new model will hold when all
-// are solved (measured: 1.9-2.0 kB per C3D4, 67-91 kB per C3D20, and up to 12 MB of a dense inverse), the temporaries of
-// the K in work, and room for their fragmentation (batches solved again without it grew by up to 160 MB).
-// Models solved before have their memory.
-static double batch_need(fx_model* const* models, const std::vector<int>& order, int K) {
-    double need = 192.0e6;
-    int fresh = 0;
-    for (int i : order) {
-        const ModelDev& d = models[i]->dev;
-        if (d.have_structure && (d.minv64.ptr || d.minv32.ptr)) continue;
-        const DenseModel& D = models[i]->dense;
-        const double e4 = (double)D.g4.size(), e20 = (double)D.g20.size();
-        const double level = e20 > 0.0 ? 0.3 * (double)D.n_nodes : (double)D.n_nodes;  // (element corners)
-        need += 2.0e3 * e4 + 80.0e3 * e20 + std::min(12.0e6, 72.0 * level * level);
-        if (fresh++ < K) need += 0.8e3 * e4 + 15.0e3 * e20;
-    }
-    return need;
-}
 
 int batch_solve(fx_ctx* ctx, fx_model* const* models, int n, const fx_solve_opts& o_in, int* status_out,
                 fx_step_stats* stats) {
@@ -1006,16 +983,14 @@ int batch_solve(fx_ctx* ctx, fx_model* const* models, int n, const fx_solve_opts
         if (rc != FX_OK) fail(rc, "batch worker context creation failed");
         ctx->workers.push_back(w);
     }
+    FX_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));  // the models' uploads on this stream are done
     std::vector<int> order(n);
-    for (int i = 0; i < n; ++i) {
-        order[i] = i;
-        ensure_dense(models[i]);
-    }
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int a, int b) { return models[a]->dense.n_nodes > models[b]->dense.n_nodes; });
-    reserve_pool(ctx->device, ctx->stream, batch_need(models, order, K));
-    // the models' uploads on this stream are done, and what was just reserved is free for the workers' streams
-    FX_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+    for (int i = 0; i < n; ++i) order[i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        ensure_dense(models[a]);
+        ensure_dense(models[b]);
+        return models[a]->dense.n_nodes > models[b]->dense.n_nodes;
+    });
     std::vector<std::vector<int>> part(K);
     std::vector<int64_t> load(K, 0);
     for (int i : order) {
