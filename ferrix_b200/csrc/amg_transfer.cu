@@ -38,6 +38,12 @@ void cub_call(Op op, DBuf<uint8_t>& tmp, cudaStream_t s) {
 
 constexpr int kSet = 512, kSetMax = 384;  // slots of a warp's hash set, distinct columns it may hold
 constexpr int kRowWarps = 8;
+// A row of a planar level whose neighbours lie in more aggregates than this (a node that many elements meet; three cells
+// in each direction are 27) keeps its tentative row. Smoothed, it joins every two of those aggregates, and the
+// Galerkin product fills all their blocks: a 205k-DOF C3D4 box beside a ball about one node, whose row reaches 75 / 130 /
+// 240 / 350 / 480 aggregates, took 20 / 31 / 64 / 110 / 177 ms a solve, and takes 17 / 23 / 29 / 37 / 45. (The whole
+// level tentative: 20 / 25 / 31 / 38 / 45.)
+constexpr int kLongRow = 64;
 
 __device__ __forceinline__ void set_clear(int* set, int lane) {
     for (int k = lane; k < kSet; k += 32) set[k] = -1;
@@ -84,13 +90,23 @@ __device__ __forceinline__ void set_write(const int* set, int* list, int lane, i
 }
 
 // column sources of a row
-struct SrcP {  // P: aggregates of the row's neighbours
+struct SrcP {  // P: aggregates of the row's neighbours, or its own alone (kLongRow; *long_rows = 1)
     FineView F;
     const int32_t* agg;
+    int* long_rows;
     __device__ __forceinline__ bool fill(int i, int lane, int* set) const {
         bool ok = true;
         for (int b = F.row_ptr[i] + lane; b < F.row_ptr[i + 1]; b += 32) ok &= set_insert(set, agg[F.col(b, i)]);
-        return ok;
+        if (F.bs != 3) return ok;
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok && set_count(set, lane) <= kLongRow) return true;
+        __syncwarp();
+        set_clear(set, lane);
+        if (lane == 0) {
+            set_insert(set, agg[i]);
+            *long_rows = 1;
+        }
+        return true;
     }
 };
 struct SrcW {  // W = A P: the P rows of the row's neighbours
@@ -188,12 +204,17 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_p_values(int n, int warps, i
     const int b1 = F.row_ptr[i + 1];
     const int r = lane < 18 ? lane / 6 : 0, c = lane % 6;
     const bool act = lane < 18;
+    bool tentative = false;  // kLongRow
     for (int b0 = F.row_ptr[i]; b0 < b1; b0 += 32) {
         int j = 0, at = 0;  // the next 32 blocks' columns and places
+        bool other = false;
         if (b0 + lane < b1) {
             j = F.col(b0 + lane, i);
             at = place(cols, u, agg[j]);
+            other = cols[at] != agg[j];
         }
+        tentative = __any_sync(0xffffffffu, other);
+        if (tentative) break;
         const int nb = min(32, b1 - b0);
         for (int q0 = 0; q0 < nb; q0 += FL) {  // warp-uniform
             double v[FL][H];
@@ -228,6 +249,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_p_values(int n, int warps, i
         double z = 0.0;
 #pragma unroll
         for (int m = 0; m < BS; ++m) z += D[rr * BS + m] * acc[p * V + 6 * m + cc];
+        if (tentative) z = 0.0;
         out[(int64_t)o0 * V + k] = (cols[p] == mya ? Q[(int64_t)i * V + o] : 0.0) - omega * z;
     }
 }
@@ -701,15 +723,16 @@ void transpose_and_interleave(Transfer& t, const int32_t* p_row, DBuf<uint8_t>& 
     }
 }
 
-// The smoothed transfer by rows; false (with t to be rebuilt) where a row is too long for it.
+// The smoothed transfer by rows; false (with t to be rebuilt) where a row is too long for it. *long_rows = 1
+// where a row of P is (kLongRow).
 bool build_by_rows(const FineView& F, int na, const int32_t* agg, const double* Q, const double* dinv, double omega,
-                   Transfer& t, DBuf<int32_t>& c_ptr, DBuf<int32_t>& c_cols, int64_t* ncb, DBuf<uint8_t>& tmp,
-                   cudaStream_t s) {
+                   Transfer& t, DBuf<int32_t>& c_ptr, DBuf<int32_t>& c_cols, int64_t* ncb, int* long_rows,
+                   DBuf<uint8_t>& tmp, cudaStream_t s) {
     if (F.nblocks <= 0 || F.nblocks > kMaxItems / 2) return false;  // (32-bit row pointers below)
     const int bs = F.bs;
     int most_p = 0;
     t.most_w = t.most_c = 0;
-    if (!row_pattern(F.n, SrcP{F, agg}, t.ptr, t.col, &t.nnz, &most_p, tmp, s)) return false;
+    if (!row_pattern(F.n, SrcP{F, agg, long_rows}, t.ptr, t.col, &t.nnz, &most_p, tmp, s)) return false;
     t.val.alloc((size_t)t.nnz * bs * 6, s);
     if (bs == 3)
         launch_rows(k_p_values<3>, 3, F, most_p, s, agg, Q, (const int32_t*)t.ptr.ptr, (const int32_t*)t.col.ptr, dinv,
@@ -740,8 +763,17 @@ bool build_transfer(const FineView& F, int na, const int32_t* agg, const double*
     t.n = n;
     t.na = na;
     t.bs = bs;
-    t.by_rows = smooth && build_by_rows(F, na, agg, Q, dinv, omega, t, c_ptr, c_cols, ncb, tmp, s);
+    DBuf<int> long_rows;
+    long_rows.alloc(1, s);
+    long_rows.zero(s);
+    t.by_rows = smooth && build_by_rows(F, na, agg, Q, dinv, omega, t, c_ptr, c_cols, ncb, long_rows.ptr, tmp, s);
     if (t.by_rows) return true;
+    if (smooth) {  // (the pair lists would smooth the long rows too)
+        int h = 0;
+        FX_CUDA_CHECK(cudaMemcpyAsync(&h, long_rows.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
+        stream_wait(s, "amg transfer rows");
+        smooth = !h;
+    }
     t.w_ptr.release();
     t.w_col.release();
     DBuf<int64_t> cnt, end;

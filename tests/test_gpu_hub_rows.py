@@ -47,3 +47,40 @@ def test_hub_rows(ball, nodes):
     p.close()
     ctx.close()
     assert err <= 1e-10, stats
+
+
+def test_setup_beside_a_hub():
+    """A node whose row reaches some 350 aggregates must not fill the coarse matrix between them: the set-up of a box with a
+    ball of 1,800 nodes about one node beside it takes at most 12 times the box's own (some 40 times
+    with that row smoothed). The least of four solves each."""
+    from scipy.spatial import ConvexHull
+
+    def setup_ms(mesh):
+        ctx = fx.Context(0)
+        p = fx.Project.from_arrays(**decks.deck_arrays(decks.DeckSpec(mesh, [(2.0e5, 0.3, None)],
+                                                                      load_total=(100.0, 50.0, -200.0))), ctx=ctx)
+        st = fx.SolutionState(p.num_dofs, p.num_nodes)
+        ms = []
+        for _ in range(4):
+            st.initialize(p)
+            ms.append(p.steps[0].solve(1, p, st)["amg_setup_ms"])
+        p.close()
+        ctx.close()
+        return min(ms)
+
+    box = decks.tet_box(16, 16, 40, 16.0, 16.0, 40.0)
+    k = np.arange(1800)
+    z = 1.0 - (2.0 * k + 1.0) / len(k)
+    phi = k * np.pi * (3.0 - np.sqrt(5.0))
+    r = np.sqrt(1.0 - z * z)
+    sphere = np.stack([r * np.cos(phi), r * np.sin(phi), z], axis=1)
+    tri = ConvexHull(sphere).simplices
+    xyz = 12.0 * np.concatenate([[[0.0, 0.0, 0.0]], sphere])
+    conn = np.concatenate([np.zeros((len(tri), 1), dtype=np.int64), tri + 1], axis=1)
+    v = np.einsum("ij,ij->i", np.cross(xyz[conn[:, 1]], xyz[conn[:, 2]]), xyz[conn[:, 3]])
+    conn[v < 0, 1], conn[v < 0, 2] = conn[v < 0, 2].copy(), conn[v < 0, 1].copy()
+    lattice = np.ones((len(xyz), 3), dtype=np.int64)
+    lattice[xyz[:, 2] < -8.4] = 0  # clamped cap
+    mesh = decks.BoxMesh(np.concatenate([box.xyz, xyz + [50.0, 8.0, 20.0]]), np.concatenate([box.conn, conn + len(box.xyz)]),
+                         4, np.concatenate([box.lattice, lattice]), box.dims, box.lengths)
+    assert setup_ms(mesh) <= 12.0 * setup_ms(box)
