@@ -30,6 +30,14 @@ constexpr double kSmoothOmega = 4.0 / 3.0 * kLmaxMargin;
 // C3D20 box, 8 nodes: 13.6 ms, 12.2 smoothed).
 constexpr int64_t kSmoothMembers = 20, kSmoothRows = 5000;
 
+// FP16 smoothing that the caller left open is given up, for FP32 values and the residual at hand, where from kTry16
+// iterations on the residual's fall so far lets expect more than 4 kTry16 in all (or twice those done). Slender and
+// stretched meshes lose the cycle to FP16's rounding as stiffness contrasts do (smoother_precision): a cantilever of 4 x 4 x
+// 160 regular C3D20 elements (43k DOF) did not converge in 3,000 iterations, 24 in FP64 (4.4 ms); 68 and 6.9 ms
+// this way. Of 413 decks, slender, flat or graded, FP16 kept to the end failed on 50 and FP64 on 4; this way 4. Where the
+// cycle itself is slow it costs up to a tenth (4k-DOF C3D20 plate 130 iterations, 7.6 ms: 140, 8.3).
+constexpr long long kTry16 = 32;
+
 template <typename Op>
 void cub_call(Op op, DBuf<uint8_t>& tmp, cudaStream_t s) {
     size_t bytes = 0;
@@ -2444,6 +2452,13 @@ void Amg::describe(ClInst& o) const {
     }
 }
 
+const float* AmgPcg::fine_fp32(const BsrStructure& S, const double* vals64, cudaStream_t s) {
+    const int64_t nv = (int64_t)S.n_groups * 36;
+    vals32_.alloc(nv, s);
+    FX_LAUNCH(k_f64_to_f32, 148 * 8, 256, 0, s, nv, vals64, vals32_.ptr);
+    return vals32_.ptr;
+}
+
 void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* dinv64, const double* xyz,
                      const CornerLevel* corner, double cell0, double node_volume, const PcgOptions& opt,
                      cudaStream_t s, AmgStats* st, bool reuse, bool persistent) {
@@ -2459,7 +2474,8 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
         in[1].vals = corner->vals.ptr;
         in[1].dinv = corner->minv.ptr;
     }
-    const bool f16 = opt.amg_fp32 && opt.amg_fp16 > 0 && !persistent;
+    if (!reuse) no16_ = false;
+    const bool f16 = opt.amg_fp32 && opt.amg_fp16 > 0 && !persistent && !no16_;
     const bool keep = keeps(S, reuse) && amg.planar() == (corner ? 2 : 1);
     // the fine level's copies for the smoother; the corner level, as the 6x6 levels, stays FP64 (with FP16 there
     // a 417k-DOF C3D20 solve takes 17.9 instead of 19.0 ms to 1e-8, 20.8 and 20.7 to 1e-10)
@@ -2474,12 +2490,7 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
     }
     // FP32 values: the FP32 smoother's; with the FP16 smoother only when the eigenvalue
     // estimate reads them (kAmgEstF16 off) instead of the FP16 values
-    if (opt.amg_fp32 && (!f16 || !kAmgEstF16)) {
-        const int64_t nv = (int64_t)S.n_groups * 36;
-        vals32_.alloc(nv, s);
-        FX_LAUNCH(k_f64_to_f32, 148 * 8, 256, 0, s, nv, vals64, vals32_.ptr);
-        in[0].vals32 = vals32_.ptr;
-    }
+    if (opt.amg_fp32 && (!f16 || !kAmgEstF16)) in[0].vals32 = fine_fp32(S, vals64, s);
     amg.set_degree(opt.amg_degree);
     kept_ = keep;
     if (keep) {
@@ -2578,14 +2589,18 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
     FX_LAUNCH(k_fin, 1, 32, 0, s, nb, part_.ptr, sc_.ptr, 1);
     FX_CUDA_CHECK(cudaMemcpyAsync(sc_.ptr + 3, sc_.ptr + 2, sizeof(double), cudaMemcpyDeviceToDevice, s));
     z2_.alloc(nd, s);
-    amg.apply(r_.ptr, z_.ptr, nullptr, nullptr, s);
-    FX_LAUNCH(k_dot_part, nb, 256, 0, s, nd, r_.ptr, z_.ptr, part_.ptr);
-    FX_LAUNCH(k_fin, 1, 32, 0, s, nb, part_.ptr, sc_.ptr, 3);
-    FX_CUDA_CHECK(cudaMemcpyAsync(p_.ptr, z_.ptr, nd * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    const AmgLevel& l0 = amg.L[0];
+    auto first_direction = [&] {
+        amg.apply(r_.ptr, z_.ptr, nullptr, nullptr, s);
+        FX_LAUNCH(k_dot_part, nb, 256, 0, s, nd, r_.ptr, z_.ptr, part_.ptr);
+        FX_LAUNCH(k_fin, 1, 32, 0, s, nb, part_.ptr, sc_.ptr, 3);
+        FX_CUDA_CHECK(cudaMemcpyAsync(p_.ptr, z_.ptr, nd * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    };
+    first_direction();
+    AmgLevel& l0 = amg.L[0];
     // flexible CG (the K-cycle makes the preconditioner vary slightly between
     // iterations): z alternates between two buffers so that r.z_old is at hand
-    const unsigned gu = grid_for(n), gx = grid_for(nd), gz = amg.apply_grid();
+    const unsigned gu = grid_for(n), gx = grid_for(nd);
+    unsigned gz = amg.apply_grid();
     int parity = 0;
     auto iteration = [&]() {
         double* zn = parity ? z_.ptr : z2_.ptr;
@@ -2620,7 +2635,8 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
     const bool graphs = opt.graphs && !debug_sync() && !amg.L[amg.planar() - 1].coarsest;
     const void* key[4] = {x, vals64, dinv64, r_.ptr};
     if (gexec_ && (!graphs || !std::equal(key, key + 4, graph_key_))) drop_graph();
-    if (graphs && !gexec_) {
+    auto capture = [&] {
+        if (!graphs || gexec_) return;
         cudaGraph_t g = nullptr;
         int64_t count = 0;
         int64_t* saved = g_launch_counter;
@@ -2643,7 +2659,8 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
         if (ci != cudaSuccess) gexec_ = nullptr;
         FX_CUDA_CHECK(ci);
         std::copy(key, key + 4, graph_key_);
-    }
+    };
+    capture();
     double h[9];
     long long it = 0;
     int rc = FX_OK;
@@ -2667,6 +2684,21 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
         if (it >= max_iter) {
             rc = FX_CONVERGENCE;
             break;
+        }
+        if (opt.amg_fp16 == 2 && l0.vals16 && it >= kTry16 &&
+            std::log(h[2] / h[3]) > std::log(rtol2) * std::min(0.5, it / (4.0 * kTry16))) {
+            no16_ = true;
+            l0.vals32 = fine_fp32(S, vals64, s);
+            l0.vals16 = nullptr;
+            l0.sq4 = nullptr;
+            amg.set_smoother_scale(nullptr, nullptr);
+            if (opt.amg_fused_coarse && !opt.amg_kcycle) amg.upload_descriptor(s);
+            drop_graph();
+            gz = amg.apply_grid();
+            parity = 0;
+            first_direction();
+            capture();
+            seen = -1.0;
         }
         int next = 4;
         if (seen > 0.0) {

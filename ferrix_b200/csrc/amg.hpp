@@ -353,10 +353,12 @@ class AmgPcg {
     DBuf<float4> sq4_;
     DBuf<float> hs_;  // FP16 smoother directions: the current V-cycle's {2^k, 2^-k}
     bool kept_ = false;
+    bool no16_ = false;  // FP16 smoothing was given up on this hierarchy (kTry16)
     bool fresh_ = false, stale_ = false;  // the hierarchy was (re)computed for this solve; should be for the next
     long long first_iters_ = 0;
     // the captured iterations, kept while the hierarchy is: what they were captured with
     void drop_graph();
+    const float* fine_fp32(const BsrStructure& S, const double* vals64, cudaStream_t s);  // into vals32_
     cudaGraphExec_t gexec_ = nullptr;
     int64_t graph_launches_ = 0;
     const void* graph_key_[4] = {nullptr, nullptr, nullptr, nullptr};

@@ -682,7 +682,7 @@ struct StepRunner {
 constexpr double kMaxContrast16 = 100.0;
 static void smoother_precision(const DenseModel& D, PcgOptions& po) {
     if (po.amg_fp16 != 0) return;
-    po.amg_fp16 = D.e_contrast <= kMaxContrast16 && 3 * D.n_nodes > kClDefaultMaxDof ? 1 : -1;
+    po.amg_fp16 = D.e_contrast <= kMaxContrast16 && 3 * D.n_nodes > kClDefaultMaxDof ? 2 : -1;
 }
 
 // Advances all runners in lockstep rounds; runners share the context stream. What is one model's own
