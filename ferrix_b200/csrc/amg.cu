@@ -2478,7 +2478,7 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
     const bool f16 = opt.amg_fp32 && opt.amg_fp16 > 0 && !persistent && !no16_;
     const bool keep = keeps(S, reuse) && amg.planar() == (corner ? 2 : 1);
     // the fine level's copies for the smoother; the corner level, as the 6x6 levels, stays FP64 (with FP16 there
-    // a 417k-DOF C3D20 solve takes 17.9 instead of 19.0 ms to 1e-8, 20.8 and 20.7 to 1e-10)
+    // a 417k-DOF C3D20 solve takes 20.4 instead of 21.5 ms to 1e-8)
     if (f16) {  // FP16 values of S A S and the scales
         sq4_.alloc((size_t)n, s);
         FX_LAUNCH(k_diag_sqrt, grid_for(n), 256, 0, s, n, S.goff.ptr, S.diag_k.ptr, vals64, sq4_.ptr);

@@ -6,7 +6,8 @@
 //     matrix like the fine one (417k-DOF box to 1e-10: 116 CG iterations without it and with
 //     unsmoothed aggregation, 36 with both, 59.2 -> 25.4 ms a solve);
 //   * aggregation by spatial binning of the level's points (nodes, then
-//     aggregate centroids) into cubic cells;
+//     aggregate centroids) into the cells of a
+//     grid that cuts their bounding box into equal parts per direction;
 //   * tentative prolongator from the six rigid-body modes (three translations,
 //     three rotations about the aggregate centroid): per aggregate a QR of the
 //     stacked near-null-space rows (one warp per aggregate, modified
@@ -292,7 +293,6 @@ inline bool dense_planar(int64_t rows) { return 3 * rows <= kDensePlanarDof; }
 // The default of the option amg_aggregate_nodes: with it the hierarchy chooses its cells (pick_cell).
 constexpr int kAmgAggregateNodes = 40;
 
-// CG on the FP64 BSR3 system preconditioned by one V-cycle per iteration.
 // CUDA-event time (ms per launch) of the fused fine-level Chebyshev step (SpMV +
 // smoother update) on the given FP64 system, with FP32 values when fp32; bytes =
 // compulsory traffic of one launch.
@@ -300,6 +300,7 @@ double profile_smoother_op(const BsrStructure& S, const double* vals64, const do
                            int reps,
                            cudaStream_t s, double* bytes);
 
+// CG on the FP64 BSR3 system preconditioned by one V-cycle per iteration.
 class AmgPcg {
    public:
     AmgPcg() = default;

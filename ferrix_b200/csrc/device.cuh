@@ -88,7 +88,7 @@ __device__ __forceinline__ T inv3(const T J[9], T Ji[9]) {
 // const __restrict__); before it only what was there before the last launch that was not chained
 // (a chain's matrices, transfers and index lists). The kernels do not let the next one start early
 // (cudaTriggerProgrammaticLaunchCompletion): CTAs that wait while the kernel ahead still works made a
-// 16k-DOF Newton solve's 2,774 iterations 131 ms, 117 without, 123 with ordinary launches.
+// 16k-DOF Newton step's 2,774 iterations 131 ms, 117 without, 123 with ordinary launches (now 103 and 108).
 __device__ __forceinline__ void chain_wait() { cudaGridDependencySynchronize(); }
 struct ChainWait {
     __device__ __forceinline__ void operator()() const { chain_wait(); }
