@@ -1841,7 +1841,7 @@ void Amg::setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz
             estimate_lmax(L[m], red_, s, false);
         }
     }
-    if (dense && cell0 <= 0.0 && dense_planar(L.back().n)) {
+    if (dense && cell0 <= 0.0 && !tentative_ && dense_planar(L.back().n)) {
         AmgLevel& l = L.back();
         l.lmax = 1.0;  // (no smoothing here)
         l.coarsest = true;
@@ -1944,6 +1944,7 @@ void Amg::setup(const PlanarIn* in, const CornerLevel* corner, const double* xyz
         }
         if (l.S0) smooth = cell0 <= 0.0 || l.n <= kSmoothRows || l.n >= kSmoothMembers * na;
         else if (planar_ == 2) smooth = true;
+        smooth &= !tentative_;
         L.emplace_back();
         AmgLevel& c = L.back();
         AmgLevel& lf = L[L.size() - 2];
@@ -2492,6 +2493,7 @@ void AmgPcg::prepare(const BsrStructure& S, const double* vals64, const double* 
     // estimate reads them (kAmgEstF16 off) instead of the FP16 values
     if (opt.amg_fp32 && (!f16 || !kAmgEstF16)) in[0].vals32 = fine_fp32(S, vals64, s);
     amg.set_degree(opt.amg_degree);
+    amg.set_tentative(opt.amg_tentative);
     kept_ = keep;
     if (keep) {
         amg.keep(in[0], st);

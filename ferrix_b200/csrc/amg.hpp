@@ -124,6 +124,8 @@ class Amg {
     uint64_t built_for = 0;  // BsrStructure::id of the last setup (0: none)
     // Chebyshev degree (1..8)
     void set_degree(int degree) { degree_ = degree; }
+    // every transfer of the next setup tentative, and no planar level the coarsest (PcgOptions)
+    void set_tentative(bool on) { tentative_ = on; }
     // FP16 smoother directions: where the V-cycle started from x = 0 finds r.D^-1 r of its
     // right-hand side (rdr) and the two floats where each V-cycle publishes its power-of-two
     // scale of the stored directions (hs); null: unscaled
@@ -196,6 +198,7 @@ class Amg {
     double alpha_ = 1.0, cheb_ratio_ = 30.0;
     bool alpha_all_ = false;
     int degree_ = 2;
+    bool tentative_ = false;
     const double* rdr_ = nullptr;
     float* hs_ = nullptr;
     float* h16_scale_slot() const;

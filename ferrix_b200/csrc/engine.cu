@@ -316,6 +316,7 @@ struct StepRunner {
     bool amg = false;
     double amg_cell = 0.0, amg_volume = 1.0;
     bool no_corner = false;  // this step's hierarchy does without a corner level
+    bool tentative = false;  // and without smoothed transfers
     DBuf<double> amg_xyz;
 
     void begin(fx_model* mm, int kk, const fx_solve_opts& oo) {
@@ -496,24 +497,27 @@ struct StepRunner {
     }
 
     // The prepared system by the multigrid CG; persistent: its set-up only.
-    void solve_amg(const PcgOptions& po, bool reuse, bool persistent) {
+    void solve_amg(PcgOptions po, bool reuse, bool persistent) {
+        po.amg_tentative = tentative;
         ModelDev& d = m->dev;
         cudaStream_t s = m->ctx->stream;
         AmgStats ast;
         const double node_volume = amg_volume / (double)std::max<int64_t>(1, planar_nodes());
+        const double cell = tentative && amg_cell <= 0.0 ? std::cbrt(kAmgAggregateNodes * node_volume) : amg_cell;
         try {
             if (persistent)
-                d.amg->prepare(d.S, d.vals64.ptr, d.minv64.ptr, amg_xyz.ptr, corner(), amg_cell, node_volume, po, s,
+                d.amg->prepare(d.S, d.vals64.ptr, d.minv64.ptr, amg_xyz.ptr, corner(), cell, node_volume, po, s,
                                &ast, reuse, true);
             else
-                csr_status = d.amg->solve(d.S, d.vals64.ptr, d.minv64.ptr, amg_xyz.ptr, corner(), amg_cell,
+                csr_status = d.amg->solve(d.S, d.vals64.ptr, d.minv64.ptr, amg_xyz.ptr, corner(), cell,
                                           node_volume, d.R.ptr, d.du.ptr, po, s, &m->ctx->launches, &csr_iters,
                                           &csr_relres, &ast, reuse);
         } catch (const Error& e) {
             // A coarse operator below the corner level may look singular where one below the nodes does not (a stiff
-            // part on flat cells 1e4 times softer): whether the system is, the latter decides.
-            if (e.status != FX_NUMERICAL || !corner()) throw;
-            no_corner = true;
+            // part on flat cells 1e4 times softer), and one by smoothed transfers where one by tentative ones does not
+            // (graded cells 20 times longer than wide): whether the system is, the last decides.
+            if (e.status != FX_NUMERICAL || tentative) throw;
+            (corner() ? no_corner : tentative) = true;
             solve_amg(po, false, persistent);
             return;
         }

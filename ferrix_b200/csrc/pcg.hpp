@@ -122,6 +122,7 @@ struct PcgOptions {
     double amg_cheb_ratio = kAmgChebRatio;  // lmax / lmin of the first-kind Chebyshev interval
     int64_t amg_persistent_max_dof = 0;     // systems up to this size: one persistent cluster launch (< 0: never)
     bool amg_fused_coarse = true;           // coarse part of each V-cycle as one cooperative launch
+    bool amg_tentative = false;             // unsmoothed transfers down to the dense level
     int amg_fp16 = -1;  // mixed, multi-launch path: FP16 values of the scaled matrix; 1 on, 2 on until slow,
                         // -1 off, 0 by the system
 };
