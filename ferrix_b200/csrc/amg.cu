@@ -8,6 +8,8 @@
 
 #include <cuda_fp16.h>
 
+#include <vector>
+
 #include "amg.hpp"
 #include "coarse_row.cuh"
 #include "corner.cuh"
@@ -30,13 +32,15 @@ constexpr double kSmoothOmega = 4.0 / 3.0 * kLmaxMargin;
 // C3D20 box, 8 nodes: 13.6 ms, 12.2 smoothed).
 constexpr int64_t kSmoothMembers = 20, kSmoothRows = 5000;
 
-// FP16 smoothing that the caller left open is given up, for FP32 values and the residual at hand, where from kTry16
-// iterations on the residual's fall so far lets expect more than 4 kTry16 in all (or twice those done). Slender and
-// stretched meshes lose the cycle to FP16's rounding as stiffness contrasts do (smoother_precision): a cantilever of 4 x 4 x
-// 160 regular C3D20 elements (43k DOF) did not converge in 3,000 iterations, 24 in FP64 (4.4 ms); 68 and 6.9 ms
-// this way. Of 413 decks, slender, flat or graded, FP16 kept to the end failed on 50 and FP64 on 4; this way 4. Where the
-// cycle itself is slow it costs up to a tenth (4k-DOF C3D20 plate 130 iterations, 7.6 ms: 140, 8.3).
-constexpr long long kTry16 = 32;
+// Whether FP16's rounding spoils the cycle, as it does on slender and stretched meshes and across stiffness contrasts
+// (smoother_precision), shows in a V-cycle of the same residual with FP32 values: the energy of the difference of the two
+// is 0.6 to 1,000 times r.z then, else 1e-5 to 3e-2. It is looked at, with smoothing that the caller left open, where from kTry16
+// iterations on (then after twice as many each) the residual's fall so far lets expect more than 4 kTry16 in
+// all, or twice those done; above kSpoilt16 the solve goes on with FP32 values from the residual at hand. A cantilever of 4 x 4 x 160
+// regular C3D20 elements (43k DOF) did not converge in 3,000 iterations, 24 in FP64 (4.4 ms);
+// 44 and 5.6 ms this way.
+constexpr long long kTry16 = 16;
+constexpr double kSpoilt16 = 0.1;
 
 template <typename Op>
 void cub_call(Op op, DBuf<uint8_t>& tmp, cudaStream_t s) {
@@ -2668,6 +2672,23 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
     int rc = FX_OK;
     const double rtol2 = opt.rtol * opt.rtol;
     const long long max_iter = kept_ ? std::min<long long>(opt.max_iter, 2 * first_iters_ + 50) : opt.max_iter;
+    long long try16 = kTry16;
+    auto smooth_fp32 = [&](bool on) {
+        l0.vals32 = on ? fine_fp32(S, vals64, s) : nullptr;
+        l0.vals16 = on ? nullptr : vals16_.ptr;
+        l0.sq4 = on ? nullptr : sq4_.ptr;
+        amg.set_smoother_scale(on ? nullptr : sc_.ptr + 2, on ? nullptr : hs_.ptr);
+        if (opt.amg_fused_coarse && !opt.amg_kcycle) amg.upload_descriptor(s);
+    };
+    auto host_dot = [&](const double* a, const double* c) {
+        std::vector<double> parts(nb);
+        FX_LAUNCH(k_dot_part, nb, 256, 0, s, nd, a, c, part_.ptr);
+        part_.download(parts.data(), parts.size(), s);
+        stream_wait(s, "amg pcg precision check");
+        double t = 0.0;
+        for (double v : parts) t += v;
+        return t;
+    };
     double seen = -1.0;  // r.D^-1 r at the check before, and the iterations queued since
     int queued = 0;
     while (true) {
@@ -2687,20 +2708,26 @@ int AmgPcg::solve(const BsrStructure& S, const double* vals64, const double* din
             rc = FX_CONVERGENCE;
             break;
         }
-        if (opt.amg_fp16 == 2 && l0.vals16 && it >= kTry16 &&
+        if (opt.amg_fp16 == 2 && l0.vals16 && it >= try16 &&
             std::log(h[2] / h[3]) > std::log(rtol2) * std::min(0.5, it / (4.0 * kTry16))) {
-            no16_ = true;
-            l0.vals32 = fine_fp32(S, vals64, s);
-            l0.vals16 = nullptr;
-            l0.sq4 = nullptr;
-            amg.set_smoother_scale(nullptr, nullptr);
-            if (opt.amg_fused_coarse && !opt.amg_kcycle) amg.upload_descriptor(s);
-            drop_graph();
-            gz = amg.apply_grid();
-            parity = 0;
-            first_direction();
-            capture();
-            seen = -1.0;
+            try16 = 2 * it;
+            smooth_fp32(true);
+            double* last = amg.kcycle() ? z_.ptr : z2_.ptr;  // V(r) with FP16
+            double* z32 = amg.kcycle() ? z2_.ptr : z_.ptr;   // (either holds nothing that is needed any more)
+            amg.apply(r_.ptr, z32, nullptr, nullptr, s);
+            const double rz = host_dot(r_.ptr, z32);
+            launch_axpby(nd, 1.0, z32, -1.0, last, z32, s);
+            level_spmv(l0, z32, nullptr, q_.ptr, s);
+            if (host_dot(z32, q_.ptr) <= kSpoilt16 * rz) {
+                smooth_fp32(false);
+            } else {
+                no16_ = true;
+                drop_graph();
+                gz = amg.apply_grid();
+                first_direction();
+                capture();
+                seen = -1.0;
+            }
         }
         int next = 4;
         if (seen > 0.0) {

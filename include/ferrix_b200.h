@@ -111,8 +111,8 @@ typedef struct {
                                    fine-level smoother reads FP16 values of the diagonally scaled matrix
                                    D^-1/2 K D^-1/2 (entries within [-1, 1]); 1 = FP16, -1 = FP32 values of K,
                                    0 = default: FP16 above 2,000 DOF where the materials' Young's moduli lie
-                                   within a factor of 100, until a solve proves slow (more than 128
-                                   iterations in prospect after 32), else FP32 */
+                                   within a factor of 100, until a slow solve (more than
+                                   64 iterations in prospect) finds its cycle spoilt by it, else FP32 */
 } fx_solve_opts;
 
 /* Preconditioner of the BSR3 PCG. */

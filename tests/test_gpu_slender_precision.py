@@ -1,5 +1,5 @@
-"""Mixed precision on slender C3D20 cantilevers, whose cycle FP16 smoothing spoils: by default it is given up after 32
-to 64 iterations, so that the mixed solve takes at most those and about the FP64 solve's iterations (a third more and four,
+"""Mixed precision on slender C3D20 cantilevers, whose cycle FP16 smoothing spoils: by default it is given up within 64
+iterations, so that the mixed solve takes at most those and about the FP64 solve's iterations (a third more and four,
 the spread that FP32 smoothing leaves), and its displacements are those of FP64 to 1e-6 (the residual target of
 1e-9 times the conditioning that these decks show, ~1e3)."""
 import numpy as np
