@@ -38,7 +38,7 @@ constexpr int64_t kSmoothMembers = 20, kSmoothRows = 5000;
 // iterations on (then after twice as many each) the residual's fall so far lets expect more than 4 kTry16 in
 // all, or twice those done; above kSpoilt16 the solve goes on with FP32 values from the residual at hand. A cantilever of 4 x 4 x 160
 // regular C3D20 elements (43k DOF) did not converge in 3,000 iterations, 24 in FP64 (4.4 ms);
-// 44 and 5.6 ms this way.
+// 44 and 5.7 ms this way.
 constexpr long long kTry16 = 16;
 constexpr double kSpoilt16 = 0.1;
 
